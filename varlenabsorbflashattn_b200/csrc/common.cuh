@@ -103,9 +103,7 @@ template <> __device__ __forceinline__ uint32_t pack2_out<__half>(float lo, floa
 //              elements apart, in lane order), 16-byte aligned
 //   my_row     index of the lane's row in the tile; rows >= n_rows are not written
 //   n_pieces   leading 16-byte pieces of the chunk that exist in the output (0..4)
-template <typename T>
-__device__ __forceinline__ void store_chunk_coalesced(uint32_t (&w)[16], T* my_chunk, long long row_stride, int my_row,
-                                                      int n_rows, int n_pieces) {
+__device__ __forceinline__ void transpose_pieces(uint32_t (&w)[16]) {
   const int lane = threadIdx.x & 31;
 #pragma unroll
   for (int m = 1; m <= 2; m <<= 1) {
@@ -123,7 +121,13 @@ __device__ __forceinline__ void store_chunk_coalesced(uint32_t (&w)[16], T* my_c
     }
   }
   // piece k now holds piece (lane & 3) of the row of lane (lane & ~3) + k
-  const int i = lane & 3;
+}
+
+template <typename T>
+__device__ __forceinline__ void store_chunk_coalesced(uint32_t (&w)[16], T* my_chunk, long long row_stride, int my_row,
+                                                      int n_rows, int n_pieces) {
+  transpose_pieces(w);
+  const int i = threadIdx.x & 3;
   if (i < n_pieces) {
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
@@ -134,6 +138,22 @@ __device__ __forceinline__ void store_chunk_coalesced(uint32_t (&w)[16], T* my_c
       }
     }
   }
+}
+
+// The same for rows at any distance from one another: off[k] = element offset of the row of lane (lane & ~3) + k,
+// negative for a row that is not written (quad_row_offsets collects them from the lanes' own offsets).
+__device__ __forceinline__ void quad_row_offsets(long long (&off)[4], long long my_off) {
+  const int quad = threadIdx.x & 28;
+#pragma unroll
+  for (int k = 0; k < 4; ++k) off[k] = __shfl_sync(0xffffffffu, my_off, quad + k);
+}
+template <typename T>
+__device__ __forceinline__ void store_chunk_rows(uint32_t (&w)[16], T* base, const long long (&off)[4]) {
+  transpose_pieces(w);
+  const int i = threadIdx.x & 3;
+#pragma unroll
+  for (int k = 0; k < 4; ++k)
+    if (off[k] >= 0) *(reinterpret_cast<uint4*>(base + off[k]) + i) = make_uint4(w[4 * k], w[4 * k + 1], w[4 * k + 2], w[4 * k + 3]);
 }
 
 __device__ __forceinline__ float warp_sum(float x) {

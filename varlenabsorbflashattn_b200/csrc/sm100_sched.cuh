@@ -70,12 +70,14 @@ struct SchedCaps {
 };
 
 // Host-side capacity bounds (no knowledge of the lengths needed).
-static inline SchedCaps sched_caps(int mode, int total_outer, int total_inner, int n_seg, int H, int sm_count, int split_len) {
+static inline SchedCaps sched_caps(int mode, int total_outer, int total_inner, int n_seg, int H, int sm_count, int split_len,
+                                   int tile_rows = kTile) {
   SchedCaps c;
-  const long long units = (long long)total_outer / kTile + n_seg + 1;
+  const long long units = (long long)total_outer / tile_rows + n_seg + 1;
   long long extra = 0;
   if (mode == kSchedFwd) {
-    extra = 2LL * sm_count + 64;
+    // a slice has at least total / (4 SMs) blocks: at most one extra item per slice's worth
+    extra = 4LL * sm_count / (H > 0 ? H : 1) + 64;
     if (split_len > 0) extra += (long long)total_inner / split_len;
   }
   long long items = (units + extra) * (H > 0 ? H : 1);
@@ -84,7 +86,8 @@ static inline SchedCaps sched_caps(int mode, int total_outer, int total_inner, i
   c.cap_combine = (int32_t)units;
   long long rows = 0;
   if (mode == kSchedFwd) {
-    rows = 512LL * sm_count / (H > 0 ? H : 1) + 256;
+    // a tile that is cut has fewer than 2 nb / slice parts
+    rows = 8LL * sm_count / (H > 0 ? H : 1) * (total_outer < tile_rows ? total_outer : tile_rows) + 256;
     if (split_len > 0) rows += 4LL * total_outer;
     if (rows > (1LL << 22)) rows = 1LL << 22;
   }

@@ -63,6 +63,27 @@ __device__ __forceinline__ Unit make_unit(const SchedParams& p, const Seg& g, in
 
 __device__ __forceinline__ int n_splits(int nb, int bs) { return (bs > 0 && nb > bs) ? (nb + bs - 1) / bs : 1; }
 
+// Inner blocks per item when the library picks the slice.  Items of total / (k * SMs) blocks keep every SM busy to
+// within 1/k of its share, whatever the lengths are (a tile longer than that is cut even if there are many
+// tiles: 40 requests of which one has a long cache).  What a cut costs is the fp32 partial result of its rows,
+// written and read once more: nothing for the one to eight rows of a decode item (as many bytes as 1/64 of a
+// key block), one key block's worth for a full 128-row tile.  Hence
+//   * slices of at least 2 blocks for few rows, 8 for full tiles;
+//   * k = 4 where a slice then still has twice that minimum, else k = 2 (500-query users with 800-block
+//     histories on 148 SMs, simulated: the busiest SM has 1.31 x the mean at k = 2, 1.07 x at 4, 1.06 x at 8);
+//   * short decode batches (below 16 blocks per SM), where a second round of items would double the time, aim at
+//     one item per SM with an eighth to spare.
+__device__ __forceinline__ int split_blocks(const SchedParams& p, int units, long long blocks, int outer) {
+  if (units <= 0) return 0;
+  const long long total = blocks * p.H, sms = p.sm_count;
+  const long long rows = min(p.tile_rows, (outer + units - 1) / units);  // mean rows of a tile
+  const long long least = 2 + 6 * rows / p.tile_rows;
+  const long long per_sm = (total + sms - 1) / sms;
+  if (per_sm < 16 && 4 * rows <= p.tile_rows) return (int)max(least, (9 * per_sm + 7) / 8);
+  const long long half = (total + 2 * sms - 1) / (2 * sms), quarter = (total + 4 * sms - 1) / (4 * sms);
+  return (int)min((long long)(1 << 24), max(least, min(half, max(quarter, 2 * least))));
+}
+
 // Monotone map of a cost to one of kBuckets buckets: 16 buckets per power of two.
 __device__ __forceinline__ int cost_bucket(long long c) {
   if (c <= 0) return 0;
@@ -134,8 +155,9 @@ __device__ __forceinline__ void sched_build(const SchedParams& p) {
   __shared__ int s_units, s_items, s_rows, s_bs, s_combine;
   __shared__ unsigned long long s_items64, s_rows64;  // pass 2 counts in 64 bits
   __shared__ long long s_blocks;
+  __shared__ int s_outer, s_longest;  // outer rows of all tiles, inner blocks of the longest tile
 
-  if (threadIdx.x == 0) { s_units = 0; s_blocks = 0; s_combine = 0; }
+  if (threadIdx.x == 0) { s_units = 0; s_blocks = 0; s_combine = 0; s_outer = 0; s_longest = 0; }
   for (int b = threadIdx.x; b < kBuckets; b += kSchedThreads) s_hist[b] = 0;
   __syncthreads();
 
@@ -147,7 +169,7 @@ __device__ __forceinline__ void sched_build(const SchedParams& p) {
   // pass 1: totals, and the cost histogram for the common case that nothing is split (one item per
   // tile); only a list that does get split goes through passes 2 and 3
   {
-    int units = 0;
+    int units = 0, outer = 0, longest = 0;
     long long blocks = 0;
     for_each_segment(p, G, [&](const Seg& g, int t0, int ts) {
       long long cost = 0;
@@ -155,7 +177,7 @@ __device__ __forceinline__ void sched_build(const SchedParams& p) {
       for (int t = t0; t < g.n_tiles; t += ts) {
         const Unit u = make_unit(p, g, t);
         const int nb = n_blocks(u.i_len);
-        if (u.i_len > 0) { units += 1; blocks += nb; }
+        if (u.i_len > 0) { units += 1; blocks += nb; outer += u.o_rows; longest = max(longest, nb); }
         cost += nb;
         items += 1;
       }
@@ -167,6 +189,11 @@ __device__ __forceinline__ void sched_build(const SchedParams& p) {
     });
     units = (int)warp_sum_ll(units);
     blocks = warp_sum_ll(blocks);
+    if (p.mode == kSchedFwd) {
+      outer = (int)warp_sum_ll(outer);
+      longest = __reduce_max_sync(0xffffffffu, longest);
+      if (lane == 0 && units) { atomicAdd(&s_outer, outer); atomicMax(&s_longest, longest); }
+    }
     if (lane == 0 && units) { atomicAdd(&s_units, units); atomicAdd((unsigned long long*)&s_blocks, (unsigned long long)blocks); }
   }
   __syncthreads();
@@ -175,15 +202,8 @@ __device__ __forceinline__ void sched_build(const SchedParams& p) {
   if (threadIdx.x == 0) {
     int bs = 0;  // 0 = never split
     if (p.mode == kSchedFwd) {
-      if (p.split_len > 0) {
-        bs = p.split_len / kTile;
-      } else {
-        const long long par = (long long)s_units * p.H;
-        if (par > 0 && par < 2LL * p.sm_count) {
-          const long long t = (s_blocks * p.H + 2LL * p.sm_count - 1) / (2LL * p.sm_count);
-          bs = (int)max(8LL, t);
-        }
-      }
+      bs = p.split_len > 0 ? p.split_len / kTile : split_blocks(p, s_units, s_blocks, s_outer);
+      if (bs >= s_longest) bs = 0;
     }
     s_bs = bs;
   }

@@ -114,17 +114,26 @@ struct FwdParams {
   const SchedHeader* header;
   const WorkItem* items;
   int H;
-  int group;  // query heads per K/V head (1 = one K/V head per query head)
+  int group;  // query heads per K/V head when an item is one query head (stack == 1)
+  int stack;  // heads stacked into a tile: tile row = (query row) * stack + (head of the stack)
+  int q_bytes;  // bytes one copy of the query tile delivers (stack * rows per tile rows of D elements)
   float scale_log2;
   int32_t* status;
   int wait_limit;  // bound of every device-side wait, in units of 65536 cycles
   long long* trace;
 };
 
-// kAbsorb = false: one item = one 128-row query tile of one head (grid of items x heads).
-// kAbsorb = true : one item = 128/H query rows of one user with all H heads stacked into the 128
-//   tile rows (row = q*H + h, the order the 64 x H x (128/H) TMA box delivers), K = V = the user's X
-//   rows (one tile serves Q.X^T as a K-major operand and P.X as an MN-major operand), D = d_kv.
+// An item is a 128-row tile of queries against a range of keys.  p.stack heads that read the same keys share
+// the tile (row = q * stack + head, the order the 64 x stack x (128 / stack) TMA box delivers), so that
+// each key tile is read and multiplied once for all of them; w.head counts such stacks.
+//   varlen, stack = 1 : 128 query rows of one head
+//   varlen, stack = G : 128 / G query rows of all G query heads of one K/V head (grouped-query batches with
+//                       few queries per segment, see launch_fwd)
+//   kAbsorb, stack = H: 128 / H query rows of one user with all H heads, K = V = the user's X rows (one tile
+//                       serves Q.X^T as a K-major operand and P.X as an MN-major operand), D = d_kv
+// Rows past the item's last query are padding.  Softmax warps whose 32 rows are all padding (a decode item
+// has one to eight rows) only follow the barriers: a row of P.V depends on its own row of P alone, so what
+// the padding rows hold never reaches a real one.
 template <typename T, int D, bool kAbsorb>
 __global__ void __launch_bounds__(kFwdThreads, 1)
 varlen_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ CUtensorMap tmap_k,
@@ -192,12 +201,12 @@ varlen_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_const
         const int idx = wq_produce(sm.wq, n, next_item, total, abort_flag);
         if (idx < 0) break;
         const WorkItem w = p.items[idx];
-        const int h = w.head;
-        const int hk = kAbsorb ? h : h / p.group;  // K/V head of this query head
+        const int h = w.head * p.stack;
+        const int hk = w.head / p.group;  // K/V head of this query head or stack
         const int nb = (w.i_len + kBlk - 1) / kBlk;
         if (nb == 0) continue;
         { TRACE_T0(); if (!mbar_wait(smem_u32(&sm.q_free), (qi & 1) ^ 1, abort_flag)) break; TRACE_ADD(0); }
-        mbar_expect_tx(smem_u32(&sm.q_full), Cfg::kTileBytes);
+        mbar_expect_tx(smem_u32(&sm.q_full), p.q_bytes);
         for (int c = 0; c < Cfg::kSub; ++c)
           tma_load_3d(smem_u32(sm.q) + c * Cfg::kSubBytes, &tmap_q, smem_u32(&sm.q_full), c * 64, h, w.o_start);
         // absorb: X is streamed once from HBM (no other CTA reads this user's keys), and a K slot is only
@@ -327,14 +336,21 @@ varlen_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_const
       const WorkItem w = p.items[idx];
       const int nb = (w.i_len + kBlk - 1) / kBlk;
       // tile row r -> (query row of the tile, head)
-      const int rq = kAbsorb ? r / p.H : r;
-      const int h = kAbsorb ? r % p.H : w.head;
+      const int rq = p.stack == 1 ? r : r / p.stack;
+      const int h = w.head * p.stack + (r - rq * p.stack);
       const bool row_ok = rq < w.o_rows;
+      const bool live = (warp & 3) * 32 < w.o_rows * p.stack;  // does any row of this warp exist?
       float m_ref = -INFINITY, l = 0.f;  // l: sum over this thread's columns only
 
       for (int b = 0; b < nb; ++b) {
         const uint32_t g = gk + b;
         { TRACE_T0(); if (!mbar_wait(smem_u32(&sm.s_full[g & 1]), (g >> 1) & 1, abort_flag)) { alive = false; break; } TRACE_ADD(8); }
+        if (!live) {
+          // nothing to compute; the arrival keeps the barrier's count
+          __syncwarp();
+          if (lane == 0) mbar_arrive(smem_u32(&sm.p_full[g & 1]));
+          continue;
+        }
         tc_fence_after();
 #ifdef VAFA_TRACE
         const long long t_sm0 = clock64();
@@ -363,7 +379,7 @@ varlen_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_const
         const int lim_diag = w.masked ? (w.diag - b * kBlk) : 0x3fffffff;  // for row 0
         const bool masked_block = lim_tail < kBlk - 1 || lim_diag < kBlk - 1;  // same for the whole CTA
         if (masked_block) {
-          const int lim = min(lim_tail, w.masked ? lim_diag + r : 0x3fffffff) - half * kHalf;
+          const int lim = min(lim_tail, w.masked ? lim_diag + rq : 0x3fffffff) - half * kHalf;
 #pragma unroll
           for (int i = 0; i < kHalf; ++i) s[i] = (i <= lim) ? s[i] : -INFINITY;
         }
@@ -472,6 +488,11 @@ varlen_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_const
 
       // ---- epilogue ----
       float l_tot = 0.f;
+      if (!live) {
+        // (the wait keeps this warp within one phase of the barrier)
+        if (nb > 0 && !mbar_wait(smem_u32(&sm.o_done[(gk - 1) % S]), ((gk - 1) / S) & 1, abort_flag)) break;
+        continue;
+      }
       if (nb > 0) {
         if (!mbar_wait(smem_u32(&sm.o_done[(gk - 1) % S]), ((gk - 1) / S) & 1, abort_flag)) break;
         tc_fence_after();
@@ -486,7 +507,9 @@ varlen_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_const
       const float lse_val = dead ? -INFINITY : m_ref + log2f(l_tot);
       if (w.partial < 0) {
         const long long row = (long long)w.o_start + rq;
-        T* optr = reinterpret_cast<T*>(p.o) + (row * p.H + h) * D;
+        T* const obase = reinterpret_cast<T*>(p.o);
+        long long off[4];
+        quad_row_offsets(off, row_ok ? (row * p.H + h) * D : -1);
 #pragma unroll
         for (int c2 = 0; c2 < D / 64; ++c2) {
           const int cc = half * (D / 64) + c2;
@@ -502,9 +525,7 @@ varlen_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_const
 #pragma unroll
           for (int i = 0; i < 16; ++i)
             pw[i] = pack2_out<T>(__uint_as_float(t[2 * i]) * inv_l, __uint_as_float(t[2 * i + 1]) * inv_l);
-          // rows of the tile are consecutive (token, head) rows of O: H*D apart (absorb: D apart)
-          store_chunk_coalesced<T>(pw, optr + cc * 32, kAbsorb ? (long long)D : (long long)p.H * D, r,
-                                   kAbsorb ? w.o_rows * p.H : w.o_rows, 4);
+          store_chunk_rows<T>(pw, obase + cc * 32, off);
         }
         if (row_ok && half == 0) p.lse[row * p.H + h] = lse_val;
       } else {
@@ -994,57 +1015,73 @@ varlen_fwd_pair_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_
 // Merge the per-split partial outputs (already normalised, fp32) with their log2-domain LSE:
 //   m = max_s lse_s;  w_s = 2^(lse_s - m);  o = sum_s w_s o_s / sum_s w_s;  lse = m + log2 sum_s w_s
 // (reference: triton_fa_varlen_v2/triton_fa_varlen_v2/kernels.py:652-734).  One warp per
-// (row, head); each lane owns D/32 consecutive columns and reads them with one vector load.
+// (row, head); each lane owns D/32 consecutive columns and reads them with one vector load, four splits in
+// flight at a time.  A CTA takes eight (row, head) pairs of a unit, `chunks` such groups per unit, so that the few
+// units of a long-history batch spread over all SMs (one CTA per unit: 124 us for 64 units of 128 rows x 4 heads
+// of 64, i.e. 41 MB).
 template <typename T, int D>
 __global__ void __launch_bounds__(256) varlen_combine_kernel(const SchedHeader* __restrict__ header,
                                                              const CombineUnit* __restrict__ units,
                                                              const float* __restrict__ partial_o,
                                                              const float* __restrict__ partial_lse, T* __restrict__ o,
-                                                             float* __restrict__ lse, int H) {
+                                                             float* __restrict__ lse, int H, int chunks) {
   constexpr int V = D / 32;  // floats per lane: 4 (D=128) or 2 (D=64)
-  const int n_units = header->n_combine;
+  constexpr int kUnroll = 4;
+  const int n_work = header->n_combine * chunks;
   const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
-  for (int u = blockIdx.x; u < n_units; u += gridDim.x) {
-    const CombineUnit cu = units[u];
-    const int n_rh = cu.q_rows * H;
-    for (int rh = wib; rh < n_rh; rh += 8) {
-      const int r = rh / H, h = rh % H;
-      float m = -INFINITY;
-      for (int s = lane; s < cu.n_splits; s += 32)
-        m = fmaxf(m, partial_lse[((long long)cu.base + (long long)s * cu.q_rows + r) * H + h]);
+  for (int i = blockIdx.x; i < n_work; i += gridDim.x) {
+    const CombineUnit cu = units[i / chunks];
+    const int rh = (i % chunks) * 8 + wib;
+    if (rh >= cu.q_rows * H) continue;
+    const int r = rh / H, h = rh % H;
+    const long long step = (long long)cu.q_rows * H;  // (row, head) entries from one split to the next
+    const long long first = ((long long)cu.base + r) * H + h;
+    float m = -INFINITY;
+    for (int s = lane; s < cu.n_splits; s += 32) m = fmaxf(m, partial_lse[first + s * step]);
 #pragma unroll
-      for (int o_ = 16; o_ > 0; o_ >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o_));
-      const float m_use = (m == -INFINITY) ? 0.f : m;
-      float acc[V];
+    for (int o_ = 16; o_ > 0; o_ >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o_));
+    const float m_use = (m == -INFINITY) ? 0.f : m;
+    float acc[V];
 #pragma unroll
-      for (int i = 0; i < V; ++i) acc[i] = 0.f;
-      float den = 0.f;
-      for (int s = 0; s < cu.n_splits; ++s) {
-        const long long prow = (long long)cu.base + (long long)s * cu.q_rows + r;
-        const float wgt = exp2f(partial_lse[prow * H + h] - m_use);
-        den += wgt;
-        const float* src = partial_o + (prow * H + h) * D + lane * V;
-        if (V == 4) {
-          const float4 f = *reinterpret_cast<const float4*>(src);
-          acc[0] += wgt * f.x; acc[1] += wgt * f.y; acc[V - 2] += wgt * f.z; acc[V - 1] += wgt * f.w;
+    for (int j = 0; j < V; ++j) acc[j] = 0.f;
+    float den = 0.f;
+    for (int s0 = 0; s0 < cu.n_splits; s0 += kUnroll) {
+      float wgt[kUnroll], f[kUnroll][V];
+#pragma unroll
+      for (int t = 0; t < kUnroll; ++t) {
+        const bool ok = s0 + t < cu.n_splits;
+        const long long e = first + (ok ? s0 + t : s0) * step;
+        wgt[t] = ok ? partial_lse[e] : -INFINITY;
+        const float* src = partial_o + e * D + lane * V;
+        if constexpr (V == 4) {
+          const float4 x = *reinterpret_cast<const float4*>(src);
+          f[t][0] = x.x; f[t][1] = x.y; f[t][2] = x.z; f[t][3] = x.w;
         } else {
-          const float2 f = *reinterpret_cast<const float2*>(src);
-          acc[0] += wgt * f.x; acc[1] += wgt * f.y;
+          const float2 x = *reinterpret_cast<const float2*>(src);
+          f[t][0] = x.x; f[t][1] = x.y;
         }
       }
-      const float inv = den == 0.f ? 0.f : 1.f / den;  // a NaN weight sum goes out as NaN
-      const long long row = (long long)cu.q_start + r;
-      T* dst = o + (row * H + h) * D + lane * V;
-      if (V == 4) {
-        uint2 pk;
-        pk.x = pack2_out<T>(acc[0] * inv, acc[1] * inv);
-        pk.y = pack2_out<T>(acc[V - 2] * inv, acc[V - 1] * inv);
-        *reinterpret_cast<uint2*>(dst) = pk;
-      } else {
-        *reinterpret_cast<uint32_t*>(dst) = pack2_out<T>(acc[0] * inv, acc[1] * inv);
+#pragma unroll
+      for (int t = 0; t < kUnroll; ++t) {
+        if (s0 + t >= cu.n_splits) break;
+        const float x = exp2f(wgt[t] - m_use);
+        den += x;
+#pragma unroll
+        for (int j = 0; j < V; ++j) acc[j] += x * f[t][j];
       }
-      if (lane == 0) lse[row * H + h] = den == 0.f ? -INFINITY : m_use + log2f(den);
     }
+    const float inv = den == 0.f ? 0.f : 1.f / den;  // a NaN weight sum goes out as NaN
+    const long long row = (long long)cu.q_start + r;
+    T* dst = o + (row * H + h) * D + lane * V;
+    if constexpr (V == 4) {
+      uint2 pk;
+      pk.x = pack2_out<T>(acc[0] * inv, acc[1] * inv);
+      pk.y = pack2_out<T>(acc[2] * inv, acc[3] * inv);
+      *reinterpret_cast<uint2*>(dst) = pk;
+    } else {
+      *reinterpret_cast<uint32_t*>(dst) = pack2_out<T>(acc[0] * inv, acc[1] * inv);
+    }
+    if (lane == 0) lse[row * H + h] = den == 0.f ? -INFINITY : m_use + log2f(den);
   }
 }
 
@@ -1063,6 +1100,17 @@ bool fwd_pair_enabled() {
   return on;
 }
 
+// Query heads stacked into one tile (see varlen_fwd_kernel).  With one item per query head a grouped-query decode
+// step reads and multiplies each key tile once per query head (from L2, for one real row in 128); stacked, once
+// per K/V head.  A stack never needs more tiles than separate heads do (ceil(q G / 128) <= G ceil(q / 128)), but
+// from 128 query rows per segment on it does not need fewer either and the separate heads keep the tile's
+// rows in one head, so the line lies there (by the mean over the batch, which is all the host knows).
+int fwd_stack(const vafa_varlen_args* a) {
+  const int h_kv = a->num_kv_heads > 0 ? a->num_kv_heads : a->num_heads;
+  const int g = a->num_heads / h_kv;
+  return (g > 1 && g <= kTile && a->total_q < (long long)kTile * a->n_seg) ? g : 1;
+}
+
 struct FwdWorkspace {
   size_t header, items, combine, plse, po, total;
   SchedCaps caps;
@@ -1072,7 +1120,9 @@ struct FwdWorkspace {
 // (the scheduler then splits less, or not at all); total > limit afterwards means it cannot fit.
 FwdWorkspace fwd_workspace(const vafa_varlen_args* a, int sm_count, size_t limit = 0) {
   FwdWorkspace w;
-  w.caps = sched_caps(kSchedFwd, a->total_q, a->total_k, a->n_seg, a->num_heads, sm_count, a->split_k_block);
+  const int stack = fwd_stack(a);
+  w.caps = sched_caps(kSchedFwd, a->total_q, a->total_k, a->n_seg, a->num_heads / stack, sm_count, a->split_k_block,
+                      kTile / stack);
   w.header = 0;
   w.items = 256;
   w.combine = w.items + align_up((size_t)w.caps.cap_items * sizeof(WorkItem), 256);
@@ -1110,15 +1160,17 @@ int launch_fwd(const vafa_varlen_args* a, cudaStream_t s, void* scratch = nullpt
   sp.header = (SchedHeader*)(base + ws.header);
   sp.items = (WorkItem*)(base + ws.items);
   sp.combine = (CombineUnit*)(base + ws.combine);
+  const int h_kv = a->num_kv_heads > 0 ? a->num_kv_heads : a->num_heads;
+  const int stack = fwd_stack(a);
+  if (stack > 1) { sp.tile_rows = kTile / stack; sp.H = h_kv; }
   // long query segments: tiles of 256 rows, worked on as two 128-row tiles per CTA
-  const bool pair = fwd_pair_enabled() && (long long)a->total_q > 160LL * a->n_seg;
+  const bool pair = fwd_pair_enabled() && stack == 1 && (long long)a->total_q > 160LL * a->n_seg;
   if (pair) sp.tile_rows = 2 * kTile;
   int rc = launch_scheduler(sp, s);
   if (rc) return rc;
 
   CUtensorMap tq, tk, tv;
-  if ((rc = encode_tmap_rows(&tq, a->q, a->dtype, a->total_q, a->num_heads, D, 128))) return rc;
-  const int h_kv = a->num_kv_heads > 0 ? a->num_kv_heads : a->num_heads;
+  if ((rc = encode_tmap_rows(&tq, a->q, a->dtype, a->total_q, a->num_heads, D, kTile / stack, stack))) return rc;
   if ((rc = encode_tmap_rows(&tk, a->k, a->dtype, a->total_k, h_kv, D, 128))) return rc;
   if ((rc = encode_tmap_rows(&tv, a->v, a->dtype, a->total_k, h_kv, D, 128))) return rc;
 
@@ -1128,7 +1180,9 @@ int launch_fwd(const vafa_varlen_args* a, cudaStream_t s, void* scratch = nullpt
   p.partial_lse = (float*)(base + ws.plse);
   p.partial_o = (float*)(base + ws.po);
   p.header = sp.header; p.items = sp.items; p.H = a->num_heads;
-  p.group = a->num_heads / h_kv;
+  p.stack = stack;
+  p.group = stack > 1 ? 1 : a->num_heads / h_kv;
+  p.q_bytes = kTile / stack * stack * D * 2;
   p.scale_log2 = a->scale * kLog2e;
   p.status = a->status;
   p.trace = nullptr;
@@ -1155,8 +1209,10 @@ int launch_fwd(const vafa_varlen_args* a, cudaStream_t s, void* scratch = nullpt
   }
   VAFA_LAUNCH_CHECK("varlen_fwd_kernel");
   LaunchScope scope(kKCombine, s);
-  varlen_combine_kernel<T, D><<<2 * sms, 256, 0, s>>>(sp.header, sp.combine, p.partial_o, p.partial_lse,
-                                                      (T*)a->o, a->lse, a->num_heads);
+  const int unit_rows = sp.tile_rows < a->total_q ? sp.tile_rows : a->total_q;
+  const int chunks = (unit_rows * a->num_heads + 7) / 8;
+  varlen_combine_kernel<T, D><<<4 * sms, 256, 0, s>>>(sp.header, sp.combine, p.partial_o, p.partial_lse,
+                                                      (T*)a->o, a->lse, a->num_heads, chunks);
   VAFA_LAUNCH_CHECK("varlen_combine_kernel");
   return 0;
 }
@@ -1206,6 +1262,8 @@ int launch_absorb_core_fwd(const AbsorbCoreArgs& a, cudaStream_t s) {
   p.o = a.axn; p.lse = a.lse; p.partial_o = nullptr; p.partial_lse = nullptr;
   p.header = sp.header; p.items = sp.items; p.H = a.H;
   p.group = 1;
+  p.stack = a.H;
+  p.q_bytes = kTile / a.H * a.H * D * 2;
   p.scale_log2 = a.scale * kLog2e;
   p.status = a.status;
   p.trace = nullptr;
