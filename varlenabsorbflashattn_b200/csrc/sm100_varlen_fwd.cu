@@ -114,9 +114,11 @@ struct FwdParams {
   const SchedHeader* header;
   const WorkItem* items;
   int H;
+  int total_q;
   int group;  // query heads per K/V head when an item is one query head (stack == 1)
   int stack;  // heads stacked into a tile: tile row = (query row) * stack + (head of the stack)
   int q_bytes;  // bytes one copy of the query tile delivers (stack * rows per tile rows of D elements)
+  int part_q;   // queries in a 16-row part of the tile (16 / stack), 0 = the tile is always loaded whole
   float scale_log2;
   int32_t* status;
   int wait_limit;  // bound of every device-side wait, in units of 65536 cycles
@@ -134,10 +136,14 @@ struct FwdParams {
 // Rows past the item's last query are padding.  Softmax warps whose 32 rows are all padding (a decode item
 // has one to eight rows) only follow the barriers: a row of P.V depends on its own row of P alone, so what
 // the padding rows hold never reaches a real one.
+// A tile that is at least half padding is loaded in 16-row parts, those without a query from past the end of q,
+// where TMA fills in zeros.  Loading the box whole puts the queries of other segments into the padding rows, and
+// multiplying those costs power: decode over 8k-32k keys ran at the 1 kW limit and 1.1-1.2 GHz.
 template <typename T, int D, bool kAbsorb>
 __global__ void __launch_bounds__(kFwdThreads, 1)
 varlen_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ CUtensorMap tmap_k,
-                  const __grid_constant__ CUtensorMap tmap_v, const FwdParams p) {
+                  const __grid_constant__ CUtensorMap tmap_v, const __grid_constant__ CUtensorMap tmap_qp,
+                  const FwdParams p) {
   using Cfg = FwdCfg<D>;
   constexpr int S = fwd_key_stages<kAbsorb>();
   constexpr int kBlk = fwd_block_keys<kAbsorb>();   // keys per block
@@ -206,9 +212,18 @@ varlen_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_const
         const int nb = (w.i_len + kBlk - 1) / kBlk;
         if (nb == 0) continue;
         { TRACE_T0(); if (!mbar_wait(smem_u32(&sm.q_free), (qi & 1) ^ 1, abort_flag)) break; TRACE_ADD(0); }
-        mbar_expect_tx(smem_u32(&sm.q_full), p.q_bytes);
-        for (int c = 0; c < Cfg::kSub; ++c)
-          tma_load_3d(smem_u32(sm.q) + c * Cfg::kSubBytes, &tmap_q, smem_u32(&sm.q_full), c * 64, h, w.o_start);
+        if (p.part_q > 0 && w.o_rows * p.stack <= kTile / 2) {
+          mbar_expect_tx(smem_u32(&sm.q_full), Cfg::kTileBytes);
+          for (int t = 0; t < kTile / 16; ++t) {
+            const int q_row = t * p.part_q < w.o_rows ? w.o_start + t * p.part_q : p.total_q;
+            for (int c = 0; c < Cfg::kSub; ++c)
+              tma_load_3d(smem_u32(sm.q) + c * Cfg::kSubBytes + t * 2048, &tmap_qp, smem_u32(&sm.q_full), c * 64, h, q_row);
+          }
+        } else {
+          mbar_expect_tx(smem_u32(&sm.q_full), p.q_bytes);
+          for (int c = 0; c < Cfg::kSub; ++c)
+            tma_load_3d(smem_u32(sm.q) + c * Cfg::kSubBytes, &tmap_q, smem_u32(&sm.q_full), c * 64, h, w.o_start);
+        }
         // absorb: X is streamed once from HBM (no other CTA reads this user's keys), and a K slot is only
         // released after P.X of its block, so the two-slot ring alone leaves the HBM latency exposed
         // (measured: the MMA issuer waited for tiles half of the time).  Tiles a few blocks ahead are
@@ -1183,6 +1198,10 @@ int launch_fwd(const vafa_varlen_args* a, cudaStream_t s, void* scratch = nullpt
   p.stack = stack;
   p.group = stack > 1 ? 1 : a->num_heads / h_kv;
   p.q_bytes = kTile / stack * stack * D * 2;
+  p.part_q = 16 % stack == 0 ? 16 / stack : 0;
+  p.total_q = a->total_q;
+  CUtensorMap tqp = tq;
+  if (p.part_q > 0 && (rc = encode_tmap_rows(&tqp, a->q, a->dtype, a->total_q, a->num_heads, D, p.part_q, stack))) return rc;
   p.scale_log2 = a->scale * kLog2e;
   p.status = a->status;
   p.trace = nullptr;
@@ -1205,7 +1224,7 @@ int launch_fwd(const vafa_varlen_args* a, cudaStream_t s, void* scratch = nullpt
     const size_t smem = sizeof(FwdSmem<D, false>) + 1024;
     VAFA_CUDA_CHECK(cudaFuncSetAttribute(varlen_fwd_kernel<T, D, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     LaunchScope scope(kKFwd, s);
-    varlen_fwd_kernel<T, D, false><<<sms, kFwdThreads, smem, s>>>(tq, tk, tv, p);
+    varlen_fwd_kernel<T, D, false><<<sms, kFwdThreads, smem, s>>>(tq, tk, tv, tqp, p);
   }
   VAFA_LAUNCH_CHECK("varlen_fwd_kernel");
   LaunchScope scope(kKCombine, s);
@@ -1264,6 +1283,10 @@ int launch_absorb_core_fwd(const AbsorbCoreArgs& a, cudaStream_t s) {
   p.group = 1;
   p.stack = a.H;
   p.q_bytes = kTile / a.H * a.H * D * 2;
+  p.part_q = 16 % a.H == 0 ? 16 / a.H : 0;
+  p.total_q = a.total_q;
+  CUtensorMap tup = tu;
+  if (p.part_q > 0 && (rc = encode_tmap_rows(&tup, a.u, a.dtype, a.total_q, a.H, D, p.part_q, a.H))) return rc;
   p.scale_log2 = a.scale * kLog2e;
   p.status = a.status;
   p.trace = nullptr;
@@ -1279,7 +1302,7 @@ int launch_absorb_core_fwd(const AbsorbCoreArgs& a, cudaStream_t s) {
   const size_t smem = sizeof(FwdSmem<D, true>) + 1024;
   VAFA_CUDA_CHECK(cudaFuncSetAttribute(varlen_fwd_kernel<T, D, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   LaunchScope scope(kKAbsorbFwd, s);
-  varlen_fwd_kernel<T, D, true><<<sms, kFwdThreads, smem, s>>>(tu, tx, tx, p);
+  varlen_fwd_kernel<T, D, true><<<sms, kFwdThreads, smem, s>>>(tu, tx, tx, tup, p);
   VAFA_LAUNCH_CHECK("varlen_fwd_kernel<absorb>");
   return 0;
 }
