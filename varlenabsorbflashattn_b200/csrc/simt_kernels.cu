@@ -372,6 +372,7 @@ int simt_attn_fwd(const SimtAttnParams& p, cudaStream_t s) {
   const long long n = (long long)p.total_q * p.H;
   if (n == 0) return 0;
   LaunchScope scope(kKSimtFwd, s);
+  if (simt_tiles_ok(p)) return simt_tiles_fwd(p, s);
   DISPATCH_T(p.dtype, simt_fwd_kernel<T><<<warp_grid(n), kWarpsPerBlock * 32, 0, s>>>(p));
   VAFA_LAUNCH_CHECK("simt_fwd_kernel");
   return 0;
@@ -391,6 +392,7 @@ int simt_attn_dq(const SimtAttnParams& p, cudaStream_t s) {
   const long long n = (long long)p.total_q * p.H;
   if (n == 0) return 0;
   LaunchScope scope(kKSimtDq, s);
+  if (simt_tiles_ok(p)) return simt_tiles_dq(p, s);
   if (p.do_f32) {
     DISPATCH_T(p.dtype, simt_dq_kernel<T, float><<<warp_grid(n), kWarpsPerBlock * 32, 0, s>>>(p));
   } else {
@@ -405,6 +407,7 @@ int simt_attn_dkv(const SimtAttnParams& p, cudaStream_t s) {
   const long long n = p.shared_kv ? (long long)p.total_k : (long long)p.total_k * p.H;
   if (n == 0) return 0;
   LaunchScope scope(kKSimtDkv, s);
+  if (simt_tiles_ok(p)) return simt_tiles_dkv(p, s);
   if (p.do_f32) {
     DISPATCH_T(p.dtype, simt_dkv_kernel<T, float><<<warp_grid(n), kWarpsPerBlock * 32, 0, s>>>(p));
   } else {

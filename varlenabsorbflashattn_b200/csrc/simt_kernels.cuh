@@ -31,6 +31,15 @@ int simt_attn_delta(const void* o, const void* d_o, float* delta, int rows, int 
 int simt_attn_dq(const SimtAttnParams& p, cudaStream_t s);
 int simt_attn_dkv(const SimtAttnParams& p, cudaStream_t s);
 
+// The tiled kernels (simt_tiles.cu): whether they take this call, and their launches.  A tile has 64 outer rows, of
+// which a warp owns eight; below kTileMinRows (stacked) query rows or keys per segment on average most of a
+// tile would be padding and the one-warp-per-row kernels stay.
+constexpr int kTileMinRows = 8;
+bool simt_tiles_ok(const SimtAttnParams& p);
+int simt_tiles_fwd(const SimtAttnParams& p, cudaStream_t s);
+int simt_tiles_dq(const SimtAttnParams& p, cudaStream_t s);
+int simt_tiles_dkv(const SimtAttnParams& p, cudaStream_t s);
+
 // C[b][m][n] = alpha * sum_k A[b][m][k] * B[b][k][n]; strides in elements; fp32 accumulate.
 struct SimtGemm {
   const void* A; const void* B; void* C;
