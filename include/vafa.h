@@ -208,6 +208,12 @@ int vafa_absorb_inner_bwd(const vafa_absorb_args* a, vafa_stream_t stream);
 int vafa_cast_from_f32(const float* src, void* dst, size_t n, int32_t dtype, vafa_stream_t stream);
 
 /* ---- housekeeping ------------------------------------------------------------------ */
+/* The host-side check of two prefix-sum arrays of n_seg + 1 entries on the device: both start at 0, end at their
+ * total, never decrease, and, with need_keys, every segment with query rows has keys.  Copies both to the host
+ * behind the work already queued on `stream` and waits for them.  Returns 0 when all holds, 1 when something does
+ * not (the caller words the error), a negative code when the copy failed or the stream is being captured. */
+int vafa_check_cu_seqlens(const int32_t* cu_q, const int32_t* cu_k, int32_t n_seg, int32_t total_q, int32_t total_k,
+                          int32_t need_keys, vafa_stream_t stream);
 int vafa_abi_version(void);
 const char* vafa_last_error(void);           /* thread-local text of the last failure */
 /* Copy the status word to the host (synchronises `stream`) and translate it: returns 0 or

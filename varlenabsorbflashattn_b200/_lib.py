@@ -5,6 +5,7 @@ raised.  Nothing here computes anything.
 """
 from __future__ import annotations
 
+import contextlib
 import ctypes as C
 import os
 import threading
@@ -23,7 +24,7 @@ STATUS_WORDS = 4
 DTYPE_CODE = {torch.float32: VAFA_F32, torch.bfloat16: VAFA_BF16, torch.float16: VAFA_F16}
 
 EXPORTS = (
-    "vafa_abi_version", "vafa_last_error", "vafa_check_status", "vafa_cast_from_f32",
+    "vafa_abi_version", "vafa_last_error", "vafa_check_status", "vafa_cast_from_f32", "vafa_check_cu_seqlens",
     "vafa_varlen_fwd_workspace_bytes", "vafa_varlen_bwd_workspace_bytes", "vafa_varlen_fwd", "vafa_varlen_bwd",
     "vafa_varlen_fwd_noalloc",
     "vafa_absorb_saved_bytes", "vafa_absorb_fwd_workspace_bytes", "vafa_absorb_bwd_workspace_bytes",
@@ -81,6 +82,8 @@ def load() -> C.CDLL:
         lib.vafa_last_error.restype = C.c_char_p
         lib.vafa_check_status.argtypes = [C.c_void_p, C.c_void_p]
         lib.vafa_check_status.restype = C.c_int
+        lib.vafa_check_cu_seqlens.argtypes = [C.c_void_p, C.c_void_p, C.c_int32, C.c_int32, C.c_int32, C.c_int32, C.c_void_p]
+        lib.vafa_check_cu_seqlens.restype = C.c_int
         lib.vafa_cast_from_f32.argtypes = [C.c_void_p, C.c_void_p, C.c_size_t, C.c_int32, C.c_void_p]
         lib.vafa_cast_from_f32.restype = C.c_int
         for name in ("vafa_varlen_fwd_workspace_bytes", "vafa_varlen_bwd_workspace_bytes"):
@@ -146,6 +149,19 @@ def sm_count(device: torch.device) -> int:
     return n
 
 
+def raw_stream(device: torch.device) -> int:
+    """The current stream of the device, as the pointer the library takes."""
+    return torch._C._cuda_getCurrentRawStream(device.index)
+
+
+_HERE = contextlib.nullcontext()
+
+
+def on_device(device: torch.device):
+    """`torch.cuda.device(device)` where that changes anything."""
+    return _HERE if torch.cuda.current_device() == device.index else torch.cuda.device(device)
+
+
 def check_status(device: torch.device) -> None:
     """Synchronise the current stream and raise if a kernel reported an error."""
     st = status_word(device)
@@ -176,6 +192,21 @@ def set_check_status(enabled: bool) -> None:
 def maybe_check_status(device: torch.device) -> None:
     if _check_after_each_op:
         check_status(device)
+
+
+def cu_seqlens_ok(cu_q: torch.Tensor, cu_k: torch.Tensor, total_q: int, total_k: int, need_keys: bool) -> bool:
+    """Whether two prefix-sum tensors (1-D int32, contiguous, on one GPU, equally long) describe the batch: one call
+    that copies both to the host and walks them there.  With torch operations on host copies the same checks
+    took over 100 us a call, all of it with the GPU idle behind the copy.  The caller words the error."""
+    n_seg = cu_q.numel() - 1
+    if cu_q.dim() != 1 or cu_k.dim() != 1 or n_seg < 1 or max(total_q, total_k) > 2**31 - 1:
+        return False
+    with on_device(cu_q.device):
+        rc = load().vafa_check_cu_seqlens(cu_q.data_ptr(), cu_k.data_ptr(), n_seg, total_q, total_k, int(need_keys),
+                                          raw_stream(cu_q.device))
+    if rc < 0:
+        check(rc, "vafa_check_cu_seqlens")
+    return rc == 0
 
 
 def workspace(nbytes: int, device: torch.device) -> torch.Tensor | None:

@@ -75,6 +75,8 @@ def _check_cu(cu: torch.Tensor, total: int, name: str) -> torch.Tensor:
 
 def _validate(cu_q, cu_k, T_q, T_k) -> None:
     assert cu_q.numel() == cu_k.numel(), "segment count mismatch q vs k"
+    if cu_q.is_cuda and _lib.cu_seqlens_ok(cu_q, cu_k, T_q, T_k, True):
+        return
     hq = _check_cu(cu_q, T_q, "cu_seqlens_q")
     hk = _check_cu(cu_k, T_k, "cu_seqlens_k")
     # reference: interface.py:109-116
@@ -111,10 +113,6 @@ def _fill(a: _lib.AbsorbArgs, device, cu_q, cu_k, T_q, T_k, d_q, d_kv, H, D_H, d
     a.status = _lib.status_word(device).data_ptr()
 
 
-def _stream() -> int:
-    return torch.cuda.current_stream().cuda_stream
-
-
 class _PackedTargetAttn(torch.autograd.Function):
     """q_raw, X, W_Q, W_K, W_V -> O, with all five gradients from the library."""
 
@@ -128,7 +126,7 @@ class _PackedTargetAttn(torch.autograd.Function):
         dev = q_raw.device
         O = torch.empty((T_q, H, D_H), dtype=q_raw.dtype, device=dev)
         lse = torch.empty((T_q, H), dtype=torch.float32, device=dev)
-        with torch.cuda.device(dev):
+        with _lib.on_device(dev):
             a = _lib.AbsorbArgs()
             _fill(a, dev, cu_q, cu_k, T_q, T_k, d_q, d_kv, H, D_H, q_raw.dtype, scale, x_w)
             a.q_raw, a.x, a.w_q, a.w_k, a.w_v = (t.data_ptr() for t in (q_raw, X, W_Q, W_K, W_V))
@@ -137,7 +135,7 @@ class _PackedTargetAttn(torch.autograd.Function):
             a.saved = saved.data_ptr()
             ws = _lib.workspace(lib.vafa_absorb_fwd_workspace_bytes(a), dev)
             a.workspace, a.workspace_bytes = _lib.ptr(ws), 0 if ws is None else ws.numel()
-            _lib.check(lib.vafa_absorb_fwd(a, _stream()), "vafa_absorb_fwd")
+            _lib.check(lib.vafa_absorb_fwd(a, _lib.raw_stream(dev)), "vafa_absorb_fwd")
             _lib.maybe_check_status(dev)
         ctx.save_for_backward(q_raw, X, W_Q, W_K, W_V, O, lse, cu_q, cu_k, saved)
         ctx.scale, ctx.group = scale, group
@@ -160,7 +158,7 @@ class _PackedTargetAttn(torch.autograd.Function):
         dq_raw, dX = torch.empty_like(q_raw), torch.empty_like(X)
         n_wq, n_wk = d_q * H * D_H, d_kv * H * D_H
         dw = torch.empty(n_wq + 2 * n_wk, dtype=torch.float32, device=dev)
-        with torch.cuda.device(dev):
+        with _lib.on_device(dev):
             a = _lib.AbsorbArgs()
             _fill(a, dev, cu_q, cu_k, T_q, T_k, d_q, d_kv, H, D_H, q_raw.dtype, ctx.scale, x_w)
             a.q_raw, a.x, a.w_q, a.w_k, a.w_v = (t.data_ptr() for t in (q_raw, X, W_Q, W_K, W_V))
@@ -169,14 +167,14 @@ class _PackedTargetAttn(torch.autograd.Function):
             ws = _lib.workspace(lib.vafa_absorb_bwd_workspace_bytes(a), dev)
             a.workspace, a.workspace_bytes = _lib.ptr(ws), 0 if ws is None else ws.numel()
             if ctx.group is None:
-                _lib.check(lib.vafa_absorb_bwd(a, _stream()), "vafa_absorb_bwd")
+                _lib.check(lib.vafa_absorb_bwd(a, _lib.raw_stream(dev)), "vafa_absorb_bwd")
             else:
                 # weight gradients first; their all-reduce (on the process group's own stream) then runs
                 # under the dX kernel and the dq_raw product, and the rounding below waits for it
                 import torch.distributed as dist
-                _lib.check(lib.vafa_absorb_bwd_phase(a, 1, _stream()), "vafa_absorb_bwd_phase(1)")
+                _lib.check(lib.vafa_absorb_bwd_phase(a, 1, _lib.raw_stream(dev)), "vafa_absorb_bwd_phase(1)")
                 work = dist.all_reduce(dw, group=ctx.group, async_op=True)
-                _lib.check(lib.vafa_absorb_bwd_phase(a, 2, _stream()), "vafa_absorb_bwd_phase(2)")
+                _lib.check(lib.vafa_absorb_bwd_phase(a, 2, _lib.raw_stream(dev)), "vafa_absorb_bwd_phase(2)")
                 work.wait()
             _lib.maybe_check_status(dev)
             if q_raw.dtype == torch.float32:
@@ -184,7 +182,7 @@ class _PackedTargetAttn(torch.autograd.Function):
             else:
                 dwc = torch.empty(dw.numel(), dtype=q_raw.dtype, device=dev)
                 _lib.check(lib.vafa_cast_from_f32(dw.data_ptr(), dwc.data_ptr(), dw.numel(),
-                                                  _lib.DTYPE_CODE[q_raw.dtype], _stream()), "vafa_cast_from_f32")
+                                                  _lib.DTYPE_CODE[q_raw.dtype], _lib.raw_stream(dev)), "vafa_cast_from_f32")
         dW_Q = dwc[:n_wq].view(d_q, H, D_H)
         dW_K = dwc[n_wq:n_wq + n_wk].view(d_kv, H, D_H)
         dW_V = dwc[n_wq + n_wk:].view(d_kv, H, D_H)
@@ -203,7 +201,7 @@ class _TargetAttnInner(torch.autograd.Function):
         dev = u.device
         O = torch.empty((T_q, H, D_H), dtype=u.dtype, device=dev)
         lse = torch.empty((T_q, H), dtype=torch.float32, device=dev)
-        with torch.cuda.device(dev):
+        with _lib.on_device(dev):
             a = _lib.AbsorbArgs()
             _fill(a, dev, cu_q, cu_k, T_q, T_k, 0, d_kv, H, D_H, u.dtype, scale, x_w)
             a.q_raw, a.x, a.w_v = u.data_ptr(), X.data_ptr(), W_V.data_ptr()
@@ -212,7 +210,7 @@ class _TargetAttnInner(torch.autograd.Function):
             a.saved = saved.data_ptr()
             ws = _lib.workspace(lib.vafa_absorb_fwd_workspace_bytes(a), dev)
             a.workspace, a.workspace_bytes = _lib.ptr(ws), 0 if ws is None else ws.numel()
-            _lib.check(lib.vafa_absorb_inner_fwd(a, _stream()), "vafa_absorb_inner_fwd")
+            _lib.check(lib.vafa_absorb_inner_fwd(a, _lib.raw_stream(dev)), "vafa_absorb_inner_fwd")
             _lib.maybe_check_status(dev)
         ctx.save_for_backward(u, X, W_V, O, lse, cu_q, cu_k, saved)
         ctx.scale = scale
@@ -233,7 +231,7 @@ class _TargetAttnInner(torch.autograd.Function):
             dO = dO.contiguous()
         du, dX = torch.empty_like(u), torch.empty_like(X)
         dw = torch.empty(d_kv * H * D_H, dtype=torch.float32, device=dev)
-        with torch.cuda.device(dev):
+        with _lib.on_device(dev):
             a = _lib.AbsorbArgs()
             _fill(a, dev, cu_q, cu_k, T_q, T_k, 0, d_kv, H, D_H, u.dtype, ctx.scale, x_w)
             a.q_raw, a.x, a.w_v = u.data_ptr(), X.data_ptr(), W_V.data_ptr()
@@ -241,7 +239,7 @@ class _TargetAttnInner(torch.autograd.Function):
             a.dq_raw, a.dx, a.dw = du.data_ptr(), dX.data_ptr(), dw.data_ptr()
             ws = _lib.workspace(lib.vafa_absorb_bwd_workspace_bytes(a), dev)
             a.workspace, a.workspace_bytes = _lib.ptr(ws), 0 if ws is None else ws.numel()
-            _lib.check(lib.vafa_absorb_inner_bwd(a, _stream()), "vafa_absorb_inner_bwd")
+            _lib.check(lib.vafa_absorb_inner_bwd(a, _lib.raw_stream(dev)), "vafa_absorb_inner_bwd")
             _lib.maybe_check_status(dev)
         dW_V = dw.view(d_kv, H, D_H).to(u.dtype)
         return du, dX, dW_V, None, None, None

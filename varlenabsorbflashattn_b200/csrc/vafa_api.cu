@@ -4,6 +4,8 @@
 #include <cstring>
 #include <atomic>
 #include <mutex>
+#include <new>
+#include <vector>
 
 #include "common.cuh"
 #include "simt_kernels.cuh"
@@ -617,6 +619,32 @@ int vafa_absorb_inner_bwd(const vafa_absorb_args* a, vafa_stream_t stream) {
 int vafa_cast_from_f32(const float* src, void* dst, size_t n, int32_t dtype, vafa_stream_t stream) {
   if (n > 0 && (!src || !dst)) return fail(VAFA_ERR_INVALID, "null pointer");
   return cast_from_f32(src, dst, n, dtype, (cudaStream_t)stream);
+}
+
+int vafa_check_cu_seqlens(const int32_t* cu_q, const int32_t* cu_k, int32_t n_seg, int32_t total_q, int32_t total_k,
+                          int32_t need_keys, vafa_stream_t stream) {
+  if (!cu_q || !cu_k || n_seg < 1) return fail(VAFA_ERR_INVALID, "check_cu_seqlens: null array or n_seg %d", n_seg);
+  const cudaStream_t s = (cudaStream_t)stream;
+  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+  VAFA_CUDA_CHECK(cudaStreamIsCapturing(s, &cap));
+  if (cap != cudaStreamCaptureStatusNone)
+    return fail(VAFA_ERR_CUDA, "cu_seqlens cannot be checked on the host while the stream is captured: switch the check off");
+  const size_t n = (size_t)n_seg + 1;
+  std::vector<int32_t> host;
+  try {
+    host.resize(cu_q == cu_k ? n : 2 * n);
+  } catch (const std::bad_alloc&) {
+    return fail(VAFA_ERR_INVALID, "check_cu_seqlens: out of host memory");
+  }
+  VAFA_CUDA_CHECK(cudaMemcpyAsync(host.data(), cu_q, n * 4, cudaMemcpyDeviceToHost, s));
+  if (cu_q != cu_k) VAFA_CUDA_CHECK(cudaMemcpyAsync(host.data() + n, cu_k, n * 4, cudaMemcpyDeviceToHost, s));
+  VAFA_CUDA_CHECK(cudaStreamSynchronize(s));
+  const int32_t* q = host.data();
+  const int32_t* k = cu_q == cu_k ? q : q + n;
+  bool ok = q[0] == 0 && k[0] == 0 && q[n_seg] == total_q && k[n_seg] == total_k;
+  for (int32_t i = 0; i < n_seg; ++i)
+    ok = ok && q[i + 1] >= q[i] && k[i + 1] >= k[i] && !(need_keys && q[i + 1] > q[i] && k[i + 1] == k[i]);
+  return ok ? 0 : 1;
 }
 
 long long vafa_set_wait_limit_cycles(long long cycles) {

@@ -143,17 +143,18 @@ class _PackedVarlenAttn(torch.autograd.Function):
         cu_k = cu_k.to(device=q.device, dtype=torch.int32).contiguous()
         assert cu_k.numel() == cu_q.numel(), \
             f"segment count mismatch: q has {cu_q.numel() - 1}, k has {cu_k.numel() - 1}"
-        _check_cu(cu_q, T_q, "cu_seqlens_q")
-        _check_cu(cu_k, T_k, "cu_seqlens_k")
+        if _validate and not _lib.cu_seqlens_ok(cu_q, cu_k, T_q, T_k, False):
+            _check_cu(cu_q, T_q, "cu_seqlens_q")
+            _check_cu(cu_k, T_k, "cu_seqlens_k")
 
         lib = _lib.load()
         o = torch.empty_like(q)
         lse = torch.empty((T_q, H), dtype=torch.float32, device=q.device)
-        with torch.cuda.device(q.device):
+        with _lib.on_device(q.device):
             a = _fill_args(q, k, v, o, lse, cu_q, cu_k, scale, causal, split_k_block)
             ws = _lib.workspace(lib.vafa_varlen_fwd_workspace_bytes(a), q.device)
             a.workspace, a.workspace_bytes = _lib.ptr(ws), 0 if ws is None else ws.numel()
-            _lib.check(lib.vafa_varlen_fwd(a, torch.cuda.current_stream().cuda_stream), "vafa_varlen_fwd")
+            _lib.check(lib.vafa_varlen_fwd(a, _lib.raw_stream(q.device)), "vafa_varlen_fwd")
             _lib.maybe_check_status(q.device)
         ctx.save_for_backward(q, k, v, o, lse, cu_q, cu_k)
         ctx.scale, ctx.causal, ctx.split_k_block = scale, causal, split_k_block
@@ -169,12 +170,12 @@ class _PackedVarlenAttn(torch.autograd.Function):
             do = do.contiguous()
         lib = _lib.load()
         dq, dk, dv = torch.empty_like(q), torch.empty_like(k), torch.empty_like(v)
-        with torch.cuda.device(q.device):
+        with _lib.on_device(q.device):
             a = _fill_args(q, k, v, o, lse, cu_q, cu_k, ctx.scale, ctx.causal, ctx.split_k_block)
             a.d_o, a.dq, a.dk, a.dv = do.data_ptr(), dq.data_ptr(), dk.data_ptr(), dv.data_ptr()
             ws = _lib.workspace(lib.vafa_varlen_bwd_workspace_bytes(a), q.device)
             a.workspace, a.workspace_bytes = _lib.ptr(ws), 0 if ws is None else ws.numel()
-            _lib.check(lib.vafa_varlen_bwd(a, torch.cuda.current_stream().cuda_stream), "vafa_varlen_bwd")
+            _lib.check(lib.vafa_varlen_bwd(a, _lib.raw_stream(q.device)), "vafa_varlen_bwd")
             _lib.maybe_check_status(q.device)
         return dq, dk, dv, None, None, None, None, None
 
