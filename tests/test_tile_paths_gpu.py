@@ -5,7 +5,7 @@ import pytest
 import torch
 
 import varlenabsorbflashattn_b200 as vb
-from oracle import make_varlen_inputs, varlen_attn_ref
+from oracle import make_absorb_inputs, make_varlen_inputs, target_attn_ref_fwd_bwd, varlen_attn_ref
 from helpers import LN2, check_close, check_lse
 
 pytestmark = pytest.mark.gpu
@@ -46,3 +46,21 @@ def test_long_segments_are_cut(ql, kl, H):
     ro, rlse = varlen_attn_ref(q, k, v, cu_q, cu_k)
     check_close("o", o, ro, torch.bfloat16)
     check_lse(lse / LN2, rlse)
+
+
+@pytest.mark.parametrize("ql,kl,H", [
+    ([16], [5000], 8),                                      # one user, one full tile
+    ([1, 16, 17, 0, 3], [700, 2048, 2047, 5, 0], 8),        # cut and uncut tiles, a second tile of one query
+    ([5, 40], [3000, 97], 4), ([3] * 24, [8] * 23 + [2048], 8)])
+def test_few_users_with_long_histories_are_cut(ql, kl, H):
+    """Absorb: up to four tiles per SM the histories are cut and the parts merged (also read by the backward)."""
+    ql = [a if b else 0 for a, b in zip(ql, kl)]
+    ins = make_absorb_inputs(ql, kl, 256, 256, H, 256 // H, torch.bfloat16, 14, x_std=0.3, w_std=0.1)
+    q_raw, X, W_Q, W_K, W_V, dO, cu_q, cu_k = ins
+    g = [t.to(DEV).requires_grad_(True) for t in (q_raw, X, W_Q, W_K, W_V)]
+    O = vb.packed_target_attn(*g, cu_seqlens_q=cu_q, cu_seqlens_k=cu_k)
+    O.backward(dO.to(DEV))
+    ref = target_attn_ref_fwd_bwd(*ins)
+    check_close("O", O, ref[0], torch.bfloat16, scale_abs=True)
+    for name, t, r in zip(("dq_raw", "dX", "dW_Q", "dW_K", "dW_V"), g, ref[2:]):
+        check_close(name, t.grad, r, torch.bfloat16, scale_abs=True)
