@@ -1,6 +1,8 @@
 """Dispatch branches of the tile kernels at the sizes where they can go wrong: stacks of heads that do and do not
 divide a 128-row tile, segments around the tile's query count, rows of padding in whole warps, slices of a
 lone long segment."""
+import math
+
 import pytest
 import torch
 
@@ -64,3 +66,45 @@ def test_few_users_with_long_histories_are_cut(ql, kl, H):
     check_close("O", O, ref[0], torch.bfloat16, scale_abs=True)
     for name, t, r in zip(("dq_raw", "dX", "dW_Q", "dW_K", "dW_V"), g, ref[2:]):
         check_close(name, t.grad, r, torch.bfloat16, scale_abs=True)
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("D", [64, 128])
+@pytest.mark.parametrize("n_seg,H,climb", [(3, 2, 12.0), (3, 2, 130.0), (160, 8, 130.0)])
+def test_scores_that_climb_past_the_first_block(dtype, D, n_seg, H, climb):
+    """Scores of later blocks far above those of the first one (by `climb` log2 units and more, in steps): tiles whose
+    reference maximum is left are done again; with many of them a CTA stops trying."""
+    L = 700
+    q, k, v, _, cu_q, cu_k = make_varlen_inputs([L] * n_seg, [L] * n_seg, H, D, dtype, 21, with_do=False)
+    # a common direction: q[..., 0] = 1, and k[..., 0] steps up every 128 keys in every other segment
+    q[..., 0] = 1.0
+    step = torch.arange(L).div(128, rounding_mode="floor").float() * climb * math.log(2.0) * math.sqrt(D) / 4
+    for s in range(0, n_seg, 2):
+        k[s * L:(s + 1) * L, :, 0] = step[:, None].to(dtype)
+    with torch.no_grad():
+        o, lse = vb.packed_varlen_attn_with_lse(q.to(DEV), k.to(DEV), v.to(DEV), cu_seqlens_q=cu_q, cu_seqlens_k=cu_k, causal=True)
+    n = min(n_seg, 4) * L
+    ro, rlse = varlen_attn_ref(q[:n], k[:n], v[:n], cu_q[:min(n_seg, 4) + 1], cu_k[:min(n_seg, 4) + 1], causal=True)
+    check_close("o", o[:n], ro, dtype)
+    # each of the D / 16 accumulation steps of a score can lose a unit in the last place of the running fp32 sum, and the
+    # exponent, the logarithm and the conversion of the LSE one more each: scores reach 110 here
+    assert ((lse[:n].cpu() - rlse).abs() <= 1e-4 + (D // 16 + 4) * 2.0 ** -23 * rlse.abs()).all()
+    assert torch.isfinite(o).all()
+
+
+def test_nan_and_infinite_scores_behind_the_first_block():
+    """Only the rows that see the bad key are touched by it."""
+    L, H, D = 400, 2, 64
+    q, k, v, _, cu_q, cu_k = make_varlen_inputs([L, L], [L, L], H, D, torch.bfloat16, 22, with_do=False)
+
+    def run(kk):
+        with torch.no_grad():
+            return vb.packed_varlen_attn(q.to(DEV), kk.to(DEV), v.to(DEV), cu_seqlens_q=cu_q, cu_seqlens_k=cu_k, causal=True)
+
+    o0 = run(k)
+    k2 = k.clone()
+    k2[300] = float("nan")
+    o1 = run(k2)
+    # the rest of the tile is done again the careful way: equal up to the rounding of P and O (2^-8 each)
+    assert (o1[:300] - o0[:300]).abs().max() <= 2e-2 and torch.equal(o1[L:], o0[L:])
+    assert torch.isnan(o1[300:L].float()).any(dim=-1).all()

@@ -43,6 +43,23 @@ using namespace ptx;
 
 constexpr int kFwdThreads = 320;  // 8 softmax warps, 1 TMA warp, 1 MMA warp
 constexpr float kRescaleThreshold = 8.0f;  // log2 units
+
+// How a tile's softmax goes (varlen_fwd_kernel).  The reference maximum of a row only keeps the exponentials in range:
+// O / l does not depend on it.  So the first block of an item sets it, and every further block is computed
+// against it as it stands: no row maximum, no exchange between the two warps that share the rows (which may then
+// run a block apart, so that one's waits lie under the other's exponentials), no rescaling of O.
+// At the end of the item the row sum tells whether all stayed in range: a sum within kMaxSum (and in fp16 every partial
+// sum within kMaxPart, which bounds P itself) proves it.  An item that fails, or holds a NaN, is written down and
+// done again at the end of the kernel by the CTA that met it, the careful way: the maximum of every
+// block, O rescaled when it moves by more than 2^8.  From kRedoGiveUp entries on the CTA takes its remaining items
+// the careful way at once, so inputs whose scores keep climbing cost a few items twice, not all.
+// DECOUPLE_FIGURES
+constexpr int kCareful = 1 << 30;   // flag on a published item index
+constexpr int kDrain = -2;          // published once: the softmax warps report that all items before it are done
+constexpr int kRedoGiveUp = 8;      // entries (each softmax warp writes its own, so one item can make eight)
+constexpr int kRedoCap = 128;       // what the items already published when the CTA gives up can add, twice over
+constexpr float kMaxSum = 1.152921504606846976e18f;  // 2^60
+constexpr float kMaxPart = 32768.f;                  // sum of one thread's exponentials of a block, fp16
 #ifndef VAFA_FWD_POLY_PERIOD
 #define VAFA_FWD_POLY_PERIOD 4
 #endif
@@ -96,6 +113,9 @@ struct FwdSmem {
   uint64_t pair_bar[4];       // the two softmax warps of one TMEM lane quadrant
   float xmax[2][2][128];      // [block parity][half][row] partial row maxima
   float xsum[2][128];         // [half][row] partial row sums at the end of an item
+  uint64_t drain;             // all softmax warps have met kDrain
+  int redo[kRedoCap];         // items to be done again
+  int n_redo;
   WorkQueue wq;
   uint32_t tmem_base;
   int abort_flag;
@@ -160,6 +180,8 @@ varlen_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_const
     sm.abort_flag = 0;
     sm.wait_limit = p.wait_limit;
     wq_init(sm.wq, 9);
+    sm.n_redo = 0;
+    mbar_init(smem_u32(&sm.drain), 8);
     for (int i = 0; i < 4; ++i) mbar_init(smem_u32(&sm.pair_bar[i]), 64);
     mbar_init(smem_u32(&sm.q_full), 1);
     mbar_init(smem_u32(&sm.q_free), 1);
@@ -203,10 +225,36 @@ varlen_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_const
     if (lane == 0) {
       uint32_t gk = 0, qi = 0;
       bool alive = true;
+      bool drained = false;
+      int n_seen = 0;  // redo entries looked at
       for (uint32_t n = 0; alive; ++n) {
-        const int idx = wq_produce(sm.wq, n, next_item, total, abort_flag);
+        const int slot = n % kWqSlots;
+        if (!mbar_wait(smem_u32(&sm.wq.empty[slot]), ((n / kWqSlots) & 1) ^ 1, abort_flag)) break;
+        int idx = -1;
+        if (!drained) {
+          idx = atomicAdd(next_item, 1);
+          if (idx >= total) {
+            idx = kDrain;
+            drained = true;
+          } else if (*(volatile int*)&sm.n_redo >= kRedoGiveUp) {
+            idx |= kCareful;
+          }
+        } else {
+          if (n_seen == 0 && !mbar_wait(smem_u32(&sm.drain), 0, abort_flag)) break;
+          const int n_redo = min(*(volatile int*)&sm.n_redo, kRedoCap);
+          while (idx < 0 && n_seen < n_redo) {
+            idx = sm.redo[n_seen];
+            for (int i = 0; i < n_seen; ++i)
+              if (sm.redo[i] == idx) { idx = -1; break; }
+            ++n_seen;
+          }
+          if (idx >= 0) idx |= kCareful;
+        }
+        sm.wq.idx[slot] = idx;
+        mbar_arrive(smem_u32(&sm.wq.full[slot]));
+        if (idx == kDrain) continue;
         if (idx < 0) break;
-        const WorkItem w = p.items[idx];
+        const WorkItem w = p.items[idx & ~kCareful];
         const int h = w.head * p.stack;
         const int hk = w.head / p.group;  // K/V head of this query head or stack
         const int nb = (w.i_len + kBlk - 1) / kBlk;
@@ -283,8 +331,9 @@ varlen_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_const
 
       for (uint32_t n = 0; alive; ++n) {
         const int idx = wq_consume_thread(sm.wq, n, abort_flag);
+        if (idx == kDrain) continue;
         if (idx < 0) break;
-        const WorkItem w = p.items[idx];
+        const WorkItem w = p.items[idx & ~kCareful];
         const int nb = (w.i_len + kBlk - 1) / kBlk;
         if (nb == 0) continue;
         { TRACE_T0(); if (!mbar_wait(smem_u32(&sm.q_full), qi & 1, abort_flag)) break; TRACE_ADD(3); }
@@ -346,8 +395,14 @@ varlen_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_const
     uint32_t gk = 0;
     bool alive = true;
     for (uint32_t n = 0; alive; ++n) {
-      const int idx = wq_consume_warp(sm.wq, n, abort_flag);
-      if (idx < 0) break;
+      const int entry = wq_consume_warp(sm.wq, n, abort_flag);
+      if (entry == kDrain) {
+        if (lane == 0) mbar_arrive(smem_u32(&sm.drain));
+        continue;
+      }
+      if (entry < 0) break;
+      const bool careful = (entry & kCareful) != 0;
+      const int idx = entry & ~kCareful;
       const WorkItem w = p.items[idx];
       const int nb = (w.i_len + kBlk - 1) / kBlk;
       // tile row r -> (query row of the tile, head)
@@ -356,6 +411,8 @@ varlen_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_const
       const bool row_ok = rq < w.o_rows;
       const bool live = (warp & 3) * 32 < w.o_rows * p.stack;  // does any row of this warp exist?
       float m_ref = -INFINITY, l = 0.f;  // l: sum over this thread's columns only
+      float worst = 0.f;                 // fp16: largest sum of a block
+      bool no_ref = false;
 
       for (int b = 0; b < nb; ++b) {
         const uint32_t g = gk + b;
@@ -398,40 +455,15 @@ varlen_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_const
 #pragma unroll
           for (int i = 0; i < kHalf; ++i) s[i] = (i <= lim) ? s[i] : -INFINITY;
         }
-        // row maximum of this half: eight independent chains of 3-input max
-        float m8[8];
-#pragma unroll
-        for (int j2 = 0; j2 < 8; ++j2) m8[j2] = max3(s[j2], s[8 + j2], s[16 + j2]);
-#pragma unroll
-        for (int i = 24; i + 16 <= kHalf; i += 16) {
-#pragma unroll
-          for (int j2 = 0; j2 < 8; ++j2) m8[j2] = max3(m8[j2], s[i + j2], s[i + 8 + j2]);
-        }
-        // 24 + 16k columns done; one more group of eight is left for both 64 and 48 columns
-#pragma unroll
-        for (int j2 = 0; j2 < 8; ++j2) m8[j2] = fmaxf(m8[j2], s[kHalf - 8 + j2]);
-        float mx = max3(max3(m8[0], m8[1], m8[2]), max3(m8[3], m8[4], m8[5]), fmaxf(m8[6], m8[7]));
-        // combine with the other half of the row
-        sm.xmax[g & 1][half][r] = mx;
-        mbar_arrive(pair_bar);
-        { TRACE_T0(); if (!mbar_wait(pair_bar, pair_cnt & 1, abort_flag)) { alive = false; break; } TRACE_ADD(12); }
-        ++pair_cnt;
-        mx = fmaxf(mx, sm.xmax[g & 1][half ^ 1][r]);
-        const float m_blk = mx * c;  // c > 0
-        float m_new = fmaxf(m_ref, m_blk);
-        const bool resc = m_new > m_ref + kRescaleThreshold;
-        if (!resc) m_new = m_ref;
-        const float alpha = resc ? ex2(m_ref - m_new) : 1.f;
-        const float m_use = (m_new == -INFINITY) ? 0.f : m_new;
         // exponents and row sums in packed pairs (one FMA-pipe instruction for two values); in unmasked
         // blocks every kPolyPeriod-th pair takes the polynomial 2^t instead of the special-function unit
         // (16 results/clk/SM).  Masked blocks keep the unit for all: it returns exactly 0 for -inf, which
         // the dead-row test (row sum == 0) relies on.
-        const uint64_t cs2 = pack_f2(c, c), nm2 = pack_f2(-m_use, -m_use);
-        uint64_t sum2[4] = {0ull, 0ull, 0ull, 0ull};
         uint32_t pk[kHalf / 2];
-        auto exps = [&](auto poly_tag) {
+        auto exps = [&](float m_use, auto poly_tag) -> float {
           constexpr bool kPoly = decltype(poly_tag)::value;
+          const uint64_t cs2 = pack_f2(c, c), nm2 = pack_f2(-m_use, -m_use);
+          uint64_t sum2[4] = {0ull, 0ull, 0ull, 0ull};
 #pragma unroll
           for (int i = 0; i < kHalf / 2; ++i) {
             const uint64_t t2 = fma_f2(pack_f2(s[2 * i], s[2 * i + 1]), cs2, nm2);
@@ -447,15 +479,49 @@ varlen_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_const
             sum2[i & 3] = add_f2(sum2[i & 3], pack_f2(p0, p1));
             pk[i] = pack_p<T>(p0, p1);
           }
-        };
-        if (masked_block) exps(std::false_type{}); else exps(std::true_type{});
-        {
           float a0, a1, b0, b1;
           unpack_f2(add_f2(sum2[0], sum2[1]), a0, a1);
           unpack_f2(add_f2(sum2[2], sum2[3]), b0, b1);
-          l = l * alpha + ((a0 + a1) + (b0 + b1));
+          return (a0 + a1) + (b0 + b1);
+        };
+        bool resc = false;
+        float alpha = 1.f;
+        if (b > 0 && !careful) {
+          const float bsum = masked_block ? exps(m_ref, std::false_type{}) : exps(m_ref, std::true_type{});
+          l += bsum;
+          if (std::is_same<T, __half>::value) worst = fmaxf(worst, bsum);
+        } else {
+          // row maximum of this half: eight independent chains of 3-input max
+          float m8[8];
+#pragma unroll
+          for (int j2 = 0; j2 < 8; ++j2) m8[j2] = max3(s[j2], s[8 + j2], s[16 + j2]);
+#pragma unroll
+          for (int i = 24; i + 16 <= kHalf; i += 16) {
+#pragma unroll
+            for (int j2 = 0; j2 < 8; ++j2) m8[j2] = max3(m8[j2], s[i + j2], s[i + 8 + j2]);
+          }
+          // 24 + 16k columns done; one more group of eight is left for both 64 and 48 columns
+#pragma unroll
+          for (int j2 = 0; j2 < 8; ++j2) m8[j2] = fmaxf(m8[j2], s[kHalf - 8 + j2]);
+          float mx = max3(max3(m8[0], m8[1], m8[2]), max3(m8[3], m8[4], m8[5]), fmaxf(m8[6], m8[7]));
+          // combine with the other half of the row
+          sm.xmax[g & 1][half][r] = mx;
+          mbar_arrive(pair_bar);
+          { TRACE_T0(); if (!mbar_wait(pair_bar, pair_cnt & 1, abort_flag)) { alive = false; break; } TRACE_ADD(12); }
+          ++pair_cnt;
+          mx = fmaxf(mx, sm.xmax[g & 1][half ^ 1][r]);
+          const float m_blk = mx * c;  // c > 0
+          float m_new = fmaxf(m_ref, m_blk);
+          resc = m_new > m_ref + kRescaleThreshold;
+          if (!resc) m_new = m_ref;
+          alpha = resc ? ex2(m_ref - m_new) : 1.f;
+          const float m_use = (m_new == -INFINITY) ? 0.f : m_new;
+          const float bsum = masked_block ? exps(m_use, std::false_type{}) : exps(m_use, std::true_type{});
+          l = l * alpha + bsum;
+          // (a row without a finite score in the first block has no reference; one that sees no key needs none)
+          m_ref = careful ? m_new : m_use;
+          no_ref = m_new == -INFINITY && !(w.masked && rq + w.diag < 0);
         }
-        m_ref = m_new;
         // kHalf probabilities -> kHalf/2 packed columns over the first half of the columns just read
         // (the MMA issuer's addressing of the K-steps is next to its P.V loop)
         if constexpr (kHalf == 64) {
@@ -469,7 +535,7 @@ varlen_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_const
           tmem_st16(s_addr, pa);
           tmem_st8(s_addr + 16, pb);
         }
-        if (b > 0 && __any_sync(0xffffffffu, resc)) {
+        if (careful && b > 0 && __any_sync(0xffffffffu, resc)) {
 #ifdef VAFA_TRACE
           tr[10] += clock64() - t_sm0;
 #endif
@@ -516,6 +582,14 @@ varlen_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_const
         if (!mbar_wait(pair_bar, pair_cnt & 1, abort_flag)) break;
         ++pair_cnt;
         l_tot = l + sm.xsum[half ^ 1][r];
+      }
+      if (nb > 1 && !careful) {
+        const bool out_of_range = row_ok && (no_ref || !(l_tot <= kMaxSum) || (std::is_same<T, __half>::value && worst > kMaxPart));
+        if (__any_sync(0xffffffffu, out_of_range) && lane == 0) {
+          // what is written below is overwritten when the item is done again
+          const int at = atomicAdd(&sm.n_redo, 1);
+          if (at < kRedoCap) sm.redo[at] = idx;
+        }
       }
       const bool dead = (nb == 0) || (l_tot == 0.f);  // a NaN row sum is not a dead row: it goes out as NaN
       const float inv_l = dead ? 0.f : 1.f / l_tot;
