@@ -281,6 +281,14 @@ __device__ __forceinline__ bool elect_one() {
   return pred != 0;
 }
 
+// The value of lane 0 in all lanes of a converged warp: tells the compiler that it is the same in all of them.
+__device__ __forceinline__ uint32_t warp_uniform(uint32_t x) { return __shfl_sync(0xffffffffu, x, 0); }
+
+// mbar_wait by all lanes of a warp, with one answer.
+__device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity, volatile int* abort_flag) {
+  return __all_sync(0xffffffffu, mbar_wait(bar, parity, abort_flag));
+}
+
 __device__ __forceinline__ float max3(float a, float b, float c) {
   float r;
   asm("max.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));

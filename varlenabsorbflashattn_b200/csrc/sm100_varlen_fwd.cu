@@ -53,7 +53,7 @@ constexpr float kRescaleThreshold = 8.0f;  // log2 units
 // done again at the end of the kernel by the CTA that met it, the careful way: the maximum of every
 // block, O rescaled when it moves by more than 2^8.  From kRedoGiveUp entries on the CTA takes its remaining items
 // the careful way at once, so inputs whose scores keep climbing cost a few items twice, not all.
-// DECOUPLE_FIGURES
+// Measured: 500-query histories, head dim 64: 710 -> 615 us; prefill of 16 sequences, head dim 128: 1229 -> 1202 us.
 constexpr int kCareful = 1 << 30;   // flag on a published item index
 constexpr int kDrain = -2;          // published once: the softmax warps report that all items before it are done
 constexpr int kRedoGiveUp = 8;      // entries (each softmax warp writes its own, so one item can make eight)
@@ -173,7 +173,7 @@ varlen_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_const
   extern __shared__ uint8_t smem_raw[];
   using Smem = FwdSmem<D, kAbsorb>;
   Smem& sm = *reinterpret_cast<Smem*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = (int)warp_uniform(threadIdx.x >> 5), lane = threadIdx.x & 31;
   volatile int* abort_flag = &sm.abort_flag;
 
   if (threadIdx.x == 0) {
@@ -303,45 +303,56 @@ varlen_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_const
     }
   } else if (warp == 9) {
     // ---------------- MMA issuer ----------------
-    if (lane == 0) {
+    // The whole warp runs this loop on warp-uniform values and one elected lane issues: descriptors then live in
+    // uniform registers, which is what the instruction takes.  With the loop inside `if (lane == 0)` every operand was
+    // moved there for every product, six moves or about 100 cycles per tcgen05.mma where the tensor pipe needs 64.
+    // Prefill of 16 sequences (32/8 heads of 128) 1202 -> 1125 us, 500-query histories (head dim 64) 615 -> 569 us.
+    {
       constexpr int kFmt = std::is_same<T, __nv_bfloat16>::value ? 1 : 0;
       constexpr uint32_t idesc_qk = make_idesc(kFmt, 0, 0, 128, kBlk);
       constexpr uint32_t idesc_pv = make_idesc(kFmt, 0, 1, 128, D);
+      const uint32_t tm = warp_uniform(tbase);
+      const uint32_t q_lo = warp_uniform(desc_lo_sw128(smem_u32(sm.q), 16));
+      const uint32_t k_lo0 = warp_uniform(desc_lo_sw128(smem_u32(sm.k[0]), 16));
+      // V tile: [keys][D] as D/64 sub tiles; 16 keys = 2 KB; sub tiles one sub tile apart (the LBO)
+      const uint32_t v_lo0 = warp_uniform(desc_lo_sw128(smem_u32(kAbsorb ? sm.k[0] : sm.v[0]), kKSubBytes));
+      constexpr uint32_t kVStage = (uint32_t)(kAbsorb ? kKTileBytes : Cfg::kTileBytes) >> 4;
       uint32_t gk = 0, qi = 0;
       bool alive = true;
 
       auto issue_qk = [&](uint32_t g, bool last) -> bool {
-        const int st = g % S;
-        const uint32_t ph = (g / S) & 1;
-        { TRACE_T0(); if (!mbar_wait(smem_u32(&sm.k_full[st]), ph, abort_flag)) return false; TRACE_ADD(4); }
+        const uint32_t st = g % S;
+        { TRACE_T0(); if (!mbar_wait_warp(smem_u32(&sm.k_full[0]) + st * 8, (g / S) & 1, abort_flag)) return false; TRACE_ADD(4); }
         tc_fence_after();
-        const uint32_t d_tmem = tbase + (g & 1) * 128;
-        const uint32_t q_lo = desc_lo_sw128(smem_u32(sm.q), 16), k_lo = desc_lo_sw128(smem_u32(sm.k[st]), 16);
+        const uint32_t d_tmem = tm + (g & 1) * 128;
+        const uint32_t k_lo = k_lo0 + st * (kKTileBytes >> 4);
+        if (elect_one()) {
 #pragma unroll
-        for (int kk = 0; kk < D / 16; ++kk) {
-          // in 16-byte units: 64-column sub tiles are a whole sub tile apart, 16 columns are 32 bytes
-          const uint32_t off_q = (kk >> 2) * (Cfg::kSubBytes >> 4) + (kk & 3) * 2;
-          const uint32_t off_k = (kk >> 2) * (kKSubBytes >> 4) + (kk & 3) * 2;
-          mma_ss2(d_tmem, q_lo + off_q, k_lo + off_k, idesc_qk, kk > 0);
+          for (int kk = 0; kk < D / 16; ++kk) {
+            // in 16-byte units: 64-column sub tiles are a whole sub tile apart, 16 columns are 32 bytes
+            const uint32_t off_q = (kk >> 2) * (Cfg::kSubBytes >> 4) + (kk & 3) * 2;
+            const uint32_t off_k = (kk >> 2) * (kKSubBytes >> 4) + (kk & 3) * 2;
+            mma_ss2(d_tmem, q_lo + off_q, k_lo + off_k, idesc_qk, kk > 0);
+          }
+          mma_commit(smem_u32(&sm.s_full[0]) + (g & 1) * 8);
+          if (last) mma_commit(smem_u32(&sm.q_free));
         }
-        mma_commit(smem_u32(&sm.s_full[g & 1]));
-        if (last) mma_commit(smem_u32(&sm.q_free));
+        __syncwarp();
         return true;
       };
 
       for (uint32_t n = 0; alive; ++n) {
-        const int idx = wq_consume_thread(sm.wq, n, abort_flag);
+        const int idx = (int)warp_uniform((uint32_t)wq_consume_warp(sm.wq, n, abort_flag));
         if (idx == kDrain) continue;
         if (idx < 0) break;
-        const WorkItem w = p.items[idx & ~kCareful];
-        const int nb = (w.i_len + kBlk - 1) / kBlk;
+        const int nb = (int)warp_uniform((uint32_t)((p.items[idx & ~kCareful].i_len + kBlk - 1) / kBlk));
         if (nb == 0) continue;
-        { TRACE_T0(); if (!mbar_wait(smem_u32(&sm.q_full), qi & 1, abort_flag)) break; TRACE_ADD(3); }
+        { TRACE_T0(); if (!mbar_wait_warp(smem_u32(&sm.q_full), qi & 1, abort_flag)) break; TRACE_ADD(3); }
         tc_fence_after();
         if (!issue_qk(gk, nb == 1)) break;
         for (int b = 0; b < nb; ++b) {
           const uint32_t g = gk + b;
-          const int st = g % S;
+          const uint32_t st = g % S;
           const uint32_t ph = (g / S) & 1;
           bool qk_pending = b + 1 < nb, qk_first = true;
           if (kAbsorb && qk_pending) {
@@ -350,8 +361,8 @@ varlen_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_const
             // latency in series with both products of every block (measured: half of this thread's time):
             // the product whose operands are there first is issued first.
             TRACE_T0();
-            const int first = mbar_wait_either(smem_u32(&sm.k_full[(g + 1) % S]), ((g + 1) / S) & 1,
-                                               smem_u32(&sm.p_full[g & 1]), (g >> 1) & 1, abort_flag);
+            const int first = (int)warp_uniform((uint32_t)mbar_wait_either(smem_u32(&sm.k_full[(g + 1) % S]), ((g + 1) / S) & 1,
+                                                                           smem_u32(&sm.p_full[g & 1]), (g >> 1) & 1, abort_flag));
             TRACE_ADD(7);
             if (first == 0) { alive = false; break; }
             qk_first = first == 1;
@@ -360,20 +371,22 @@ varlen_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_const
             if (!issue_qk(g + 1, b + 2 == nb)) { alive = false; break; }
             qk_pending = false;
           }
-          { TRACE_T0(); if (!mbar_wait(smem_u32(&sm.p_full[g & 1]), (g >> 1) & 1, abort_flag)) { alive = false; break; } TRACE_ADD(5); }
-          if (!kAbsorb) { TRACE_T0(); if (!mbar_wait(smem_u32(&sm.v_full[st]), ph, abort_flag)) { alive = false; break; } TRACE_ADD(6); }
+          { TRACE_T0(); if (!mbar_wait_warp(smem_u32(&sm.p_full[0]) + (g & 1) * 8, (g >> 1) & 1, abort_flag)) { alive = false; break; } TRACE_ADD(5); }
+          if (!kAbsorb) { TRACE_T0(); if (!mbar_wait_warp(smem_u32(&sm.v_full[0]) + st * 8, ph, abort_flag)) { alive = false; break; } TRACE_ADD(6); }
           tc_fence_after();
-          const uint32_t a_tmem = tbase + (g & 1) * 128;
-          // V tile: [keys][D] as D/64 sub tiles; 16 keys = 2 KB; sub tiles one sub tile apart (the LBO)
-          const uint32_t v_lo = desc_lo_sw128(smem_u32(kAbsorb ? sm.k[st] : sm.v[st]), kKSubBytes);
+          const uint32_t a_tmem = tm + (g & 1) * 128;
+          const uint32_t v_lo = v_lo0 + st * kVStage;
           // P: each softmax thread packed its kHalf columns into the first kHalf/2 of them, so K-step kk
           // (16 keys = 8 packed columns) sits at column (kk / steps_per_half) * kHalf + (kk % steps_per_half) * 8
           constexpr int kStepsPerHalf = kHalf / 16;
+          if (elect_one()) {
 #pragma unroll
-          for (int kk = 0; kk < kBlk / 16; ++kk)
-            mma_ts2(tbase + Cfg::kOCol, a_tmem + (kk / kStepsPerHalf) * kHalf + (kk % kStepsPerHalf) * 8, v_lo + kk * (2048 >> 4),
-                    idesc_pv, (b > 0 || kk > 0) ? 1u : 0u);
-          mma_commit(smem_u32(&sm.o_done[st]));
+            for (int kk = 0; kk < kBlk / 16; ++kk)
+              mma_ts2(tm + Cfg::kOCol, a_tmem + (kk / kStepsPerHalf) * kHalf + (kk % kStepsPerHalf) * 8, v_lo + kk * (2048 >> 4),
+                      idesc_pv, (b > 0 || kk > 0) ? 1u : 0u);
+            mma_commit(smem_u32(&sm.o_done[0]) + st * 8);
+          }
+          __syncwarp();
           if (qk_pending && !issue_qk(g + 1, b + 2 == nb)) { alive = false; break; }
         }
         gk += nb;
