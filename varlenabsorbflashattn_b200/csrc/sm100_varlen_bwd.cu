@@ -138,7 +138,7 @@ varlen_bwd_kernel(const __grid_constant__ CUtensorMap tmap_outer_a, const __grid
   using Smem = BwdSmem<D, kDKV, kAbsorb>;
   constexpr int S = Smem::kS;
   Smem& sm = *reinterpret_cast<Smem*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = (int)warp_uniform(threadIdx.x >> 5), lane = threadIdx.x & 31;
   volatile int* abort_flag = &sm.abort_flag;
 
   if (threadIdx.x == 0) {
@@ -258,24 +258,32 @@ varlen_bwd_kernel(const __grid_constant__ CUtensorMap tmap_outer_a, const __grid
     }
   } else if (warp == 9) {
     // ---------------- MMA issuer ----------------
-    if (lane == 0) {
+    // The whole warp on warp-uniform values, one elected lane issues (see varlen_fwd_kernel). Production
+    // widths: dU 439 -> 383 us, dX 487 -> 478.
+    {
       constexpr int kFmt = std::is_same<T, __nv_bfloat16>::value ? 1 : 0;
       constexpr uint32_t idesc_xy = make_idesc(kFmt, 0, 0, 128, kInner);  // outer(128) x inner(64), both K-major
       constexpr uint32_t idesc_acc = make_idesc(kFmt, 0, 1, 128, D);      // A from TMEM, B MN-major
       uint32_t gk = 0, qi = 0;
       bool alive = true;
+      const uint32_t tm = warp_uniform(tbase);
+      const uint32_t oa_lo = warp_uniform(desc_lo_sw128(smem_u32(sm.outer_a), 16));
+      const uint32_t ob_lo = warp_uniform(desc_lo_sw128(smem_u32((kAbsorb && kDKV) ? sm.outer_a : sm.outer_b), 16));
+      const uint32_t ia_lo0 = warp_uniform(desc_lo_sw128(smem_u32(sm.inner_a[0]), 16));
+      const uint32_t ib_lo0 = warp_uniform(desc_lo_sw128(smem_u32((kAbsorb && !kDKV) ? sm.inner_a[0] : sm.inner_b[0]), 16));
+      const uint32_t ma_lo0 = warp_uniform(desc_lo_sw128(smem_u32(sm.inner_a[0]), Cfg::kInnerSubBytes));
+      const uint32_t mb_lo0 = warp_uniform(desc_lo_sw128(smem_u32((kAbsorb && !kDKV) ? sm.inner_a[0] : sm.inner_b[0]), Cfg::kInnerSubBytes));
+      constexpr uint32_t kStage16 = Cfg::kInnerBytes >> 4;
 
       auto issue_xy = [&](uint32_t g, bool last) -> bool {
-        const int st = g % S;
+        const uint32_t st = g % S;
         const uint32_t ph = (g / S) & 1;
-        { TRACE_T0(); if (!mbar_wait(smem_u32(&sm.in_full[st]), ph, abort_flag)) return false; TRACE_ADD(4); }
+        { TRACE_T0(); if (!mbar_wait_warp(smem_u32(&sm.in_full[0]) + st * 8, ph, abort_flag)) return false; TRACE_ADD(4); }
         tc_fence_after();
-        const uint32_t x_tmem = tbase + Cfg::kXCol + (g & 1) * kInner;
-        const uint32_t y_tmem = tbase + Cfg::kYCol + (g & 1) * kInner;
-        const uint32_t oa_lo = desc_lo_sw128(smem_u32(sm.outer_a), 16);
-        const uint32_t ob_lo = desc_lo_sw128(smem_u32((kAbsorb && kDKV) ? sm.outer_a : sm.outer_b), 16);
-        const uint32_t ia_lo = desc_lo_sw128(smem_u32(sm.inner_a[st]), 16);
-        const uint32_t ib_lo = desc_lo_sw128(smem_u32((kAbsorb && !kDKV) ? sm.inner_a[st] : sm.inner_b[st]), 16);
+        const uint32_t x_tmem = tm + Cfg::kXCol + (g & 1) * kInner;
+        const uint32_t y_tmem = tm + Cfg::kYCol + (g & 1) * kInner;
+        const uint32_t ia_lo = ia_lo0 + st * kStage16, ib_lo = ib_lo0 + st * kStage16;
+        if (elect_one()) {
 #pragma unroll
         for (int kk = 0; kk < D / 16; ++kk) {
           const uint32_t offo = (kk >> 2) * (Cfg::kOuterSubBytes >> 4) + (kk & 3) * 2;  // 16-byte units
@@ -288,8 +296,10 @@ varlen_bwd_kernel(const __grid_constant__ CUtensorMap tmap_outer_a, const __grid
           const uint32_t offi = (kk >> 2) * (Cfg::kInnerSubBytes >> 4) + (kk & 3) * 2;
           mma_ss2(y_tmem, ob_lo + offo, ib_lo + offi, idesc_xy, kk > 0);
         }
-        mma_commit(smem_u32(&sm.xy_full[g & 1]));
+        mma_commit(smem_u32(&sm.xy_full[0]) + (g & 1) * 8);
         if (last) mma_commit(smem_u32(&sm.outer_free));
+        }
+        __syncwarp();
         return true;
       };
 
@@ -302,13 +312,12 @@ varlen_bwd_kernel(const __grid_constant__ CUtensorMap tmap_outer_a, const __grid
       // draws items until one has inner blocks; waits for its outer tile and issues its first score products
       auto start_next_item = [&]() -> bool {
         while (true) {
-          const int idx = wq_consume_thread(sm.wq, n_next++, abort_flag);
+          const int idx = (int)warp_uniform((uint32_t)wq_consume_warp(sm.wq, n_next++, abort_flag));
           if (idx < 0) return false;
-          const WorkItem w = p.items[idx];
-          nb_next = (w.i_len + ib - 1) / ib;
+          nb_next = (int)warp_uniform((uint32_t)((p.items[idx].i_len + ib - 1) / ib));
           if (nb_next > 0) break;
         }
-        { TRACE_T0(); if (!mbar_wait(smem_u32(&sm.outer_full), qi & 1, abort_flag)) return false; TRACE_ADD(3); }
+        { TRACE_T0(); if (!mbar_wait_warp(smem_u32(&sm.outer_full), qi & 1, abort_flag)) return false; TRACE_ADD(3); }
         tc_fence_after();
         ++qi;
         return issue_xy(gk, nb_next == 1);
@@ -326,33 +335,35 @@ varlen_bwd_kernel(const __grid_constant__ CUtensorMap tmap_outer_a, const __grid
           } else {
             have = start_next_item();
           }
-          const int st = g % S;
-          { TRACE_T0(); if (!mbar_wait(smem_u32(&sm.ds_full[g & 1]), (g >> 1) & 1, abort_flag)) { alive = false; break; } TRACE_ADD(7); }
+          const uint32_t st = g % S;
+          { TRACE_T0(); if (!mbar_wait_warp(smem_u32(&sm.ds_full[0]) + (g & 1) * 8, (g >> 1) & 1, abort_flag)) { alive = false; break; } TRACE_ADD(7); }
           tc_fence_after();
-          const uint32_t x_tmem = tbase + Cfg::kXCol + (g & 1) * kInner;
-          const uint32_t y_tmem = tbase + Cfg::kYCol + (g & 1) * kInner;
+          const uint32_t x_tmem = tm + Cfg::kXCol + (g & 1) * kInner;
+          const uint32_t y_tmem = tm + Cfg::kYCol + (g & 1) * kInner;
           const uint32_t acc = (b > 0) ? 1u : 0u;
-          const uint32_t ma_lo = desc_lo_sw128(smem_u32(sm.inner_a[st]), Cfg::kInnerSubBytes);
-          const uint32_t mb_lo = desc_lo_sw128(smem_u32((kAbsorb && !kDKV) ? sm.inner_a[st] : sm.inner_b[st]), Cfg::kInnerSubBytes);
+          const uint32_t ma_lo = ma_lo0 + st * kStage16, mb_lo = mb_lo0 + st * kStage16;
+          if (elect_one()) {
           if (!kDKV) {
             // dQ += dS . K_g     (dS in X, 16-bit packed; K block MN-major)
 #pragma unroll
             for (int kk = 0; kk < kInner / 16; ++kk)
-              mma_ts2(tbase + Cfg::kAcc0, x_tmem + (kk >> 1) * 32 + (kk & 1) * 8, ma_lo + kk * (2048 >> 4), idesc_acc,
+              mma_ts2(tm + Cfg::kAcc0, x_tmem + (kk >> 1) * 32 + (kk & 1) * 8, ma_lo + kk * (2048 >> 4), idesc_acc,
                       (acc | (kk > 0)) ? 1u : 0u);
           } else {
             // dV += P^T . dO_g ;  dK += dS^T . Q_g
 #pragma unroll
             for (int kk = 0; kk < kInner / 16; ++kk)
-              mma_ts2(tbase + Cfg::kAcc0, x_tmem + (kk >> 1) * 32 + (kk & 1) * 8, mb_lo + kk * (2048 >> 4), idesc_acc,
+              mma_ts2(tm + Cfg::kAcc0, x_tmem + (kk >> 1) * 32 + (kk & 1) * 8, mb_lo + kk * (2048 >> 4), idesc_acc,
                       (acc | (kk > 0)) ? 1u : 0u);
 #pragma unroll
             for (int kk = 0; kk < kInner / 16; ++kk)
-              mma_ts2(tbase + (kAbsorb ? Cfg::kAcc0 : Cfg::kAcc1), y_tmem + (kk >> 1) * 32 + (kk & 1) * 8, ma_lo + kk * (2048 >> 4),
+              mma_ts2(tm + (kAbsorb ? Cfg::kAcc0 : Cfg::kAcc1), y_tmem + (kk >> 1) * 32 + (kk & 1) * 8, ma_lo + kk * (2048 >> 4),
                       idesc_acc, (kAbsorb || acc || kk > 0) ? 1u : 0u);
           }
-          mma_commit(smem_u32(&sm.in_empty[st]));
+          mma_commit(smem_u32(&sm.in_empty[0]) + st * 8);
           if (b + 1 == nb) mma_commit(smem_u32(&sm.acc_done));
+          }
+          __syncwarp();
         }
       }
     }

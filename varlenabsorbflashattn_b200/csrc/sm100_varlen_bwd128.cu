@@ -163,7 +163,7 @@ varlen_bwd128_kernel(const __grid_constant__ CUtensorMap tmap_outer_a, const __g
   extern __shared__ uint8_t smem_raw[];
   using Smem = Smem128<D, kDKV>;
   Smem& sm = *reinterpret_cast<Smem*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = (int)warp_uniform(threadIdx.x >> 5), lane = threadIdx.x & 31;
   volatile int* abort_flag = &sm.abort_flag;
 
   if (threadIdx.x == 0) {
@@ -270,100 +270,112 @@ varlen_bwd128_kernel(const __grid_constant__ CUtensorMap tmap_outer_a, const __g
   } else if (warp == kMmaWarp) {
     VAFA_REG_DEC();
     // ---------------- MMA issuer ----------------
-    if (lane == 0) {
+    // The whole warp on warp-uniform values, one elected lane issues (see varlen_fwd_kernel). 34 k-token
+    // training batch (16 heads of 128): dQ 507 -> 485 us, dK/dV 665 -> 641; 500-query histories: 911 -> 885, 1284 -> 1171.
+    {
       constexpr int kFmt = std::is_same<T, __nv_bfloat16>::value ? 1 : 0;
       constexpr uint32_t idesc_xy = make_idesc(kFmt, 0, 0, 128, kIn);  // both operands K-major
       constexpr uint32_t idesc_acc = make_idesc(kFmt, 0, 1, 128, D);   // A from TMEM, B MN-major
+      constexpr uint32_t kTile16 = Cfg::kTileBytes >> 4;
       uint32_t gk = 0, qi = 0;
       bool alive = true;
-      const uint32_t oa_lo = desc_lo_sw128(smem_u32(sm.outer_a), 16), ob_lo = desc_lo_sw128(smem_u32(sm.outer_b), 16);
-      const uint32_t ones_lo = desc_lo_sw128(smem_u32(sm.ones), 16);
+      const uint32_t tm = warp_uniform(tbase);
+      const uint32_t oa_lo = warp_uniform(desc_lo_sw128(smem_u32(sm.outer_a), 16)), ob_lo = warp_uniform(desc_lo_sw128(smem_u32(sm.outer_b), 16));
+      const uint32_t ones_lo = warp_uniform(desc_lo_sw128(smem_u32(sm.ones), 16));
+      const uint32_t ia_lo0 = warp_uniform(desc_lo_sw128(smem_u32(sm.inner_a[0]), 16)), ib_lo0 = warp_uniform(desc_lo_sw128(smem_u32(sm.inner_b[0]), 16));
+      const uint32_t aug_lo0 = warp_uniform(desc_lo_sw128(smem_u32(sm.aug[0][0]), 16));
+      const uint32_t ma_lo0 = warp_uniform(desc_lo_sw128(smem_u32(sm.inner_a[0]), Cfg::kSubBytes));
+      const uint32_t mb_lo0 = warp_uniform(desc_lo_sw128(smem_u32(sm.inner_b[0]), Cfg::kSubBytes));
 
       // X(g) = outerA . innerA(g)^T  (+ fold step)
       auto issue_x = [&](uint32_t g) -> bool {
-        const int sa = g % SA;
-        { TRACE_T0(); if (!mbar_wait(smem_u32(&sm.a_full[sa]), (g / SA) & 1, abort_flag)) return false; TRACE_ADD(4); }
+        const uint32_t sa = g % SA;
+        { TRACE_T0(); if (!mbar_wait_warp(smem_u32(&sm.a_full[0]) + sa * 8, (g / SA) & 1, abort_flag)) return false; TRACE_ADD(4); }
         tc_fence_after();
         TRACE_T0();
-        const uint32_t x_tmem = tbase + Cfg::kX + (kDKV ? 0u : (g & 1) * 128u);
-        const uint32_t ia_lo = desc_lo_sw128(smem_u32(sm.inner_a[sa]), 16);
+        const uint32_t x_tmem = tm + Cfg::kX + (kDKV ? 0u : (g & 1) * 128u);
+        const uint32_t ia_lo = ia_lo0 + sa * kTile16;
+        if (elect_one()) {
 #pragma unroll
-        for (int kk = 0; kk < D / 16; ++kk) {
-          const uint32_t off = (kk >> 2) * (Cfg::kSubBytes >> 4) + (kk & 3) * 2;  // 16-byte units
-          mma_ss2(x_tmem, oa_lo + off, ia_lo + off, idesc_xy, kk > 0);
+          for (int kk = 0; kk < D / 16; ++kk) {
+            const uint32_t off = (kk >> 2) * (Cfg::kSubBytes >> 4) + (kk & 3) * 2;  // 16-byte units
+            mma_ss2(x_tmem, oa_lo + off, ia_lo + off, idesc_xy, kk > 0);
+          }
+          if (kDKV) mma_ss2h(x_tmem, ones_lo, aug_lo0 + sa * (2 * kAugBytes >> 4), idesc_xy, 1u, kDescHiSw32);
+          mma_commit(smem_u32(&sm.x_full[0]) + (kDKV ? 0u : (g & 1) * 8));
         }
-        if (kDKV) mma_ss2h(x_tmem, ones_lo, desc_lo_sw128(smem_u32(sm.aug[sa][0]), 16), idesc_xy, 1u, kDescHiSw32);
-        mma_commit(smem_u32(&sm.x_full[kDKV ? 0 : (g & 1)]));
+        __syncwarp();
         TRACE_ADD(14);
         return true;
       };
       // Y(g) = outerB . innerB(g)^T  (+ fold step); the last one of an item releases the outer tiles
       auto issue_y = [&](uint32_t g, bool last) -> bool {
-        const int sa = g % SA, sb = g % SB;
-        { TRACE_T0(); if (!mbar_wait(smem_u32(&sm.b_full[sb]), (g / SB) & 1, abort_flag)) return false; TRACE_ADD(5); }
+        const uint32_t sa = g % SA, sb = g % SB;
+        { TRACE_T0(); if (!mbar_wait_warp(smem_u32(&sm.b_full[0]) + sb * 8, (g / SB) & 1, abort_flag)) return false; TRACE_ADD(5); }
         tc_fence_after();
         TRACE_T0();
-        const uint32_t ib_lo = desc_lo_sw128(smem_u32(sm.inner_b[sb]), 16);
+        const uint32_t ib_lo = ib_lo0 + sb * kTile16;
+        if (elect_one()) {
 #pragma unroll
-        for (int kk = 0; kk < D / 16; ++kk) {
-          const uint32_t off = (kk >> 2) * (Cfg::kSubBytes >> 4) + (kk & 3) * 2;
-          mma_ss2(tbase + Cfg::kY, ob_lo + off, ib_lo + off, idesc_xy, kk > 0);
+          for (int kk = 0; kk < D / 16; ++kk) {
+            const uint32_t off = (kk >> 2) * (Cfg::kSubBytes >> 4) + (kk & 3) * 2;
+            mma_ss2(tm + Cfg::kY, ob_lo + off, ib_lo + off, idesc_xy, kk > 0);
+          }
+          if (kDKV) mma_ss2h(tm + Cfg::kY, ones_lo, aug_lo0 + sa * (2 * kAugBytes >> 4) + (kAugBytes >> 4), idesc_xy, 1u, kDescHiSw32);
+          mma_commit(smem_u32(&sm.y_full));
+          if (!kDKV) mma_commit(smem_u32(&sm.b_empty[0]) + sb * 8);  // V is read by this product only
+          if (last) mma_commit(smem_u32(&sm.outer_free));
         }
-        if (kDKV) mma_ss2h(tbase + Cfg::kY, ones_lo, desc_lo_sw128(smem_u32(sm.aug[sa][1]), 16), idesc_xy, 1u, kDescHiSw32);
-        mma_commit(smem_u32(&sm.y_full));
-        if (!kDKV) mma_commit(smem_u32(&sm.b_empty[sb]));  // V is read by this product only
-        if (last) mma_commit(smem_u32(&sm.outer_free));
+        __syncwarp();
         TRACE_ADD(14);
         return true;
       };
-      // ACC (+)= A[TMEM, 16-bit packed: K-step kk at column (kk/2)*32 + (kk%2)*8] . B[shared, MN-major]
-      auto issue_acc = [&](uint32_t d_tmem, uint32_t a_tmem, const uint8_t* b_tile, bool first) {
+      // ACC (+)= A[TMEM, 16-bit packed: K-step kk at column (kk/2)*32 + (kk%2)*8] . B[shared, MN-major], then the
+      // commits the caller lists (0: none)
+      auto issue_acc = [&](uint32_t d_tmem, uint32_t a_tmem, uint32_t b_lo, bool first, uint32_t bar0, uint32_t bar1) {
         TRACE_T0();
-        const uint32_t b_lo = desc_lo_sw128(smem_u32(b_tile), Cfg::kSubBytes);
+        if (elect_one()) {
 #pragma unroll
-        for (int kk = 0; kk < kIn / 16; ++kk)
-          mma_ts2(d_tmem, a_tmem + (kk >> 1) * 32 + (kk & 1) * 8, b_lo + kk * (2048 >> 4), idesc_acc, (!first || kk > 0) ? 1u : 0u);
+          for (int kk = 0; kk < kIn / 16; ++kk)
+            mma_ts2(d_tmem, a_tmem + (kk >> 1) * 32 + (kk & 1) * 8, b_lo + kk * (2048 >> 4), idesc_acc, (!first || kk > 0) ? 1u : 0u);
+          mma_commit(bar0);
+          if (bar1 != 0) mma_commit(bar1);
+        }
+        __syncwarp();
         TRACE_ADD(2);
       };
 
       for (uint32_t n = 0; alive; ++n) {
-        const int idx = wq_consume_thread(sm.wq, n, abort_flag);
+        const int idx = (int)warp_uniform((uint32_t)wq_consume_warp(sm.wq, n, abort_flag));
         if (idx < 0) break;
-        const WorkItem w = p.items[idx];
-        const int nb = ((w.i_len + kIn - 1) / kIn) * (kDKV ? p.group : 1);  // blocks of the item, over all its query heads
+        // blocks of the item, over all its query heads
+        const int nb = (int)warp_uniform((uint32_t)(((p.items[idx].i_len + kIn - 1) / kIn) * (kDKV ? p.group : 1)));
         if (nb == 0) continue;
-        { TRACE_T0(); if (!mbar_wait(smem_u32(&sm.outer_full), qi & 1, abort_flag)) break; TRACE_ADD(3); }
+        { TRACE_T0(); if (!mbar_wait_warp(smem_u32(&sm.outer_full), qi & 1, abort_flag)) break; TRACE_ADD(3); }
         tc_fence_after();
         if (!issue_x(gk) || !issue_y(gk, nb == 1)) break;
         if (!kDKV && nb > 1 && !issue_x(gk + 1)) break;
         for (int b = 0; b < nb; ++b) {
           const uint32_t g = gk + b;
-          const int sa = g % SA, sb = g % SB;
+          const uint32_t sa = g % SA, sb = g % SB;
+          const uint32_t a_empty = smem_u32(&sm.a_empty[0]) + sa * 8, b_empty = smem_u32(&sm.b_empty[0]) + sb * 8;
+          const uint32_t done = b + 1 < nb ? 0u : smem_u32(&sm.acc_done);
           if (kDKV) {
-            { TRACE_T0(); if (!mbar_wait(smem_u32(&sm.p_full), g & 1, abort_flag)) { alive = false; break; } TRACE_ADD(6); }
+            { TRACE_T0(); if (!mbar_wait_warp(smem_u32(&sm.p_full), g & 1, abort_flag)) { alive = false; break; } TRACE_ADD(6); }
             tc_fence_after();
-            issue_acc(tbase + Cfg::kAcc0, tbase + Cfg::kX, sm.inner_b[sb], b == 0);  // dV += P^T dO
-            mma_commit(smem_u32(&sm.b_empty[sb]));
+            issue_acc(tm + Cfg::kAcc0, tm + Cfg::kX, mb_lo0 + sb * kTile16, b == 0, b_empty, 0);  // dV += P^T dO
             if (b + 1 < nb && !issue_x(g + 1)) { alive = false; break; }
-            { TRACE_T0(); if (!mbar_wait(smem_u32(&sm.ds_full), g & 1, abort_flag)) { alive = false; break; } TRACE_ADD(7); }
+            { TRACE_T0(); if (!mbar_wait_warp(smem_u32(&sm.ds_full), g & 1, abort_flag)) { alive = false; break; } TRACE_ADD(7); }
             tc_fence_after();
-            issue_acc(tbase + Cfg::kAcc1, tbase + Cfg::kY, sm.inner_a[sa], b == 0);  // dK += dS^T Q
-            mma_commit(smem_u32(&sm.a_empty[sa]));
-            if (b + 1 < nb) {
-              if (!issue_y(g + 1, b + 2 == nb)) { alive = false; break; }
-            } else {
-              mma_commit(smem_u32(&sm.acc_done));
-            }
+            issue_acc(tm + Cfg::kAcc1, tm + Cfg::kY, ma_lo0 + sa * kTile16, b == 0, a_empty, done);  // dK += dS^T Q
+            if (b + 1 < nb && !issue_y(g + 1, b + 2 == nb)) { alive = false; break; }
           } else {
-            { TRACE_T0(); if (!mbar_wait(smem_u32(&sm.ds_full), g & 1, abort_flag)) { alive = false; break; } TRACE_ADD(7); }
+            { TRACE_T0(); if (!mbar_wait_warp(smem_u32(&sm.ds_full), g & 1, abort_flag)) { alive = false; break; } TRACE_ADD(7); }
             tc_fence_after();
-            issue_acc(tbase + Cfg::kAcc0, tbase + Cfg::kX + (g & 1) * 128u, sm.inner_a[sa], b == 0);  // dQ += dS K
-            mma_commit(smem_u32(&sm.a_empty[sa]));
+            issue_acc(tm + Cfg::kAcc0, tm + Cfg::kX + (g & 1) * 128u, ma_lo0 + sa * kTile16, b == 0, a_empty, done);  // dQ += dS K
             if (b + 1 < nb) {
               if (!issue_y(g + 1, b + 2 == nb)) { alive = false; break; }
               if (b + 2 < nb && !issue_x(g + 2)) { alive = false; break; }
-            } else {
-              mma_commit(smem_u32(&sm.acc_done));
             }
           }
         }
