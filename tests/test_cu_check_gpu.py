@@ -1,0 +1,29 @@
+"""The host-side cu_seqlens check of tensors on the GPU: what it refuses, and with which error."""
+import pytest
+import torch
+
+import varlenabsorbflashattn_b200 as vb
+
+pytestmark = pytest.mark.gpu
+
+
+def _cu(*v):
+    return torch.tensor(v, dtype=torch.int32, device="cuda")
+
+
+@pytest.mark.parametrize("cu_q,cu_k,text", [
+    ((1, 4), (0, 6), "cu_seqlens_q"), ((0, 3), (0, 6), "cu_seqlens_q"), ((0, 4), (0, 7), "cu_seqlens_k"),
+    ((0, 5, 4), (0, 2, 6), "cu_seqlens_q"), ((0, 2, 4), (0, 7, 6), "cu_seqlens_k"), ((0,), (0,), "at least 2")])
+def test_bad_arrays_are_refused(cu_q, cu_k, text):
+    q, k, v = (torch.randn(n, 1, 64, device="cuda", dtype=torch.bfloat16) for n in (4, 6, 6))
+    with pytest.raises(ValueError, match=text):
+        vb.packed_varlen_attn(q, k, v, cu_seqlens_q=_cu(*cu_q), cu_seqlens_k=_cu(*cu_k))
+
+
+@pytest.mark.parametrize("n_seg", [1, 5000])
+def test_good_arrays_pass(n_seg):
+    x = torch.randn(3 * n_seg, 1, 64, device="cuda", dtype=torch.bfloat16)
+    cu = torch.arange(0, 3 * n_seg + 1, 3, device="cuda", dtype=torch.int64)
+    a = vb.packed_varlen_attn(x, x, x, cu_seqlens_q=cu, cu_seqlens_k=cu.clone())
+    c32 = cu.to(torch.int32)
+    assert torch.equal(a, vb.packed_varlen_attn(x, x, x, cu_seqlens_q=c32, cu_seqlens_k=c32))
