@@ -83,17 +83,23 @@ constexpr int kThreads = kEw * 32 + (VAFA_BWD_SETMAXNREG ? 128 : 64);  // + 1 TM
 __device__ __forceinline__ void tmem_ld_cols(uint32_t taddr, uint32_t (&r)[64]) { tmem_ld64(taddr, r); }
 __device__ __forceinline__ void tmem_ld_cols(uint32_t taddr, uint32_t (&r)[32]) { tmem_ld32(taddr, r); }
 constexpr int kIn = 128;       // rows per inner block
-// One pair of exponentials in kPolyPeriod can take the polynomial 2^t on the FMA pipe instead of the
-// special-function unit; 0 = none.  In these kernels none is fastest (measured: period 4 costs 3-5 % on long
-// non-causal batches and 2.5 % on the 1 M-token causal batch): per score they already issue five integer-pipe
-// instructions (two rounding adds and a byte permute for each of P and dS), that pipe runs at half rate and is
-// the busiest one, and the polynomial adds six more per pair.  The forward, with one rounding per score,
-// keeps period 4.
-#ifndef VAFA_BWD_POLY_PERIOD
-#define VAFA_BWD_POLY_PERIOD 0
+// One pair of exponentials in this many takes the polynomial 2^t on the FMA pipe instead of the special-function unit;
+// 0 = none.  With head dim 64 a block has half the products per exponential, so the unit is what the dQ kernel waits
+// for: 500-query histories 906 us without, 823 us with every fourth pair (832 with every eighth).  With head dim 128 it
+// is level (489 / 496 / 489 us on a 34 k-token batch).  The dK/dV kernel would gain 3 % with head dim 64 (1172 -> 1135
+// us), but the clamp of the polynomial turns a NaN exponent into about 1e-38, and a thread there meets a diverged query
+// row in single columns only, which would then miss from dK and dV; in the dQ kernel it is the thread's whole row.
+// bf16 only: there the error of dQ against 64 bits is the same in six digits, in fp16 it grew in the fourth.
+// -DVAFA_BWD_POLY_PERIOD sets it for both kernels and head dims.
+template <typename T, int D, bool kDKV>
+constexpr bool use_poly(int i) {
+#ifdef VAFA_BWD_POLY_PERIOD
+  constexpr int kPeriod = VAFA_BWD_POLY_PERIOD;
+#else
+  constexpr int kPeriod = !kDKV && D == 64 && std::is_same<T, __nv_bfloat16>::value ? 4 : 0;
 #endif
-constexpr int kPolyPeriod = VAFA_BWD_POLY_PERIOD;
-constexpr bool use_poly(int i) { return kPolyPeriod > 0 && (i % (kPolyPeriod > 0 ? kPolyPeriod : 1)) == kPolyPeriod - 1; }
+  return kPeriod > 0 && i % (kPeriod > 0 ? kPeriod : 1) == kPeriod - 1;
+}
 constexpr int kAugBytes = 128 * 32;  // one fold tile: 128 rows x 16 elements, 32-byte swizzle
 
 template <int D, bool kDKV>
@@ -439,15 +445,14 @@ varlen_bwd128_kernel(const __grid_constant__ CUtensorMap tmap_outer_a, const __g
           uint32_t xs[kC];
           tmem_ld_cols(x_addr + grp * kC, xs);
           tmem_wait_ld();
-          // exponent t = c X' (dK/dV: the product already holds S - lse/c) or c S - lse, in pairs; every
-          // kPolyPeriod-th pair takes the polynomial 2^t on the FMA pipe, the others the special-function unit
+          // exponent t = c X' (dK/dV: the product already holds S - lse/c) or c S - lse, in pairs
           const uint64_t c2 = pack_f2(c, c), nl2 = pack_f2(neg_lse, neg_lse);
 #pragma unroll
           for (int i = 0; i < kC / 2; ++i) {
             const uint64_t x2 = pack_f2(__uint_as_float(xs[2 * i]), __uint_as_float(xs[2 * i + 1]));
             const uint64_t t2 = kDKV ? mul_f2(x2, c2) : fma_f2(x2, c2, nl2);
             float p0, p1;
-            if (use_poly(i)) {
+            if (use_poly<T, D, kDKV>(i)) {
               ex2_poly2(t2, p0, p1);
             } else {
               float t0, t1;
