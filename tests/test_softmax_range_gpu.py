@@ -1,0 +1,72 @@
+"""The forward's softmax against a fixed reference, on scores that leave its range: every further block of an item runs
+against the maximum of the first one, so what lies far above it has to be noticed, in whichever column it stands."""
+import math
+
+import pytest
+import torch
+
+import varlenabsorbflashattn_b200 as vb
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda"
+GAPS = (14.0, 59.0, 100.0, 128.6, 150.0, 200.0, 255.0, 300.0, 400.0)  # log2 units above the first block
+
+
+def _cu(lens):
+    return torch.tensor([0] + list(lens), dtype=torch.int64).cumsum(0).int().to(DEV)
+
+
+def _ref(q, k, v, scale):
+    """Every segment with the same lengths, [n, Lq, H, D] x [n, Lk, H, D], in 64 bits."""
+    S = torch.einsum("nqhd,nkhd->nhqk", q.double(), k.double()) * scale
+    return torch.einsum("nhqk,nkhd->nqhd", S.softmax(-1), v.double()), S.logsumexp(-1).transpose(1, 2)
+
+
+def _lse_tol(ref, D):
+    # each of the D / 16 accumulation steps of a score can lose a unit in the last place of the running fp32 sum, and the
+    # exponent, the logarithm and the conversion of the LSE one more each
+    return 1e-4 + (D // 16 + 4) * 2.0 ** -23 * ref.abs()
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("D", [64, 128])
+@pytest.mark.parametrize("Lq", [1, 130])
+def test_one_key_far_above_the_first_block(dtype, D, Lq):
+    """One key of the second of three blocks stands alone, segment by segment in another column of its block."""
+    n, L, H = 128, 384, 2
+    g = torch.Generator(device=DEV).manual_seed(31)
+    q, k, v = (torch.randn(n, m, H, D, device=DEV, generator=g).to(dtype) for m in (Lq, L, L))
+    q[..., 0] = 8.0
+    k[..., 0] = 0.0
+    at = torch.arange(n, device=DEV)
+    for gap in GAPS:
+        k[at, 128 + at, :, 0] = gap * math.log(2.0) * math.sqrt(D) / 8.0
+        with torch.no_grad():
+            o, lse = vb.packed_varlen_attn_with_lse(q.view(-1, H, D), k.view(-1, H, D), v.view(-1, H, D),
+                                                    cu_seqlens_q=_cu([Lq] * n), cu_seqlens_k=_cu([L] * n))
+        ro, rlse = _ref(q, k, v, D ** -0.5)
+        # P and O are rounded to the type, half an eps each
+        assert (o.view_as(q).double() - ro).abs().max() <= torch.finfo(dtype).eps * v.abs().max() + 1e-3, gap
+        err = (lse.view(n, Lq, H).double() - rlse).abs()
+        assert (err <= _lse_tol(rlse, D)).all(), (gap, err.max().item())
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+def test_one_key_far_above_the_first_block_absorb(dtype):
+    """The same in the absorb kernel's 96-key blocks, whose keys are the values."""
+    n, L, H, D_H, d = 96, 288, 8, 32, 256
+    g = torch.Generator(device=DEV).manual_seed(32)
+    u = (0.3 * torch.randn(n, 2, H, d, device=DEV, generator=g)).to(dtype)
+    X = torch.randn(n, L, d, device=DEV, generator=g).to(dtype)
+    W_V = (torch.randn(d, H, D_H, device=DEV, generator=g) / 16.0).to(dtype)
+    u[..., 0] = 8.0
+    X[..., 0] = 0.0
+    W_V[0] = 0.0  # the column that raises a key is not seen in its value
+    at = torch.arange(n, device=DEV)
+    for gap in GAPS:
+        X[at, 96 + at, 0] = gap * math.log(2.0) * math.sqrt(D_H) / 8.0
+        with torch.no_grad():
+            O = vb.target_attn_inner(u.view(-1, H, d), X.view(-1, d), W_V, _cu([2] * n), _cu([L] * n))
+        xs = X.unsqueeze(2).expand(n, L, H, d)
+        ro = torch.einsum("nqhk,khd->nqhd", _ref(u, xs, xs, D_H ** -0.5)[0], W_V.double())
+        assert (O.view_as(ro).double() - ro).abs().max() <= 3e-2, gap  # alphaX is rounded as well

@@ -48,8 +48,10 @@ constexpr float kRescaleThreshold = 8.0f;  // log2 units
 // O / l does not depend on it.  So the first block of an item sets it, and every further block is computed
 // against it as it stands: no row maximum, no exchange between the two warps that share the rows (which may then
 // run a block apart, so that one's waits lie under the other's exponentials), no rescaling of O.
-// At the end of the item the row sum tells whether all stayed in range: a sum within kMaxSum (and in fp16 every partial
-// sum within kMaxPart, which bounds P itself) proves it.  An item that fails, or holds a NaN, is written down and
+// At the end of the item the row sum tells whether the exponentials of the special-function unit stayed in range: a sum
+// within kMaxSum (and in fp16 every partial sum within kMaxPart, which bounds P itself) proves it.  Those of the
+// polynomial it cannot vouch for: from 2^128 on they run into the sign bit and come out as anything, small or negative.
+// Their largest exponent is kept instead, one 3-input maximum per pair.  An item that fails, or holds a NaN, is written down and
 // done again at the end of the kernel by the CTA that met it, the careful way: the maximum of every
 // block, O rescaled when it moves by more than 2^8.  From kRedoGiveUp entries on the CTA takes its remaining items
 // the careful way at once, so inputs whose scores keep climbing cost a few items twice, not all.
@@ -60,6 +62,7 @@ constexpr int kRedoGiveUp = 8;      // entries (each softmax warp writes its own
 constexpr int kRedoCap = 128;       // what the items already published when the CTA gives up can add, twice over
 constexpr float kMaxSum = 1.152921504606846976e18f;  // 2^60
 constexpr float kMaxPart = 32768.f;                  // sum of one thread's exponentials of a block, fp16
+constexpr float kMaxExp = 60.f;                      // exponent of a polynomial
 #ifndef VAFA_FWD_POLY_PERIOD
 #define VAFA_FWD_POLY_PERIOD 4
 #endif
@@ -425,6 +428,7 @@ varlen_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_const
       const bool live = (warp & 3) * 32 < w.o_rows * p.stack;  // does any row of this warp exist?
       float m_ref = -INFINITY, l = 0.f;  // l: sum over this thread's columns only
       float worst = 0.f;                 // fp16: largest sum of a block
+      float t_max = 0.f;                 // largest exponent given to the polynomial
       bool no_ref = false;
 
       for (int b = 0; b < nb; ++b) {
@@ -481,11 +485,12 @@ varlen_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_const
           for (int i = 0; i < kHalf / 2; ++i) {
             const uint64_t t2 = fma_f2(pack_f2(s[2 * i], s[2 * i + 1]), cs2, nm2);
             float p0, p1;
+            float t0, t1;
+            unpack_f2(t2, t0, t1);
             if (kPoly && (i % kPolyPeriod == kPolyPeriod - 1)) {
+              t_max = max3(t_max, t0, t1);
               ex2_poly2(t2, p0, p1);
             } else {
-              float t0, t1;
-              unpack_f2(t2, t0, t1);
               p0 = ex2(t0);
               p1 = ex2(t1);
             }
@@ -597,7 +602,8 @@ varlen_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_const
         l_tot = l + sm.xsum[half ^ 1][r];
       }
       if (nb > 1 && !careful) {
-        const bool out_of_range = row_ok && (no_ref || !(l_tot <= kMaxSum) || (std::is_same<T, __half>::value && worst > kMaxPart));
+        const bool out_of_range = row_ok && (no_ref || !(l_tot <= kMaxSum) || t_max > kMaxExp ||
+                                             (std::is_same<T, __half>::value && worst > kMaxPart));
         if (__any_sync(0xffffffffu, out_of_range) && lane == 0) {
           // what is written below is overwritten when the item is done again
           const int at = atomicAdd(&sm.n_redo, 1);
