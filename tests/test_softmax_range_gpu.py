@@ -1,6 +1,9 @@
 """The forward's softmax against a fixed reference, on scores that leave its range: every further block of an item runs
 against the maximum of the first one, so what lies far above it has to be noticed, in whichever column it stands."""
 import math
+import os
+import subprocess
+import sys
 
 import pytest
 import torch
@@ -70,3 +73,32 @@ def test_one_key_far_above_the_first_block_absorb(dtype):
         xs = X.unsqueeze(2).expand(n, L, H, d)
         ro = torch.einsum("nqhk,khd->nqhd", _ref(u, xs, xs, D_H ** -0.5)[0], W_V.double())
         assert (O.view_as(ro).double() - ro).abs().max() <= 3e-2, gap  # alphaX is rounded as well
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("D", [64, 128])
+@pytest.mark.parametrize("Lq,L", [(3, 128), (3, 384), (200, 384)])
+@pytest.mark.parametrize("bad", [float("nan"), float("inf")])
+def test_a_nan_or_infinite_score_reaches_its_rows_from_every_column(dtype, D, Lq, L, bad):
+    """Softmax of a row with a NaN or +inf score is NaN; the key stands in another column of the last block of each segment."""
+    n, H = 128, 2
+    g = torch.Generator(device=DEV).manual_seed(33)
+    q, k, v = (torch.randn(n, m, H, D, device=DEV, generator=g).to(dtype) for m in (Lq, L, L))
+    q[..., 0] = 1.0
+    at = torch.arange(n, device=DEV)
+    k[at, L - 128 + at, 0, 0] = bad
+    with torch.no_grad():
+        o, lse = vb.packed_varlen_attn_with_lse(q.view(-1, H, D), k.view(-1, H, D), v.view(-1, H, D),
+                                                cu_seqlens_q=_cu([Lq] * n), cu_seqlens_k=_cu([L] * n))
+    o, lse = o.view(n, Lq, H, D), lse.view(n, Lq, H)
+    assert torch.isnan(o[:, :, 0]).all() and torch.isnan(lse[:, :, 0]).all()
+    assert torch.isfinite(o[:, :, 1]).all() and torch.isfinite(lse[:, :, 1]).all()
+
+
+def test_the_same_in_the_two_tile_kernel():
+    """Segments of more than 160 query rows go there with VAFA_FWD_PAIR=1 (read once per process)."""
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    r = subprocess.run([sys.executable, "-m", "pytest", __file__, "-q", "-x", "-m", "gpu", "-k", "from_every_column and 200",
+                        "-p", "no:cacheprovider"], env=dict(os.environ, VAFA_FWD_PAIR="1"), cwd=root, capture_output=True, text=True,
+                       timeout=600)
+    assert r.returncode == 0 and "8 passed" in r.stdout, r.stdout[-3000:] + r.stderr[-2000:]

@@ -294,6 +294,12 @@ __device__ __forceinline__ float max3(float a, float b, float c) {
   asm("max.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
   return r;
 }
+// The same, NaN if one of them is.
+__device__ __forceinline__ float max3_nan(float a, float b, float c) {
+  float r;
+  asm("max.NaN.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+  return r;
+}
 
 // 1-D bulk copy global -> shared (16-byte aligned addresses, size a multiple of 16 bytes).
 __device__ __forceinline__ void bulk_load_1d(uint32_t smem_dst, const void* gsrc, uint32_t bytes, uint32_t bar) {
@@ -336,7 +342,7 @@ __device__ __forceinline__ uint64_t add_f2(uint64_t a, uint64_t b) {
 // 2^t for a pair without the special-function unit (16 results/clk/SM, the limit of the softmax
 // loops): n = round(t) by the magic-number add, f = t - n in [-0.5, 0.5], 2^f by a degree-4
 // polynomial (max relative error 2.7e-6), n added into the exponent field.  t is clamped at -126,
-// so -inf and very negative arguments give about 1e-38 instead of 0.
+// so -inf, very negative arguments and NaN give about 1e-38 instead of 0 or NaN; from 128 on the result is meaningless.
 __device__ __forceinline__ void ex2_poly2(uint64_t t2, float& r0, float& r1) {
   float a, b;
   unpack_f2(t2, a, b);

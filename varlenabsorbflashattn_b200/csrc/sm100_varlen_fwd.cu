@@ -51,8 +51,8 @@ constexpr float kRescaleThreshold = 8.0f;  // log2 units
 // At the end of the item the row sum tells whether the exponentials of the special-function unit stayed in range: a sum
 // within kMaxSum (and in fp16 every partial sum within kMaxPart, which bounds P itself) proves it.  Those of the
 // polynomial it cannot vouch for: from 2^128 on they run into the sign bit and come out as anything, small or negative.
-// Their largest exponent is kept instead, one 3-input maximum per pair.  An item that fails, or holds a NaN, is written down and
-// done again at the end of the kernel by the CTA that met it, the careful way: the maximum of every
+// Their largest exponent is kept instead, one 3-input maximum per pair, which also keeps a NaN that the polynomial would
+// make a zero of: the row sum takes it over.  An item that fails is written down and done again at the end of the kernel by the CTA that met it, the careful way: the maximum of every
 // block, O rescaled when it moves by more than 2^8.  From kRedoGiveUp entries on the CTA takes its remaining items
 // the careful way at once, so inputs whose scores keep climbing cost a few items twice, not all.
 // Measured: 500-query histories, head dim 64: 710 -> 615 us; prefill of 16 sequences, head dim 128: 1229 -> 1202 us.
@@ -488,7 +488,7 @@ varlen_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_const
             float t0, t1;
             unpack_f2(t2, t0, t1);
             if (kPoly && (i % kPolyPeriod == kPolyPeriod - 1)) {
-              t_max = max3(t_max, t0, t1);
+              t_max = max3_nan(t_max, t0, t1);
               ex2_poly2(t2, p0, p1);
             } else {
               p0 = ex2(t0);
@@ -595,6 +595,7 @@ varlen_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_const
       if (nb > 0) {
         if (!mbar_wait(smem_u32(&sm.o_done[(gk - 1) % S]), ((gk - 1) / S) & 1, abort_flag)) break;
         tc_fence_after();
+        if (isnan(t_max)) l = t_max;
         sm.xsum[half][r] = l;
         mbar_arrive(pair_bar);
         if (!mbar_wait(pair_bar, pair_cnt & 1, abort_flag)) break;
@@ -943,6 +944,7 @@ varlen_fwd_pair_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_
       const int my_nb = z.nb_t[t], my_rows = z.rows_t[t];
       const int h = w.head;
       float m_ref = -INFINITY, l = 0.f;
+      float t_max = 0.f;  // largest exponent given to the polynomial: keeps a NaN that it would make a zero of
 
       for (int b = 0; b < my_nb; ++b, ++cnt) {
         const uint32_t g = gk + b;
@@ -999,11 +1001,12 @@ varlen_fwd_pair_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_
               const int e = 64 * hf + 2 * i;
               const uint64_t t2 = fma_f2(pack_f2(s[e], s[e + 1]), cs2, nm2);
               float p0, p1;
+              float t0, t1;
+              unpack_f2(t2, t0, t1);
               if (kPoly && (i % kPolyPeriod == kPolyPeriod - 1)) {
+                t_max = max3_nan(t_max, t0, t1);
                 ex2_poly2(t2, p0, p1);
               } else {
-                float t0, t1;
-                unpack_f2(t2, t0, t1);
                 p0 = ex2(t0);
                 p1 = ex2(t1);
               }
@@ -1051,6 +1054,7 @@ varlen_fwd_pair_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_
         ++n_ready;
         tc_fence_after();
       }
+      if (isnan(t_max)) l = t_max;
       const bool row_ok = r < my_rows;
       const bool dead = (my_nb == 0) || (l == 0.f);  // a NaN row sum is not a dead row: it goes out as NaN
       const float inv_l = dead ? 0.f : 1.f / l;
