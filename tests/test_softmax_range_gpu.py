@@ -102,3 +102,32 @@ def test_the_same_in_the_two_tile_kernel():
                         "-p", "no:cacheprovider"], env=dict(os.environ, VAFA_FWD_PAIR="1"), cwd=root, capture_output=True, text=True,
                        timeout=600)
     assert r.returncode == 0 and "8 passed" in r.stdout, r.stdout[-3000:] + r.stderr[-2000:]
+
+
+def _climbing(dtype, D, n, L, H, climb, every):
+    """Self-attention batch in which every `every`-th segment climbs by `climb` log2 units from block to block."""
+    g = torch.Generator(device=DEV).manual_seed(34)
+    q, k, v = (torch.randn(n, L, H, D, device=DEV, generator=g).to(dtype) for _ in range(3))
+    q[..., 0] = 1.0
+    step = torch.arange(L, device=DEV).div(128, rounding_mode="floor").float() * climb * math.log(2.0) * math.sqrt(D)
+    k[::every, :, :, 0] = step[:, None].to(dtype)
+    return q, k, v
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("D,climb,every", [(64, 30.0, 2), (128, 30.0, 7), (128, 12.0, 2)])
+def test_results_do_not_depend_on_the_rest_of_the_batch(dtype, D, climb, every):
+    """Where a few segments leave the range, all come out with the same bits in every run and in a batch of their own."""
+    n, L, H = 96, 640, 4
+    q, k, v = _climbing(dtype, D, n, L, H, climb, every)
+
+    def run(a, b):
+        with torch.no_grad():
+            return vb.packed_varlen_attn_with_lse(*(t[a:b].reshape(-1, H, D) for t in (q, k, v)),
+                                                  cu_seqlens_q=_cu([L] * (b - a)), cu_seqlens_k=_cu([L] * (b - a)), causal=True)
+
+    full = run(0, n)
+    for _ in range(4):
+        assert all(torch.equal(x, y) for x, y in zip(run(0, n), full))
+    for a, b in ((0, 12), (12, 13), (13, 60), (60, n)):
+        assert all(torch.equal(x, y[a * L:b * L]) for x, y in zip(run(a, b), full)), (a, b)

@@ -48,21 +48,32 @@ constexpr float kRescaleThreshold = 8.0f;  // log2 units
 // O / l does not depend on it.  So the first block of an item sets it, and every further block is computed
 // against it as it stands: no row maximum, no exchange between the two warps that share the rows (which may then
 // run a block apart, so that one's waits lie under the other's exponentials), no rescaling of O.
-// At the end of the item the row sum tells whether the exponentials of the special-function unit stayed in range: a sum
-// within kMaxSum (and in fp16 every partial sum within kMaxPart, which bounds P itself) proves it.  Those of the
-// polynomial it cannot vouch for: from 2^128 on they run into the sign bit and come out as anything, small or negative.
-// Their largest exponent is kept instead, one 3-input maximum per pair, which also keeps a NaN that the polynomial would
-// make a zero of: the row sum takes it over.  An item that fails is written down and done again at the end of the kernel by the CTA that met it, the careful way: the maximum of every
-// block, O rescaled when it moves by more than 2^8.  From kRedoGiveUp entries on the CTA takes its remaining items
-// the careful way at once, so inputs whose scores keep climbing cost a few items twice, not all.
-// Measured: 500-query histories, head dim 64: 710 -> 615 us; prefill of 16 sequences, head dim 128: 1229 -> 1202 us.
+// At the end of the item each thread knows whether its exponents stayed below kStay: for those of the special-function
+// unit the largest sum of a block tells, which bounds them; those of the polynomial, which from 2^128 on run into the
+// sign bit and come out as anything, by their maximum (one 3-input instruction per pair, which also keeps a NaN
+// that the polynomial would make a zero of: the row sum takes it over).
+// An item where they did not goes to the CTA's own list and is done again the careful way: the maximum of every block,
+// O rescaled when it moves by more than kStay + 1/2.  Where the exponents stay below kStay that never happens, so both
+// ways give the same bits; how an item is done may therefore depend on timing, what comes out does not.
+// Doing an item twice is what inputs of large spread must not pay for: the lists begin with the longest items, and a CTA
+// of a decode batch has four in all.  So a pair of warps does its first item of several blocks the careful way, and
+// goes on without only if the exponents of that one stayed below kNear; from the first item of the CTA on that does not, all
+// are done the careful way.  In fp16, whose range a spread of a few units leaves, so are all items of at most 32 rows:
+// one row tells too little about the next, and a decode batch, bound by HBM, loses 0 to 1.5 % by it.
+// Measured, forward in fp16 with scores of standard deviation 1 / 4 / 8 (us; one column per rule: maximum in every block |
+// every item without, failed ones again at the end | this one):
+//   16 causal sequences, 32/8 heads of 128    970 989 992 | 903 1285 1338 | 910 1007 1019
+//   16 users x 500 queries, 4 heads of 64     490 497 497 | 318  624  488 | 337  392  384
+//   64 decode requests, 8 heads of 128        302 302 302 | 302  345  462 | 302  302  306
+// In bf16 the second and the third rule are level up to 8 (prefill 876 / 888, histories 341 / 355), the first takes 949 and 531.
+template <typename T> constexpr float kStay = std::is_same<T, __half>::value ? 15.f : 59.f;
+template <typename T> constexpr float kStayPart = std::is_same<T, __half>::value ? 0x1p15f : 0x1p59f;  // 2^kStay
+template <typename T> constexpr float kNear = std::is_same<T, __half>::value ? 11.f : 40.f;
+template <typename T> constexpr float kNearPart = std::is_same<T, __half>::value ? 0x1p11f : 0x1p40f;
 constexpr int kCareful = 1 << 30;   // flag on a published item index
-constexpr int kDrain = -2;          // published once: the softmax warps report that all items before it are done
-constexpr int kRedoGiveUp = 8;      // entries (each softmax warp writes its own, so one item can make eight)
-constexpr int kRedoCap = 128;       // what the items already published when the CTA gives up can add, twice over
-constexpr float kMaxSum = 1.152921504606846976e18f;  // 2^60
-constexpr float kMaxPart = 32768.f;                  // sum of one thread's exponentials of a block, fp16
-constexpr float kMaxExp = 60.f;                      // exponent of a polynomial
+constexpr int kItemMask = kCareful - 1;
+constexpr int kDrain = -2;          // the softmax warps report that all items before it are done
+constexpr int kRedoCap = 4;         // one entry per pair of warps
 #ifndef VAFA_FWD_POLY_PERIOD
 #define VAFA_FWD_POLY_PERIOD 4
 #endif
@@ -116,9 +127,10 @@ struct FwdSmem {
   uint64_t pair_bar[4];       // the two softmax warps of one TMEM lane quadrant
   float xmax[2][2][128];      // [block parity][half][row] partial row maxima
   float xsum[2][128];         // [half][row] partial row sums at the end of an item
+  int xflag[2][4];            // [half][pair] 1: an exponent left the range, 2: one came near, or left it in another pair
   uint64_t drain;             // all softmax warps have met kDrain
-  int redo[kRedoCap];         // items to be done again
-  int n_redo;
+  int redo[kRedoCap];         // items to be done again; -1 = not written
+  int n_redo;                 // entries written so far
   WorkQueue wq;
   uint32_t tmem_base;
   int abort_flag;
@@ -184,6 +196,7 @@ varlen_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_const
     sm.wait_limit = p.wait_limit;
     wq_init(sm.wq, 9);
     sm.n_redo = 0;
+    for (int i = 0; i < kRedoCap; ++i) sm.redo[i] = -1;
     mbar_init(smem_u32(&sm.drain), 8);
     for (int i = 0; i < 4; ++i) mbar_init(smem_u32(&sm.pair_bar[i]), 64);
     mbar_init(smem_u32(&sm.q_full), 1);
@@ -228,36 +241,39 @@ varlen_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_const
     if (lane == 0) {
       uint32_t gk = 0, qi = 0;
       bool alive = true;
-      bool drained = false;
-      int n_seen = 0;  // redo entries looked at
+      bool exhausted = false, dirty = true;  // dirty: items were published since the last kDrain
+      uint32_t n_drain = 0;
+      int n_seen = 0;                        // redo entries taken
       for (uint32_t n = 0; alive; ++n) {
         const int slot = n % kWqSlots;
         if (!mbar_wait(smem_u32(&sm.wq.empty[slot]), ((n / kWqSlots) & 1) ^ 1, abort_flag)) break;
         int idx = -1;
-        if (!drained) {
+        while (idx < 0 && n_seen < kRedoCap) {
+          idx = ((volatile int*)sm.redo)[n_seen];
+          if (idx < 0) break;
+          for (int i = 0; i < n_seen; ++i)
+            if (sm.redo[i] == idx) { idx = -1; break; }  // the pairs of a CTA write an item's entry one by one
+          ++n_seen;
+        }
+        if (idx < 0 && !exhausted) {
           idx = atomicAdd(next_item, 1);
-          if (idx >= total) {
-            idx = kDrain;
-            drained = true;
-          } else if (*(volatile int*)&sm.n_redo >= kRedoGiveUp) {
-            idx |= kCareful;
-          }
-        } else {
-          if (n_seen == 0 && !mbar_wait(smem_u32(&sm.drain), 0, abort_flag)) break;
-          const int n_redo = min(*(volatile int*)&sm.n_redo, kRedoCap);
-          while (idx < 0 && n_seen < n_redo) {
-            idx = sm.redo[n_seen];
-            for (int i = 0; i < n_seen; ++i)
-              if (sm.redo[i] == idx) { idx = -1; break; }
-            ++n_seen;
-          }
-          if (idx >= 0) idx |= kCareful;
+          if (idx >= total) { idx = -1; exhausted = true; }
+        }
+        if (idx >= 0) {
+          dirty = true;
+        } else if (dirty) {
+          idx = kDrain;
+          dirty = false;
         }
         sm.wq.idx[slot] = idx;
         mbar_arrive(smem_u32(&sm.wq.full[slot]));
-        if (idx == kDrain) continue;
+        if (idx == kDrain) {
+          if (!mbar_wait(smem_u32(&sm.drain), n_drain & 1, abort_flag)) break;
+          ++n_drain;
+          continue;
+        }
         if (idx < 0) break;
-        const WorkItem w = p.items[idx & ~kCareful];
+        const WorkItem w = p.items[idx & kItemMask];
         const int h = w.head * p.stack;
         const int hk = w.head / p.group;  // K/V head of this query head or stack
         const int nb = (w.i_len + kBlk - 1) / kBlk;
@@ -348,7 +364,7 @@ varlen_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_const
         const int idx = (int)warp_uniform((uint32_t)wq_consume_warp(sm.wq, n, abort_flag));
         if (idx == kDrain) continue;
         if (idx < 0) break;
-        const int nb = (int)warp_uniform((uint32_t)((p.items[idx & ~kCareful].i_len + kBlk - 1) / kBlk));
+        const int nb = (int)warp_uniform((uint32_t)((p.items[idx & kItemMask].i_len + kBlk - 1) / kBlk));
         if (nb == 0) continue;
         { TRACE_T0(); if (!mbar_wait_warp(smem_u32(&sm.q_full), qi & 1, abort_flag)) break; TRACE_ADD(3); }
         tc_fence_after();
@@ -410,6 +426,7 @@ varlen_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_const
     const float c = p.scale_log2;
     uint32_t gk = 0;
     bool alive = true;
+    bool known = false, wary = false;  // the pair has done an item of several blocks; one of the CTA came near the limit
     for (uint32_t n = 0; alive; ++n) {
       const int entry = wq_consume_warp(sm.wq, n, abort_flag);
       if (entry == kDrain) {
@@ -417,9 +434,10 @@ varlen_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_const
         continue;
       }
       if (entry < 0) break;
-      const bool careful = (entry & kCareful) != 0;
-      const int idx = entry & ~kCareful;
+      const int idx = entry & kItemMask;
       const WorkItem w = p.items[idx];
+      const bool few = std::is_same<T, __half>::value && w.o_rows * p.stack <= 32;
+      const bool careful = few || wary || !known || (entry & kCareful) != 0;
       const int nb = (w.i_len + kBlk - 1) / kBlk;
       // tile row r -> (query row of the tile, head)
       const int rq = p.stack == 1 ? r : r / p.stack;
@@ -427,9 +445,9 @@ varlen_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_const
       const bool row_ok = rq < w.o_rows;
       const bool live = (warp & 3) * 32 < w.o_rows * p.stack;  // does any row of this warp exist?
       float m_ref = -INFINITY, l = 0.f;  // l: sum over this thread's columns only
-      float worst = 0.f;                 // fp16: largest sum of a block
+      float worst = 0.f;                 // largest sum of a block behind the first
       float t_max = 0.f;                 // largest exponent given to the polynomial
-      bool no_ref = false;
+      bool no_ref = false, moved = false;
 
       for (int b = 0; b < nb; ++b) {
         const uint32_t g = gk + b;
@@ -503,12 +521,8 @@ varlen_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_const
           return (a0 + a1) + (b0 + b1);
         };
         bool resc = false;
-        float alpha = 1.f;
-        if (b > 0 && !careful) {
-          const float bsum = masked_block ? exps(m_ref, std::false_type{}) : exps(m_ref, std::true_type{});
-          l += bsum;
-          if (std::is_same<T, __half>::value) worst = fmaxf(worst, bsum);
-        } else {
+        float alpha = 1.f, m_use = m_ref;
+        if (b == 0 || careful) {
           // row maximum of this half: eight independent chains of 3-input max
           float m8[8];
 #pragma unroll
@@ -528,17 +542,20 @@ varlen_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_const
           { TRACE_T0(); if (!mbar_wait(pair_bar, pair_cnt & 1, abort_flag)) { alive = false; break; } TRACE_ADD(12); }
           ++pair_cnt;
           mx = fmaxf(mx, sm.xmax[g & 1][half ^ 1][r]);
-          const float m_blk = mx * c;  // c > 0
-          float m_new = fmaxf(m_ref, m_blk);
-          resc = m_new > m_ref + kRescaleThreshold;
-          if (!resc) m_new = m_ref;
+          // (c > 0; the exponent of the largest score in the arithmetic of the exponents, so that it is the largest of them)
+          resc = fmaf(mx, c, -m_ref) > kStay<T> + 0.5f;
+          const float m_new = resc ? mx * c : m_ref;
           alpha = resc ? ex2(m_ref - m_new) : 1.f;
-          const float m_use = (m_new == -INFINITY) ? 0.f : m_new;
-          const float bsum = masked_block ? exps(m_use, std::false_type{}) : exps(m_use, std::true_type{});
-          l = l * alpha + bsum;
+          m_use = (m_new == -INFINITY) ? 0.f : m_new;
           // (a row without a finite score in the first block has no reference; one that sees no key needs none)
           m_ref = careful ? m_new : m_use;
           no_ref = m_new == -INFINITY && !(w.masked && rq + w.diag < 0);
+        }
+        const float bsum = masked_block ? exps(m_use, std::false_type{}) : exps(m_use, std::true_type{});
+        l = l * alpha + bsum;
+        if (b > 0) {
+          worst = fmaxf(worst, bsum);
+          moved = moved || resc;
         }
         // kHalf probabilities -> kHalf/2 packed columns over the first half of the columns just read
         // (the MMA issuer's addressing of the K-steps is next to its P.V loop)
@@ -596,20 +613,23 @@ varlen_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_const
         if (!mbar_wait(smem_u32(&sm.o_done[(gk - 1) % S]), ((gk - 1) / S) & 1, abort_flag)) break;
         tc_fence_after();
         if (isnan(t_max)) l = t_max;
+        const bool left = row_ok && nb > 1 && (no_ref || moved || worst > kStayPart<T> || t_max > kStay<T>);
+        const bool near = row_ok && (worst > kNearPart<T> || t_max > kNear<T>);
+        int flags = (__any_sync(0xffffffffu, left) ? 1 : 0) | (__any_sync(0xffffffffu, near) ? 2 : 0);
+        if (lane == 0) {
+          if (*(volatile int*)&sm.n_redo > 0) flags |= 2;
+          sm.xflag[half][warp & 3] = flags;
+        }
         sm.xsum[half][r] = l;
         mbar_arrive(pair_bar);
         if (!mbar_wait(pair_bar, pair_cnt & 1, abort_flag)) break;
         ++pair_cnt;
         l_tot = l + sm.xsum[half ^ 1][r];
-      }
-      if (nb > 1 && !careful) {
-        const bool out_of_range = row_ok && (no_ref || !(l_tot <= kMaxSum) || t_max > kMaxExp ||
-                                             (std::is_same<T, __half>::value && worst > kMaxPart));
-        if (__any_sync(0xffffffffu, out_of_range) && lane == 0) {
-          // what is written below is overwritten when the item is done again
-          const int at = atomicAdd(&sm.n_redo, 1);
-          if (at < kRedoCap) sm.redo[at] = idx;
-        }
+        flags = sm.xflag[0][warp & 3] | sm.xflag[1][warp & 3];
+        wary = wary || flags != 0;
+        known = known || nb > 1;
+        // (what is written below is overwritten when the item is done again)
+        if ((flags & 1) && !careful && half == 0 && lane == 0) ((volatile int*)sm.redo)[atomicAdd(&sm.n_redo, 1)] = idx | kCareful;
       }
       const bool dead = (nb == 0) || (l_tot == 0.f);  // a NaN row sum is not a dead row: it goes out as NaN
       const float inv_l = dead ? 0.f : 1.f / l_tot;
