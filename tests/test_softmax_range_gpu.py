@@ -131,3 +131,26 @@ def test_results_do_not_depend_on_the_rest_of_the_batch(dtype, D, climb, every):
         assert all(torch.equal(x, y) for x, y in zip(run(0, n), full))
     for a, b in ((0, 12), (12, 13), (13, 60), (60, n)):
         assert all(torch.equal(x, y[a * L:b * L]) for x, y in zip(run(a, b), full)), (a, b)
+
+
+@pytest.mark.parametrize("D", [64, 128])
+@pytest.mark.parametrize("Lq,n", [(640, 8), (640, 90), (2, 90)])
+def test_large_values_under_climbing_scores(D, Lq, n):
+    """bf16 values near 2^100 under scores that climb by up to 40: P.V stays finite, as P does not grow with them."""
+    L, H = 640, 2
+    q, k, v = _climbing(torch.bfloat16, D, n, L, H, 10.0, 2)
+    q = q[:, :Lq].contiguous()
+    v = (v.float() * 2.0 ** 100).to(torch.bfloat16)
+
+    def run(a, b):
+        with torch.no_grad():
+            return vb.packed_varlen_attn(*(t[a:b].reshape(-1, H, D) for t in (q, k, v)), cu_seqlens_q=_cu([Lq] * (b - a)),
+                                         cu_seqlens_k=_cu([L] * (b - a)), split_k_block=L)  # (how keys are cut depends on the batch)
+
+    o = run(0, n)
+    ro, _ = _ref(q[:8], k[:8], v[:8], D ** -0.5)
+    # P and O are rounded to the type, half an eps each
+    assert (o[:8 * Lq].view_as(ro).double() - ro).abs().max() <= (torch.finfo(o.dtype).eps + 1e-3) * v.abs().max().double()
+    for _ in range(3):
+        assert torch.equal(run(0, n), o)
+    assert torch.equal(run(3, 8), o[3 * Lq:8 * Lq])

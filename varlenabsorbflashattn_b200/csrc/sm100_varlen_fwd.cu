@@ -66,14 +66,22 @@ constexpr float kRescaleThreshold = 8.0f;  // log2 units
 //   16 users x 500 queries, 4 heads of 64     490 497 497 | 318  624  488 | 337  392  384
 //   64 decode requests, 8 heads of 128        302 302 302 | 302  345  462 | 302  302  306
 // In bf16 the second and the third rule are level up to 8 (prefill 876 / 888, histories 341 / 355), the first takes 949 and 531.
+// A bf16 P of up to 2^kStay can overflow O where V is large, which one of up to 2^8 would not: an item with partial sums
+// above 2^8 and a value of O that is not finite is done again the strict way, O rescaled when the maximum moves by 2^8.
 template <typename T> constexpr float kStay = std::is_same<T, __half>::value ? 15.f : 59.f;
 template <typename T> constexpr float kStayPart = std::is_same<T, __half>::value ? 0x1p15f : 0x1p59f;  // 2^kStay
 template <typename T> constexpr float kNear = std::is_same<T, __half>::value ? 11.f : 40.f;
 template <typename T> constexpr float kNearPart = std::is_same<T, __half>::value ? 0x1p11f : 0x1p40f;
-constexpr int kCareful = 1 << 30;   // flag on a published item index
-constexpr int kItemMask = kCareful - 1;
+constexpr float kLargePart = 256.f;
+constexpr int kCareful = 1 << 30;   // flags on a published item index
+constexpr int kStrict = 1 << 29;
+constexpr int kItemMask = kStrict - 1;
 constexpr int kDrain = -2;          // the softmax warps report that all items before it are done
-constexpr int kRedoCap = 4;         // one entry per pair of warps
+// Entries of the list that can wait at a time.  An item leaves at most eight (one per warp), of which the careful ones come
+// once per pair and kernel.  At most seven items lie between the producer and the slowest warp (four published, one in
+// each role), and while entries wait the producer publishes them instead of new items; of these only the careful
+// ones, four at most, leave new entries.
+constexpr int kRedoCap = 128;
 #ifndef VAFA_FWD_POLY_PERIOD
 #define VAFA_FWD_POLY_PERIOD 4
 #endif
@@ -127,9 +135,9 @@ struct FwdSmem {
   uint64_t pair_bar[4];       // the two softmax warps of one TMEM lane quadrant
   float xmax[2][2][128];      // [block parity][half][row] partial row maxima
   float xsum[2][128];         // [half][row] partial row sums at the end of an item
-  int xflag[2][4];            // [half][pair] 1: an exponent left the range, 2: one came near, or left it in another pair
+  int xflag[2][4];            // [half][pair] 1: an exponent left the range, 2: one came near, or left it in another pair, 4: a large sum
   uint64_t drain;             // all softmax warps have met kDrain
-  int redo[kRedoCap];         // items to be done again; -1 = not written
+  int redo[kRedoCap];         // ring of items to be done again, each with its flag; -1 = free
   int n_redo;                 // entries written so far
   WorkQueue wq;
   uint32_t tmem_base;
@@ -242,18 +250,30 @@ varlen_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_const
       uint32_t gk = 0, qi = 0;
       bool alive = true;
       bool exhausted = false, dirty = true;  // dirty: items were published since the last kDrain
-      uint32_t n_drain = 0;
-      int n_seen = 0;                        // redo entries taken
+      uint32_t n_drain = 0, n_seen = 0;      // kDrain so far, redo entries taken
+      int recent[4] = {-1, -1, -1, -1};      // the last of them: the warps of a CTA write an item's entry one by one
       for (uint32_t n = 0; alive; ++n) {
         const int slot = n % kWqSlots;
         if (!mbar_wait(smem_u32(&sm.wq.empty[slot]), ((n / kWqSlots) & 1) ^ 1, abort_flag)) break;
         int idx = -1;
-        while (idx < 0 && n_seen < kRedoCap) {
-          idx = ((volatile int*)sm.redo)[n_seen];
-          if (idx < 0) break;
-          for (int i = 0; i < n_seen; ++i)
-            if (sm.redo[i] == idx) { idx = -1; break; }  // the pairs of a CTA write an item's entry one by one
+        while (idx < 0) {
+          volatile int* const entry = &sm.redo[n_seen % kRedoCap];
+          const int e = *entry;
+          if (e < 0) break;
+          *entry = -1;
           ++n_seen;
+          // A pass covers all warps' rows, a strict one also in place of a careful one (which, coming after it, would
+          // write the strict entry again)
+          bool known = false, covered = false;
+          for (int i = 0; i < 4; ++i) {
+            if (recent[i] < 0 || (recent[i] & kItemMask) != (e & kItemMask)) continue;
+            known = true;
+            covered = recent[i] == e || (recent[i] & kStrict) != 0;
+            if (!covered) recent[i] = e;
+          }
+          if (covered) continue;
+          if (!known) { recent[3] = recent[2]; recent[2] = recent[1]; recent[1] = recent[0]; recent[0] = e; }
+          idx = e;
         }
         if (idx < 0 && !exhausted) {
           idx = atomicAdd(next_item, 1);
@@ -426,6 +446,7 @@ varlen_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_const
     const float c = p.scale_log2;
     uint32_t gk = 0;
     bool alive = true;
+    auto again = [&](int entry) { *(volatile int*)&sm.redo[atomicAdd(&sm.n_redo, 1) % kRedoCap] = entry; };
     bool known = false, wary = false;  // the pair has done an item of several blocks; one of the CTA came near the limit
     for (uint32_t n = 0; alive; ++n) {
       const int entry = wq_consume_warp(sm.wq, n, abort_flag);
@@ -437,7 +458,8 @@ varlen_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_const
       const int idx = entry & kItemMask;
       const WorkItem w = p.items[idx];
       const bool few = std::is_same<T, __half>::value && w.o_rows * p.stack <= 32;
-      const bool careful = few || wary || !known || (entry & kCareful) != 0;
+      const bool strict = (entry & kStrict) != 0;
+      const bool careful = few || wary || !known || strict || (entry & kCareful) != 0;
       const int nb = (w.i_len + kBlk - 1) / kBlk;
       // tile row r -> (query row of the tile, head)
       const int rq = p.stack == 1 ? r : r / p.stack;
@@ -543,7 +565,7 @@ varlen_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_const
           ++pair_cnt;
           mx = fmaxf(mx, sm.xmax[g & 1][half ^ 1][r]);
           // (c > 0; the exponent of the largest score in the arithmetic of the exponents, so that it is the largest of them)
-          resc = fmaf(mx, c, -m_ref) > kStay<T> + 0.5f;
+          resc = fmaf(mx, c, -m_ref) > (strict ? kRescaleThreshold : kStay<T> + 0.5f);
           const float m_new = resc ? mx * c : m_ref;
           alpha = resc ? ex2(m_ref - m_new) : 1.f;
           m_use = (m_new == -INFINITY) ? 0.f : m_new;
@@ -604,6 +626,16 @@ varlen_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_const
 
       // ---- epilogue ----
       float l_tot = 0.f;
+      constexpr bool kBf16 = std::is_same<T, __nv_bfloat16>::value;
+      bool check_o = false;
+      uint64_t not_finite = 0ull;  // a pair of zeros, NaN once a value of O is not finite
+      auto look = [&](const uint32_t (&t)[32]) {
+        if (kBf16 && check_o) {
+#pragma unroll
+          for (int i = 0; i < 16; ++i)
+            not_finite = fma_f2(pack_f2(__uint_as_float(t[2 * i]), __uint_as_float(t[2 * i + 1])), 0ull, not_finite);
+        }
+      };
       if (!live) {
         // (the wait keeps this warp within one phase of the barrier)
         if (nb > 0 && !mbar_wait(smem_u32(&sm.o_done[(gk - 1) % S]), ((gk - 1) / S) & 1, abort_flag)) break;
@@ -615,7 +647,9 @@ varlen_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_const
         if (isnan(t_max)) l = t_max;
         const bool left = row_ok && nb > 1 && (no_ref || moved || worst > kStayPart<T> || t_max > kStay<T>);
         const bool near = row_ok && (worst > kNearPart<T> || t_max > kNear<T>);
-        int flags = (__any_sync(0xffffffffu, left) ? 1 : 0) | (__any_sync(0xffffffffu, near) ? 2 : 0);
+        const bool large = kBf16 && row_ok && !strict && worst > kLargePart;
+        int flags = (__any_sync(0xffffffffu, left) ? 1 : 0) | (__any_sync(0xffffffffu, near) ? 2 : 0) |
+                    (__any_sync(0xffffffffu, large) ? 4 : 0);
         if (lane == 0) {
           if (*(volatile int*)&sm.n_redo > 0) flags |= 2;
           sm.xflag[half][warp & 3] = flags;
@@ -626,10 +660,12 @@ varlen_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_const
         ++pair_cnt;
         l_tot = l + sm.xsum[half ^ 1][r];
         flags = sm.xflag[0][warp & 3] | sm.xflag[1][warp & 3];
-        wary = wary || flags != 0;
+        wary = wary || (flags & 3) != 0;
         known = known || nb > 1;
         // (what is written below is overwritten when the item is done again)
-        if ((flags & 1) && !careful && half == 0 && lane == 0) ((volatile int*)sm.redo)[atomicAdd(&sm.n_redo, 1)] = idx | kCareful;
+        const bool failed = (flags & 1) != 0 && !careful;
+        if (failed && half == 0 && lane == 0) again(idx | kCareful);
+        check_o = kBf16 && !failed && (flags & 4) != 0;
       }
       const bool dead = (nb == 0) || (l_tot == 0.f);  // a NaN row sum is not a dead row: it goes out as NaN
       const float inv_l = dead ? 0.f : 1.f / l_tot;
@@ -650,6 +686,7 @@ varlen_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_const
 #pragma unroll
             for (int i = 0; i < 32; ++i) t[i] = 0u;
           }
+          look(t);
           uint32_t pw[16];
 #pragma unroll
           for (int i = 0; i < 16; ++i)
@@ -671,6 +708,7 @@ varlen_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_const
 #pragma unroll
             for (int i = 0; i < 32; ++i) t[i] = 0u;
           }
+          look(t);
           if (row_ok) {
             float4* dst = reinterpret_cast<float4*>(optr + cc * 32);
 #pragma unroll
@@ -685,6 +723,11 @@ varlen_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_const
           }
         }
         if (row_ok && half == 0) p.partial_lse[prow * p.H + h] = lse_val;
+      }
+      if (kBf16 && check_o) {
+        float a, b;
+        unpack_f2(not_finite, a, b);
+        if (__any_sync(0xffffffffu, row_ok && isnan(a + b) && !isnan(l_tot)) && lane == 0) again(idx | kStrict);
       }
       // the TMEM reads of O above finish (tcgen05.wait::ld) before this thread's next p_full arrival,
       // and the next item's first P.V, which overwrites O, is issued only after that arrival
