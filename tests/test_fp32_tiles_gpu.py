@@ -64,3 +64,36 @@ def test_rows_that_are_not_seen_may_hold_anything():
     o1, dq1 = run(k2, v2)
     for a, b in ((o0, o1), (dq0, dq1)):
         assert torch.equal(a[:60], b[:60]) and torch.equal(a[70:], b[70:])
+
+
+@pytest.mark.parametrize("dtype,D", [(torch.float32, 32), (torch.float32, 64), (torch.float32, 256), (torch.bfloat16, 32), (torch.float16, 256)])
+@pytest.mark.parametrize("Lk", [40, 900])  # one CTA of a cluster, several
+@pytest.mark.parametrize("where", ["q nan", "k nan", "k inf"])
+def test_a_visible_nan_or_infinity_does_not_vanish(dtype, D, Lk, where):
+    """It reaches the rows that see it in O, LSE and dQ, and no others."""
+    H = 2
+    q, k, v, do, cu_q, cu_k = make_varlen_inputs([16, 20], [Lk, 30], H, D, dtype, 8)
+    if where == "q nan":
+        q[5, 1, 3] = float("nan")
+        rows = [5]
+    else:
+        q[..., 3] = 1.0
+        k[Lk - 3, 1, 3] = float(where[2:])
+        rows = list(range(16))
+    g = [t.to(DEV).requires_grad_(True) for t in (q, k, v)]
+    o, lse = vb.packed_varlen_attn_with_lse(*g, cu_seqlens_q=cu_q, cu_seqlens_k=cu_k)
+    o.backward(do.to(DEV))
+    hit = torch.zeros(36, H, dtype=torch.bool, device=DEV)
+    hit[rows, 1] = True
+    for t in (o, g[0].grad):
+        assert torch.isnan(t[hit].float()).all() and torch.isfinite(t[~hit].float()).all()
+    assert torch.isnan(lse[hit]).all() and torch.isfinite(lse[~hit]).all()
+
+
+def test_a_visible_nan_does_not_vanish_absorb():
+    ins = make_absorb_inputs([16, 3], [700, 64], 72, 130, 4, 32, torch.float32, 9, x_std=0.1, w_std=0.1)
+    q_raw, X, W_Q, W_K, W_V, _, cu_q, cu_k = ins
+    X[690, 7] = float("nan")
+    with torch.no_grad():
+        O = vb.packed_target_attn(*(t.to(DEV) for t in (q_raw, X, W_Q, W_K, W_V)), cu_seqlens_q=cu_q, cu_seqlens_k=cu_k)
+    assert torch.isnan(O[:16]).all() and torch.isfinite(O[16:]).all()

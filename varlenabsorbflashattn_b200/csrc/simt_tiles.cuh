@@ -437,7 +437,7 @@ __global__ void __launch_bounds__(kThreads) tile_fwd_kernel(const TileParams p) 
     } else {
       st_f[r] = 1.f;
     }
-    const bool dead = !(lt > 0.f);
+    const bool dead = lt == 0.f;  // a NaN row sum is not a dead row: it goes out as NaN
     st_d[r] = dead ? 0.f : 1.f / lt;
     if (t.rank == 0 && r < rows)
       p.lse[p.stack > 1 ? row0 + r : (row0 + r) * p.H + t.h] = dead ? -INFINITY : mt + log2f(lt);
