@@ -37,6 +37,20 @@ def test_abi_version(lib):
     assert lib.vafa_abi_version() == 3
 
 
+@pytest.mark.parametrize("version,missing", [(2, ()), (3, ("vafa_check_cu_seqlens",))])
+def test_a_library_that_does_not_fit_is_named(lib, monkeypatch, version, missing):
+    """Another ABI version, or this one from before a function was added: an error that says to rebuild."""
+    class Old:
+        def __init__(self, path):
+            for n in set(_lib.EXPORTS) - set(missing):
+                setattr(self, n, lambda: version)
+
+    monkeypatch.setattr(_lib, "_lib", None)
+    monkeypatch.setattr(_lib.C, "CDLL", Old)
+    with pytest.raises(RuntimeError, match="ABI version mismatch.*" + "".join(missing) + ".*rebuild"):
+        _lib.load()
+
+
 def test_struct_sizes_match_header():
     # 11 pointers + 7 int32 + float + 3 int32 (+pad) + pointer + size_t + pointer + num_kv_heads (int32, padded to 8)
     assert C.sizeof(_lib.VarlenArgs) == 11 * 8 + 12 * 4 + 3 * 8 + 8

@@ -23,6 +23,7 @@ STATUS_WORDS = 4
 
 DTYPE_CODE = {torch.float32: VAFA_F32, torch.bfloat16: VAFA_BF16, torch.float16: VAFA_F16}
 
+ABI_VERSION = 3
 EXPORTS = (
     "vafa_abi_version", "vafa_last_error", "vafa_check_status", "vafa_cast_from_f32", "vafa_check_cu_seqlens",
     "vafa_varlen_fwd_workspace_bytes", "vafa_varlen_bwd_workspace_bytes", "vafa_varlen_fwd", "vafa_varlen_bwd",
@@ -78,6 +79,11 @@ def load() -> C.CDLL:
                 f"{LIB_PATH} is missing: build it with `python -m varlenabsorbflashattn_b200.build` "
                 "(there is no fallback implementation)")
         lib = C.CDLL(LIB_PATH)
+        # a library of another version, or one built before a function was added to this one
+        missing = [n for n in EXPORTS if not hasattr(lib, n)]
+        if missing or lib.vafa_abi_version() != ABI_VERSION:
+            raise RuntimeError("libvafa_b200.so: ABI version mismatch"
+                               + (f" (no {', '.join(missing)})" if missing else "") + "; rebuild")
         lib.vafa_abi_version.restype = C.c_int
         lib.vafa_last_error.restype = C.c_char_p
         lib.vafa_check_status.argtypes = [C.c_void_p, C.c_void_p]
@@ -111,8 +117,6 @@ def load() -> C.CDLL:
         lib.vafa_profile_kernel_name.restype = C.c_char_p
         lib.vafa_profile_read.argtypes = [C.c_int, C.POINTER(C.c_double), C.POINTER(C.c_longlong),
                                           C.POINTER(C.c_longlong)]
-        if lib.vafa_abi_version() != 3:
-            raise RuntimeError("libvafa_b200.so: ABI version mismatch; rebuild")
         _lib = lib
     return _lib
 
