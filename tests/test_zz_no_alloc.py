@@ -115,3 +115,19 @@ def test_noalloc_rejects_oversized_batches_and_unsupported_shapes():
     cu4 = torch.tensor([0, 4], dtype=torch.int32, device=dev)
     b = _args(q32, q32, q32, torch.empty_like(q32), lse[:4], cu4, cu4, False)
     assert lib.vafa_varlen_fwd_noalloc(C.byref(b), torch.cuda.current_stream(dev).cuda_stream) == -2
+
+
+def test_noalloc_takes_every_list_of_whole_tiles_that_fits():
+    """One head, 346 490 segments of one query and one key: 32 B of item and 16 B of combine unit for each of 349 197
+    possible tiles are 21 KB short of the built-in array, which leaves little room for slices and none for partials."""
+    lib = _lib.load()
+    dev = torch.device("cuda", 0)
+    n_seg = 346_490
+    assert 0 < (16 << 20) - 48 * (n_seg + n_seg // 128 + 1) < 21_000
+    cu = torch.arange(n_seg + 1, dtype=torch.int32, device=dev)
+    q, v = (torch.randn(n_seg, 1, 64, device=dev).to(torch.bfloat16) for _ in range(2))
+    o, lse = torch.empty_like(q), torch.empty(n_seg, 1, dtype=torch.float32, device=dev)
+    a = _args(q, q, v, o, lse, cu, cu, False)
+    _lib.check(lib.vafa_varlen_fwd_noalloc(C.byref(a), torch.cuda.current_stream(dev).cuda_stream), "vafa_varlen_fwd_noalloc")
+    _lib.check_status(dev)
+    assert torch.equal(o, v)                           # one key: its value

@@ -1297,7 +1297,7 @@ struct FwdWorkspace {
   SchedCaps caps;
 };
 
-// `limit` > 0 shrinks the split-K partial area so that the whole layout fits in `limit` bytes
+// `limit` > 0 shrinks the split-K partial area and the room for slices in the item list so that the whole layout fits in `limit` bytes
 // (the scheduler then splits less, or not at all); total > limit afterwards means it cannot fit.
 FwdWorkspace fwd_workspace(const vafa_varlen_args* a, int sm_count, size_t limit = 0) {
   FwdWorkspace w;
@@ -1306,8 +1306,15 @@ FwdWorkspace fwd_workspace(const vafa_varlen_args* a, int sm_count, size_t limit
                       kTile / stack);
   w.header = 0;
   w.items = 256;
+  const size_t combine_bytes = align_up((size_t)w.caps.cap_combine * sizeof(CombineUnit), 256);
+  if (limit > 0) {
+    // a list of whole tiles (cap_combine per head or stack) is all that has to fit; items for slices are what is left
+    const size_t whole = (size_t)w.caps.cap_combine * (a->num_heads / stack), lists = w.items + combine_bytes + 256;
+    const size_t room = limit > lists ? (limit - lists) / sizeof(WorkItem) : 0;
+    if (room < (size_t)w.caps.cap_items) w.caps.cap_items = (int32_t)(room > whole ? room : whole);
+  }
   w.combine = w.items + align_up((size_t)w.caps.cap_items * sizeof(WorkItem), 256);
-  w.plse = w.combine + align_up((size_t)w.caps.cap_combine * sizeof(CombineUnit), 256);
+  w.plse = w.combine + combine_bytes;
   if (limit > 0) {
     const size_t per_row = (size_t)a->num_heads * (a->head_dim + 1) * 4;
     const size_t room = limit > w.plse + 1024 ? limit - w.plse - 1024 : 0;
