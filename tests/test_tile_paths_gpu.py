@@ -52,10 +52,10 @@ def test_long_segments_are_cut(ql, kl, H):
 
 @pytest.mark.parametrize("ql,kl,H", [
     ([16], [5000], 8),                                      # one user, one full tile
-    ([1, 16, 17, 0, 3], [700, 2048, 2047, 5, 0], 8),        # cut and uncut tiles, a second tile of one query
+    ([1, 16, 17, 0, 3], [700, 2048, 2047, 5, 0], 8),        # a second tile of one query
     ([5, 40], [3000, 97], 4), ([3] * 24, [8] * 23 + [2048], 8)])
-def test_few_users_with_long_histories_are_cut(ql, kl, H):
-    """Absorb: up to four tiles per SM the histories are cut and the parts merged (also read by the backward)."""
+def test_few_users_with_long_histories(ql, kl, H):
+    """Absorb: fewer tiles than SMs, histories of many blocks and of one, a tile of one query."""
     ql = [a if b else 0 for a, b in zip(ql, kl)]
     ins = make_absorb_inputs(ql, kl, 256, 256, H, 256 // H, torch.bfloat16, 14, x_std=0.3, w_std=0.1)
     q_raw, X, W_Q, W_K, W_V, dO, cu_q, cu_k = ins

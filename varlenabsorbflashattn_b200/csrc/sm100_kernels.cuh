@@ -56,7 +56,7 @@ struct AbsorbCoreArgs {
   int x_width;
   int lists_built;     // the tile list was already built by sm100_absorb_core_fwd_lists() (ordered before this call)
 };
-size_t sm100_absorb_core_fwd_workspace_bytes(int total_q, int total_k, int n_seg, int H, int sm_count);
+size_t sm100_absorb_core_fwd_workspace_bytes(int total_q, int n_seg, int H);
 int sm100_absorb_core_fwd(const AbsorbCoreArgs& a, cudaStream_t s);
 
 // Backward of the attention core: dU [T_q,H,256] (scaled) and dX [T_k,256] from u, X, dAlphaX

@@ -1200,7 +1200,7 @@ __global__ void __launch_bounds__(256) varlen_combine_kernel(const SchedHeader* 
                                                              const float* __restrict__ partial_o,
                                                              const float* __restrict__ partial_lse, T* __restrict__ o,
                                                              float* __restrict__ lse, int H, int chunks) {
-  constexpr int V = D / 32;  // floats per lane: 8 (D=256), 4 (D=128) or 2 (D=64)
+  constexpr int V = D / 32;  // floats per lane: 4 (D=128) or 2 (D=64)
   constexpr int kUnroll = 4;
   const int n_work = header->n_combine * chunks;
   const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
@@ -1228,12 +1228,9 @@ __global__ void __launch_bounds__(256) varlen_combine_kernel(const SchedHeader* 
         const long long e = first + (ok ? s0 + t : s0) * step;
         wgt[t] = ok ? partial_lse[e] : -INFINITY;
         const float* src = partial_o + e * D + lane * V;
-        if constexpr (V >= 4) {
-#pragma unroll
-          for (int j = 0; j < V; j += 4) {
-            const float4 x = *reinterpret_cast<const float4*>(src + j);
-            f[t][j] = x.x; f[t][j + 1] = x.y; f[t][j + 2] = x.z; f[t][j + 3] = x.w;
-          }
+        if constexpr (V == 4) {
+          const float4 x = *reinterpret_cast<const float4*>(src);
+          f[t][0] = x.x; f[t][1] = x.y; f[t][2] = x.z; f[t][3] = x.w;
         } else {
           const float2 x = *reinterpret_cast<const float2*>(src);
           f[t][0] = x.x; f[t][1] = x.y;
@@ -1251,14 +1248,11 @@ __global__ void __launch_bounds__(256) varlen_combine_kernel(const SchedHeader* 
     const float inv = den == 0.f ? 0.f : 1.f / den;  // a NaN weight sum goes out as NaN
     const long long row = (long long)cu.q_start + r;
     T* dst = o + (row * H + h) * D + lane * V;
-    if constexpr (V >= 4) {
-#pragma unroll
-      for (int j = 0; j < V; j += 4) {
-        uint2 pk;
-        pk.x = pack2_out<T>(acc[j] * inv, acc[j + 1] * inv);
-        pk.y = pack2_out<T>(acc[j + 2] * inv, acc[j + 3] * inv);
-        *reinterpret_cast<uint2*>(dst + j) = pk;
-      }
+    if constexpr (V == 4) {
+      uint2 pk;
+      pk.x = pack2_out<T>(acc[0] * inv, acc[1] * inv);
+      pk.y = pack2_out<T>(acc[2] * inv, acc[3] * inv);
+      *reinterpret_cast<uint2*>(dst) = pk;
     } else {
       *reinterpret_cast<uint32_t*>(dst) = pack2_out<T>(acc[0] * inv, acc[1] * inv);
     }
@@ -1410,48 +1404,32 @@ int launch_fwd(const vafa_varlen_args* a, cudaStream_t s, void* scratch = nullpt
 }
 
 struct AbsorbCoreWs {
-  size_t header, items, combine, plse, po, total;
+  size_t header, items, total;
   SchedCaps caps;
-  bool split;
 };
 
-// A request batch of a few users is as slow as its longest history: with at most four tiles per SM the histories are
-// cut (see split_blocks) and the parts merged by the combine kernel.  Measured, 32 users of 8-2048 keys: 34 us in one
-// pass, 23 + 5 us cut and merged.
-// Larger batches fill the chip with whole users and keep their one pass; the mean is all the host knows.
-AbsorbCoreWs absorb_core_ws(int total_q, int total_k, int n_seg, int H, int sms) {
+AbsorbCoreWs absorb_core_ws(int total_q, int n_seg, int H) {
   AbsorbCoreWs w;
   const int tile_rows = kTile / H;
-  const long long units = (long long)total_q / tile_rows + n_seg;
-  w.split = units <= 4LL * sms;
   w.caps.cap_items = total_q / tile_rows + n_seg + 1;
   w.caps.cap_combine = 0;
   w.caps.cap_rows = 0;
-  if (w.split) {
-    w.caps = sched_caps(kSchedFwd, total_q, total_k, n_seg, 1, sms, 0, tile_rows);
-    // (a partial row is H x 256 floats; a list that needs more than this is cut into longer slices)
-    const int most = 2 * sms * tile_rows;
-    if (w.caps.cap_rows > most) w.caps.cap_rows = most;
-  }
   w.header = 0;
   w.items = 256;
-  w.combine = w.items + align_up((size_t)w.caps.cap_items * sizeof(WorkItem), 256);
-  w.plse = w.combine + align_up((size_t)w.caps.cap_combine * sizeof(CombineUnit), 256);
-  w.po = w.plse + align_up((size_t)w.caps.cap_rows * H * 4, 256);
-  w.total = w.po + align_up((size_t)w.caps.cap_rows * H * 256 * 4, 256);
+  w.total = w.items + align_up((size_t)w.caps.cap_items * sizeof(WorkItem), 256);
   return w;
 }
 
 SchedParams absorb_fwd_sched_params(const AbsorbCoreArgs& a, int sms) {
-  const AbsorbCoreWs ws = absorb_core_ws(a.total_q, a.total_k, a.n_seg, a.H, sms);
+  const AbsorbCoreWs ws = absorb_core_ws(a.total_q, a.n_seg, a.H);
   char* base = (char*)a.workspace;
   SchedParams sp;
-  sp.cu_q = a.cu_q; sp.cu_k = a.cu_k; sp.n_seg = a.n_seg; sp.mode = ws.split ? kSchedFwd : kSchedDq;  // dQ mode: no split-K
+  sp.cu_q = a.cu_q; sp.cu_k = a.cu_k; sp.n_seg = a.n_seg; sp.mode = kSchedDq;  // no split-K
   sp.causal = 0; sp.H = 1; sp.sm_count = sms; sp.split_len = 0; sp.tile_rows = kTile / a.H;
-  sp.cap_items = ws.caps.cap_items; sp.cap_combine = ws.caps.cap_combine; sp.cap_rows = ws.caps.cap_rows;
+  sp.cap_items = ws.caps.cap_items; sp.cap_combine = 0; sp.cap_rows = 0;
   sp.header = (SchedHeader*)(base + ws.header);
   sp.items = (WorkItem*)(base + ws.items);
-  sp.combine = (CombineUnit*)(base + ws.combine);
+  sp.combine = nullptr;
   return sp;
 }
 
@@ -1467,10 +1445,7 @@ int launch_absorb_core_fwd(const AbsorbCoreArgs& a, cudaStream_t s) {
   if ((rc = encode_tmap_rows(&tx, a.x, a.dtype, a.total_k, 1, a.x_width, fwd_block_keys<true>()))) return rc;
   FwdParams p;
   p.wait_limit = wait_limit_units();
-  const AbsorbCoreWs ws = absorb_core_ws(a.total_q, a.total_k, a.n_seg, a.H, sms);
-  p.o = a.axn; p.lse = a.lse;
-  p.partial_lse = (float*)((char*)a.workspace + ws.plse);
-  p.partial_o = (float*)((char*)a.workspace + ws.po);
+  p.o = a.axn; p.lse = a.lse; p.partial_o = nullptr; p.partial_lse = nullptr;
   p.header = sp.header; p.items = sp.items; p.H = a.H;
   p.group = 1;
   p.stack = a.H;
@@ -1493,26 +1468,15 @@ int launch_absorb_core_fwd(const AbsorbCoreArgs& a, cudaStream_t s) {
 #endif
   const size_t smem = sizeof(FwdSmem<D, true>) + 1024;
   VAFA_CUDA_CHECK(cudaFuncSetAttribute(varlen_fwd_kernel<T, D, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  {
-    LaunchScope scope(kKAbsorbFwd, s);
-    varlen_fwd_kernel<T, D, true><<<sms, kFwdThreads, smem, s>>>(tu, tx, tx, tup, p);
-  }
+  LaunchScope scope(kKAbsorbFwd, s);
+  varlen_fwd_kernel<T, D, true><<<sms, kFwdThreads, smem, s>>>(tu, tx, tx, tup, p);
   VAFA_LAUNCH_CHECK("varlen_fwd_kernel<absorb>");
-  if (ws.split) {
-    LaunchScope scope(kKCombine, s);
-    const int unit_rows = sp.tile_rows < a.total_q ? sp.tile_rows : a.total_q;
-    varlen_combine_kernel<T, D><<<4 * sms, 256, 0, s>>>(sp.header, sp.combine, p.partial_o, p.partial_lse, (T*)a.axn, a.lse, a.H,
-                                                        (unit_rows * a.H + 7) / 8);
-    VAFA_LAUNCH_CHECK("varlen_combine_kernel");
-  }
   return 0;
 }
 
 }  // namespace
 
-size_t sm100_absorb_core_fwd_workspace_bytes(int total_q, int total_k, int n_seg, int H, int sm_count) {
-  return absorb_core_ws(total_q, total_k, n_seg, H, resolve_sm_count(sm_count)).total;
-}
+size_t sm100_absorb_core_fwd_workspace_bytes(int total_q, int n_seg, int H) { return absorb_core_ws(total_q, n_seg, H).total; }
 
 int sm100_absorb_core_fwd_lists(const AbsorbCoreArgs& a, cudaStream_t s) {
   return launch_scheduler(absorb_fwd_sched_params(a, resolve_sm_count(a.sm_count)), s);

@@ -245,7 +245,7 @@ size_t absorb_fwd_ws_bytes(const vafa_absorb_args* a, bool inner) {
   const AbsorbFast f = absorb_fast(a, inner);
   size_t n = 0;
   if (f.prologue) n += align_up((size_t)a->d_q * a->num_heads * a->d_kv * elem_size(a->dtype), 256);
-  if (f.core) n += sm100_absorb_core_fwd_workspace_bytes(a->total_q, a->total_k, a->n_seg, a->num_heads, a->sm_count);
+  if (f.core) n += sm100_absorb_core_fwd_workspace_bytes(a->total_q, a->n_seg, a->num_heads);
   return n;
 }
 
