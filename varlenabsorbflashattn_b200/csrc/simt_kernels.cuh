@@ -32,9 +32,14 @@ int simt_attn_dq(const SimtAttnParams& p, cudaStream_t s);
 int simt_attn_dkv(const SimtAttnParams& p, cudaStream_t s);
 
 // The tiled kernels (simt_tiles.cu): whether they take this call, and their launches.  A tile has 64 outer rows, of
-// which a warp owns eight; below kTileMinRows (stacked) query rows or keys per segment on average most of a
-// tile would be padding and the one-warp-per-row kernels stay.
+// which a warp owns eight, and walks blocks of 32 or 64 inner rows; below eight (stacked) query rows or keys per segment on
+// average most of a tile is padding, and a segment of few rows by few keys does not pay for the tile's loads.
+// Measured, one warp per row | tiles (us), forward of 512 segments, fp32, 8 heads of 128, query rows x keys each: 8x8
+// 94 | 199, 8x16 226 | 249, 12x12 264 | 254; 1 head: 8x16 27 | 37, 16x8 29 | 35, 8x32 44 | 40, 16x16 46 | 38,
+// 32x8 49 | 38; backward 8x8 56 | 95, 16x8 83 | 99, 8x16 87 | 97, 16x16 132 | 103.  1024 users of one target (8 stacked rows), 16
+// keys each: 71 | 108, of 4 targets, 16 keys: 249 | 185.  Hence the line at 256 scores a segment.
 constexpr int kTileMinRows = 8;
+constexpr double kTileMinScores = 256.;
 bool simt_tiles_ok(const SimtAttnParams& p);
 int simt_tiles_fwd(const SimtAttnParams& p, cudaStream_t s);
 int simt_tiles_dq(const SimtAttnParams& p, cudaStream_t s);

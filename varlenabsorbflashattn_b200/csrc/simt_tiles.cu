@@ -10,7 +10,9 @@ bool simt_tiles_ok(const SimtAttnParams& a) {
   if (a.shared_kv && (a.q_row != a.H * a.q_head || a.do_row != a.H * a.do_head || a.causal || !a.do_f32)) return false;
   if (!a.shared_kv && a.do_f32) return false;
   const int stack = a.shared_kv ? a.H : 1;
-  if ((long long)a.total_q * stack < (long long)kTileMinRows * a.n_seg || a.total_k < (long long)kTileMinRows * a.n_seg) return false;
+  const long long rows = (long long)a.total_q * stack;
+  if (rows < (long long)kTileMinRows * a.n_seg || a.total_k < (long long)kTileMinRows * a.n_seg) return false;
+  if ((double)rows * a.total_k < kTileMinScores * a.n_seg * a.n_seg) return false;
   const long long heads = a.shared_kv ? 1 : a.H;
   return max_slots(a.total_q, stack, a.n_seg) * heads < (1LL << 31) / kMaxSplits &&
          max_slots(a.total_k, 1, a.n_seg) * heads < (1LL << 31) / kMaxSplits;
