@@ -17,7 +17,8 @@ DEV = "cuda"
     ([64, 65, 63, 1, 0, 129], [64, 63, 65, 33, 7, 0]),
     ([100, 8, 31], [1000, 513, 32]),           # several ranks of a cluster per tile
     ([300], [20]),                             # more queries than keys: causal rows without a key
-    ([8] * 40, [31] * 40), ([8] * 40, [32] * 40), ([16] * 9, [15] * 9), ([16] * 9, [16] * 9)])  # either side of the line
+    ([8] * 40, [31] * 40), ([8] * 40, [32] * 40), ([16] * 9, [15] * 9), ([16] * 9, [16] * 9),  # either side of the line
+    ([20] * 3, [127] * 3), ([20] * 3, [128] * 3), ([20] * 3, [320] * 3)])  # one rank, two, eight
 def test_varlen_fp32(D, causal, ql, kl):
     q, k, v, do, cu_q, cu_k = make_varlen_inputs(ql, kl, 3, D, torch.float32, 5)
     g = [t.to(DEV).requires_grad_(True) for t in (q, k, v)]

@@ -695,12 +695,16 @@ inline int vec4(const void* p, int64_t row, int64_t head, int D, int es) {
 inline long long max_slots(long long tokens, int stack, int n_seg) { return tokens * stack / kRows + n_seg; }
 
 // Cluster size: CTAs that share an outer tile.  The lengths are not known here, only their mean, and the longest
-// segment decides the time of a ragged batch, so the tile is shared as far as the mean segment has an inner block
-// of 64 rows for each rank, until the grid holds eight tiles per SM.
+// segment decides the time of a ragged batch, so the tile is shared while the mean segment has inner blocks of
+// 64 rows for more than the ranks so far, until the grid holds eight tiles per SM.  With no more blocks than ranks
+// the new ranks of most tiles return at once, and each costs a launch slot with the tile's shared memory: forward of
+// users of one target, fp32, one rank more from as many blocks as ranks | from one more: 1024 users x 64 keys 267 | 153 us, 512 x 64
+// 126 | 81, 1024 x 96 339 | 241; 64 users x 8 targets x 370 keys 128 | 130.
+// (A grid of less than two CTAs per SM has room for them, and the segments above the mean use them.)
 inline int pick_splits(long long tiles, long long inner_rows, int n_seg) {
   const long long mean = inner_rows / n_seg, sms = sm_count();
   int n = 1;
-  while (n < kMaxSplits && tiles * n < 8 * sms && mean >= 64 * n) n *= 2;
+  while (n < kMaxSplits && tiles * n < 8 * sms && mean >= 64 * (tiles * n < 2 * sms ? n : n + 1)) n *= 2;
   return n;
 }
 
