@@ -92,7 +92,8 @@ def test_scores_that_climb_past_the_first_block(dtype, D, n_seg, H, climb):
     assert torch.isfinite(o).all()
 
 
-def test_nan_and_infinite_scores_behind_the_first_block():
+@pytest.mark.parametrize("bad", [float("nan"), float("inf")])
+def test_nan_and_infinite_scores_behind_the_first_block(bad):
     """Only the rows that see the bad key are touched by it."""
     L, H, D = 400, 2, 64
     q, k, v, _, cu_q, cu_k = make_varlen_inputs([L, L], [L, L], H, D, torch.bfloat16, 22, with_do=False)
@@ -103,8 +104,8 @@ def test_nan_and_infinite_scores_behind_the_first_block():
 
     o0 = run(k)
     k2 = k.clone()
-    k2[300] = float("nan")
+    k2[300] = bad
     o1 = run(k2)
-    # the rest of the tile is done again the careful way: equal up to the rounding of P and O (2^-8 each)
+    # (with an infinite score the rest of the tile is done again: equal at least up to the rounding of P and O, 2^-8 each)
     assert (o1[:300] - o0[:300]).abs().max() <= 2e-2 and torch.equal(o1[L:], o0[L:])
     assert torch.isnan(o1[300:L].float()).any(dim=-1).all()

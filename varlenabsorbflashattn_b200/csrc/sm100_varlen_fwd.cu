@@ -5,13 +5,14 @@
 //   warps 0-7  softmax + epilogue: two threads per query row of the 128-row tile (TMEM lane = row),
 //              each owning half of the score and output columns
 //   warp 8     TMA producer (one lane): Q tile once per item, K and V tiles through a ring
-//   warp 9     tcgen05.mma issuer (one lane) and TMEM owner
+//   warp 9     tcgen05.mma issuer (the converged warp, one elected lane issues) and TMEM owner
 // TMEM (512 columns): S0 [0,128), S1 [128,256) fp32 scores, double buffered; the 16-bit
 // probabilities P overwrite the first 64 columns of their S buffer; O accumulator at [256,256+D).
 //
-// Per KV block g:  S[g&1] = Q K_g^T  ->  softmax warps read S, write P, rescale O when the
-// running maximum moved by more than 2^8  ->  O += P V_g.  S for block g+1 is issued before
-// block g's P is ready, so the tensor pipe works on the next scores while the softmax runs.
+// Per KV block g:  S[g&1] = Q K_g^T  ->  softmax warps read S, write P (against the maximum of the item's first
+// block, or, where that may not do, a maximum that follows and an O that is rescaled: see kStay)  ->  O += P V_g.
+// S for block g+1 is issued before block g's P is ready, so the tensor pipe works on the next scores while the
+// softmax runs.
 //
 // Numerics follow the reference kernels (triton_fa_varlen_v2/triton_fa_varlen_v2/kernels.py:
 // 127-166): scores scaled by scale*log2(e) in fp32 after the dot, exp2-domain online softmax,
@@ -199,12 +200,12 @@ varlen_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_const
   const int warp = (int)warp_uniform(threadIdx.x >> 5), lane = threadIdx.x & 31;
   volatile int* abort_flag = &sm.abort_flag;
 
+  for (int i = threadIdx.x; i < kRedoCap; i += kFwdThreads) sm.redo[i] = -1;
   if (threadIdx.x == 0) {
     sm.abort_flag = 0;
     sm.wait_limit = p.wait_limit;
     wq_init(sm.wq, 9);
     sm.n_redo = 0;
-    for (int i = 0; i < kRedoCap; ++i) sm.redo[i] = -1;
     mbar_init(smem_u32(&sm.drain), 8);
     for (int i = 0; i < 4; ++i) mbar_init(smem_u32(&sm.pair_bar[i]), 64);
     mbar_init(smem_u32(&sm.q_full), 1);
@@ -436,8 +437,9 @@ varlen_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_const
     // ---------------- softmax + epilogue (warps 0-7) ----------------
     // Two threads per tile row: thread (r, half) owns score columns [64*half, 64*half+64) of every
     // block and output columns [D/2*half, D/2*(half+1)).  The two halves of a row sit in warps w and
-    // w+4 (same TMEM lane quadrant) and exchange their partial row maximum through shared memory;
-    // two warps per scheduler also give the exp2-heavy loop a second instruction stream to overlap.
+    // w+4 (same TMEM lane quadrant) and exchange their partial row maximum, in blocks that take one, and their
+    // row sums through shared memory; two warps per scheduler also give the exp2-heavy loop a second
+    // instruction stream to overlap.
     const int r = threadIdx.x & 127;
     const int half = threadIdx.x >> 7;
     const uint32_t pair_bar = smem_u32(&sm.pair_bar[warp & 3]);
@@ -765,10 +767,10 @@ varlen_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_const
 // block (TMEM round trips, barriers) is paid once per 128 scores of a thread instead of once per 64.
 // Under the causal mask tile A ends one block before tile B; barriers of a tile are indexed by the tile's own
 // block count.
-// Opt-in (environment variable VAFA_FWD_PAIR=1, read once per process): measured on a B200 it is 4 % faster than
-// the one-tile kernel above on long non-causal segments (8 x 8192: 4.40 against 4.60 ms), 6-14 % slower on
-// causal batches (tile A idles through tile B's last block of every item) and on batches of short segments
-// (half as many items, so the scheduler splits keys more often), and level on the 500-query production shapes.
+// Opt-in (environment variable VAFA_FWD_PAIR=1, read once per process).  Its issuer still runs in one lane and it takes
+// the maximum of every block; measured on a B200 against the one-tile kernel above, which does neither any more: 8 x 8192
+// non-causal 4.31 against 3.74 ms, 37 causal sequences (62 k tokens, 32 heads) 3.51 against 3.22, 64 causal sequences (16
+// heads) 0.65 against 0.52, 500-query histories (4 heads of 64) 0.41 against 0.37.
 template <int D>
 struct PairSmem {
   alignas(1024) uint8_t q[2][FwdCfg<D>::kTileBytes];
