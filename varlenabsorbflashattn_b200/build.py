@@ -52,7 +52,7 @@ def _digest() -> str:
 
 
 def _extra_flags() -> list[str]:
-    """Additional nvcc flags from VAFA_NVCC_FLAGS (e.g. -DVAFA_BWD_EW_WARPS=16), for experiments."""
+    """Additional nvcc flags from VAFA_NVCC_FLAGS (e.g. -DVAFA_FWD_POLY_PERIOD=3), for experiments."""
     return os.environ.get("VAFA_NVCC_FLAGS", "").split()
 
 

@@ -29,6 +29,7 @@ constexpr int kWqSlots = 4;
 struct WorkQueue {
   uint64_t full[kWqSlots], empty[kWqSlots];
   int idx[kWqSlots];
+  WorkItem item[kWqSlots];  // (kernels that publish the item itself: its load from global memory is paid once, ahead of time)
 };
 
 // consumers = number of arrivals per slot: one per consuming warp (or single consuming thread)
@@ -56,6 +57,32 @@ __device__ __forceinline__ int wq_consume_warp(WorkQueue& q, uint32_t n, volatil
   const int slot = n % kWqSlots;
   if (!ptx::mbar_wait(ptx::smem_u32(&q.full[slot]), (n / kWqSlots) & 1, abort_flag)) return -1;
   const int idx = q.idx[slot];
+  __syncwarp();
+  if ((threadIdx.x & 31) == 0) ptx::mbar_arrive(ptx::smem_u32(&q.empty[slot]));
+  return idx;
+}
+
+// The same with the item: the producer reads it and publishes it beside its index, so that no consumer waits for global
+// memory between two items.
+__device__ __forceinline__ void wq_publish_item(WorkQueue& q, uint32_t n, int idx, const WorkItem& w) {
+  const int slot = n % kWqSlots;
+  q.idx[slot] = idx;
+  q.item[slot] = w;
+  ptx::mbar_arrive(ptx::smem_u32(&q.full[slot]));
+}
+__device__ __forceinline__ int wq_produce_item(WorkQueue& q, uint32_t n, int* counter, int total, const WorkItem* items, WorkItem& w,
+                                               volatile int* abort_flag) {
+  if (!ptx::mbar_wait(ptx::smem_u32(&q.empty[n % kWqSlots]), ((n / kWqSlots) & 1) ^ 1, abort_flag)) return -1;
+  int idx = atomicAdd(counter, 1);
+  if (idx < total) w = items[idx]; else idx = -1;
+  wq_publish_item(q, n, idx, w);
+  return idx;
+}
+__device__ __forceinline__ int wq_consume_item(WorkQueue& q, uint32_t n, WorkItem& w, volatile int* abort_flag) {
+  const int slot = n % kWqSlots;
+  if (!ptx::mbar_wait(ptx::smem_u32(&q.full[slot]), (n / kWqSlots) & 1, abort_flag)) return -1;
+  const int idx = q.idx[slot];
+  w = q.item[slot];
   __syncwarp();
   if ((threadIdx.x & 31) == 0) ptx::mbar_arrive(ptx::smem_u32(&q.empty[slot]));
   return idx;

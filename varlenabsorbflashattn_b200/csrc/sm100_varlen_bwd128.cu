@@ -5,17 +5,17 @@
 //   dK/dV : one 128-row key tile per item (outer = K, V), walks the segment's query rows (inner = Q, dO)
 // All score products are M128 x N128 MMAs (N = 64 measured 56 % of the tensor rate).
 //
-// The element-wise work of a block is split in two phases, so that with single score buffers the
-// tensor pipe always has the other phase's product to run:
+// The element-wise work of a block is split in two phases:
 //   phase 1:  P  = 2^(c X - lse)          needs X = outerA . innerA^T
 //   phase 2:  dS = P (Y - delta)          needs Y = outerB . innerB^T
-// dK/dV (TMEM: X [0,128) Y [128,256) dV [256,384) dK [384,512)), issue order in steady state
-//     dV += P^T dO(g) ; X(g+1)   |   dK += dS^T Q(g) ; Y(g+1)
-//   P^T overwrites X and dS^T overwrites Y in place (16-bit, packed); the next X is issued behind
-//   the product that reads P^T, the next Y behind the product that reads dS^T (the pipe runs in order).
-// dQ (TMEM: X0 [0,128) X1 [128,256) Y [256,384) dQ [384,512)), steady state
-//     dQ += dS K(g) ; Y(g+1) ; X(g+2)
-//   dS overwrites X[g&1] in place; the scores of block g+1 are already there when phase 1 of g+1 starts.
+// and a score buffer is free again as soon as the element-wise warps have it in registers:
+// dK/dV (TMEM: X [0,128) Y [128,256) dV [256,384) dK [384,512)).  X(g+1) runs under phase 1 of block g; P^T and dS^T (16-bit,
+// packed) go over the halves of Y as those are read.  Steady state:  dV += P^T dO(g) ; dK += dS^T Q(g) ; Y(g+1) ; X(g+2)
+// dQ (TMEM: X0 [0,128) X1 [128,256) Y [256,384) dQ [384,512)).  dS overwrites X[g&1] in place.  Steady state:
+// Y(g+1) ; dQ += dS K(g) ; X(g+2)
+// With P^T in place of X the dK/dV warps waited for every X behind dV, and the dQ warps for Y behind dQ.  dQ / dK/dV before and
+// now: 500-query histories (head dim 64) 843 / 1174 -> 776 / 968 us, 158 k causal tokens (32 heads of 128, at the power limit)
+// 7892 / 10453 -> 7833 / 10353, 42 k causal tokens (16 heads of 128) 492 / 654 -> 480 / 650.
 //
 // In the dK/dV kernel a thread owns a key row, so lse and delta vary along its columns.  Instead of
 // reading them per element from shared memory (measured: about 1000 cycles per block), they are
@@ -46,42 +46,15 @@ using namespace ptx;
 #define TRACE_ADD(slot)
 #endif
 
-// Element-wise warps: 8 (two per TMEM lane quadrant, 64 score columns per thread) or 16 (four per quadrant, 32
-// columns per thread).  The backward needs no row statistics, so the columns of a row split freely.
-#ifndef VAFA_BWD_EW_WARPS
-#define VAFA_BWD_EW_WARPS 8
-#endif
-constexpr int kEw = VAFA_BWD_EW_WARPS;
-// Rounding of P and dS to the I/O type: pack2 (two adds and a byte permute on the integer pipe) or pack2_out (one
-// conversion on the special-function pipe, which also runs the exponentials).  Measured: the dK/dV kernel, with two
-// roundings per score, is 0.5-1.7 % faster with the conversion; the dQ kernel is level to 1.5 % slower with it.
-template <typename T, bool kDKV>
-__device__ __forceinline__ uint32_t pack_bwd(float lo, float hi) {
-  if constexpr (kDKV) return pack2_out<T>(lo, hi);
-  else return pack2<T>(lo, hi);
-}
-static_assert(kEw == 8 || kEw == 16, "element-wise warps");
+constexpr int kEw = 8;  // element-wise warps: two per TMEM lane quadrant, 64 score columns per thread
 constexpr int kGroups = kEw / 4;        // column groups of a row
 constexpr int kC = 128 / kGroups;       // score columns per thread
 constexpr int kTmaWarp = kEw, kMmaWarp = kEw + 1;
-// Registers are granted per four warps, so ten warps leave every thread 168.  With two spare warps the
-// producer / issuer warp group can hand most of its share to the element-wise warp groups (setmaxnreg), which
-// then have 216 each (build with -DVAFA_BWD_SETMAXNREG=1; eight element-wise warps only).
-#ifndef VAFA_BWD_SETMAXNREG
-#define VAFA_BWD_SETMAXNREG 0
-#endif
-static_assert(!VAFA_BWD_SETMAXNREG || kEw == 8, "register hand-over is laid out for eight element-wise warps");
-constexpr int kThreads = kEw * 32 + (VAFA_BWD_SETMAXNREG ? 128 : 64);  // + 1 TMA warp, 1 MMA warp (+ 2 spare)
-#if VAFA_BWD_SETMAXNREG
-#define VAFA_REG_DEC() asm volatile("setmaxnreg.dec.sync.aligned.u32 72;")
-#define VAFA_REG_INC() asm volatile("setmaxnreg.inc.sync.aligned.u32 216;")
-#else
-#define VAFA_REG_DEC()
-#define VAFA_REG_INC()
-#endif
-// one tcgen05.ld for a thread's kC columns
-__device__ __forceinline__ void tmem_ld_cols(uint32_t taddr, uint32_t (&r)[64]) { tmem_ld64(taddr, r); }
-__device__ __forceinline__ void tmem_ld_cols(uint32_t taddr, uint32_t (&r)[32]) { tmem_ld32(taddr, r); }
+// Registers are granted per four warps, so ten warps leave every thread 168, which is enough for dQ.  A dK/dV thread holds P
+// in both precisions beside the scores: there two spare warps fill up the producer / issuer warp group, which hands most
+// of its share to the element-wise warp groups (setmaxnreg: 216 registers each; 500-query histories 1088 us without, 997 with them).
+template <bool kDKV> constexpr int bwd_threads() { return kEw * 32 + (kDKV ? 128 : 64); }  // + 1 TMA warp, 1 MMA warp (+ 2 spare)
+static_assert(256 * 216 + 128 * 72 <= 384 * 168, "setmaxnreg draws on the registers of the launch");
 constexpr int kIn = 128;       // rows per inner block
 // One pair of exponentials in this many takes the polynomial 2^t on the FMA pipe instead of the special-function unit;
 // 0 = none.  With head dim 64 a block has half the products per exponential, so the unit is what the dQ kernel waits
@@ -108,6 +81,16 @@ struct Cfg128 {
   // block; ring B holds V (dQ: read once) or dO (dK/dV)
   static constexpr int kSA = kDKV ? (D == 128 ? 2 : 4) : (D == 128 ? 3 : 6);
   static constexpr int kSB = (D == 128) ? 2 : 4;
+  // Slot of block g's tile.  dQ: two rings.  dK/dV: one pool in which Q(g+S) takes the slot of dO(g) and dO(g+S) that of
+  // Q(g): dO(g) is done with after dV(g), one product before Q(g), and X(g+2), issued a block ahead, is what needs
+  // its tile first.
+  __device__ static __forceinline__ uint32_t slot_a(uint32_t g) {
+    return kDKV ? g % kSA + ((g / kSA) & 1) * kSA : g % kSA;
+  }
+  __device__ static __forceinline__ uint32_t slot_b(uint32_t g) {
+    return kDKV ? g % kSA + (((g / kSA) & 1) ^ 1) * kSA : kSA + g % kSB;
+  }
+  static_assert(!kDKV || kSA == kSB, "one pool");
   static constexpr int kSub = D / 64;
   static constexpr int kSubBytes = 128 * 128;  // 128 rows x 128 B
   static constexpr int kTileBytes = kSub * kSubBytes;
@@ -122,14 +105,13 @@ struct Smem128 {
   using Cfg = Cfg128<D, kDKV>;
   alignas(1024) uint8_t outer_a[Cfg::kTileBytes];
   alignas(1024) uint8_t outer_b[Cfg::kTileBytes];
-  alignas(1024) uint8_t inner_a[Cfg::kSA][Cfg::kTileBytes];
-  alignas(1024) uint8_t inner_b[Cfg::kSB][Cfg::kTileBytes];
+  alignas(1024) uint8_t inner[Cfg::kSA + Cfg::kSB][Cfg::kTileBytes];
   alignas(1024) uint8_t aug[kDKV ? Cfg::kSA : 1][2][kDKV ? kAugBytes : 16];  // [slot][lse, delta]
   alignas(1024) uint8_t ones[kDKV ? kAugBytes : 16];
   alignas(8) uint64_t outer_full, outer_free;
-  uint64_t a_full[Cfg::kSA], a_empty[Cfg::kSA];
-  uint64_t b_full[Cfg::kSB], b_empty[Cfg::kSB];
+  uint64_t full[Cfg::kSA + Cfg::kSB], empty[Cfg::kSA + Cfg::kSB];  // per slot of `inner`
   uint64_t x_full[2], y_full, p_full, ds_full, acc_done;
+  uint64_t score_free;  // dK/dV: X of a block, dQ: Y of a block is in the element-wise warps' registers
   WorkQueue wq;
   uint32_t tmem_base;
   int abort_flag;
@@ -160,7 +142,7 @@ struct Params128 {
 constexpr uint32_t kDescHiSw32 = (256u >> 4) | (1u << 14) | (6u << 29);
 
 template <typename T, int D, bool kDKV>
-__global__ void __launch_bounds__(kThreads, 1)
+__global__ void __launch_bounds__(bwd_threads<kDKV>(), 1)
 varlen_bwd128_kernel(const __grid_constant__ CUtensorMap tmap_outer_a, const __grid_constant__ CUtensorMap tmap_outer_b,
                      const __grid_constant__ CUtensorMap tmap_inner_a, const __grid_constant__ CUtensorMap tmap_inner_b,
                      const __grid_constant__ CUtensorMap tmap_aug, const Params128 p) {
@@ -178,19 +160,16 @@ varlen_bwd128_kernel(const __grid_constant__ CUtensorMap tmap_outer_a, const __g
     wq_init(sm.wq, kEw + 1);
     mbar_init(smem_u32(&sm.outer_full), 1);
     mbar_init(smem_u32(&sm.outer_free), 1);
-    for (int i = 0; i < SA; ++i) {
-      mbar_init(smem_u32(&sm.a_full[i]), 1);
-      mbar_init(smem_u32(&sm.a_empty[i]), 1);
-    }
-    for (int i = 0; i < SB; ++i) {
-      mbar_init(smem_u32(&sm.b_full[i]), 1);
-      mbar_init(smem_u32(&sm.b_empty[i]), 1);
+    for (int i = 0; i < SA + SB; ++i) {
+      mbar_init(smem_u32(&sm.full[i]), 1);
+      mbar_init(smem_u32(&sm.empty[i]), 1);
     }
     mbar_init(smem_u32(&sm.x_full[0]), 1);
     mbar_init(smem_u32(&sm.x_full[1]), 1);
     mbar_init(smem_u32(&sm.y_full), 1);
     mbar_init(smem_u32(&sm.p_full), kEw);   // one arrival per element-wise warp
     mbar_init(smem_u32(&sm.ds_full), kEw);
+    mbar_init(smem_u32(&sm.score_free), kEw);
     mbar_init(smem_u32(&sm.acc_done), 1);
     fence_barrier_init();
   }
@@ -230,20 +209,26 @@ varlen_bwd128_kernel(const __grid_constant__ CUtensorMap tmap_outer_a, const __g
 
   // each setmaxnreg sits inside its own role's branch: after a join the compiler assumes the smaller budget
   if (warp > kMmaWarp) {
-    VAFA_REG_DEC();  // spare warps of the third warp group
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 72;");  // spare warps of the third warp group
   } else if (warp == kTmaWarp) {
-    VAFA_REG_DEC();
+    if constexpr (kDKV) asm volatile("setmaxnreg.dec.sync.aligned.u32 72;");
     // ---------------- TMA producer ----------------
     if (lane == 0) {
       uint32_t gk = 0, qi = 0;
       bool alive = true;
       for (uint32_t n = 0; alive; ++n) {
-        const int idx = wq_produce(sm.wq, n, next_item, total, abort_flag);
+        WorkItem w;
+        const int idx = wq_produce_item(sm.wq, n, next_item, total, p.items, w, abort_flag);
         if (idx < 0) break;
-        const WorkItem w = p.items[idx];
         const int h = w.head;
         const int nb = (w.i_len + kIn - 1) / kIn;
         if (nb == 0) continue;
+        // the outer tiles are single-buffered and no CTA may have read them yet: while the item before is finished they
+        // come into L2 (dQ of the 42 k tokens 490 -> 484 us with this and the items passed on in shared memory)
+        for (int c = 0; c < Cfg::kSub; ++c) {
+          tma_prefetch_3d(&tmap_outer_a, c * 64, h, w.o_start);
+          tma_prefetch_3d(&tmap_outer_b, c * 64, h, w.o_start);
+        }
         if (!mbar_wait(smem_u32(&sm.outer_free), (qi & 1) ^ 1, abort_flag)) break;
         mbar_expect_tx(smem_u32(&sm.outer_full), 2 * Cfg::kTileBytes);
         for (int c = 0; c < Cfg::kSub; ++c) {
@@ -252,29 +237,30 @@ varlen_bwd128_kernel(const __grid_constant__ CUtensorMap tmap_outer_a, const __g
         }
         const int nbt = kDKV ? nb * p.group : nb;
         for (int bb = 0; bb < nbt; ++bb, ++gk) {
-          const int sa = gk % SA, sb = gk % SB;
+          const uint32_t sa = Cfg::slot_a(gk), sb = Cfg::slot_b(gk);
           const int b = kDKV ? bb % nb : bb;
           const int hin = kDKV ? h * p.group + bb / nb : h / p.group;  // head of the inner tensors
           const int row = w.i_start + b * kIn;
-          { TRACE_T0(); if (!mbar_wait(smem_u32(&sm.a_empty[sa]), ((gk / SA) & 1) ^ 1, abort_flag)) { alive = false; break; } TRACE_ADD(0); }
-          mbar_expect_tx(smem_u32(&sm.a_full[sa]), Cfg::kTileBytes + (kDKV ? 2 * kAugBytes : 0));
+          { TRACE_T0(); if (!mbar_wait(smem_u32(&sm.empty[sa]), ((gk / SA) & 1) ^ 1, abort_flag)) { alive = false; break; } TRACE_ADD(0); }
+          mbar_expect_tx(smem_u32(&sm.full[sa]), Cfg::kTileBytes + (kDKV ? 2 * kAugBytes : 0));
           for (int c = 0; c < Cfg::kSub; ++c)
-            tma_load_3d(smem_u32(sm.inner_a[sa]) + c * Cfg::kSubBytes, &tmap_inner_a, smem_u32(&sm.a_full[sa]), c * 64, hin, row);
+            tma_load_3d(smem_u32(sm.inner[sa]) + c * Cfg::kSubBytes, &tmap_inner_a, smem_u32(&sm.full[sa]), c * 64, hin, row);
           if (kDKV) {
-            // fold pieces of the block's 128 query rows: elements [0,16) for lse, [16,32) for delta
-            tma_load_3d(smem_u32(sm.aug[sa][0]), &tmap_aug, smem_u32(&sm.a_full[sa]), 0, hin, row);
-            tma_load_3d(smem_u32(sm.aug[sa][1]), &tmap_aug, smem_u32(&sm.a_full[sa]), 16, hin, row);
+            // fold pieces of the block's 128 query rows: elements [0,16) for lse, [16,32) for delta; X and Y of the block
+            // that used them last were done when dV of that block released this slot
+            tma_load_3d(smem_u32(sm.aug[gk % SA][0]), &tmap_aug, smem_u32(&sm.full[sa]), 0, hin, row);
+            tma_load_3d(smem_u32(sm.aug[gk % SA][1]), &tmap_aug, smem_u32(&sm.full[sa]), 16, hin, row);
           }
-          { TRACE_T0(); if (!mbar_wait(smem_u32(&sm.b_empty[sb]), ((gk / SB) & 1) ^ 1, abort_flag)) { alive = false; break; } TRACE_ADD(1); }
-          mbar_expect_tx(smem_u32(&sm.b_full[sb]), Cfg::kTileBytes);
+          { TRACE_T0(); if (!mbar_wait(smem_u32(&sm.empty[sb]), ((gk / SB) & 1) ^ 1, abort_flag)) { alive = false; break; } TRACE_ADD(1); }
+          mbar_expect_tx(smem_u32(&sm.full[sb]), Cfg::kTileBytes);
           for (int c = 0; c < Cfg::kSub; ++c)
-            tma_load_3d(smem_u32(sm.inner_b[sb]) + c * Cfg::kSubBytes, &tmap_inner_b, smem_u32(&sm.b_full[sb]), c * 64, hin, row);
+            tma_load_3d(smem_u32(sm.inner[sb]) + c * Cfg::kSubBytes, &tmap_inner_b, smem_u32(&sm.full[sb]), c * 64, hin, row);
         }
         ++qi;
       }
     }
   } else if (warp == kMmaWarp) {
-    VAFA_REG_DEC();
+    if constexpr (kDKV) asm volatile("setmaxnreg.dec.sync.aligned.u32 72;");
     // ---------------- MMA issuer ----------------
     // The whole warp on warp-uniform values, one elected lane issues (see varlen_fwd_kernel). 34 k-token
     // training batch (16 heads of 128): dQ 507 -> 485 us, dK/dV 665 -> 641; 500-query histories: 911 -> 885, 1284 -> 1171.
@@ -288,26 +274,28 @@ varlen_bwd128_kernel(const __grid_constant__ CUtensorMap tmap_outer_a, const __g
       const uint32_t tm = warp_uniform(tbase);
       const uint32_t oa_lo = warp_uniform(desc_lo_sw128(smem_u32(sm.outer_a), 16)), ob_lo = warp_uniform(desc_lo_sw128(smem_u32(sm.outer_b), 16));
       const uint32_t ones_lo = warp_uniform(desc_lo_sw128(smem_u32(sm.ones), 16));
-      const uint32_t ia_lo0 = warp_uniform(desc_lo_sw128(smem_u32(sm.inner_a[0]), 16)), ib_lo0 = warp_uniform(desc_lo_sw128(smem_u32(sm.inner_b[0]), 16));
+      const uint32_t in_lo0 = warp_uniform(desc_lo_sw128(smem_u32(sm.inner[0]), 16));
       const uint32_t aug_lo0 = warp_uniform(desc_lo_sw128(smem_u32(sm.aug[0][0]), 16));
-      const uint32_t ma_lo0 = warp_uniform(desc_lo_sw128(smem_u32(sm.inner_a[0]), Cfg::kSubBytes));
-      const uint32_t mb_lo0 = warp_uniform(desc_lo_sw128(smem_u32(sm.inner_b[0]), Cfg::kSubBytes));
+      const uint32_t mn_lo0 = warp_uniform(desc_lo_sw128(smem_u32(sm.inner[0]), Cfg::kSubBytes));
+      const uint32_t full0 = smem_u32(&sm.full[0]), empty0 = smem_u32(&sm.empty[0]);
 
       // X(g) = outerA . innerA(g)^T  (+ fold step)
       auto issue_x = [&](uint32_t g) -> bool {
-        const uint32_t sa = g % SA;
-        { TRACE_T0(); if (!mbar_wait_warp(smem_u32(&sm.a_full[0]) + sa * 8, (g / SA) & 1, abort_flag)) return false; TRACE_ADD(4); }
+        const uint32_t sa = Cfg::slot_a(g);
+        // (the score buffer: block g - 1 has been read)
+        if (kDKV) { TRACE_T0(); if (!mbar_wait_warp(smem_u32(&sm.score_free), (g & 1) ^ 1, abort_flag)) return false; TRACE_ADD(10); }
+        { TRACE_T0(); if (!mbar_wait_warp(full0 + sa * 8, (g / SA) & 1, abort_flag)) return false; TRACE_ADD(4); }
         tc_fence_after();
         TRACE_T0();
         const uint32_t x_tmem = tm + Cfg::kX + (kDKV ? 0u : (g & 1) * 128u);
-        const uint32_t ia_lo = ia_lo0 + sa * kTile16;
+        const uint32_t ia_lo = in_lo0 + sa * kTile16;
         if (elect_one()) {
 #pragma unroll
           for (int kk = 0; kk < D / 16; ++kk) {
             const uint32_t off = (kk >> 2) * (Cfg::kSubBytes >> 4) + (kk & 3) * 2;  // 16-byte units
             mma_ss2(x_tmem, oa_lo + off, ia_lo + off, idesc_xy, kk > 0);
           }
-          if (kDKV) mma_ss2h(x_tmem, ones_lo, aug_lo0 + sa * (2 * kAugBytes >> 4), idesc_xy, 1u, kDescHiSw32);
+          if (kDKV) mma_ss2h(x_tmem, ones_lo, aug_lo0 + (g % SA) * (2 * kAugBytes >> 4), idesc_xy, 1u, kDescHiSw32);
           mma_commit(smem_u32(&sm.x_full[0]) + (kDKV ? 0u : (g & 1) * 8));
         }
         __syncwarp();
@@ -316,34 +304,36 @@ varlen_bwd128_kernel(const __grid_constant__ CUtensorMap tmap_outer_a, const __g
       };
       // Y(g) = outerB . innerB(g)^T  (+ fold step); the last one of an item releases the outer tiles
       auto issue_y = [&](uint32_t g, bool last) -> bool {
-        const uint32_t sa = g % SA, sb = g % SB;
-        { TRACE_T0(); if (!mbar_wait_warp(smem_u32(&sm.b_full[0]) + sb * 8, (g / SB) & 1, abort_flag)) return false; TRACE_ADD(5); }
+        const uint32_t sb = Cfg::slot_b(g);
+        if (!kDKV) { TRACE_T0(); if (!mbar_wait_warp(smem_u32(&sm.score_free), (g & 1) ^ 1, abort_flag)) return false; TRACE_ADD(10); }
+        { TRACE_T0(); if (!mbar_wait_warp(full0 + sb * 8, (g / SB) & 1, abort_flag)) return false; TRACE_ADD(5); }
         tc_fence_after();
         TRACE_T0();
-        const uint32_t ib_lo = ib_lo0 + sb * kTile16;
+        const uint32_t ib_lo = in_lo0 + sb * kTile16;
         if (elect_one()) {
 #pragma unroll
           for (int kk = 0; kk < D / 16; ++kk) {
             const uint32_t off = (kk >> 2) * (Cfg::kSubBytes >> 4) + (kk & 3) * 2;
             mma_ss2(tm + Cfg::kY, ob_lo + off, ib_lo + off, idesc_xy, kk > 0);
           }
-          if (kDKV) mma_ss2h(tm + Cfg::kY, ones_lo, aug_lo0 + sa * (2 * kAugBytes >> 4) + (kAugBytes >> 4), idesc_xy, 1u, kDescHiSw32);
+          if (kDKV) mma_ss2h(tm + Cfg::kY, ones_lo, aug_lo0 + (g % SA) * (2 * kAugBytes >> 4) + (kAugBytes >> 4), idesc_xy, 1u, kDescHiSw32);
           mma_commit(smem_u32(&sm.y_full));
-          if (!kDKV) mma_commit(smem_u32(&sm.b_empty[0]) + sb * 8);  // V is read by this product only
+          if (!kDKV) mma_commit(empty0 + sb * 8);  // V is read by this product only
           if (last) mma_commit(smem_u32(&sm.outer_free));
         }
         __syncwarp();
         TRACE_ADD(14);
         return true;
       };
-      // ACC (+)= A[TMEM, 16-bit packed: K-step kk at column (kk/2)*32 + (kk%2)*8] . B[shared, MN-major], then the
-      // commits the caller lists (0: none)
+      // ACC (+)= A[TMEM, 16-bit packed] . B[shared, MN-major], then the commits the caller lists (0: none).  A holds the
+      // kC columns of an element-wise thread in kC / 2 at the thread's first column (dQ: dS, dK/dV: P) or in the kC / 2
+      // behind (dS)
       auto issue_acc = [&](uint32_t d_tmem, uint32_t a_tmem, uint32_t b_lo, bool first, uint32_t bar0, uint32_t bar1) {
         TRACE_T0();
         if (elect_one()) {
 #pragma unroll
           for (int kk = 0; kk < kIn / 16; ++kk)
-            mma_ts2(d_tmem, a_tmem + (kk >> 1) * 32 + (kk & 1) * 8, b_lo + kk * (2048 >> 4), idesc_acc, (!first || kk > 0) ? 1u : 0u);
+            mma_ts2(d_tmem, a_tmem + (kk / (kC / 16)) * kC + (kk % (kC / 16)) * 8, b_lo + kk * (2048 >> 4), idesc_acc, (!first || kk > 0) ? 1u : 0u);
           mma_commit(bar0);
           if (bar1 != 0) mma_commit(bar1);
         }
@@ -352,38 +342,33 @@ varlen_bwd128_kernel(const __grid_constant__ CUtensorMap tmap_outer_a, const __g
       };
 
       for (uint32_t n = 0; alive; ++n) {
-        const int idx = (int)warp_uniform((uint32_t)wq_consume_warp(sm.wq, n, abort_flag));
+        WorkItem w;
+        const int idx = (int)warp_uniform((uint32_t)wq_consume_item(sm.wq, n, w, abort_flag));
         if (idx < 0) break;
         // blocks of the item, over all its query heads
-        const int nb = (int)warp_uniform((uint32_t)(((p.items[idx].i_len + kIn - 1) / kIn) * (kDKV ? p.group : 1)));
+        const int nb = (int)warp_uniform((uint32_t)(((w.i_len + kIn - 1) / kIn) * (kDKV ? p.group : 1)));
         if (nb == 0) continue;
         { TRACE_T0(); if (!mbar_wait_warp(smem_u32(&sm.outer_full), qi & 1, abort_flag)) break; TRACE_ADD(3); }
         tc_fence_after();
         if (!issue_x(gk) || !issue_y(gk, nb == 1)) break;
-        if (!kDKV && nb > 1 && !issue_x(gk + 1)) break;
+        if (nb > 1 && !issue_x(gk + 1)) break;
         for (int b = 0; b < nb; ++b) {
           const uint32_t g = gk + b;
-          const uint32_t sa = g % SA, sb = g % SB;
-          const uint32_t a_empty = smem_u32(&sm.a_empty[0]) + sa * 8, b_empty = smem_u32(&sm.b_empty[0]) + sb * 8;
+          const uint32_t sa = Cfg::slot_a(g), sb = Cfg::slot_b(g);
           const uint32_t done = b + 1 < nb ? 0u : smem_u32(&sm.acc_done);
+          // the other operand's scores of the next block: dQ as soon as those of this one have been read
+          if (!kDKV && b + 1 < nb && !issue_y(g + 1, b + 2 == nb)) { alive = false; break; }
           if (kDKV) {
             { TRACE_T0(); if (!mbar_wait_warp(smem_u32(&sm.p_full), g & 1, abort_flag)) { alive = false; break; } TRACE_ADD(6); }
             tc_fence_after();
-            issue_acc(tm + Cfg::kAcc0, tm + Cfg::kX, mb_lo0 + sb * kTile16, b == 0, b_empty, 0);  // dV += P^T dO
-            if (b + 1 < nb && !issue_x(g + 1)) { alive = false; break; }
-            { TRACE_T0(); if (!mbar_wait_warp(smem_u32(&sm.ds_full), g & 1, abort_flag)) { alive = false; break; } TRACE_ADD(7); }
-            tc_fence_after();
-            issue_acc(tm + Cfg::kAcc1, tm + Cfg::kY, ma_lo0 + sa * kTile16, b == 0, a_empty, done);  // dK += dS^T Q
-            if (b + 1 < nb && !issue_y(g + 1, b + 2 == nb)) { alive = false; break; }
-          } else {
-            { TRACE_T0(); if (!mbar_wait_warp(smem_u32(&sm.ds_full), g & 1, abort_flag)) { alive = false; break; } TRACE_ADD(7); }
-            tc_fence_after();
-            issue_acc(tm + Cfg::kAcc0, tm + Cfg::kX + (g & 1) * 128u, ma_lo0 + sa * kTile16, b == 0, a_empty, done);  // dQ += dS K
-            if (b + 1 < nb) {
-              if (!issue_y(g + 1, b + 2 == nb)) { alive = false; break; }
-              if (b + 2 < nb && !issue_x(g + 2)) { alive = false; break; }
-            }
+            issue_acc(tm + Cfg::kAcc0, tm + Cfg::kY, mn_lo0 + sb * kTile16, b == 0, empty0 + sb * 8, 0);  // dV += P^T dO
           }
+          { TRACE_T0(); if (!mbar_wait_warp(smem_u32(&sm.ds_full), g & 1, abort_flag)) { alive = false; break; } TRACE_ADD(7); }
+          tc_fence_after();
+          if (kDKV) issue_acc(tm + Cfg::kAcc1, tm + Cfg::kY + kC / 2, mn_lo0 + sa * kTile16, b == 0, empty0 + sa * 8, done);  // dK += dS^T Q
+          else issue_acc(tm + Cfg::kAcc0, tm + Cfg::kX + (g & 1) * 128u, mn_lo0 + sa * kTile16, b == 0, empty0 + sa * 8, done);  // dQ += dS K
+          if (kDKV && b + 1 < nb && !issue_y(g + 1, b + 2 == nb)) { alive = false; break; }
+          if (b + 2 < nb && !issue_x(g + 2)) { alive = false; break; }
         }
         gk += nb;
         ++qi;
@@ -391,7 +376,7 @@ varlen_bwd128_kernel(const __grid_constant__ CUtensorMap tmap_outer_a, const __g
     }
   } else {
     // ---------------- element-wise warps + epilogue (warps 0-7) ----------------
-    VAFA_REG_INC();
+    if constexpr (kDKV) asm volatile("setmaxnreg.inc.sync.aligned.u32 216;");
     // thread -> outer row r = tid % 128 (TMEM lane; a warp may only touch lane quadrant warp % 4);
     // warps 0-3 take inner columns [0,64) of every block, warps 4-7 columns [64,128)
     const int r = threadIdx.x & 127;
@@ -400,10 +385,16 @@ varlen_bwd128_kernel(const __grid_constant__ CUtensorMap tmap_outer_a, const __g
     const float c = p.scale_log2;
     uint32_t gk = 0, qi = 0;
     bool alive = true;
+    // the warp has the scores of a block in registers: their columns may be written again
+    auto score_read = [&] {
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(smem_u32(&sm.score_free));
+    };
     for (uint32_t n = 0; alive; ++n) {
-      const int idx = wq_consume_warp(sm.wq, n, abort_flag);
+      WorkItem w;
+      const int idx = wq_consume_item(sm.wq, n, w, abort_flag);
       if (idx < 0) break;
-      const WorkItem w = p.items[idx];
       const int h = w.head;
       const int nb1 = (w.i_len + kIn - 1) / kIn;      // blocks per query head
       const int nb = nb1 * (kDKV ? p.group : 1);
@@ -437,14 +428,16 @@ varlen_bwd128_kernel(const __grid_constant__ CUtensorMap tmap_outer_a, const __g
         const long long t_p1 = clock64();
 #endif
         float pf[kC];
+        uint32_t pp[kC / 2];
         // masked blocks (tails, the causal diagonal) take their own copy of the loop: folded into one
         // loop the two compares and the select per element ran in every block
         auto phase1 = [&](auto mask_tag) {
           constexpr bool kMask = decltype(mask_tag)::value;
           // this thread's columns [kC * grp, kC * grp + kC) in one load
           uint32_t xs[kC];
-          tmem_ld_cols(x_addr + grp * kC, xs);
+          tmem_ld64(x_addr + grp * kC, xs);
           tmem_wait_ld();
+          if (kDKV) score_read();
           // exponent t = c X' (dK/dV: the product already holds S - lse/c) or c S - lse, in pairs
           const uint64_t c2 = pack_f2(c, c), nl2 = pack_f2(neg_lse, neg_lse);
 #pragma unroll
@@ -468,26 +461,13 @@ varlen_bwd128_kernel(const __grid_constant__ CUtensorMap tmap_outer_a, const __g
             pf[2 * i] = p0;
             pf[2 * i + 1] = p1;
           }
-          if (kDKV) {
-            // P^T in place: each 32-column chunk becomes 16 packed columns over its own first half
+          if constexpr (kDKV) {
 #pragma unroll
-            for (int q2 = 0; q2 < kC / 32; ++q2) {
-              uint32_t pp[16];
-#pragma unroll
-              for (int i = 0; i < 16; ++i) pp[i] = pack_bwd<T, kDKV>(pf[q2 * 32 + 2 * i], pf[q2 * 32 + 2 * i + 1]);
-              tmem_st16(x_addr + (grp * (kC / 32) + q2) * 32, pp);
-            }
+            for (int i = 0; i < kC / 2; ++i) pp[i] = pack2_out<T>(pf[2 * i], pf[2 * i + 1]);
           }
         };
         // warp-uniform choice: the TMEM loads and stores inside are .sync.aligned
         if (__any_sync(0xffffffffu, need_mask)) phase1(std::true_type{}); else phase1(std::false_type{});
-        if (kDKV) {
-          tmem_wait_st();
-          tc_fence_before();
-          __syncwarp();
-          if (lane == 0) mbar_arrive(smem_u32(&sm.p_full));
-        }
-
 #ifdef VAFA_TRACE
         tr[12] += clock64() - t_p1;
 #endif
@@ -497,27 +477,44 @@ varlen_bwd128_kernel(const __grid_constant__ CUtensorMap tmap_outer_a, const __g
 #ifdef VAFA_TRACE
         const long long t_p2 = clock64();
 #endif
-        {
-          uint32_t ys[kC];
+        // dS of half the thread's columns.  dK/dV: the product already holds dP - delta.  Masked columns have P = 0
+        // exactly, and the other factor is finite there (rows of a neighbouring segment, or zero fill past the end)
+        uint32_t dd[kC / 2];
+        auto phase2 = [&](const uint32_t (&ys)[kC / 2], int q2) {
           const uint64_t nd2 = pack_f2(-my_delta, -my_delta);
-          tmem_ld_cols(y_addr + grp * kC, ys);
-          tmem_wait_ld();
 #pragma unroll
-          for (int q2 = 0; q2 < kC / 32; ++q2) {
-            uint32_t dd[16];
-#pragma unroll
-            for (int i = 0; i < 16; ++i) {
-              // dK/dV: the product already holds dP - delta.  Masked columns have P = 0 exactly, and the
-              // other factor is finite there (rows of a neighbouring segment, or zero fill past the end)
-              uint64_t y2 = pack_f2(__uint_as_float(ys[q2 * 32 + 2 * i]), __uint_as_float(ys[q2 * 32 + 2 * i + 1]));
-              if (!kDKV) y2 = add_f2(y2, nd2);
-              float d0, d1;
-              unpack_f2(mul_f2(pack_f2(pf[q2 * 32 + 2 * i], pf[q2 * 32 + 2 * i + 1]), y2), d0, d1);
-              dd[i] = pack_bwd<T, kDKV>(d0, d1);
-            }
-            // dQ: dS over the scores just consumed (X[g&1]); dK/dV: dS^T over dP^T (Y); in place as above
-            tmem_st16((kDKV ? y_addr : x_addr) + (grp * (kC / 32) + q2) * 32, dd);
+          for (int i = 0; i < kC / 4; ++i) {
+            const int at = q2 * (kC / 2) + 2 * i;
+            uint64_t y2 = pack_f2(__uint_as_float(ys[2 * i]), __uint_as_float(ys[2 * i + 1]));
+            if (!kDKV) y2 = add_f2(y2, nd2);
+            float d0, d1;
+            unpack_f2(mul_f2(pack_f2(pf[at], pf[at + 1]), y2), d0, d1);
+            dd[at / 2] = pack2_out<T>(d0, d1);
           }
+        };
+        uint32_t y0[kC / 2], y1[kC / 2];
+        tmem_ld32(y_addr + grp * kC, y0);
+        if constexpr (kDKV) {
+          // P^T, then dS^T go over the two halves of this thread's columns of dP^T as they are read
+          tmem_wait_ld();
+          tmem_st32(y_addr + grp * kC, pp);
+          tmem_ld32(y_addr + grp * kC + kC / 2, y1);
+          phase2(y0, 0);
+          tmem_wait_st();
+          tc_fence_before();
+          __syncwarp();
+          if (lane == 0) mbar_arrive(smem_u32(&sm.p_full));
+          tmem_wait_ld();
+          phase2(y1, 1);
+          tmem_st32(y_addr + grp * kC + kC / 2, dd);
+        } else {
+          // dS over the scores just consumed (X[g&1])
+          tmem_ld32(y_addr + grp * kC + kC / 2, y1);
+          tmem_wait_ld();
+          score_read();
+          phase2(y0, 0);
+          phase2(y1, 1);
+          tmem_st32(x_addr + grp * kC, dd);
         }
         tmem_wait_st();
         tc_fence_before();
@@ -543,8 +540,8 @@ varlen_bwd128_kernel(const __grid_constant__ CUtensorMap tmap_outer_a, const __g
         T* optr = reinterpret_cast<T*>(which == 0 ? p.out0 : p.out1) + out_row * D;
         // dV unscaled; dQ and dK scaled; dQ rows that saw no key are exact zeros (the polynomial 2^t
         // leaves about 1e-38 where the special-function unit gives 0)
-        // a row whose lse or delta is NaN (the forward saw a NaN, or dO holds one) goes out as NaN: the packed
-        // dS operand cannot carry it (see pack2)
+        // a row whose lse or delta is NaN (the forward saw a NaN, or dO holds one) goes out as NaN: the polynomial
+        // 2^t would make a number of it
         const float poison = kDKV ? 0.f : ((neg_lse == -INFINITY ? 0.f : neg_lse * 0.f) + my_delta * 0.f);
         const float mul = (kDKV && which == 0) ? 1.f : ((!kDKV && neg_lse == -INFINITY) ? 0.f : p.scale + poison);
         const uint32_t acc_col = which == 0 ? Cfg::kAcc0 : Cfg::kAcc1;
@@ -568,7 +565,7 @@ varlen_bwd128_kernel(const __grid_constant__ CUtensorMap tmap_outer_a, const __g
   }
 
 #ifdef VAFA_TRACE
-  if (p.trace != nullptr && (threadIdx.x == 0 || threadIdx.x == 256 || threadIdx.x == 288)) {
+  if (p.trace != nullptr && (threadIdx.x == 0 || threadIdx.x == kTmaWarp * 32 || threadIdx.x == kMmaWarp * 32)) {
     tr[15] = clock64() - t_begin;
     for (int i = 0; i < 16; ++i)
       if (tr[i] != 0) p.trace[((long long)(kDKV ? 1 : 0) * 256 + blockIdx.x) * 16 + i] = tr[i];
@@ -623,7 +620,7 @@ static int launch128(const Bwd128Launch& L, cudaStream_t s) {
     VAFA_CUDA_CHECK(cudaFuncSetAttribute(varlen_bwd128_kernel<T, D, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     {
       LaunchScope scope(kKBwdDq, s);
-      varlen_bwd128_kernel<T, D, false><<<L.sms, kThreads, smem, s>>>(q128, do128, k128, v128, aug, p);
+      varlen_bwd128_kernel<T, D, false><<<L.sms, bwd_threads<false>(), smem, s>>>(q128, do128, k128, v128, aug, p);
     }
     VAFA_LAUNCH_CHECK("varlen_bwd128_kernel<dQ>");
   }
@@ -635,7 +632,7 @@ static int launch128(const Bwd128Launch& L, cudaStream_t s) {
     VAFA_CUDA_CHECK(cudaFuncSetAttribute(varlen_bwd128_kernel<T, D, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     {
       LaunchScope scope(kKBwdDkv, s);
-      varlen_bwd128_kernel<T, D, true><<<L.sms, kThreads, smem, s>>>(k128, v128, q128, do128, aug, p);
+      varlen_bwd128_kernel<T, D, true><<<L.sms, bwd_threads<true>(), smem, s>>>(k128, v128, q128, do128, aug, p);
     }
     VAFA_LAUNCH_CHECK("varlen_bwd128_kernel<dKV>");
   }
