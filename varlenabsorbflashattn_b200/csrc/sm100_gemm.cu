@@ -1,10 +1,13 @@
 // Dense product for the absorb operator's prologue and epilogue:
 //   C[M, N] = A[M, K] . B[K, N]        (16-bit operands, fp32 accumulation, 16-bit result; K = 256 k)
-// K = 256: one persistent CTA per SM keeps its 256 x 256 slice of B in shared memory (128 KB,
-// MN-major) and streams 128-row tiles of A through a second buffer.  K = 512, 768, ...: the B slice of
-// each 256-deep chunk is streamed with the A chunk instead and the chunks accumulate in TMEM.  The
-// accumulator (256 TMEM columns) is double buffered so the epilogue of tile i overlaps the load and
-// MMAs of tile i+1.
+// One persistent CTA per SM owns a 256-column slice of C and walks 128-row tiles of it.  K is taken 64 deep: a chunk of A
+// (16 KB) has a slot of its own, so the loads of the next tile start while the current one is multiplied.  K = 256: the
+// CTA's 256 x 256 slice of B stays in shared memory (128 KB, MN-major) beside five slots; K = 512, 768, ...: a slot holds the
+// chunk of B (32 KB) too, and there are four.  The accumulator (256 TMEM columns) is double buffered, so the epilogue
+// of tile i overlaps the products of tile i + 1; a row's pieces leave through the lane transpose of common.cuh.
+// Bound by L2 and HBM (a row of the stacked operands is 4 KB).  With one 64 KB tile of A at a time its load, its products and the
+// next load ran one after the other: the six products of a training step of 1024 users 113 -> 90 us, at raw widths 968 / 216
+// 134 -> 99.
 // It stands in for the two torch matmuls of the reference's prologue
 // (triton_target_attn_absorb/triton_target_attn_absorb/interface.py:434-435, here as one product
 // with the pre-multiplied W_Q W_K^T) and for the per-head W_V projection the reference does at the
@@ -24,11 +27,17 @@ using namespace ptx;
 constexpr int kGemmThreads = 192;
 constexpr int kK = 256;
 constexpr int kNTile = 256;
+constexpr int kChunk = 64;                       // depth of a slot
+constexpr int kAChunk = 128 * 128;               // 128 rows x 64 of A
+constexpr int kBSub = kChunk * 128;              // 64 k-rows x 64 columns of B
+constexpr int kBChunk = 4 * kBSub;
+constexpr int kResidentSlots = 5, kStreamSlots = 4, kMaxSlots = 5;
+constexpr int kBufBytes = 4 * kBChunk + kResidentSlots * kAChunk;
+static_assert(kStreamSlots * (kAChunk + kBChunk) <= kBufBytes, "streamed slots fit where the resident slice and its slots do");
 
 struct GemmSmem {
-  alignas(1024) uint8_t b[4][kK * 128];    // 4 column chunks of 64: [256 k-rows x 128 B] each
-  alignas(1024) uint8_t a[4][128 * 128];   // 4 k chunks of 64: [128 rows x 128 B] each
-  alignas(8) uint64_t b_full, a_full, a_empty, acc_full[2], acc_empty[2];
+  alignas(1024) uint8_t buf[kBufBytes];  // resident: B slice, then A slots; streamed: slots of A chunk and B chunk
+  alignas(8) uint64_t b_full[4], full[kMaxSlots], empty[kMaxSlots], acc_full[2], acc_empty[2];
   uint32_t tmem_base;
   int abort_flag;
   int wait_limit;  // read by the bounded waits as abort_flag[1]: keep it right behind abort_flag
@@ -41,24 +50,28 @@ struct GemmParams {
   int ldc;
   int n_tiles;     // N / 256
   int m_tiles;     // ceil(M / 128)
-  int k_chunks;    // K / 256
+  int k_chunks;    // K / 64
   int diag_heads;  // 0: full rows
   int wait_limit;  // bound of every device-side wait, in units of 65536 cycles
 };
 
-template <typename T>
+template <typename T, bool kResident>
 __global__ void __launch_bounds__(kGemmThreads, 1)
 gemm_nn_k256_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b, const GemmParams p) {
+  constexpr uint32_t kSlots = kResident ? kResidentSlots : kStreamSlots;
+  constexpr uint32_t kFirst = kResident ? 4 * kBChunk : 0, kSlot = kResident ? kAChunk : kAChunk + kBChunk;
   extern __shared__ uint8_t smem_raw[];
   GemmSmem& sm = *reinterpret_cast<GemmSmem*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = (int)warp_uniform(threadIdx.x >> 5), lane = threadIdx.x & 31;
   volatile int* abort_flag = &sm.abort_flag;
   if (threadIdx.x == 0) {
     sm.abort_flag = 0;
     sm.wait_limit = p.wait_limit;
-    mbar_init(smem_u32(&sm.b_full), 1);
-    mbar_init(smem_u32(&sm.a_full), 1);
-    mbar_init(smem_u32(&sm.a_empty), 1);
+    for (int i = 0; i < 4; ++i) mbar_init(smem_u32(&sm.b_full[i]), 1);
+    for (int i = 0; i < kMaxSlots; ++i) {
+      mbar_init(smem_u32(&sm.full[i]), 1);
+      mbar_init(smem_u32(&sm.empty[i]), 1);
+    }
     for (int i = 0; i < 2; ++i) {
       mbar_init(smem_u32(&sm.acc_full[i]), 1);
       mbar_init(smem_u32(&sm.acc_empty[i]), 128);
@@ -82,91 +95,100 @@ gemm_nn_k256_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
   const int groups = gridDim.x / p.n_tiles;  // CTAs per column tile (grid is a multiple of n_tiles)
   const int n_tile = blockIdx.x % p.n_tiles;
   const int m_first = blockIdx.x / p.n_tiles;
+  const uint32_t buf0 = smem_u32(sm.buf);
 
   if (warp == 4) {
     if (lane == 0) {
-      const bool resident = p.k_chunks == 1;
-      if (resident) {
-        mbar_expect_tx(smem_u32(&sm.b_full), 4 * kK * 128);
-        for (int c = 0; c < 4; ++c) tma_load_3d(smem_u32(sm.b[c]), &tmap_b, smem_u32(&sm.b_full), n_tile * kNTile + c * 64, 0, 0);
-      }
+      auto load_b = [&](uint32_t dst, uint32_t bar, int kc) {
+        for (int c = 0; c < 4; ++c) tma_load_3d(dst + c * kBSub, &tmap_b, bar, n_tile * kNTile + c * 64, 0, kc * kChunk);
+      };
       uint32_t it = 0;
       bool alive = true;
       for (int m = m_first; alive && m < p.m_tiles; m += groups) {
         for (int kc = 0; kc < p.k_chunks; ++kc, ++it) {
-          if (!mbar_wait(smem_u32(&sm.a_empty), (it & 1) ^ 1, abort_flag)) { alive = false; break; }
-          mbar_expect_tx(smem_u32(&sm.a_full), 4 * 128 * 128 + (resident ? 0 : 4 * kK * 128));
-          for (int c = 0; c < 4; ++c)
-            tma_load_3d(smem_u32(sm.a[c]), &tmap_a, smem_u32(&sm.a_full), kc * kK + c * 64, 0, m * 128);
-          if (!resident)
-            for (int c = 0; c < 4; ++c)
-              tma_load_3d(smem_u32(sm.b[c]), &tmap_b, smem_u32(&sm.a_full), n_tile * kNTile + c * 64, 0, kc * kK);
+          const uint32_t slot = it % kSlots, bar = smem_u32(&sm.full[0]) + slot * 8, dst = buf0 + kFirst + slot * kSlot;
+          if (!mbar_wait(smem_u32(&sm.empty[0]) + slot * 8, ((it / kSlots) & 1) ^ 1, abort_flag)) { alive = false; break; }
+          mbar_expect_tx(bar, kSlot);
+          tma_load_3d(dst, &tmap_a, bar, kc * kChunk, 0, m * 128);
+          if (!kResident) load_b(dst + kAChunk, bar, kc);
+          if (kResident && m == m_first) {
+            const uint32_t b_bar = smem_u32(&sm.b_full[kc]);
+            mbar_expect_tx(b_bar, kBChunk);
+            load_b(buf0 + kc * kBChunk, b_bar, kc);
+          }
         }
       }
     }
   } else if (warp == 5) {
-    if (lane == 0) {
-      constexpr int kFmt = std::is_same<T, __nv_bfloat16>::value ? 1 : 0;
-      constexpr uint32_t idesc = make_idesc(kFmt, 0, 1, 128, kNTile);
-      bool ok = p.k_chunks > 1 || mbar_wait(smem_u32(&sm.b_full), 0, abort_flag);
-      uint32_t it = 0, tile = 0;
-      for (int m = m_first; ok && m < p.m_tiles; m += groups, ++tile) {
-        const uint32_t buf = tile & 1;
-        if (!mbar_wait(smem_u32(&sm.acc_empty[buf]), ((tile >> 1) & 1) ^ 1, abort_flag)) break;
-        for (int kc = 0; kc < p.k_chunks; ++kc, ++it) {
-          if (!mbar_wait(smem_u32(&sm.a_full), it & 1, abort_flag)) { ok = false; break; }
-          tc_fence_after();
+    // the whole warp on warp-uniform values, one elected lane issues (see varlen_fwd_kernel)
+    constexpr int kFmt = std::is_same<T, __nv_bfloat16>::value ? 1 : 0;
+    constexpr uint32_t idesc = make_idesc(kFmt, 0, 1, 128, kNTile);
+    const uint32_t tm = warp_uniform(tbase);
+    const uint32_t a_lo0 = warp_uniform(desc_lo_sw128(buf0 + kFirst, 16));
+    const uint32_t b_lo0 = warp_uniform(desc_lo_sw128(buf0 + (kResident ? 0 : kAChunk), kBSub));
+    bool ok = true;
+    uint32_t it = 0, tile = 0;
+    for (int m = m_first; ok && m < p.m_tiles; m += groups, ++tile) {
+      const uint32_t buf = tile & 1;
+      if (!mbar_wait_warp(smem_u32(&sm.acc_empty[0]) + buf * 8, ((tile >> 1) & 1) ^ 1, abort_flag)) break;
+      for (int kc = 0; kc < p.k_chunks; ++kc, ++it) {
+        const uint32_t slot = it % kSlots;
+        if (kResident && tile == 0 && !mbar_wait_warp(smem_u32(&sm.b_full[0]) + kc * 8, 0, abort_flag)) { ok = false; break; }
+        if (!mbar_wait_warp(smem_u32(&sm.full[0]) + slot * 8, (it / kSlots) & 1, abort_flag)) { ok = false; break; }
+        tc_fence_after();
+        const uint32_t a_lo = a_lo0 + slot * (kSlot >> 4), b_lo = b_lo0 + (kResident ? (uint32_t)kc * (kBChunk >> 4) : slot * (kSlot >> 4));
+        if (elect_one()) {
 #pragma unroll
-          for (int kk = 0; kk < kK / 16; ++kk) {
-            const uint64_t da = make_desc_sw128(smem_u32(sm.a[kk >> 2]) + (kk & 3) * 32, 16, 1024);
-            const uint64_t db = make_desc_sw128(smem_u32(sm.b[0]) + kk * 2048, kK * 128, 1024);
-            mma_ss(tbase + buf * kNTile, da, db, idesc, (kc > 0 || kk > 0) ? 1u : 0u);
-          }
-          mma_commit(smem_u32(&sm.a_empty));
+          for (int kk = 0; kk < kChunk / 16; ++kk)
+            mma_ss2(tm + buf * kNTile, a_lo + kk * 2, b_lo + kk * (2048 >> 4), idesc, (kc > 0 || kk > 0) ? 1u : 0u);
+          mma_commit(smem_u32(&sm.empty[0]) + slot * 8);
+          if (kc == p.k_chunks - 1) mma_commit(smem_u32(&sm.acc_full[0]) + buf * 8);
         }
-        if (ok) mma_commit(smem_u32(&sm.acc_full[buf]));
+        __syncwarp();
       }
     }
   } else {
     const int r = threadIdx.x;
     const uint32_t lane_base = tbase + ((uint32_t)(warp * 32) << 16);
-    T* C = reinterpret_cast<T*>(p.C);
+    T* const C = reinterpret_cast<T*>(p.C);
     uint32_t it = 0;
     for (int m = m_first; m < p.m_tiles; m += groups, ++it) {
       const uint32_t buf = it & 1;
       if (!mbar_wait(smem_u32(&sm.acc_full[buf]), (it >> 1) & 1, abort_flag)) break;
       tc_fence_after();
       const long long row = (long long)m * 128 + r;
-      const bool row_ok = row < p.M;
-      int c_begin = 0, c_end = kNTile / 32;
-      long long col0 = (long long)n_tile * kNTile;  // first output column of chunk c_begin
-      if (p.diag_heads > 0) {
-        const int per = (kNTile / p.diag_heads) / 32;  // 32-column chunks per head block
-        c_begin = (int)(row % p.diag_heads) * per;
-        c_end = c_begin + per;
-        col0 = 0;
-      }
-      // c_begin/c_end differ per thread in diag mode, but tcgen05.ld is warp-collective: walk all
-      // chunks uniformly and keep only this thread's range
-      for (int cc = 0; cc < kNTile / 32; ++cc) {
-        if (p.diag_heads > 0) {
-          const bool any = __any_sync(0xffffffffu, cc >= c_begin && cc < c_end);
-          if (!any) continue;
-        }
+      const int rows = (int)min(128LL, p.M - (long long)m * 128);
+      auto ld = [&](int cc, uint32_t (&pw)[16]) {
         uint32_t t[32];
         tmem_ld32(lane_base + buf * kNTile + cc * 32, t);
         tmem_wait_ld();
-        if (row_ok && cc >= c_begin && cc < c_end) {
-          uint4* dst = reinterpret_cast<uint4*>(C + row * p.ldc + col0 + (cc - c_begin) * 32);
 #pragma unroll
-          for (int v4 = 0; v4 < 4; ++v4) {
-            uint4 u;
-            u.x = pack2_out<T>(__uint_as_float(t[8 * v4 + 0]), __uint_as_float(t[8 * v4 + 1]));
-            u.y = pack2_out<T>(__uint_as_float(t[8 * v4 + 2]), __uint_as_float(t[8 * v4 + 3]));
-            u.z = pack2_out<T>(__uint_as_float(t[8 * v4 + 4]), __uint_as_float(t[8 * v4 + 5]));
-            u.w = pack2_out<T>(__uint_as_float(t[8 * v4 + 6]), __uint_as_float(t[8 * v4 + 7]));
-            dst[v4] = u;
+        for (int i = 0; i < 16; ++i) pw[i] = pack2_out<T>(__uint_as_float(t[2 * i]), __uint_as_float(t[2 * i + 1]));
+      };
+      if (p.diag_heads == 0) {
+#pragma unroll 2
+        for (int cc = 0; cc < kNTile / 32; ++cc) {
+          uint32_t pw[16];
+          ld(cc, pw);
+          store_chunk_coalesced<T>(pw, C + row * p.ldc + (long long)n_tile * kNTile + cc * 32, p.ldc, r, rows, 4);
+        }
+      } else {
+        // row m keeps the 256 / diag_heads columns of its own head.  tcgen05.ld is warp-collective: all chunks are walked
+        // and each lane keeps its own, so that a chunk of all rows leaves in one go
+        const int per = (kNTile / p.diag_heads) / 32;  // 32-column chunks per head
+        const int mine = (int)(row % p.diag_heads);
+        for (int j = 0; j < per; ++j) {
+          uint32_t keep[16];
+#pragma unroll
+          for (int i = 0; i < 16; ++i) keep[i] = 0u;
+          for (int h = 0; h < p.diag_heads; ++h) {
+            if (!__any_sync(0xffffffffu, mine == h)) continue;
+            uint32_t pw[16];
+            ld(h * per + j, pw);
+#pragma unroll
+            for (int i = 0; i < 16; ++i) keep[i] = mine == h ? pw[i] : keep[i];
           }
+          store_chunk_coalesced<T>(keep, C + row * p.ldc + j * 32, p.ldc, r, rows, 4);
         }
       }
       tc_fence_before();
@@ -182,6 +204,15 @@ gemm_nn_k256_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
     __syncthreads();
   }
   if (warp == 5) tmem_dealloc(tbase, 512);
+}
+
+template <typename T, bool kResident>
+int launch_gemm_nn(const CUtensorMap& ta, const CUtensorMap& tb, const GemmParams& p, int grid, cudaStream_t s) {
+  const size_t smem = sizeof(GemmSmem) + 1024;
+  VAFA_CUDA_CHECK(cudaFuncSetAttribute(gemm_nn_k256_kernel<T, kResident>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  gemm_nn_k256_kernel<T, kResident><<<grid, kGemmThreads, smem, s>>>(ta, tb, p);
+  VAFA_LAUNCH_CHECK("gemm_nn_k256_kernel");
+  return 0;
 }
 
 }  // namespace
@@ -200,7 +231,7 @@ int sm100_gemm_nn_k256(const GemmNNArgs& g, cudaStream_t s) {
   p.wait_limit = wait_limit_units();
   p.C = g.C; p.M = g.M; p.ldc = g.ldc; p.n_tiles = g.N / kNTile; p.m_tiles = (int)((g.M + 127) / 128);
   p.diag_heads = g.diag_heads;
-  p.k_chunks = g.lda / kK;
+  p.k_chunks = g.lda / kChunk;
   int groups = sms / p.n_tiles;
   if (groups < 1) groups = 1;
   if (groups > p.m_tiles) groups = p.m_tiles;
@@ -210,18 +241,12 @@ int sm100_gemm_nn_k256(const GemmNNArgs& g, cudaStream_t s) {
   // K = lda (A rows densely packed), a multiple of 256; B is [K, N] densely packed
   if (g.lda < kK || g.lda % kK != 0 || g.ldb != g.N) return fail(VAFA_ERR_UNSUPPORTED, "gemm_nn_k256: K=%d ldb=%d not supported", g.lda, g.ldb);
   if ((rc = encode_tmap_rows(&ta, g.A, g.dtype, g.M, 1, g.lda, 128))) return rc;
-  if ((rc = encode_tmap_rows(&tb, g.B, g.dtype, g.lda, 1, g.N, 256))) return rc;
-  const size_t smem = sizeof(GemmSmem) + 1024;
+  if ((rc = encode_tmap_rows(&tb, g.B, g.dtype, g.lda, 1, g.N, kChunk))) return rc;
   LaunchScope scope(kKAbsorbGemm, s);
-  if (g.dtype == VAFA_BF16) {
-    VAFA_CUDA_CHECK(cudaFuncSetAttribute(gemm_nn_k256_kernel<__nv_bfloat16>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    gemm_nn_k256_kernel<__nv_bfloat16><<<grid, kGemmThreads, smem, s>>>(ta, tb, p);
-  } else {
-    VAFA_CUDA_CHECK(cudaFuncSetAttribute(gemm_nn_k256_kernel<__half>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    gemm_nn_k256_kernel<__half><<<grid, kGemmThreads, smem, s>>>(ta, tb, p);
-  }
-  VAFA_LAUNCH_CHECK("gemm_nn_k256_kernel");
-  return 0;
+  const bool resident = g.lda == kK;
+  if (g.dtype == VAFA_BF16)
+    return resident ? launch_gemm_nn<__nv_bfloat16, true>(ta, tb, p, grid, s) : launch_gemm_nn<__nv_bfloat16, false>(ta, tb, p, grid, s);
+  return resident ? launch_gemm_nn<__half, true>(ta, tb, p, grid, s) : launch_gemm_nn<__half, false>(ta, tb, p, grid, s);
 }
 
 }  // namespace vafa
