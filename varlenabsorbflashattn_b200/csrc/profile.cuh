@@ -25,6 +25,7 @@ enum KernelId {
   kKAbsorbGemmTn,
   kKBwdFused,
   kKBwdDqFin,
+  kKAbsorbBwdDxu,
   kKCount
 };
 

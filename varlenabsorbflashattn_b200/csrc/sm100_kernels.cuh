@@ -72,10 +72,25 @@ struct AbsorbCoreBwdArgs {
   int32_t* status;
   int x_width;         // row width of x and dx (<= 256)
   int lists_built;     // the tile lists were already built by sm100_absorb_core_bwd_lists()
-  int which;           // 0: both kernels; 1: the dU kernel only; 2: the dX kernel only
+  int which;           // 0: dU and dX; 1: dU only; 2: dX only
 };
+// dU and dX of the users in the list (1 to 64 / H queries, at least one key) in one kernel.
+struct AbsorbDxuLaunch {
+  const void* u; const void* x; const void* dax;
+  const float* nl; const float* nd;  // planar rows of sm100_absorb_ld()
+  void* du; void* dx;
+  const void* header; const void* items;
+  int total_q, total_k, H, dtype, x_width, sms;
+  int which;  // as in AbsorbCoreBwdArgs
+  float scale;
+  int32_t* status;
+};
+int sm100_absorb_dxu_launch(const AbsorbDxuLaunch& L, cudaStream_t s);
 size_t sm100_absorb_core_bwd_workspace_bytes(int total_q, int total_k, int n_seg, int H);
 int sm100_absorb_core_bwd(const AbsorbCoreBwdArgs& a, cudaStream_t s);
+// The users of few queries, which sm100_absorb_core_bwd() leaves out where this is true: on any stream, lists built before.
+bool sm100_absorb_one_pass(const AbsorbCoreBwdArgs& a);
+int sm100_absorb_core_bwd_one_pass(const AbsorbCoreBwdArgs& a, cudaStream_t s);
 // The tile lists depend on cu_seqlens only: these build them on their own (on any stream the caller
 // orders before the core call), so that the single-CTA list builder runs beside the projections.
 int sm100_absorb_core_fwd_lists(const AbsorbCoreArgs& a, cudaStream_t s);

@@ -42,6 +42,19 @@ __device__ __forceinline__ bool mbar_try_wait(uint32_t bar, uint32_t parity) {
   return ok != 0;
 }
 
+// The same without the wait that try_wait may take before it answers.
+__device__ __forceinline__ bool mbar_test_wait(uint32_t bar, uint32_t parity) {
+  uint32_t ok;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t}"
+      : "=r"(ok)
+      : "r"(bar), "r"(parity)
+      : "memory");
+  return ok != 0;
+}
+
 // Bounded wait.  `abort_flag` is a shared-memory word any role sets when it gives up, so that
 // the other roles leave their waits promptly.  Returns false when the wait did not complete.
 // The word after it (abort_flag[1]) holds the limit in units of 65536 clock cycles; the kernel copies it
@@ -69,15 +82,16 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatil
 }
 
 // Waits until either barrier has completed its phase: 1 = the first one is ready (checked first),
-// 2 = only the second one, 0 = the bounded wait ran out or another role gave up.
+// 2 = only the second one, 0 = the bounded wait ran out or another role gave up.  (With try_wait the thread sleeps on one
+// of the two for microseconds while the other completes.)
 __device__ __forceinline__ int mbar_wait_either(uint32_t bar_a, uint32_t parity_a, uint32_t bar_b, uint32_t parity_b,
                                                 volatile int* abort_flag) {
   const long long t0 = clock64();
   const long long limit = wait_limit_cycles(abort_flag);
   uint32_t spins = 0;
   while (true) {
-    if (mbar_try_wait(bar_a, parity_a)) return 1;
-    if (mbar_try_wait(bar_b, parity_b)) return 2;
+    if (mbar_test_wait(bar_a, parity_a)) return 1;
+    if (mbar_test_wait(bar_b, parity_b)) return 2;
     if ((++spins & 63u) == 0u) {
       if (*abort_flag != 0) return 0;
       if (clock64() - t0 > limit) {
@@ -307,6 +321,23 @@ __device__ __forceinline__ void bulk_load_1d(uint32_t smem_dst, const void* gsrc
                ::"r"(smem_dst), "l"(reinterpret_cast<uint64_t>(gsrc)), "r"(bytes), "r"(bar)
                : "memory");
 }
+
+// Tiled store of a box from shared memory, as a bulk operation of the current group.
+__device__ __forceinline__ void tma_store_3d(const CUtensorMap* m, uint32_t smem_src, int c0, int c1, int c2) {
+  asm volatile("cp.async.bulk.tensor.3d.global.shared::cta.tile.bulk_group [%0, {%2, %3, %4}], [%1];"
+               ::"l"(reinterpret_cast<uint64_t>(m)), "r"(smem_src), "r"(c0), "r"(c1), "r"(c2)
+               : "memory");
+}
+__device__ __forceinline__ void bulk_store_commit() { asm volatile("cp.async.bulk.commit_group;" ::: "memory"); }
+// 1-D bulk copy shared -> global, in a bulk group of its own (same alignment).
+__device__ __forceinline__ void bulk_store_1d(void* gdst, uint32_t smem_src, uint32_t bytes) {
+  asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;\n\tcp.async.bulk.commit_group;"
+               ::"l"(reinterpret_cast<uint64_t>(gdst)), "r"(smem_src), "r"(bytes)
+               : "memory");
+}
+// The thread's bulk stores have read their shared memory / are complete.
+__device__ __forceinline__ void bulk_store_wait_read() { asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory"); }
+__device__ __forceinline__ void bulk_store_wait() { asm volatile("cp.async.bulk.wait_group 0;" ::: "memory"); }
 
 __device__ __forceinline__ float ex2(float x) {
   float y;

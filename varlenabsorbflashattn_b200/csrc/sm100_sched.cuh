@@ -40,7 +40,7 @@ struct alignas(256) SchedHeader {
   int32_t n_combine;
   int32_t n_partial_rows;
   int32_t block_len;   // inner blocks per split that was finally used (0 = no split)
-  int32_t reserved0;
+  int32_t next_item_2; // counter of a second kernel that walks the same list
   int32_t next_item;   // dynamic scheduling counter
   int32_t pad[2];
 };
@@ -56,6 +56,8 @@ struct SchedParams {
   int32_t H;
   int32_t sm_count;
   int32_t split_len;    // forced inner slice length (multiple of 128), 0 = automatic
+  // > 0: only segments with 1 to that many query rows and at least one key; < 0: all but those
+  int32_t short_rows = 0;
   int32_t tile_rows = kTile;  // outer rows per tile in the forward / dQ modes (absorb: 128 / H)
   int32_t cap_items;
   int32_t cap_combine;
@@ -96,7 +98,7 @@ static inline SchedCaps sched_caps(int mode, int total_outer, int total_inner, i
 }
 
 int launch_scheduler(const SchedParams& p, cudaStream_t s);
-// two independent tile lists in one launch (one CTA each)
-int launch_scheduler_pair(const SchedParams& a, const SchedParams& b, cudaStream_t s);
+// three independent tile lists in one launch (one CTA each)
+int launch_scheduler_three(const SchedParams& a, const SchedParams& b, const SchedParams& c, cudaStream_t s);
 
 }  // namespace vafa

@@ -33,6 +33,10 @@ __device__ __forceinline__ Seg load_seg(const SchedParams& p, int s) {
   g.k0 = p.cu_k[s]; g.Lk = p.cu_k[s + 1] - g.k0;
   g.off = g.Lk - g.Lq;
   g.n_tiles = (p.mode == kSchedDkv) ? (g.Lk + kTile - 1) / kTile : (g.Lq + p.tile_rows - 1) / p.tile_rows;
+  if (p.short_rows != 0) {
+    const bool is_short = g.Lq > 0 && g.Lq <= abs(p.short_rows) && g.Lk > 0;
+    if (is_short != (p.short_rows > 0)) g.n_tiles = 0;
+  }
   return g;
 }
 
@@ -372,7 +376,7 @@ __device__ __forceinline__ void sched_build(const SchedParams& p) {
     h.n_combine = s_combine;
     h.n_partial_rows = s_rows;
     h.block_len = bs;
-    h.reserved0 = 0;
+    h.next_item_2 = 0;
     h.next_item = 0;
     h.pad[0] = h.pad[1] = 0;
     *p.header = h;

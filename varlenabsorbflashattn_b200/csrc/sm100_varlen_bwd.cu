@@ -891,8 +891,8 @@ namespace {
 #endif
 
 struct AbsorbBwdWs {
-  size_t hdr_du, hdr_dx, items_du, items_dx, total;
-  int cap_du, cap_dx;
+  size_t hdr_du, hdr_dx, hdr_dxu, items_du, items_dx, items_dxu, total;
+  int cap_du, cap_dx, cap_dxu;
 };
 
 AbsorbBwdWs absorb_bwd_ws(int total_q, int total_k, int n_seg, int H) {
@@ -901,15 +901,22 @@ AbsorbBwdWs absorb_bwd_ws(int total_q, int total_k, int n_seg, int H) {
   w.cap_dx = total_k / kTile + n_seg + 1;
   w.hdr_du = 0;
   w.hdr_dx = 256;
-  w.items_du = 512;
+  w.cap_dxu = n_seg;
+  w.hdr_dxu = 512;
+  w.items_du = 768;
   w.items_dx = w.items_du + align_up((size_t)w.cap_du * sizeof(WorkItem), 256);
-  w.total = w.items_dx + align_up((size_t)w.cap_dx * sizeof(WorkItem), 256);
+  w.items_dxu = w.items_dx + align_up((size_t)w.cap_dx * sizeof(WorkItem), 256);
+  w.total = w.items_dxu + align_up((size_t)w.cap_dxu * sizeof(WorkItem), 256);
   return w;
 }
 
 struct AbsorbBwdSched {
-  SchedParams du, dx;
+  SchedParams du, dx, dxu;
 };
+
+// Users whose stacked query rows fill at most half a tile go through one kernel for dU and dX
+// (sm100_absorb_bwd.cu).  It rounds P / scale, which a 16-bit type holds as well as P unless the scale is extreme.
+bool absorb_one_pass(float scale) { return scale >= 1.f / 256.f && scale <= 256.f; }
 
 AbsorbBwdSched absorb_bwd_sched_params(const AbsorbCoreBwdArgs& a, int sms) {
   const AbsorbBwdWs ws = absorb_bwd_ws(a.total_q, a.total_k, a.n_seg, a.H);
@@ -924,6 +931,15 @@ AbsorbBwdSched absorb_bwd_sched_params(const AbsorbCoreBwdArgs& a, int sms) {
   SchedParams& sk = r.dx;
   sk.mode = kSchedDkv; sk.tile_rows = kTile; sk.cap_items = ws.cap_dx;
   sk.header = (SchedHeader*)(base + ws.hdr_dx); sk.items = (WorkItem*)(base + ws.items_dx);
+  r.dxu = sq;
+  r.dxu.tile_rows = kInner / a.H; r.dxu.cap_items = ws.cap_dxu;
+  r.dxu.header = (SchedHeader*)(base + ws.hdr_dxu); r.dxu.items = (WorkItem*)(base + ws.items_dxu);
+  if (absorb_one_pass(a.scale)) {
+    r.dxu.short_rows = kInner / a.H;
+    sq.short_rows = sk.short_rows = -(kInner / a.H);
+  } else {
+    r.dxu.n_seg = 0;
+  }
   return r;
 }
 
@@ -935,7 +951,7 @@ int launch_absorb_core_bwd(const AbsorbCoreBwdArgs& a, cudaStream_t s) {
   const SchedParams& sq = sch.du;
   const SchedParams& sk = sch.dx;
   int rc;
-  if (!a.lists_built && (rc = launch_scheduler_pair(sq, sk, s))) return rc;
+  if (!a.lists_built && (rc = launch_scheduler_three(sq, sk, sch.dxu, s))) return rc;
 
   CUtensorMap u128, g128, x64, x128, u64, g64;
   if ((rc = encode_tmap_rows(&u128, a.u, a.dtype, a.total_q, a.H, D, kTile / a.H, a.H))) return rc;
@@ -987,7 +1003,18 @@ size_t sm100_absorb_core_bwd_workspace_bytes(int total_q, int total_k, int n_seg
 
 int sm100_absorb_core_bwd_lists(const AbsorbCoreBwdArgs& a, cudaStream_t s) {
   const AbsorbBwdSched sch = absorb_bwd_sched_params(a, resolve_sm_count_bwd(a.sm_count));
-  return launch_scheduler_pair(sch.du, sch.dx, s);
+  return launch_scheduler_three(sch.du, sch.dx, sch.dxu, s);
+}
+
+bool sm100_absorb_one_pass(const AbsorbCoreBwdArgs& a) { return absorb_one_pass(a.scale); }
+
+int sm100_absorb_core_bwd_one_pass(const AbsorbCoreBwdArgs& a, cudaStream_t s) {
+  const int sms = resolve_sm_count_bwd(a.sm_count);
+  const SchedParams list = absorb_bwd_sched_params(a, sms).dxu;
+  const long long pad = sm100_absorb_ld_pad((long long)a.total_q * a.H);
+  const float* nl = reinterpret_cast<const float*>((const float2*)a.ld + pad);
+  return sm100_absorb_dxu_launch({a.u, a.x, a.dax, nl, nl + pad, a.du, a.dx, list.header, list.items, a.total_q, a.total_k, a.H, a.dtype,
+                                  a.x_width, sms, a.which, a.scale, a.status}, s);
 }
 
 int sm100_absorb_core_bwd(const AbsorbCoreBwdArgs& a, cudaStream_t s) {

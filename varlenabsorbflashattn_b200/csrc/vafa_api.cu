@@ -344,6 +344,21 @@ bool absorb_bwd_core_fast(const vafa_absorb_args* a, bool inner) {
   return f.core && f.epilogue && (64 % a->num_heads) == 0 && al(a->d_o) && al(a->dx) && al(a->dq_raw);
 }
 
+// The attention core's backward: the users of few queries on the side stream, the others on the caller's.  Each of the three
+// kernels fills the GPU; which is queued where decides only whose blocks take over the SMs as the other's run out.
+int absorb_core_bwd(const AbsorbCoreBwdArgs& cb, cudaStream_t s) {
+  SideGuard side(s);
+  int rc;
+  if (sm100_absorb_one_pass(cb)) {
+    if ((rc = side_fork(s, &side.ss))) return rc;
+    rc = sm100_absorb_core_bwd_one_pass(cb, side.ss->stream);
+    const int rd = side_done(side.ss);
+    if (rc || rd) return rc ? rc : rd;
+  }
+  if ((rc = sm100_absorb_core_bwd(cb, s))) return rc;
+  return side.join();
+}
+
 // phase: 0 = the whole backward; 1 = everything the weight gradients need (and du); 2 = the rest (dX and
 // dq_raw), reading what phase 1 left in the workspace.  Only the tensor-core chain can be cut: on the
 // other paths phase 1 is the whole backward and phase 2 nothing.
@@ -380,7 +395,7 @@ int absorb_backward(const vafa_absorb_args* a, bool inner, int phase, cudaStream
     cb.ld = ex;
     cb.lists_built = 1;
     cb.which = 2;
-    if ((rc = sm100_absorb_core_bwd(cb, s))) return rc;
+    if ((rc = absorb_core_bwd(cb, s))) return rc;
     void* wqt = ex + x.ld + x.bexp + x.sched + x.tn;
     if ((rc = sm100_transpose(a->w_q, wqt, dq, H * dh, a->dtype, s))) return rc;
     GemmNNArgs gq{dp, wqt, a->dq_raw, Tq, dq, H * dh, dq, dq, a->dtype, 0, a->sm_count};
@@ -419,7 +434,7 @@ int absorb_backward(const vafa_absorb_args* a, bool inner, int phase, cudaStream
     cb.ld = ld;
     cb.which = cut ? 1 : 0;
     if ((rc = side.join())) return rc;
-    if ((rc = sm100_absorb_core_bwd(cb, s))) return rc;
+    if ((rc = absorb_core_bwd(cb, s))) return rc;
   } else {
     // dax_h = dO_h W_V_h^T                  fp32 [T_q, H, d_kv]
     SimtGemm g1{a->d_o, a->w_v, dax, a->dtype, a->dtype, VAFA_F32, Tq, dkv, dh, H,
