@@ -214,6 +214,13 @@ int vafa_cast_from_f32(const float* src, void* dst, size_t n, int32_t dtype, vaf
  * not (the caller words the error), a negative code when the copy failed or the stream is being captured. */
 int vafa_check_cu_seqlens(const int32_t* cu_q, const int32_t* cu_k, int32_t n_seg, int32_t total_q, int32_t total_k,
                           int32_t need_keys, vafa_stream_t stream);
+/* The forward calls with that check in them, done on the device by the first kernel of the call; the host reads
+ * the verdict while the kernels queued behind it run.  Same arguments as vafa_varlen_fwd, vafa_absorb_fwd and
+ * vafa_absorb_inner_fwd (the latter two with need_keys).  Return 1 for bad prefix sums: nothing has been read or
+ * written by them, and the outputs are undefined. */
+int vafa_varlen_fwd_checked(const vafa_varlen_args* a, vafa_stream_t stream);
+int vafa_absorb_fwd_checked(const vafa_absorb_args* a, vafa_stream_t stream);
+int vafa_absorb_inner_fwd_checked(const vafa_absorb_args* a, vafa_stream_t stream);
 int vafa_abi_version(void);
 const char* vafa_last_error(void);           /* thread-local text of the last failure */
 /* Copy the status word to the host (synchronises `stream`) and translate it: returns 0 or

@@ -27,7 +27,7 @@ ABI_VERSION = 3
 EXPORTS = (
     "vafa_abi_version", "vafa_last_error", "vafa_check_status", "vafa_cast_from_f32", "vafa_check_cu_seqlens",
     "vafa_varlen_fwd_workspace_bytes", "vafa_varlen_bwd_workspace_bytes", "vafa_varlen_fwd", "vafa_varlen_bwd",
-    "vafa_varlen_fwd_noalloc",
+    "vafa_varlen_fwd_noalloc", "vafa_varlen_fwd_checked", "vafa_absorb_fwd_checked", "vafa_absorb_inner_fwd_checked",
     "vafa_absorb_saved_bytes", "vafa_absorb_fwd_workspace_bytes", "vafa_absorb_bwd_workspace_bytes",
     "vafa_absorb_fwd", "vafa_absorb_bwd", "vafa_absorb_bwd_phase", "vafa_absorb_inner_fwd", "vafa_absorb_inner_bwd",
     "vafa_profile_enable", "vafa_profile_kernel_count", "vafa_profile_kernel_name", "vafa_profile_read",
@@ -95,13 +95,14 @@ def load() -> C.CDLL:
         for name in ("vafa_varlen_fwd_workspace_bytes", "vafa_varlen_bwd_workspace_bytes"):
             getattr(lib, name).argtypes = [C.POINTER(VarlenArgs)]
             getattr(lib, name).restype = C.c_size_t
-        for name in ("vafa_varlen_fwd", "vafa_varlen_bwd", "vafa_varlen_fwd_noalloc"):
+        for name in ("vafa_varlen_fwd", "vafa_varlen_bwd", "vafa_varlen_fwd_noalloc", "vafa_varlen_fwd_checked"):
             getattr(lib, name).argtypes = [C.POINTER(VarlenArgs), C.c_void_p]
             getattr(lib, name).restype = C.c_int
         for name in ("vafa_absorb_saved_bytes", "vafa_absorb_fwd_workspace_bytes", "vafa_absorb_bwd_workspace_bytes"):
             getattr(lib, name).argtypes = [C.POINTER(AbsorbArgs)]
             getattr(lib, name).restype = C.c_size_t
-        for name in ("vafa_absorb_fwd", "vafa_absorb_bwd", "vafa_absorb_inner_fwd", "vafa_absorb_inner_bwd"):
+        for name in ("vafa_absorb_fwd", "vafa_absorb_bwd", "vafa_absorb_inner_fwd", "vafa_absorb_inner_bwd",
+                     "vafa_absorb_fwd_checked", "vafa_absorb_inner_fwd_checked"):
             getattr(lib, name).argtypes = [C.POINTER(AbsorbArgs), C.c_void_p]
             getattr(lib, name).restype = C.c_int
         lib.vafa_absorb_bwd_phase.argtypes = [C.POINTER(AbsorbArgs), C.c_int32, C.c_void_p]
@@ -196,21 +197,6 @@ def set_check_status(enabled: bool) -> None:
 def maybe_check_status(device: torch.device) -> None:
     if _check_after_each_op:
         check_status(device)
-
-
-def cu_seqlens_ok(cu_q: torch.Tensor, cu_k: torch.Tensor, total_q: int, total_k: int, need_keys: bool) -> bool:
-    """Whether two prefix-sum tensors (1-D int32, contiguous, on one GPU, equally long) describe the batch: one call
-    that copies both to the host and walks them there.  With torch operations on host copies the same checks
-    took over 100 us a call, all of it with the GPU idle behind the copy.  The caller words the error."""
-    n_seg = cu_q.numel() - 1
-    if cu_q.dim() != 1 or cu_k.dim() != 1 or n_seg < 1 or max(total_q, total_k) > 2**31 - 1:
-        return False
-    with on_device(cu_q.device):
-        rc = load().vafa_check_cu_seqlens(cu_q.data_ptr(), cu_k.data_ptr(), n_seg, total_q, total_k, int(need_keys),
-                                          raw_stream(cu_q.device))
-    if rc < 0:
-        check(rc, "vafa_check_cu_seqlens")
-    return rc == 0
 
 
 def workspace(nbytes: int, device: torch.device) -> torch.Tensor | None:

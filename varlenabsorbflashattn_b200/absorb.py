@@ -75,13 +75,19 @@ def _check_cu(cu: torch.Tensor, total: int, name: str) -> torch.Tensor:
 
 def _validate(cu_q, cu_k, T_q, T_k) -> None:
     assert cu_q.numel() == cu_k.numel(), "segment count mismatch q vs k"
-    if cu_q.is_cuda and _lib.cu_seqlens_ok(cu_q, cu_k, T_q, T_k, True):
-        return
     hq = _check_cu(cu_q, T_q, "cu_seqlens_q")
     hk = _check_cu(cu_k, T_k, "cu_seqlens_k")
     # reference: interface.py:109-116
     if bool((((hq[1:] - hq[:-1]) > 0) & ((hk[1:] - hk[:-1]) <= 0)).any()):
         raise ValueError("segments with q_len > 0 must have k_len > 0")
+
+
+def _failed(rc: int, what: str, cu_q, cu_k, T_q: int, T_k: int) -> None:
+    """The error of a forward call that did not return 0: 1 where the library found the prefix sums bad."""
+    if rc > 0:
+        _validate(cu_q, cu_k, T_q, T_k)
+        raise ValueError("cu_seqlens_q / cu_seqlens_k do not describe the batch")
+    _lib.check(rc, what)
 
 
 def _chunk_rows(cu: torch.Tensor, bt: int) -> torch.Tensor:
@@ -101,14 +107,14 @@ def prepare_target_attn_indices(cu_seqlens_q: torch.Tensor, cu_seqlens_k: torch.
     return _chunk_rows(cu_seqlens_q, _BT_Q), _chunk_rows(cu_seqlens_k, _BT_K)
 
 
-def _fill(a: _lib.AbsorbArgs, device, cu_q, cu_k, T_q, T_k, d_q, d_kv, H, D_H, dtype, scale, x_width=0) -> None:
+def _fill(a: _lib.AbsorbArgs, device, cu_q, cu_k, T_q, T_k, d_q, d_kv, H, D_H, dtype, scale, x_width, impl) -> None:
     a.x_width = 0 if x_width == d_kv else x_width
     a.cu_seqlens_q, a.cu_seqlens_k = cu_q.data_ptr(), cu_k.data_ptr()
     a.n_seg, a.total_q, a.total_k = cu_q.numel() - 1, T_q, T_k
     a.d_q, a.d_kv, a.num_heads, a.head_dim = d_q, d_kv, H, D_H
     a.dtype = _lib.DTYPE_CODE[dtype]
     a.scale = float(scale)
-    a.impl = _impl_code()
+    a.impl = impl
     a.sm_count = _lib.sm_count(device)
     a.status = _lib.status_word(device).data_ptr()
 
@@ -117,7 +123,7 @@ class _PackedTargetAttn(torch.autograd.Function):
     """q_raw, X, W_Q, W_K, W_V -> O, with all five gradients from the library."""
 
     @staticmethod
-    def forward(ctx, q_raw, X, W_Q, W_K, W_V, cu_q, cu_k, scale, group):
+    def forward(ctx, q_raw, X, W_Q, W_K, W_V, cu_q, cu_k, scale, group, check, impl):
         lib = _lib.load()
         T_q, d_q = q_raw.shape
         T_k, x_w = X.shape
@@ -128,14 +134,17 @@ class _PackedTargetAttn(torch.autograd.Function):
         lse = torch.empty((T_q, H), dtype=torch.float32, device=dev)
         with _lib.on_device(dev):
             a = _lib.AbsorbArgs()
-            _fill(a, dev, cu_q, cu_k, T_q, T_k, d_q, d_kv, H, D_H, q_raw.dtype, scale, x_w)
-            a.q_raw, a.x, a.w_q, a.w_k, a.w_v = (t.data_ptr() for t in (q_raw, X, W_Q, W_K, W_V))
+            _fill(a, dev, cu_q, cu_k, T_q, T_k, d_q, d_kv, H, D_H, q_raw.dtype, scale, x_w, impl)
+            a.q_raw, a.x = q_raw.data_ptr(), X.data_ptr()
+            a.w_q, a.w_k, a.w_v = W_Q.data_ptr(), W_K.data_ptr(), W_V.data_ptr()
             a.o, a.lse = O.data_ptr(), lse.data_ptr()
             saved = torch.empty(max(1, lib.vafa_absorb_saved_bytes(a)), dtype=torch.uint8, device=dev)
             a.saved = saved.data_ptr()
             ws = _lib.workspace(lib.vafa_absorb_fwd_workspace_bytes(a), dev)
             a.workspace, a.workspace_bytes = _lib.ptr(ws), 0 if ws is None else ws.numel()
-            _lib.check(lib.vafa_absorb_fwd(a, _lib.raw_stream(dev)), "vafa_absorb_fwd")
+            rc = (lib.vafa_absorb_fwd_checked if check else lib.vafa_absorb_fwd)(a, _lib.raw_stream(dev))
+            if rc != 0:
+                _failed(rc, "vafa_absorb_fwd", cu_q, cu_k, T_q, T_k)
             _lib.maybe_check_status(dev)
         ctx.save_for_backward(q_raw, X, W_Q, W_K, W_V, O, lse, cu_q, cu_k, saved)
         ctx.scale, ctx.group = scale, group
@@ -160,7 +169,7 @@ class _PackedTargetAttn(torch.autograd.Function):
         dw = torch.empty(n_wq + 2 * n_wk, dtype=torch.float32, device=dev)
         with _lib.on_device(dev):
             a = _lib.AbsorbArgs()
-            _fill(a, dev, cu_q, cu_k, T_q, T_k, d_q, d_kv, H, D_H, q_raw.dtype, ctx.scale, x_w)
+            _fill(a, dev, cu_q, cu_k, T_q, T_k, d_q, d_kv, H, D_H, q_raw.dtype, ctx.scale, x_w, _impl_code())
             a.q_raw, a.x, a.w_q, a.w_k, a.w_v = (t.data_ptr() for t in (q_raw, X, W_Q, W_K, W_V))
             a.o, a.lse, a.saved, a.d_o = O.data_ptr(), lse.data_ptr(), saved.data_ptr(), dO.data_ptr()
             a.dq_raw, a.dx, a.dw = dq_raw.data_ptr(), dX.data_ptr(), dw.data_ptr()
@@ -186,14 +195,14 @@ class _PackedTargetAttn(torch.autograd.Function):
         dW_Q = dwc[:n_wq].view(d_q, H, D_H)
         dW_K = dwc[n_wq:n_wq + n_wk].view(d_kv, H, D_H)
         dW_V = dwc[n_wq + n_wk:].view(d_kv, H, D_H)
-        return dq_raw, dX, dW_Q, dW_K, dW_V, None, None, None, None
+        return dq_raw, dX, dW_Q, dW_K, dW_V, None, None, None, None, None, None
 
 
 class _TargetAttnInner(torch.autograd.Function):
     """u, X, W_V -> O: counterpart of _TargetAttnFunction (reference interface.py:141-321)."""
 
     @staticmethod
-    def forward(ctx, u, X, W_V, cu_q, cu_k, scale):
+    def forward(ctx, u, X, W_V, cu_q, cu_k, scale, check, impl):
         lib = _lib.load()
         T_q, H, d_kv = u.shape
         T_k, x_w = X.shape
@@ -203,14 +212,16 @@ class _TargetAttnInner(torch.autograd.Function):
         lse = torch.empty((T_q, H), dtype=torch.float32, device=dev)
         with _lib.on_device(dev):
             a = _lib.AbsorbArgs()
-            _fill(a, dev, cu_q, cu_k, T_q, T_k, 0, d_kv, H, D_H, u.dtype, scale, x_w)
+            _fill(a, dev, cu_q, cu_k, T_q, T_k, 0, d_kv, H, D_H, u.dtype, scale, x_w, impl)
             a.q_raw, a.x, a.w_v = u.data_ptr(), X.data_ptr(), W_V.data_ptr()
             a.o, a.lse = O.data_ptr(), lse.data_ptr()
             saved = torch.empty(max(1, lib.vafa_absorb_saved_bytes(a)), dtype=torch.uint8, device=dev)
             a.saved = saved.data_ptr()
             ws = _lib.workspace(lib.vafa_absorb_fwd_workspace_bytes(a), dev)
             a.workspace, a.workspace_bytes = _lib.ptr(ws), 0 if ws is None else ws.numel()
-            _lib.check(lib.vafa_absorb_inner_fwd(a, _lib.raw_stream(dev)), "vafa_absorb_inner_fwd")
+            rc = (lib.vafa_absorb_inner_fwd_checked if check else lib.vafa_absorb_inner_fwd)(a, _lib.raw_stream(dev))
+            if rc != 0:
+                _failed(rc, "vafa_absorb_inner_fwd", cu_q, cu_k, T_q, T_k)
             _lib.maybe_check_status(dev)
         ctx.save_for_backward(u, X, W_V, O, lse, cu_q, cu_k, saved)
         ctx.scale = scale
@@ -233,7 +244,7 @@ class _TargetAttnInner(torch.autograd.Function):
         dw = torch.empty(d_kv * H * D_H, dtype=torch.float32, device=dev)
         with _lib.on_device(dev):
             a = _lib.AbsorbArgs()
-            _fill(a, dev, cu_q, cu_k, T_q, T_k, 0, d_kv, H, D_H, u.dtype, ctx.scale, x_w)
+            _fill(a, dev, cu_q, cu_k, T_q, T_k, 0, d_kv, H, D_H, u.dtype, ctx.scale, x_w, _impl_code())
             a.q_raw, a.x, a.w_v = u.data_ptr(), X.data_ptr(), W_V.data_ptr()
             a.o, a.lse, a.saved, a.d_o = O.data_ptr(), lse.data_ptr(), saved.data_ptr(), dO.data_ptr()
             a.dq_raw, a.dx, a.dw = du.data_ptr(), dX.data_ptr(), dw.data_ptr()
@@ -242,12 +253,13 @@ class _TargetAttnInner(torch.autograd.Function):
             _lib.check(lib.vafa_absorb_inner_bwd(a, _lib.raw_stream(dev)), "vafa_absorb_inner_bwd")
             _lib.maybe_check_status(dev)
         dW_V = dw.view(d_kv, H, D_H).to(u.dtype)
-        return du, dX, dW_V, None, None, None
+        return du, dX, dW_V, None, None, None, None, None
 
 
-def _padded_widths(dtype: torch.dtype, d_q: Optional[int], d_kv: int, H: int) -> Optional[Tuple[Optional[int], int]]:
+def _padded_widths(dtype: torch.dtype, d_q: Optional[int], d_kv: int, H: int,
+                   impl: int = _lib.IMPL_AUTO) -> Optional[Tuple[Optional[int], int]]:
     """(d_q, d_kv) to pad to so that the tcgen05 kernels apply, or None to leave the inputs alone."""
-    if os.environ.get("VAFA_IMPL", "auto").lower() == "simt":
+    if impl == _lib.IMPL_SIMT:
         return None
     if dtype not in (torch.bfloat16, torch.float16) or d_kv > 256 or H < 1 or 128 % H != 0:
         return None
@@ -281,11 +293,14 @@ def _next_pow2(x: int) -> int:
 
 
 def _common_checks(dtype_tensors, device_tensors, D_H, d_kv) -> None:
-    assert all(t.dtype == dtype_tensors[0].dtype for t in dtype_tensors), \
-        "inputs must share dtype, got " + "/".join(str(t.dtype) for t in dtype_tensors)
-    assert dtype_tensors[0].dtype in _lib.DTYPE_CODE, f"dtype {dtype_tensors[0].dtype} not supported"
-    assert all(t.is_cuda for t in device_tensors), "all inputs must be CUDA"
-    assert all(t.device == device_tensors[0].device for t in device_tensors), "inputs must be on same device"
+    dtype, device = dtype_tensors[0].dtype, device_tensors[0].device
+    for t in dtype_tensors:
+        assert t.dtype == dtype, "inputs must share dtype, got " + "/".join(str(t.dtype) for t in dtype_tensors)
+    assert dtype in _lib.DTYPE_CODE, f"dtype {dtype} not supported"
+    for t in device_tensors:
+        assert t.is_cuda, "all inputs must be CUDA"
+    for t in device_tensors:
+        assert t.device == device, "inputs must be on same device"
     assert D_H in _SUPPORTED_D_H, f"D_H {D_H} not supported"
     assert _next_pow2(d_kv) <= 512, f"D_KV={d_kv} pads to {_next_pow2(d_kv)}, which is too large"
 
@@ -317,14 +332,15 @@ def target_attn_inner(
         scale = 1.0 / math.sqrt(D_H)
     cu_q = cu_seqlens_q.to(device=u.device, dtype=torch.int32).contiguous()
     cu_k = cu_seqlens_k.to(device=u.device, dtype=torch.int32).contiguous()
-    if validate:
+    if validate and (cu_q.dim() != 1 or cu_q.numel() < 2 or cu_q.shape != cu_k.shape):
         _validate(cu_q, cu_k, T_q, T_k)
-    pad = _padded_widths(u.dtype, None, d_kv, H)
+    impl = _impl_code()
+    pad = _padded_widths(u.dtype, None, d_kv, H, impl)
     if pad is not None:
         u, W_V = _pad_last(u, pad[1]), _pad_first(W_V, pad[1])
         if not _narrow_x_ok(d_kv, H, D_H, T_q, T_k):
             X = _pad_last(X, pad[1])
-    O, _ = _TargetAttnInner.apply(u.contiguous(), X.contiguous(), W_V.contiguous(), cu_q, cu_k, float(scale))
+    O, _ = _TargetAttnInner.apply(u.contiguous(), X.contiguous(), W_V.contiguous(), cu_q, cu_k, float(scale), validate, impl)
     return O
 
 
@@ -383,14 +399,15 @@ def packed_target_attn(
         scale = 1.0 / math.sqrt(D_H)
     cu_q = cu_seqlens_q.to(device=q_raw.device, dtype=torch.int32).contiguous()
     cu_k = cu_seqlens_k.to(device=q_raw.device, dtype=torch.int32).contiguous()
-    if validate:
+    if validate and (cu_q.dim() != 1 or cu_q.numel() < 2 or cu_q.shape != cu_k.shape):
         _validate(cu_q, cu_k, T_q, T_k)
-    pad = _padded_widths(q_raw.dtype, d_q, d_kv, H)
+    impl = _impl_code()
+    pad = _padded_widths(q_raw.dtype, d_q, d_kv, H, impl)
     if pad is not None:
         q_raw, W_Q = _pad_last(q_raw, pad[0]), _pad_first(W_Q, pad[0])
         W_K, W_V = _pad_first(W_K, pad[1]), _pad_first(W_V, pad[1])
         if not _narrow_x_ok(d_kv, H, D_H, T_q, T_k):
             X = _pad_last(X, pad[1])
     O, _ = _PackedTargetAttn.apply(q_raw.contiguous(), X.contiguous(), W_Q.contiguous(), W_K.contiguous(),
-                                   W_V.contiguous(), cu_q, cu_k, float(scale), weight_grad_group)
+                                   W_V.contiguous(), cu_q, cu_k, float(scale), weight_grad_group, validate, impl)
     return O

@@ -34,6 +34,7 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32) simt_fwd_kernel(SimtAttnP
   const SegInfo s = load_seg(p.cu_q, p.cu_k, seg);
   const int i = row - s.q0;
   int kend = p.causal ? min(s.Lk, i + s.Lk - s.Lq + 1) : s.Lk;
+  if (p.guard && (s.k0 < 0 || (int64_t)s.k0 + kend > p.total_k)) return;
   const int nd = (p.D + 31) >> 5;
   const float c = p.scale * kLog2e;
 

@@ -24,6 +24,7 @@ struct SimtAttnParams {
                   // (scale*dK_h + dV_h) into dk [total_k, D]
   int dtype;      // q/k/v/o/dq/dk/dv
   int do_f32;     // 1: d_o is fp32 regardless of dtype
+  int guard;      // forward: cu_q / cu_k are being checked beside this call: segments that leave the tensors are passed over
 };
 
 int simt_attn_fwd(const SimtAttnParams& p, cudaStream_t s);

@@ -52,6 +52,7 @@ struct TileParams {
   int vec_q, vec_k, vec_v, vec_do, vec_o;   // rows can be read / written four elements at a time
   int causal;
   float scale;
+  int total_q, total_k, guard;  // guard: see SimtAttnParams
 };
 
 template <int DP> struct Dim {
@@ -325,6 +326,9 @@ __global__ void __launch_bounds__(kThreads) tile_fwd_kernel(const TileParams p) 
   const Tile t = find_tile(p, p.cu_q, p.stack);
   if (!t.any) return;  // the same for the whole cluster
   const int q0 = p.cu_q[t.seg], Lq = p.cu_q[t.seg + 1] - q0, k0 = p.cu_k[t.seg], Lk = p.cu_k[t.seg + 1] - k0;
+  if (p.guard && (t.row0 < 0 || q0 < 0 || k0 < 0 || p.cu_q[t.seg + 1] < q0 || p.cu_q[t.seg + 1] > p.total_q ||
+                  p.cu_k[t.seg + 1] < k0 || p.cu_k[t.seg + 1] > p.total_k))
+    return;
   const long long row0 = (long long)q0 * p.stack + t.row0;  // first row of the tile in the whole batch
   const int rows = (int)min((long long)kRows, (long long)Lq * p.stack - t.row0);
   const int i0 = (int)t.row0;  // causal: stack is 1
@@ -726,6 +730,7 @@ inline TileParams tile_params(const SimtAttnParams& a) {
   p.vec_do = vec4(a.d_o, p.do_row, p.do_head, a.D, a.do_f32 ? 4 : es);
   p.vec_o = 0;
   p.causal = a.causal; p.scale = a.scale;
+  p.total_q = a.total_q; p.total_k = a.total_k; p.guard = a.guard;
   p.splits = 1; p.slots = 0;
   return p;
 }

@@ -1,6 +1,7 @@
 // tcgen05 / TMA kernels for sm_100a: host-side launchers.
 #pragma once
 #include "common.cuh"
+#include "sm100_sched.cuh"
 
 namespace vafa {
 
@@ -10,7 +11,8 @@ bool sm100_varlen_bwd_supported(const vafa_varlen_args* a);
 
 size_t sm100_varlen_fwd_workspace_bytes(const vafa_varlen_args* a);
 size_t sm100_varlen_bwd_workspace_bytes(const vafa_varlen_args* a);
-int sm100_varlen_fwd(const vafa_varlen_args* a, cudaStream_t s);
+// check: also look over the prefix sums (not null: see CuCheck)
+int sm100_varlen_fwd(const vafa_varlen_args* a, cudaStream_t s, CuCheck* check = nullptr);
 int sm100_varlen_bwd(const vafa_varlen_args* a, cudaStream_t s);
 // forward with the library's built-in scratch array instead of a workspace
 int sm100_varlen_fwd_noalloc(const vafa_varlen_args* a, cudaStream_t s);
@@ -55,6 +57,7 @@ struct AbsorbCoreArgs {
   int32_t* status;
   int x_width;
   int lists_built;     // the tile list was already built by sm100_absorb_core_fwd_lists() (ordered before this call)
+  CuCheck* check;      // not null: the prefix sums are looked over when the list is built
 };
 size_t sm100_absorb_core_fwd_workspace_bytes(int total_q, int n_seg, int H);
 int sm100_absorb_core_fwd(const AbsorbCoreArgs& a, cudaStream_t s);

@@ -47,6 +47,16 @@ struct alignas(256) SchedHeader {
 
 enum SchedMode { kSchedFwd = 0, kSchedDq = 1, kSchedDkv = 2 };
 
+// A forward call's check of its prefix sums: done by the list builder, whose verdict (0 good, 1 bad) goes to pinned host
+// memory; `done` is recorded behind it, so that the host reads it while the kernels queued behind the builder run.
+// For bad prefix sums the list is empty, and no kernel reads or writes a row.
+struct CuCheck {
+  int32_t* verdict;
+  cudaEvent_t done;
+  int32_t total_q, total_k, need_keys;
+  bool queued;
+};
+
 struct SchedParams {
   const int32_t* cu_q;
   const int32_t* cu_k;
@@ -65,6 +75,8 @@ struct SchedParams {
   SchedHeader* header;
   WorkItem* items;
   CombineUnit* combine;
+  int32_t* verdict = nullptr;  // see CuCheck; null: the prefix sums are taken as they are
+  int32_t check_q = 0, check_k = 0, need_keys = 0;
 };
 
 struct SchedCaps {
@@ -97,7 +109,9 @@ static inline SchedCaps sched_caps(int mode, int total_outer, int total_inner, i
   return c;
 }
 
-int launch_scheduler(const SchedParams& p, cudaStream_t s);
+int launch_scheduler(const SchedParams& p, cudaStream_t s, CuCheck* check = nullptr);
+// the check on its own, for calls that build no list (their kernels pass over segments that leave the tensors)
+int launch_cu_check(const int32_t* cu_q, const int32_t* cu_k, int n_seg, cudaStream_t s, CuCheck* check);
 // three independent tile lists in one launch (one CTA each)
 int launch_scheduler_three(const SchedParams& a, const SchedParams& b, const SchedParams& c, cudaStream_t s);
 

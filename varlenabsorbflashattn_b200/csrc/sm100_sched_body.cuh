@@ -154,6 +154,18 @@ __device__ __forceinline__ void for_each_segment(const SchedParams& p, int G, F 
   }
 }
 
+// Whether the prefix sums are bad, for the whole CTA; the verdict goes to the host.
+__device__ __forceinline__ bool cu_check(const SchedParams& p) {
+  bool bad = threadIdx.x == 0 && (p.cu_q[0] != 0 || p.cu_k[0] != 0 || p.cu_q[p.n_seg] != p.check_q || p.cu_k[p.n_seg] != p.check_k);
+  for (int i = threadIdx.x; i < p.n_seg; i += blockDim.x) {
+    const int q0 = p.cu_q[i], q1 = p.cu_q[i + 1], k0 = p.cu_k[i], k1 = p.cu_k[i + 1];
+    bad = bad || q1 < q0 || k1 < k0 || (p.need_keys && q1 > q0 && k1 == k0);
+  }
+  bad = __syncthreads_or(bad) != 0;
+  if (threadIdx.x == 0) *p.verdict = bad ? 1 : 0;
+  return bad;
+}
+
 __device__ __forceinline__ void sched_build(const SchedParams& p) {
   __shared__ int s_hist[kBuckets];
   __shared__ int s_units, s_items, s_rows, s_bs, s_combine;
@@ -161,6 +173,12 @@ __device__ __forceinline__ void sched_build(const SchedParams& p) {
   __shared__ long long s_blocks;
   __shared__ int s_outer, s_longest;  // outer rows of all tiles, inner blocks of the longest tile
 
+  if (p.verdict != nullptr) {
+    if (cu_check(p)) {
+      if (threadIdx.x == 0) *p.header = SchedHeader{};
+      return;
+    }
+  }
   if (threadIdx.x == 0) { s_units = 0; s_blocks = 0; s_combine = 0; s_outer = 0; s_longest = 0; }
   for (int b = threadIdx.x; b < kBuckets; b += kSchedThreads) s_hist[b] = 0;
   __syncthreads();

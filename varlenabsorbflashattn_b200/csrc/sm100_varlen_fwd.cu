@@ -1333,7 +1333,7 @@ int resolve_sm_count(int given) {
 // `scratch` == nullptr: the caller's workspace with the default layout; otherwise the given
 // buffer of `scratch_bytes` with a layout shrunk to fit it.
 template <typename T, int D>
-int launch_fwd(const vafa_varlen_args* a, cudaStream_t s, void* scratch = nullptr, size_t scratch_bytes = 0) {
+int launch_fwd(const vafa_varlen_args* a, cudaStream_t s, void* scratch = nullptr, size_t scratch_bytes = 0, CuCheck* check = nullptr) {
   const int sms = resolve_sm_count(a->sm_count);
   const FwdWorkspace ws = fwd_workspace(a, sms, scratch ? scratch_bytes : 0);
   char* base = scratch ? (char*)scratch : (char*)a->workspace;
@@ -1350,7 +1350,7 @@ int launch_fwd(const vafa_varlen_args* a, cudaStream_t s, void* scratch = nullpt
   // long query segments: tiles of 256 rows, worked on as two 128-row tiles per CTA
   const bool pair = fwd_pair_enabled() && stack == 1 && (long long)a->total_q > 160LL * a->n_seg;
   if (pair) sp.tile_rows = 2 * kTile;
-  int rc = launch_scheduler(sp, s);
+  int rc = launch_scheduler(sp, s, check);
   if (rc) return rc;
 
   CUtensorMap tq, tk, tv;
@@ -1440,7 +1440,7 @@ int launch_absorb_core_fwd(const AbsorbCoreArgs& a, cudaStream_t s) {
   constexpr int D = 256;
   const int sms = resolve_sm_count(a.sm_count);
   const SchedParams sp = absorb_fwd_sched_params(a, sms);
-  int rc = a.lists_built ? 0 : launch_scheduler(sp, s);
+  int rc = a.lists_built ? 0 : launch_scheduler(sp, s, a.check);
   if (rc) return rc;
   CUtensorMap tu, tx;
   if ((rc = encode_tmap_rows(&tu, a.u, a.dtype, a.total_q, a.H, D, kTile / a.H, a.H))) return rc;
@@ -1481,7 +1481,7 @@ int launch_absorb_core_fwd(const AbsorbCoreArgs& a, cudaStream_t s) {
 size_t sm100_absorb_core_fwd_workspace_bytes(int total_q, int n_seg, int H) { return absorb_core_ws(total_q, n_seg, H).total; }
 
 int sm100_absorb_core_fwd_lists(const AbsorbCoreArgs& a, cudaStream_t s) {
-  return launch_scheduler(absorb_fwd_sched_params(a, resolve_sm_count(a.sm_count)), s);
+  return launch_scheduler(absorb_fwd_sched_params(a, resolve_sm_count(a.sm_count)), s, a.check);
 }
 
 int sm100_absorb_core_fwd(const AbsorbCoreArgs& a, cudaStream_t s) {
@@ -1501,11 +1501,11 @@ size_t sm100_varlen_fwd_workspace_bytes(const vafa_varlen_args* a) {
   return fwd_workspace(a, resolve_sm_count(a->sm_count)).total;
 }
 
-int sm100_varlen_fwd(const vafa_varlen_args* a, cudaStream_t s) {
+int sm100_varlen_fwd(const vafa_varlen_args* a, cudaStream_t s, CuCheck* check) {
   if (a->dtype == VAFA_BF16) {
-    return a->head_dim == 128 ? launch_fwd<__nv_bfloat16, 128>(a, s) : launch_fwd<__nv_bfloat16, 64>(a, s);
+    return a->head_dim == 128 ? launch_fwd<__nv_bfloat16, 128>(a, s, nullptr, 0, check) : launch_fwd<__nv_bfloat16, 64>(a, s, nullptr, 0, check);
   }
-  return a->head_dim == 128 ? launch_fwd<__half, 128>(a, s) : launch_fwd<__half, 64>(a, s);
+  return a->head_dim == 128 ? launch_fwd<__half, 128>(a, s, nullptr, 0, check) : launch_fwd<__half, 64>(a, s, nullptr, 0, check);
 }
 
 // ---------------- forward without any allocation by anyone ------------------------------------

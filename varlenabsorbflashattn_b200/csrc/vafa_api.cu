@@ -249,9 +249,13 @@ size_t absorb_fwd_ws_bytes(const vafa_absorb_args* a, bool inner) {
   return n;
 }
 
-int absorb_forward(const vafa_absorb_args* a, bool inner, cudaStream_t s) {
+int absorb_forward(const vafa_absorb_args* a, bool inner, cudaStream_t s, CuCheck* check = nullptr) {
   const AbsorbSizes z = absorb_sizes(a);
   const AbsorbFast fast = absorb_fast(a, inner);
+  if (check != nullptr && !fast.core) {
+    const int rc = launch_cu_check(a->cu_seqlens_q, a->cu_seqlens_k, a->n_seg, s, check);
+    if (rc) return rc;
+  }
   char* sv = (char*)a->saved;
   char* ws = (char*)a->workspace;
   const int H = a->num_heads, dh = a->head_dim, dkv = a->d_kv, Tq = a->total_q;
@@ -261,7 +265,7 @@ int absorb_forward(const vafa_absorb_args* a, bool inner, cudaStream_t s) {
   // the tile list is built on the side stream while the projection runs
   SideGuard side(s);
   AbsorbCoreArgs c{nullptr, a->x, nullptr, a->lse, a->cu_seqlens_q, a->cu_seqlens_k, a->n_seg, Tq, a->total_k, H, a->dtype,
-                   a->scale, a->sm_count, nullptr, a->status, x_width_of(a), 0};
+                   a->scale, a->sm_count, nullptr, a->status, x_width_of(a), 0, check};
   if (fast.core) {
     c.workspace = ws + ((!inner && fast.prologue) ? align_up((size_t)a->d_q * H * dkv * elem_size(a->dtype), 256) : 0);
     if (!inner) {
@@ -306,6 +310,7 @@ int absorb_forward(const vafa_absorb_args* a, bool inner, cudaStream_t s) {
     if ((rc = sm100_absorb_core_fwd(c, s))) return rc;
   } else {
     SimtAttnParams p = simt_from_absorb(a, u, axn);
+    p.guard = check != nullptr;
     if ((rc = simt_attn_fwd(p, s))) return rc;
   }
   if (fast.epilogue) {
@@ -317,6 +322,53 @@ int absorb_forward(const vafa_absorb_args* a, bool inner, cudaStream_t s) {
   SimtGemm g3{axn, a->w_v, a->o, a->dtype, a->dtype, a->dtype, Tq, dh, dkv, H,
               (int64_t)H * dkv, 1, dkv, (int64_t)H * dh, 1, dh, (int64_t)H * dh, 1, dh, 1.f};
   return simt_gemm(g3, s);
+}
+
+// Where the verdict of a checked forward call arrives: one pinned word and one event per thread and device (a call
+// waits for its verdict before it returns, so a thread has one at a time).  Given back when the thread ends.
+struct VerdictSlot {
+  int32_t* word = nullptr;
+  cudaEvent_t done = nullptr;
+  ~VerdictSlot() {
+    if (done) cudaEventDestroy(done);
+    if (word) cudaFreeHost(word);
+  }
+};
+
+// Runs `launch(CuCheck*)`, which queues the list builder and the kernels behind it, then waits for the builder's verdict.
+// Returns 1 for bad prefix sums.  The GPU has the call's kernels to run while the host waits: with the arrays copied
+// to the host and walked there first, it stood idle for the 60-100 us until the first launch, on every call.
+template <typename F>
+int checked(int total_q, int total_k, int need_keys, F launch) {
+  static thread_local VerdictSlot slots[kMaxSideDevices];
+  int dev = -1;
+  VAFA_CUDA_CHECK(cudaGetDevice(&dev));
+  if (dev < 0 || dev >= kMaxSideDevices) return fail(VAFA_ERR_UNSUPPORTED, "device ordinal %d out of range", dev);
+  VerdictSlot& slot = slots[dev];
+  if (!slot.word) {
+    // (another thread may be capturing a stream, which an allocation would otherwise break)
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    VAFA_CUDA_CHECK(cudaThreadExchangeStreamCaptureMode(&mode));
+    cudaError_t e = slot.done ? cudaSuccess : cudaEventCreateWithFlags(&slot.done, cudaEventDisableTiming);
+    if (e == cudaSuccess) e = cudaHostAlloc((void**)&slot.word, sizeof(int32_t), cudaHostAllocPortable | cudaHostAllocMapped);
+    cudaThreadExchangeStreamCaptureMode(&mode);
+    VAFA_CUDA_CHECK(e);
+  }
+  *(volatile int32_t*)slot.word = 1;
+  CuCheck c{slot.word, slot.done, total_q, total_k, need_keys, false};
+  const int rc = launch(&c);
+  // (on an error behind the builder's launch too: its write must not meet the next call's word)
+  if (c.queued) VAFA_CUDA_CHECK(cudaEventSynchronize(slot.done));
+  if (rc) return rc;
+  return *(volatile int32_t*)slot.word != 0 ? 1 : 0;
+}
+
+int not_while_captured(cudaStream_t s) {
+  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+  VAFA_CUDA_CHECK(cudaStreamIsCapturing(s, &cap));
+  if (cap != cudaStreamCaptureStatusNone)
+    return fail(VAFA_ERR_CUDA, "cu_seqlens cannot be checked on the host while the stream is captured: switch the check off");
+  return 0;
 }
 
 // Extra backward scratch of the tcgen05 path, placed after the regions both paths share.
@@ -518,17 +570,26 @@ size_t vafa_varlen_bwd_workspace_bytes(const vafa_varlen_args* a) {
   return align_up((size_t)a->total_q * a->num_heads * 4, 256);
 }
 
-int vafa_varlen_fwd(const vafa_varlen_args* a, vafa_stream_t stream) {
+static int varlen_fwd_call(const vafa_varlen_args* a, bool check, cudaStream_t s) {
   int rc = check_varlen(a, false);
   if (rc) return rc;
-  cudaStream_t s = (cudaStream_t)stream;
   const int impl = pick_impl(a->impl, varlen_fwd_tc_ok(a), "varlen_fwd");
   if (impl < 0) return impl;
   if (impl == 0 && is_gqa(a)) return fail(VAFA_ERR_UNSUPPORTED, "num_kv_heads != num_heads needs the tcgen05 kernels (bf16/fp16, head_dim 64/128)");
   if ((rc = need_ws(a->workspace, a->workspace_bytes, vafa_varlen_fwd_workspace_bytes(a)))) return rc;
-  if (impl == 1) return sm100_varlen_fwd(a, s);
-  return simt_attn_fwd(simt_from_varlen(a), s);
+  SimtAttnParams p = simt_from_varlen(a);
+  if (!check) return impl == 1 ? sm100_varlen_fwd(a, s) : simt_attn_fwd(p, s);
+  if ((rc = not_while_captured(s))) return rc;
+  return checked(a->total_q, a->total_k, 0, [&](CuCheck* c) -> int {
+    if (impl == 1) return sm100_varlen_fwd(a, s, c);
+    if (const int e = launch_cu_check(a->cu_seqlens_q, a->cu_seqlens_k, a->n_seg, s, c)) return e;
+    p.guard = 1;
+    return simt_attn_fwd(p, s);
+  });
 }
+
+int vafa_varlen_fwd(const vafa_varlen_args* a, vafa_stream_t stream) { return varlen_fwd_call(a, false, (cudaStream_t)stream); }
+int vafa_varlen_fwd_checked(const vafa_varlen_args* a, vafa_stream_t stream) { return varlen_fwd_call(a, true, (cudaStream_t)stream); }
 
 int vafa_varlen_fwd_noalloc(const vafa_varlen_args* a, vafa_stream_t stream) {
   int rc = check_varlen(a, false);
@@ -584,15 +645,21 @@ static int check_x_width(const vafa_absorb_args* a, bool fast) {
   return 0;
 }
 
-int vafa_absorb_fwd(const vafa_absorb_args* a, vafa_stream_t stream) {
-  int rc = check_absorb(a, false, false);
+static int absorb_fwd_call(const vafa_absorb_args* a, bool inner, bool check, cudaStream_t s) {
+  int rc = check_absorb(a, false, inner);
   if (rc) return rc;
-  if ((rc = check_x_width(a, absorb_fast(a, false).core))) return rc;
-  const int impl = pick_impl(a->impl, absorb_fast(a, false).core, "absorb_fwd");
+  const bool core = absorb_fast(a, inner).core;
+  if ((rc = check_x_width(a, core))) return rc;
+  const int impl = pick_impl(a->impl, core, inner ? "absorb_inner_fwd" : "absorb_fwd");
   if (impl < 0) return impl;
-  if ((rc = need_ws(a->workspace, a->workspace_bytes, absorb_fwd_ws_bytes(a, false)))) return rc;
-  return absorb_forward(a, false, (cudaStream_t)stream);
+  if ((rc = need_ws(a->workspace, a->workspace_bytes, absorb_fwd_ws_bytes(a, inner)))) return rc;
+  if (!check) return absorb_forward(a, inner, s);
+  if ((rc = not_while_captured(s))) return rc;
+  return checked(a->total_q, a->total_k, 1, [&](CuCheck* c) { return absorb_forward(a, inner, s, c); });
 }
+
+int vafa_absorb_fwd(const vafa_absorb_args* a, vafa_stream_t stream) { return absorb_fwd_call(a, false, false, (cudaStream_t)stream); }
+int vafa_absorb_fwd_checked(const vafa_absorb_args* a, vafa_stream_t stream) { return absorb_fwd_call(a, false, true, (cudaStream_t)stream); }
 int vafa_absorb_bwd(const vafa_absorb_args* a, vafa_stream_t stream) {
   int rc = check_absorb(a, true, false);
   if (rc) return rc;
@@ -612,15 +679,8 @@ int vafa_absorb_bwd_phase(const vafa_absorb_args* a, int32_t phase, vafa_stream_
   if ((rc = need_ws(a->workspace, a->workspace_bytes, vafa_absorb_bwd_workspace_bytes(a)))) return rc;
   return absorb_backward(a, false, phase, (cudaStream_t)stream);
 }
-int vafa_absorb_inner_fwd(const vafa_absorb_args* a, vafa_stream_t stream) {
-  int rc = check_absorb(a, false, true);
-  if (rc) return rc;
-  if ((rc = check_x_width(a, absorb_fast(a, true).core))) return rc;
-  const int impl = pick_impl(a->impl, absorb_fast(a, true).core, "absorb_inner_fwd");
-  if (impl < 0) return impl;
-  if ((rc = need_ws(a->workspace, a->workspace_bytes, absorb_fwd_ws_bytes(a, true)))) return rc;
-  return absorb_forward(a, true, (cudaStream_t)stream);
-}
+int vafa_absorb_inner_fwd(const vafa_absorb_args* a, vafa_stream_t stream) { return absorb_fwd_call(a, true, false, (cudaStream_t)stream); }
+int vafa_absorb_inner_fwd_checked(const vafa_absorb_args* a, vafa_stream_t stream) { return absorb_fwd_call(a, true, true, (cudaStream_t)stream); }
 int vafa_absorb_inner_bwd(const vafa_absorb_args* a, vafa_stream_t stream) {
   int rc = check_absorb(a, true, true);
   if (rc) return rc;
@@ -640,10 +700,7 @@ int vafa_check_cu_seqlens(const int32_t* cu_q, const int32_t* cu_k, int32_t n_se
                           int32_t need_keys, vafa_stream_t stream) {
   if (!cu_q || !cu_k || n_seg < 1) return fail(VAFA_ERR_INVALID, "check_cu_seqlens: null array or n_seg %d", n_seg);
   const cudaStream_t s = (cudaStream_t)stream;
-  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-  VAFA_CUDA_CHECK(cudaStreamIsCapturing(s, &cap));
-  if (cap != cudaStreamCaptureStatusNone)
-    return fail(VAFA_ERR_CUDA, "cu_seqlens cannot be checked on the host while the stream is captured: switch the check off");
+  if (const int rc = not_while_captured(s)) return rc;
   const size_t n = (size_t)n_seg + 1;
   std::vector<int32_t> host;
   try {

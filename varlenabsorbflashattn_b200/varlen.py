@@ -90,6 +90,13 @@ def _check_cu(cu: torch.Tensor, total: int, name: str) -> None:
         raise ValueError(f"{name} must be non-decreasing (found negative segment length)")
 
 
+def _refuse_cu(cu_q: torch.Tensor, cu_k: torch.Tensor, T_q: int, T_k: int) -> None:
+    """The error for prefix sums that the library found bad."""
+    _check_cu(cu_q, T_q, "cu_seqlens_q")
+    _check_cu(cu_k, T_k, "cu_seqlens_k")
+    raise ValueError("cu_seqlens_q / cu_seqlens_k do not describe the batch")
+
+
 def _as_thd(x: torch.Tensor, name: str) -> Tuple[torch.Tensor, bool]:
     # reference: interface.py:121-150
     if x.dim() == 4:
@@ -143,9 +150,9 @@ class _PackedVarlenAttn(torch.autograd.Function):
         cu_k = cu_k.to(device=q.device, dtype=torch.int32).contiguous()
         assert cu_k.numel() == cu_q.numel(), \
             f"segment count mismatch: q has {cu_q.numel() - 1}, k has {cu_k.numel() - 1}"
-        if _validate and not _lib.cu_seqlens_ok(cu_q, cu_k, T_q, T_k, False):
-            _check_cu(cu_q, T_q, "cu_seqlens_q")
-            _check_cu(cu_k, T_k, "cu_seqlens_k")
+        check = _validate
+        if check and (cu_q.dim() != 1 or cu_q.numel() < 2 or cu_k.dim() != 1):
+            _refuse_cu(cu_q, cu_k, T_q, T_k)
 
         lib = _lib.load()
         o = torch.empty_like(q)
@@ -154,7 +161,10 @@ class _PackedVarlenAttn(torch.autograd.Function):
             a = _fill_args(q, k, v, o, lse, cu_q, cu_k, scale, causal, split_k_block)
             ws = _lib.workspace(lib.vafa_varlen_fwd_workspace_bytes(a), q.device)
             a.workspace, a.workspace_bytes = _lib.ptr(ws), 0 if ws is None else ws.numel()
-            _lib.check(lib.vafa_varlen_fwd(a, _lib.raw_stream(q.device)), "vafa_varlen_fwd")
+            rc = (lib.vafa_varlen_fwd_checked if check else lib.vafa_varlen_fwd)(a, _lib.raw_stream(q.device))
+            if rc > 0:
+                _refuse_cu(cu_q, cu_k, T_q, T_k)
+            _lib.check(rc, "vafa_varlen_fwd")
             _lib.maybe_check_status(q.device)
         ctx.save_for_backward(q, k, v, o, lse, cu_q, cu_k)
         ctx.scale, ctx.causal, ctx.split_k_block = scale, causal, split_k_block
