@@ -50,7 +50,8 @@ struct GemmParams {
   int ldc;
   int n_tiles;     // N / 256
   int m_tiles;     // ceil(M / 128)
-  int k_chunks;    // K / 64
+  int k_chunks;    // K / 64, or those of a column tile's block
+  int k_block;     // rows of B between the blocks of neighbouring column tiles, 0: B is full
   int diag_heads;  // 0: full rows
   int wait_limit;  // bound of every device-side wait, in units of 65536 cycles
 };
@@ -95,12 +96,13 @@ gemm_nn_k256_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
   const int groups = gridDim.x / p.n_tiles;  // CTAs per column tile (grid is a multiple of n_tiles)
   const int n_tile = blockIdx.x % p.n_tiles;
   const int m_first = blockIdx.x / p.n_tiles;
+  const int kc0 = n_tile * p.k_block / kChunk;
   const uint32_t buf0 = smem_u32(sm.buf);
 
   if (warp == 4) {
     if (lane == 0) {
       auto load_b = [&](uint32_t dst, uint32_t bar, int kc) {
-        for (int c = 0; c < 4; ++c) tma_load_3d(dst + c * kBSub, &tmap_b, bar, n_tile * kNTile + c * 64, 0, kc * kChunk);
+        for (int c = 0; c < 4; ++c) tma_load_3d(dst + c * kBSub, &tmap_b, bar, n_tile * kNTile + c * 64, 0, (kc0 + kc) * kChunk);
       };
       uint32_t it = 0;
       bool alive = true;
@@ -109,7 +111,7 @@ gemm_nn_k256_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
           const uint32_t slot = it % kSlots, bar = smem_u32(&sm.full[0]) + slot * 8, dst = buf0 + kFirst + slot * kSlot;
           if (!mbar_wait(smem_u32(&sm.empty[0]) + slot * 8, ((it / kSlots) & 1) ^ 1, abort_flag)) { alive = false; break; }
           mbar_expect_tx(bar, kSlot);
-          tma_load_3d(dst, &tmap_a, bar, kc * kChunk, 0, m * 128);
+          tma_load_3d(dst, &tmap_a, bar, (kc0 + kc) * kChunk, 0, m * 128);
           if (!kResident) load_b(dst + kAChunk, bar, kc);
           if (kResident && m == m_first) {
             const uint32_t b_bar = smem_u32(&sm.b_full[kc]);
@@ -221,6 +223,8 @@ int sm100_gemm_nn_k256(const GemmNNArgs& g, cudaStream_t s) {
   if (g.M <= 0) return 0;
   if (g.N % kNTile != 0 || (g.diag_heads > 0 && (g.N != kNTile || (kNTile / g.diag_heads) % 32 != 0)))
     return fail(VAFA_ERR_UNSUPPORTED, "gemm_nn_k256: N=%d diag_heads=%d not supported", g.N, g.diag_heads);
+  if (g.k_block > 0 && (g.lda != kK || (g.N / kNTile) * g.k_block != kK || (kChunk % g.k_block != 0 && g.k_block % kChunk != 0)))
+    return fail(VAFA_ERR_UNSUPPORTED, "gemm_nn_k256: blocks of %d rows not supported", g.k_block);
   int sms = g.sm_count;
   if (sms <= 0) {
     int dev = 0;
@@ -231,7 +235,8 @@ int sm100_gemm_nn_k256(const GemmNNArgs& g, cudaStream_t s) {
   p.wait_limit = wait_limit_units();
   p.C = g.C; p.M = g.M; p.ldc = g.ldc; p.n_tiles = g.N / kNTile; p.m_tiles = (int)((g.M + 127) / 128);
   p.diag_heads = g.diag_heads;
-  p.k_chunks = g.lda / kChunk;
+  p.k_block = g.k_block;
+  p.k_chunks = g.k_block > 0 ? (g.k_block + kChunk - 1) / kChunk : g.lda / kChunk;
   int groups = sms / p.n_tiles;
   if (groups < 1) groups = 1;
   if (groups > p.m_tiles) groups = p.m_tiles;

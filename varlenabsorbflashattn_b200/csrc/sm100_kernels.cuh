@@ -114,6 +114,8 @@ struct GemmNNArgs {
   const void* A; const void* B; void* C;
   long long M; int N; int lda, ldb, ldc;
   int dtype; int diag_heads; int sm_count;
+  int k_block = 0;  // > 0: B is block diagonal, column tile j has rows [j k_block, (j + 1) k_block) only (K = 256; 32 or a
+                    // multiple of 64): the products with its zero rows are left out
 };
 int sm100_gemm_nn_k256(const GemmNNArgs& g, cudaStream_t s);
 

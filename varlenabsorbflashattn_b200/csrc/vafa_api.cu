@@ -373,7 +373,7 @@ int not_while_captured(cudaStream_t s) {
 
 // Extra backward scratch of the tcgen05 path, placed after the regions both paths share.
 struct AbsorbBwdExtra {
-  size_t ld, bexp, sched, tn, wqt;
+  size_t ld, bexp, sched, tn, wqt, tnv;
 };
 
 AbsorbBwdExtra absorb_bwd_extra(const vafa_absorb_args* a) {
@@ -386,6 +386,7 @@ AbsorbBwdExtra absorb_bwd_extra(const vafa_absorb_args* a) {
   const int q_chunks = a->d_q >= 256 ? a->d_q / 256 : 1;
   const size_t t2 = sm100_gemm_tn_workspace_bytes(a->total_q, q_chunks, 256, a->sm_count);
   x.tn = t1 > t2 ? t1 : t2;
+  x.tnv = t1;  // dW_V's own: it runs beside the rest
   x.wqt = align_up((size_t)256 * (a->d_q > 256 ? a->d_q : 256) * elem_size(a->dtype), 256);
   return x;
 }
@@ -409,6 +410,20 @@ int absorb_core_bwd(const AbsorbCoreBwdArgs& cb, cudaStream_t s) {
   }
   if ((rc = sm100_absorb_core_bwd(cb, s))) return rc;
   return side.join();
+}
+
+// The parts of the backward that wait for nothing but the forward: dW_V, p = q_raw W_Q (into `saved`), and W_Q^T (at `wqt`, with
+// dW_V's scratch behind it).
+int absorb_bwd_beside(const vafa_absorb_args* a, bool inner, const void* axn, char* wqt, float* dWV, cudaStream_t s) {
+  const int H = a->num_heads, dh = a->head_dim, Tq = a->total_q, dq = a->d_q;
+  int rc;
+  // dW_V[kv,h,dd] = sum_t axn[t,h,kv] dO[t,h,dd]
+  GemmTNArgs tv{axn, a->d_o, dWV, wqt + absorb_bwd_extra(a).wqt, Tq, a->dtype, H, H, 64, 32, H * dh, dh, dh, (long long)H * dh, a->sm_count};
+  if ((rc = sm100_gemm_tn(tv, s))) return rc;
+  if (inner) return 0;
+  GemmNNArgs gp{a->q_raw, a->w_q, a->saved, Tq, H * dh, dq, H * dh, H * dh, a->dtype, 0, a->sm_count};
+  if ((rc = sm100_gemm_nn_k256(gp, s))) return rc;
+  return sm100_transpose(a->w_q, wqt, dq, H * dh, a->dtype, s);
 }
 
 // phase: 0 = the whole backward; 1 = everything the weight gradients need (and du); 2 = the rest (dX and
@@ -448,8 +463,7 @@ int absorb_backward(const vafa_absorb_args* a, bool inner, int phase, cudaStream
     cb.lists_built = 1;
     cb.which = 2;
     if ((rc = absorb_core_bwd(cb, s))) return rc;
-    void* wqt = ex + x.ld + x.bexp + x.sched + x.tn;
-    if ((rc = sm100_transpose(a->w_q, wqt, dq, H * dh, a->dtype, s))) return rc;
+    void* wqt = ex + x.ld + x.bexp + x.sched + x.tn;  // transposed in phase 1
     GemmNNArgs gq{dp, wqt, a->dq_raw, Tq, dq, H * dh, dq, dq, a->dtype, 0, a->sm_count};
     return sm100_gemm_nn_k256(gq, s);
   }
@@ -462,16 +476,11 @@ int absorb_backward(const vafa_absorb_args* a, bool inner, int phase, cudaStream
     if (rc || rd) return rc ? rc : rd;
     cb.lists_built = 1;
   }
-  if (!inner && absorb_fast(a, false).prologue) {
-    // the tcgen05 prologue goes straight to u; the weight-gradient chain below needs p = q_raw W_Q
-    if (fast_chain) {
-      GemmNNArgs gp{a->q_raw, a->w_q, sv, Tq, H * dh, dq, H * dh, H * dh, a->dtype, 0, a->sm_count};
-      if ((rc = sm100_gemm_nn_k256(gp, s))) return rc;
-    } else {
-      SimtGemm gp{a->q_raw, a->w_q, sv, a->dtype, a->dtype, a->dtype, Tq, H * dh, dq, 1,
-                  dq, 1, 0, (int64_t)H * dh, 1, 0, (int64_t)H * dh, 1, 0, 1.f};
-      if ((rc = simt_gemm(gp, s))) return rc;
-    }
+  if (!inner && absorb_fast(a, false).prologue && !fast_chain) {
+    // the tcgen05 prologue goes straight to u; the weight gradients need p = q_raw W_Q
+    SimtGemm gp{a->q_raw, a->w_q, sv, a->dtype, a->dtype, a->dtype, Tq, H * dh, dq, 1,
+                dq, 1, 0, (int64_t)H * dh, 1, 0, (int64_t)H * dh, 1, 0, 1.f};
+    if ((rc = simt_gemm(gp, s))) return rc;
   }
   if (absorb_bwd_core_fast(a, inner)) {
     // tcgen05 path: dAlphaX = dO . Bexp (one dense product over all heads), then the dU and dX kernels
@@ -480,13 +489,23 @@ int absorb_backward(const vafa_absorb_args* a, bool inner, int phase, cudaStream
     void* ld = ex;
     void* bexp = ex + x.ld;
     if ((rc = sm100_absorb_expand_wv(a->w_v, bexp, H, dh, dkv, a->dtype, s))) return rc;
-    GemmNNArgs gd{a->d_o, bexp, dax, Tq, H * dkv, H * dh, H * dkv, H * dkv, a->dtype, 0, a->sm_count};
+    GemmNNArgs gd{a->d_o, bexp, dax, Tq, H * dkv, H * dh, H * dkv, H * dkv, a->dtype, 0, a->sm_count, dh};
     if ((rc = sm100_gemm_nn_k256(gd, s))) return rc;
     if ((rc = sm100_absorb_ld(a->o, a->d_o, a->lse, ld, (long long)Tq * H, dh, a->scale, a->dtype, s))) return rc;
     cb.ld = ld;
     cb.which = cut ? 1 : 0;
-    if ((rc = side.join())) return rc;
+    SideStream* const ss = side.ss;
+    if ((rc = side.join())) return rc;  // the lists
+    if (fast_chain) {
+      // what needs the forward's results only, beside the products above and the kernels below (1024 users of 1-16 queries: about
+      // 30 us of launches and gaps that stood in the row before)
+      rc = absorb_bwd_beside(a, inner, axn, ex + x.ld + x.bexp + x.sched + x.tn, dWV, ss->stream);
+      const int rd = side_done(ss);
+      side.ss = ss;
+      if (rc || rd) return rc ? rc : rd;
+    }
     if ((rc = absorb_core_bwd(cb, s))) return rc;
+    if ((rc = side.join())) return rc;
   } else {
     // dax_h = dO_h W_V_h^T                  fp32 [T_q, H, d_kv]
     SimtGemm g1{a->d_o, a->w_v, dax, a->dtype, a->dtype, VAFA_F32, Tq, dkv, dh, H,
@@ -503,9 +522,6 @@ int absorb_backward(const vafa_absorb_args* a, bool inner, int phase, cudaStream
     char* ex = ws + z.dax + z.delta + z.du + z.dp + x.ld + x.bexp + x.sched;
     void* tn_ws = ex;
     void* wqt = ex + x.tn;
-    // dW_V[kv,h,dd] = sum_t axn[t,h,kv] dO[t,h,dd]
-    GemmTNArgs tv{axn, a->d_o, dWV, tn_ws, Tq, a->dtype, H, H, 64, 32, H * dh, dh, dh, (long long)H * dh, a->sm_count};
-    if ((rc = sm100_gemm_tn(tv, s))) return rc;
     if (inner) return 0;
     // dp[(t,h), dd] = sum_kv du[t,h,kv] W_K[kv,h,dd]: stacked rows against all of W_K, own head's block kept
     GemmNNArgs gdp{du, a->w_k, dp, (long long)Tq * H, H * dh, dkv, H * dh, dh, a->dtype, H, a->sm_count};
@@ -521,7 +537,6 @@ int absorb_backward(const vafa_absorb_args* a, bool inner, int phase, cudaStream
     if ((rc = sm100_gemm_tn(tq, s))) return rc;
     if (cut) return 0;  // phase 1 ends with the last weight gradient
     // dq_raw = dp W_Q^T   (W_Q is [d_q, H*D_H]; its transpose [H*D_H, d_q])
-    if ((rc = sm100_transpose(a->w_q, wqt, dq, H * dh, a->dtype, s))) return rc;
     GemmNNArgs gq{dp, wqt, a->dq_raw, Tq, dq, H * dh, dq, dq, a->dtype, 0, a->sm_count};
     return sm100_gemm_nn_k256(gq, s);
   }
@@ -631,7 +646,7 @@ size_t vafa_absorb_bwd_workspace_bytes(const vafa_absorb_args* a) {
   size_t n = z.dax + z.delta + z.du + z.dp;
   if (a->impl != VAFA_IMPL_SIMT && a->d_kv == 256 && a->dtype != VAFA_F32) {
     const AbsorbBwdExtra x = absorb_bwd_extra(a);
-    n += x.ld + x.bexp + x.sched + x.tn + x.wqt;
+    n += x.ld + x.bexp + x.sched + x.tn + x.wqt + x.tnv;
   }
   return n;
 }
