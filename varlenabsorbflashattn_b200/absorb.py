@@ -149,11 +149,14 @@ class _PackedTargetAttn(torch.autograd.Function):
         ctx.save_for_backward(q_raw, X, W_Q, W_K, W_V, O, lse, cu_q, cu_k, saved)
         ctx.scale, ctx.group = scale, group
         ctx.mark_non_differentiable(lse)
+        ctx.set_materialize_grads(False)  # no zeros are filled in for lse
         return O, lse
 
     @staticmethod
     def backward(ctx, dO, _dlse):
         q_raw, X, W_Q, W_K, W_V, O, lse, cu_q, cu_k, saved = ctx.saved_tensors
+        if dO is None:
+            dO = torch.zeros_like(O)
         lib = _lib.load()
         T_q, d_q = q_raw.shape
         T_k, x_w = X.shape
@@ -226,11 +229,14 @@ class _TargetAttnInner(torch.autograd.Function):
         ctx.save_for_backward(u, X, W_V, O, lse, cu_q, cu_k, saved)
         ctx.scale = scale
         ctx.mark_non_differentiable(lse)
+        ctx.set_materialize_grads(False)  # no zeros are filled in for lse
         return O, lse
 
     @staticmethod
     def backward(ctx, dO, _dlse):
         u, X, W_V, O, lse, cu_q, cu_k, saved = ctx.saved_tensors
+        if dO is None:
+            dO = torch.zeros_like(O)
         lib = _lib.load()
         T_q, H, d_kv = u.shape
         T_k, x_w = X.shape

@@ -42,7 +42,8 @@ struct alignas(256) SchedHeader {
   int32_t block_len;   // inner blocks per split that was finally used (0 = no split)
   int32_t next_item_2; // counter of a second kernel that walks the same list
   int32_t next_item;   // dynamic scheduling counter
-  int32_t pad[2];
+  int32_t combine_rows; // most rows of a combine unit
+  int32_t pad;
 };
 
 enum SchedMode { kSchedFwd = 0, kSchedDq = 1, kSchedDkv = 2 };

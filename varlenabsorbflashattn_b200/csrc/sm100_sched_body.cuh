@@ -168,7 +168,7 @@ __device__ __forceinline__ bool cu_check(const SchedParams& p) {
 
 __device__ __forceinline__ void sched_build(const SchedParams& p) {
   __shared__ int s_hist[kBuckets];
-  __shared__ int s_units, s_items, s_rows, s_bs, s_combine;
+  __shared__ int s_units, s_items, s_rows, s_bs, s_combine, s_combine_rows;
   __shared__ unsigned long long s_items64, s_rows64;  // pass 2 counts in 64 bits
   __shared__ long long s_blocks;
   __shared__ int s_outer, s_longest;  // outer rows of all tiles, inner blocks of the longest tile
@@ -179,7 +179,7 @@ __device__ __forceinline__ void sched_build(const SchedParams& p) {
       return;
     }
   }
-  if (threadIdx.x == 0) { s_units = 0; s_blocks = 0; s_combine = 0; s_outer = 0; s_longest = 0; }
+  if (threadIdx.x == 0) { s_units = 0; s_blocks = 0; s_combine = 0; s_combine_rows = 0; s_outer = 0; s_longest = 0; }
   for (int b = threadIdx.x; b < kBuckets; b += kSchedThreads) s_hist[b] = 0;
   __syncthreads();
 
@@ -335,6 +335,7 @@ __device__ __forceinline__ void sched_build(const SchedParams& p) {
               CombineUnit cu;
               cu.q_start = u.o_start; cu.q_rows = u.o_rows; cu.n_splits = ns;
               cu.base = atomicAdd(&s_rows, ns * u.o_rows);
+              atomicMax(&s_combine_rows, u.o_rows);
               p.combine[c0 + k++] = cu;
             }
           }
@@ -396,7 +397,8 @@ __device__ __forceinline__ void sched_build(const SchedParams& p) {
     h.block_len = bs;
     h.next_item_2 = 0;
     h.next_item = 0;
-    h.pad[0] = h.pad[1] = 0;
+    h.combine_rows = s_combine_rows;
+    h.pad = 0;
     *p.header = h;
   }
 }

@@ -1201,9 +1201,12 @@ __global__ void __launch_bounds__(256) varlen_combine_kernel(const SchedHeader* 
                                                              const CombineUnit* __restrict__ units,
                                                              const float* __restrict__ partial_o,
                                                              const float* __restrict__ partial_lse, T* __restrict__ o,
-                                                             float* __restrict__ lse, int H, int chunks) {
+                                                             float* __restrict__ lse, int H) {
   constexpr int V = D / 32;  // floats per lane: 4 (D=128) or 2 (D=64)
   constexpr int kUnroll = 4;
+  // eight (row, head) pairs of a unit at a time; a decode unit has one row of the 128 / G that its tile has room for, and going
+  // by the room made 14 dependent loads of a CTA to find one unit with something to do (64 requests of 32 / 8 heads: 12.8 -> 10.7 us between events)
+  const int chunks = (header->combine_rows * H + 7) / 8;
   const int n_work = header->n_combine * chunks;
   const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
   for (int i = blockIdx.x; i < n_work; i += gridDim.x) {
@@ -1397,10 +1400,8 @@ int launch_fwd(const vafa_varlen_args* a, cudaStream_t s, void* scratch = nullpt
   }
   VAFA_LAUNCH_CHECK("varlen_fwd_kernel");
   LaunchScope scope(kKCombine, s);
-  const int unit_rows = sp.tile_rows < a->total_q ? sp.tile_rows : a->total_q;
-  const int chunks = (unit_rows * a->num_heads + 7) / 8;
   varlen_combine_kernel<T, D><<<4 * sms, 256, 0, s>>>(sp.header, sp.combine, p.partial_o, p.partial_lse,
-                                                      (T*)a->o, a->lse, a->num_heads, chunks);
+                                                      (T*)a->o, a->lse, a->num_heads);
   VAFA_LAUNCH_CHECK("varlen_combine_kernel");
   return 0;
 }

@@ -169,11 +169,14 @@ class _PackedVarlenAttn(torch.autograd.Function):
         ctx.save_for_backward(q, k, v, o, lse, cu_q, cu_k)
         ctx.scale, ctx.causal, ctx.split_k_block = scale, causal, split_k_block
         ctx.mark_non_differentiable(lse)
+        ctx.set_materialize_grads(False)  # no zeros are filled in for lse
         return o, lse
 
     @staticmethod
     def backward(ctx, do, _dlse):
         q, k, v, o, lse, cu_q, cu_k = ctx.saved_tensors
+        if do is None:
+            do = torch.zeros_like(o)
         if do.dtype != q.dtype:
             do = do.to(q.dtype)
         if not do.is_contiguous():
