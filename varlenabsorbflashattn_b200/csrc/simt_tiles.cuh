@@ -87,11 +87,34 @@ template <typename T> __device__ __forceinline__ void store4(T* p, float4 f) {
   }
 }
 
+// 16 bytes from global to shared memory without a register on the way; `bytes` = 0 writes zeros and reads nothing.
+__device__ __forceinline__ void copy16_async(float* dst, const float* src, int bytes) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(ptx::smem_u32(dst)), "l"(src), "r"(bytes) : "memory");
+}
+// The thread's copies so far have arrived (load_tile: before the barrier that publishes the tile).
+__device__ __forceinline__ void tile_arrived() { asm volatile("cp.async.wait_all;" ::: "memory"); }
+
 // kN rows of DP columns into shared memory; rows past n_valid, rows `keep` refuses and columns past D become zeros.
+// fp32 rows that can be read four elements at a time are all on their way at once, several tiles together; through registers,
+// eight loads at a time, a CTA waited four times for its first two tiles.  Forward | dQ | dK/dV, registers -> now: 64 users of
+// 1-16 targets, widths 256, 217 -> 160 | 238 -> 211 | 211 -> 185 us; 148 users x 2048 keys 1114 -> 766 | 1431 -> 1084 | 1796 -> 1426.
+// (A second set of tiles, filled while the first is multiplied: 156 | 213 | 183 and 736 | 1084 | 1408.)
 template <int DP, int kN, typename T, typename Keep>
 __device__ __forceinline__ void load_tile(float* dst, const T* src, int64_t row_stride, int n_valid, int D, int vec, Keep keep) {
   constexpr int kQuads = DP / 4;
   constexpr int kIters = kN * kQuads / kThreads;
+  if constexpr (sizeof(T) == 4) {
+    if (vec) {
+#pragma unroll 4
+      for (int it = 0; it < kIters; ++it) {
+        const int i = it * kThreads + threadIdx.x;
+        const int r = i / kQuads, c = (i % kQuads) * 4;
+        const bool ok = r < n_valid && c < D && keep(r);
+        copy16_async(dst + r * Dim<DP>::kStride + c, ok ? src + r * row_stride + c : src, ok ? 16 : 0);
+      }
+      return;
+    }
+  }
 #pragma unroll 8
   for (int it = 0; it < kIters; ++it) {
     const int i = it * kThreads + threadIdx.x;
@@ -206,14 +229,23 @@ __device__ __forceinline__ Tile find_tile(const TileParams& p, const int32_t* cu
   const long long unit = blockIdx.x / (unsigned)p.splits;
   t.h = (int)(unit % p.heads);
   const long long slot = unit / p.heads;
-  int lo = 0, hi = p.n_seg;  // first slot of lo <= slot < first slot of hi
-  while (hi - lo > 1) {
-    const int mid = (lo + hi) >> 1;
-    if ((long long)cu[mid] * stack / kRows + mid <= slot) lo = mid; else hi = mid;
+  // First slots grow from segment to segment; all threads look at once.  (A binary search is a chain of global loads, a
+  // third of a microsecond each.)
+  __shared__ int seg;
+  if (threadIdx.x == 0) seg = -1;
+  __syncthreads();
+  for (int i = threadIdx.x; i < p.n_seg; i += kThreads) {
+    const long long lo = (long long)cu[i] * stack / kRows + i, hi = (long long)cu[i + 1] * stack / kRows + i + 1;
+    if (lo <= slot && slot < hi) seg = i;
   }
-  t.seg = lo;
-  t.row0 = (slot - ((long long)cu[lo] * stack / kRows + lo)) * kRows;
-  t.any = t.row0 < (long long)(cu[lo + 1] - cu[lo]) * stack;
+  __syncthreads();
+  t.seg = seg;
+  t.any = t.seg >= 0;
+  t.row0 = 0;
+  if (t.any) {
+    t.row0 = (slot - ((long long)cu[t.seg] * stack / kRows + t.seg)) * kRows;
+    t.any = t.row0 < (long long)(cu[t.seg + 1] - cu[t.seg]) * stack;
+  }
   return t;
 }
 
@@ -364,6 +396,7 @@ __global__ void __launch_bounds__(kThreads) tile_fwd_kernel(const TileParams p) 
     __syncthreads();
     load_tile<DP, C>(sk, kb + (int64_t)j0 * p.k_row, p.k_row, n_keys, p.D, p.vec_k, KeepAll());
     if (!kShared) load_tile<DP, C>(sv, vb + (int64_t)j0 * p.v_row, p.v_row, n_keys, p.D, p.vec_v, KeepAll());
+    tile_arrived();
     __syncthreads();
     if (!live) continue;
     float s[4][J];
@@ -415,6 +448,7 @@ __global__ void __launch_bounds__(kThreads) tile_fwd_kernel(const TileParams p) 
     }
     __syncwarp();
   }
+  tile_arrived();  // a share without a block has waited for nothing yet, and the rows' buffer is used again below
 
   // row statistics: the lanes of a row hold the sums of their own columns
 #pragma unroll
@@ -523,6 +557,7 @@ __global__ void __launch_bounds__(kThreads) tile_dq_kernel(const TileParams p) {
     __syncthreads();
     load_tile<DP, C>(sk, kb + (int64_t)j0 * p.k_row, p.k_row, n_keys, p.D, p.vec_k, KeepAll());
     if (!kShared) load_tile<DP, C>(sv, vb + (int64_t)j0 * p.v_row, p.v_row, n_keys, p.D, p.vec_v, KeepAll());
+    tile_arrived();
     __syncthreads();
     if (!live) continue;
     float s[4][J], dp[4][J];
@@ -550,6 +585,7 @@ __global__ void __launch_bounds__(kThreads) tile_dq_kernel(const TileParams p) {
     }
     __syncwarp();
   }
+  tile_arrived();  // a share without a block has waited for nothing yet
   __syncthreads();
   reduce_store<DP>(p, acc, sq, n_ranks, t.rank, rows, (T*)p.dq + t.h * p.q_head + row0 * p.q_row, p.q_row, p.vec_o,
                    [&](int) { return 1.f; },
@@ -627,6 +663,7 @@ __global__ void __launch_bounds__(kThreads) tile_dkv_kernel(const TileParams p) 
     auto seen = [&](int r) { return st_lse[r] != -INFINITY; };
     load_tile<DP, C>(sq, (const T*)p.q + t.h * p.q_head + g0 * p.q_row, p.q_row, n_in, p.D, p.vec_q, seen);
     load_tile<DP, C>(sd, (const TDO*)p.d_o + t.h * p.do_head + g0 * p.do_row, p.do_row, n_in, p.D, p.vec_do, seen);
+    tile_arrived();
     __syncthreads();
     if (!live) continue;
     float s[4][J], dp[4][J];
@@ -667,6 +704,7 @@ __global__ void __launch_bounds__(kThreads) tile_dkv_kernel(const TileParams p) 
     }
     __syncwarp();
   }
+  tile_arrived();  // a share without a block has waited for nothing yet
   __syncthreads();
   const float mul = kShared ? 1.f : p.scale;
   if (kShared) {
