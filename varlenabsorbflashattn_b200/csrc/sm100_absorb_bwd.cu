@@ -5,21 +5,26 @@
 // Keys are the rows of all products (TMEM lanes), so nothing is computed for the 64 to 120 padding rows that a
 // 128-row tile of the user's queries would have.  Per tile
 //     S  = X U^T, Y = X dAlphaX^T                                    [128 keys, R query rows]
-//     P  = 2^(c S - lse) / scale,  dS = P (scale Y - scale delta)    16-bit, to shared memory
-//     dU^T += X^T dS                                                 [256, R]   TMEM, for the whole item
-//     dX  = scale (P dAlphaX + dS U)                                 [128 keys, 256]
-// P and dS lie in shared memory as [key][row] tiles with the 128-byte swizzle, which the tensor core reads as the K-major
-// A operand of dX and as the MN-major B operand of dU^T alike, and S and Y are free once they have been read, so those of
-// the next tile can run under this one's element-wise work.  dX leaves through the slot of its X tile, which dU^T was the last to
+//     P  = 2^(c S - lse),  dS = P (Y - delta),  dS' = P (scale Y - scale delta)
+//     dU^T += X^T dS                                                 [256, R]   TMEM, for the whole item; dU = scale (dU^T)^T
+//     dX  = (w P dAlphaX + w dS' U) / w                              [128 keys, 256]
+// What is rounded to 16 bits is what the pair rounds, P and dS' in dX, dS in dU, so the results differ from the pair's in the order
+// of the fp32 sums alone.  w is a power of two that changes no bit of P or dS', but keeps dS' of fp16 out of the subnormal numbers
+// when the scale is small (see range_factor).  dS lies in shared memory as a [key][row] tile
+// with the 128-byte swizzle, the MN-major B operand of dU^T; P and dS' go over the columns of Y as those are read, as the
+// A operands of dX.  S is free once it has been read, so that of the next tile runs under this one's element-wise work;
+// Y follows dX, under its epilogue.  dX leaves through the slot of its X tile, which dU^T was the last to
 // read: the rows of a tile are one piece of the output, and a warp of its own sends them off with one bulk copy.
 // (Stored from registers, in pieces of 64 bytes per row, the 55 KB of a tile held the warps up for 4400 of 7500 cycles.)
-// TMEM (512 columns): S [0,64) Y [64,128) dX [128,384) dU^T [384,448) (d_kv 0-127) and [448,512) (128-255).
+// TMEM (512 columns): S [0,64) Y, later P and dS' [64,128) dX [128,384) dU^T [384,448) (d_kv 0-127) and [448,512) (128-255).
 //
 // The pair of kernels reads X twice, and its dU kernel multiplies 128-row query tiles by 64-key blocks: 4600 tensor cycles per 128
 // keys where the three products here that replace it take 2300.  What bounds it: X in and dX out are 110 KB per tile at
 // a width of 216, 4800 cycles of an SM's share of HBM, against about 3300 cycles of products.
 // A step of 1137 users of 1-10 queries over 2048 keys of width 216: 1649 us with the pair for all, 1288 with this kernel for the 80 %
 // it takes; of 1024 users of 1-16 queries over 8-2048 keys of width 256: 551 and 529.
+// Rounding one P / scale and one dS for both results instead, with P as a second shared-memory tile, was 0.5 % faster (1175 and 1180 us of
+// the first step as it is now, 421 and 424 of the second), but moved dX by 0.17 to 0.27 % and lost bits of fp16 at scales above 1.
 //
 // Reference: triton_target_attn_absorb/triton_target_attn_absorb/kernels.py:287-474 (dU, dX).
 #include <cuda.h>
@@ -53,11 +58,10 @@ struct DxuSmem {
   alignas(1024) uint8_t u[4 * kRowSub];
   alignas(1024) uint8_t g[4 * kRowSub];
   alignas(1024) uint8_t x[2][4 * kKeySub];
-  alignas(1024) uint8_t p[kTile * 128];
   alignas(1024) uint8_t ds[kTile * 128];
-  alignas(16) float nl[2][kRows], nd[2][kRows];  // [item parity]: -lse - log2(scale) (-inf past the last row), -scale delta
+  alignas(16) float nl[2][kRows], nd[2][kRows], nds[2][kRows];  // [item parity]: -lse (-inf past the last row), -delta, -scale delta
   alignas(8) uint64_t ug_full, ug_empty, x_full[2], x_empty[2];
-  uint64_t sy_full, sy_free, pds_full, dx_done, nl_full, stage_full[2];
+  uint64_t sy_full, s_free, pds_full, dx_done, nl_full, stage_full[2];
   WorkQueue wq;
   uint32_t tmem_base;
   int abort_flag;
@@ -68,14 +72,16 @@ static_assert(sizeof(DxuSmem) + 1024 <= 227 * 1024, "shared memory budget");
 struct DxuParams {
   void* du;
   void* dx;
-  const float* nl;  // planar -lse and -delta * scale per stacked row
-  const float* nd;
+  const float2* ld;  // (lse, delta) per stacked row
+  const float* nl;   // the same planar, as -lse and -delta * scale
+  const float* nds;
   const SchedHeader* header;
   const WorkItem* items;  // o_start / o_rows: the user's queries, i_start / i_len: the user's keys
   int H;
   int x_width;
   int which;  // 0: dU and dX; 1: dU only; 2: dX only (a backward in two phases; the same bits as both at once)
-  float scale, scale_log2, log2_scale;
+  float scale, scale_log2;
+  float range, inv_range;  // w, 1 / w
   int32_t* status;
   int wait_limit;  // bound of every device-side wait, in units of 65536 cycles
   long long* trace;
@@ -108,7 +114,7 @@ absorb_dxu_kernel(const __grid_constant__ CUtensorMap tmap_u, const __grid_const
       mbar_init(smem_u32(&sm.stage_full[i]), 8);  // one arrival per element-wise warp
     }
     mbar_init(smem_u32(&sm.sy_full), 1);
-    mbar_init(smem_u32(&sm.sy_free), 8);
+    mbar_init(smem_u32(&sm.s_free), 8);
     mbar_init(smem_u32(&sm.pds_full), 8);
     mbar_init(smem_u32(&sm.dx_done), 1);
     mbar_init(smem_u32(&sm.nl_full), kRows);
@@ -207,37 +213,41 @@ absorb_dxu_kernel(const __grid_constant__ CUtensorMap tmap_u, const __grid_const
     // ---------------- MMA issuer: the whole warp on warp-uniform values, one elected lane issues ----------------
     constexpr int kFmt = std::is_same<T, __nv_bfloat16>::value ? 1 : 0;
     constexpr uint32_t idesc_du = make_idesc(kFmt, 1, 1, 128, kRows);  // both operands MN-major
-    constexpr uint32_t idesc_dx = make_idesc(kFmt, 0, 1, 128, kKv);    // A K-major, B MN-major
+    constexpr uint32_t idesc_dx = make_idesc(kFmt, 0, 1, 128, kKv);    // A from TMEM, B MN-major
     const uint32_t tm = warp_uniform(tbase);
     const uint32_t u_k = warp_uniform(desc_lo_sw128(smem_u32(sm.u), 16)), g_k = warp_uniform(desc_lo_sw128(smem_u32(sm.g), 16));
     const uint32_t u_mn = warp_uniform(desc_lo_sw128(smem_u32(sm.u), kRowSub)), g_mn = warp_uniform(desc_lo_sw128(smem_u32(sm.g), kRowSub));
     const uint32_t x_k0 = warp_uniform(desc_lo_sw128(smem_u32(sm.x[0]), 16)), x_mn0 = warp_uniform(desc_lo_sw128(smem_u32(sm.x[0]), kKeySub));
-    const uint32_t p_k = warp_uniform(desc_lo_sw128(smem_u32(sm.p), 16)), ds_k = warp_uniform(desc_lo_sw128(smem_u32(sm.ds), 16));
     const uint32_t ds_mn = warp_uniform(desc_lo_sw128(smem_u32(sm.ds), kKeySub));
     constexpr uint32_t kStage16 = 4 * kKeySub >> 4;
     uint32_t gk = 0, qi = 0;
     bool alive = true;
 
-    // S and Y of tile g over the first `n` query rows
-    auto issue_sy = [&](uint32_t g, uint32_t n) -> bool {
-      { TRACE_T0(); if (!mbar_wait_warp(smem_u32(&sm.sy_free), (g & 1) ^ 1, abort_flag)) return false; TRACE_ADD(5); }  // those of tile g - 1 have been read
+    // S or Y of tile g over the first `n` query rows
+    auto issue_score = [&](uint32_t g, uint32_t n, uint32_t col, uint32_t b_lo) {
+      const uint32_t x_lo = x_k0 + (g & 1) * kStage16;
+      const uint32_t idesc = make_idesc(kFmt, 0, 0, 128, 0) | (n >> 3) << 17;
+#pragma unroll
+      for (int kk = 0; kk < kKv / 16; ++kk)
+        mma_ss2(tm + col, x_lo + (kk >> 2) * (kKeySub >> 4) + (kk & 3) * 2, b_lo + (kk >> 2) * (kRowSub >> 4) + (kk & 3) * 2, idesc, kk > 0);
+    };
+    auto issue_s = [&](uint32_t g, uint32_t n) -> bool {
+      { TRACE_T0(); if (!mbar_wait_warp(smem_u32(&sm.s_free), (g & 1) ^ 1, abort_flag)) return false; TRACE_ADD(5); }  // that of tile g - 1 has been read
       { TRACE_T0(); if (!mbar_wait_warp(smem_u32(&sm.x_full[0]) + (g & 1) * 8, (g >> 1) & 1, abort_flag)) return false; TRACE_ADD(4); }
       tc_fence_after();
       TRACE_T0();
-      const uint32_t x_lo = x_k0 + (g & 1) * kStage16;
-      const uint32_t idesc = make_idesc(kFmt, 0, 0, 128, 0) | (n >> 3) << 17;
-      if (elect_one()) {
-#pragma unroll
-        for (int which = 0; which < 2; ++which)
-#pragma unroll
-          for (int kk = 0; kk < kKv / 16; ++kk)
-            mma_ss2(tm + (which ? kYCol : kSCol), x_lo + (kk >> 2) * (kKeySub >> 4) + (kk & 3) * 2,
-                    (which ? g_k : u_k) + (kk >> 2) * (kRowSub >> 4) + (kk & 3) * 2, idesc, kk > 0);
-        mma_commit(smem_u32(&sm.sy_full));
-      }
+      if (elect_one()) issue_score(g, n, kSCol, u_k);
       __syncwarp();
       TRACE_ADD(2);
       return true;
+    };
+    // (behind dX of tile g - 1, which reads P and dS' from these columns: the pipe runs in order)
+    auto issue_y = [&](uint32_t g, uint32_t n) {
+      if (elect_one()) {
+        issue_score(g, n, kYCol, g_k);
+        mma_commit(smem_u32(&sm.sy_full));
+      }
+      __syncwarp();
     };
 
     for (uint32_t n = 0; alive; ++n) {
@@ -251,16 +261,17 @@ absorb_dxu_kernel(const __grid_constant__ CUtensorMap tmap_u, const __grid_const
       { TRACE_T0(); if (!mbar_wait_warp(smem_u32(&sm.ug_full), qi & 1, abort_flag)) break; TRACE_ADD(3); }
       ++qi;
       tc_fence_after();
-      if (!issue_sy(gk, row_steps * 16)) break;
+      if (!issue_s(gk, row_steps * 16)) break;
+      issue_y(gk, row_steps * 16);
       for (int t = 0; t < nt; ++t) {
         const uint32_t g = gk + t;
         // the next tile's scores, where the tile is there before P and dS of this one
-        bool sy_due = t + 1 < nt;
-        if (sy_due) {
+        bool s_due = t + 1 < nt;
+        if (s_due) {
           const int first = (int)warp_uniform((uint32_t)mbar_wait_either(smem_u32(&sm.x_full[0]) + ((g + 1) & 1) * 8, ((g + 1) >> 1) & 1,
                                                                          smem_u32(&sm.pds_full), g & 1, abort_flag));
-          if (first == 0 || (first == 1 && !issue_sy(g + 1, row_steps * 16))) { alive = false; break; }
-          sy_due = first != 1;
+          if (first == 0 || (first == 1 && !issue_s(g + 1, row_steps * 16))) { alive = false; break; }
+          s_due = first != 1;
         }
         { TRACE_T0(); if (!mbar_wait_warp(smem_u32(&sm.pds_full), g & 1, abort_flag)) { alive = false; break; } TRACE_ADD(6); }
         tc_fence_after();
@@ -277,14 +288,16 @@ absorb_dxu_kernel(const __grid_constant__ CUtensorMap tmap_u, const __grid_const
 #pragma unroll
           for (int kk = 0; kk < kRows / 16; ++kk) {
             if (kk >= row_steps || p.which == 1) break;
-            mma_ss2(tm + kDxCol, p_k + kk * 2, g_mn + kk * (2048 >> 4), idesc_dx, kk > 0 ? 1u : 0u);
-            mma_ss2(tm + kDxCol, ds_k + kk * 2, u_mn + kk * (2048 >> 4), idesc_dx, 1u);
+            const uint32_t a = tm + kYCol + (kk >> 1) * 32 + (kk & 1) * 8;  // a thread's 32 columns: 16 of P, 16 of dS'
+            mma_ts2(tm + kDxCol, a, g_mn + kk * (2048 >> 4), idesc_dx, kk > 0 ? 1u : 0u);
+            mma_ts2(tm + kDxCol, a + 16, u_mn + kk * (2048 >> 4), idesc_dx, 1u);
           }
           mma_commit(smem_u32(&sm.dx_done));
           if (t + 1 == nt) mma_commit(smem_u32(&sm.ug_empty));
         }
         __syncwarp();
-        if (sy_due && !issue_sy(g + 1, row_steps * 16)) { alive = false; break; }
+        if (s_due && !issue_s(g + 1, row_steps * 16)) { alive = false; break; }
+        if (t + 1 < nt) issue_y(g + 1, row_steps * 16);
       }
       gk += nt;
     }
@@ -295,10 +308,10 @@ absorb_dxu_kernel(const __grid_constant__ CUtensorMap tmap_u, const __grid_const
     const int r = threadIdx.x & 127;
     const int half = threadIdx.x >> 7;
     const uint32_t lane_base = tbase + ((uint32_t)((warp & 3) * 32) << 16);
-    const uint64_t c2 = pack_f2(p.scale_log2, p.scale_log2), s2 = pack_f2(p.scale, p.scale);
+    const uint64_t c2 = pack_f2(p.scale_log2, p.scale_log2), s2 = pack_f2(p.scale, p.scale), w2 = pack_f2(p.range, p.range);
     uint32_t gk = 0, par = 0;
     bool alive = true;
-    // dX of the tile, scaled and rounded, over its X tile (see boxed_dx)
+    // dX of the tile, scaled back and rounded, over its X tile (see boxed_dx)
     auto epilogue_dx = [&](uint8_t* stage, int rows) {
       if (p.which == 1) return;
       const bool boxed = boxed_dx(p.x_width, rows);
@@ -312,7 +325,7 @@ absorb_dxu_kernel(const __grid_constant__ CUtensorMap tmap_u, const __grid_const
         tmem_wait_ld();
 #pragma unroll
         for (int i = 0; i < 16; ++i)
-          pw[i] = pack2_out<T>(__uint_as_float(t[2 * i]) * p.scale, __uint_as_float(t[2 * i + 1]) * p.scale);
+          pw[i] = pack2_out<T>(__uint_as_float(t[2 * i]) * p.inv_range, __uint_as_float(t[2 * i + 1]) * p.inv_range);
         // (rows past the last are left out: with rows of 512 bytes each is a bank conflict)
         uint8_t* const dst = boxed ? stage + (cc >> 1) * kKeySub + r * 128 : stage + (r * p.x_width + cc * 32) * 2;
         const int turn = boxed ? r & 7 : 0, first = boxed ? (cc & 1) * 4 : 0;
@@ -356,8 +369,9 @@ absorb_dxu_kernel(const __grid_constant__ CUtensorMap tmap_u, const __grid_const
       if (threadIdx.x < kRows) {
         const int t = threadIdx.x;
         const long long at = (long long)w.o_start * p.H + t;
-        sm.nl[par][t] = t < rows ? p.nl[at] - p.log2_scale : -INFINITY;
-        sm.nd[par][t] = t < rows ? p.nd[at] : 0.f;
+        sm.nl[par][t] = t < rows ? p.nl[at] : -INFINITY;
+        sm.nd[par][t] = t < rows ? -p.ld[at].y : 0.f;
+        sm.nds[par][t] = t < rows ? p.nds[at] : 0.f;
         mbar_arrive(smem_u32(&sm.nl_full));
       }
       if (!mbar_wait(smem_u32(&sm.nl_full), par, abort_flag)) break;
@@ -372,7 +386,7 @@ absorb_dxu_kernel(const __grid_constant__ CUtensorMap tmap_u, const __grid_const
         tr[11] += 1;
         long long t_c = clock64();
 #endif
-        uint32_t pp[16], dd[16];
+        uint32_t pd[32], dd[16];  // w P and w dS', dS
         uint32_t xs[32], ys[32];
         if (active) {
           tmem_ld32(lane_base + kSCol + half * 32, xs);
@@ -381,39 +395,44 @@ absorb_dxu_kernel(const __grid_constant__ CUtensorMap tmap_u, const __grid_const
         }
         tc_fence_before();
         __syncwarp();
-        if (lane == 0) mbar_arrive(smem_u32(&sm.sy_free));
+        if (lane == 0) mbar_arrive(smem_u32(&sm.s_free));
         if (active) {
           const float2* nlp = reinterpret_cast<const float2*>(&sm.nl[par][half * 32]);
           const float2* ndp = reinterpret_cast<const float2*>(&sm.nd[par][half * 32]);
+          const float2* ndsp = reinterpret_cast<const float2*>(&sm.nds[par][half * 32]);
           const bool row_ok = r < keys;
 #pragma unroll
           for (int i = 0; i < 16; ++i) {
-            const float2 n2 = nlp[i], d2 = ndp[i];
-            float t0, t1, e0, e1;
+            const float2 n2 = nlp[i], d2 = ndp[i], ds2 = ndsp[i];
+            const uint64_t y2 = pack_f2(__uint_as_float(ys[2 * i]), __uint_as_float(ys[2 * i + 1]));
+            float t0, t1, w0, w1, e0, e1, f0, f1;
             unpack_f2(fma_f2(pack_f2(__uint_as_float(xs[2 * i]), __uint_as_float(xs[2 * i + 1])), c2, pack_f2(n2.x, n2.y)), t0, t1);
-            const float p0 = ex2(t0), p1 = ex2(t1);
-            const uint64_t u2 = fma_f2(pack_f2(__uint_as_float(ys[2 * i]), __uint_as_float(ys[2 * i + 1])), s2, pack_f2(d2.x, d2.y));
-            unpack_f2(mul_f2(pack_f2(p0, p1), u2), e0, e1);
-            pp[i] = row_ok ? pack2_out<T>(p0, p1) : 0u;
-            dd[i] = row_ok ? pack2_out<T>(e0, e1) : 0u;
+            const uint64_t p2 = pack_f2(ex2(t0), ex2(t1)), wp2 = mul_f2(p2, w2);
+            unpack_f2(wp2, w0, w1);
+            unpack_f2(mul_f2(wp2, fma_f2(y2, s2, pack_f2(ds2.x, ds2.y))), e0, e1);
+            unpack_f2(mul_f2(p2, add_f2(y2, pack_f2(d2.x, d2.y))), f0, f1);
+            pd[i] = row_ok ? pack2_out<T>(w0, w1) : 0u;
+            pd[16 + i] = row_ok ? pack2_out<T>(e0, e1) : 0u;
+            dd[i] = row_ok ? pack2_out<T>(f0, f1) : 0u;
           }
         }
 #ifdef VAFA_TRACE
         tr[12] += clock64() - t_c;
 #endif
         if (active) {
+          tmem_st32(lane_base + kYCol + half * 32, pd);
 #pragma unroll
           for (int j = 0; j < 4; ++j) {
             const uint32_t off = r * 128 + (((half * 4 + j) ^ (r & 7)) << 4);
-            *reinterpret_cast<uint4*>(sm.p + off) = make_uint4(pp[4 * j], pp[4 * j + 1], pp[4 * j + 2], pp[4 * j + 3]);
             *reinterpret_cast<uint4*>(sm.ds + off) = make_uint4(dd[4 * j], dd[4 * j + 1], dd[4 * j + 2], dd[4 * j + 3]);
           }
+          tmem_wait_st();
           fence_proxy_async();
         }
         tc_fence_before();
         __syncwarp();
         if (lane == 0) mbar_arrive(smem_u32(&sm.pds_full));
-        // the tile's products: they have read P and dS and, with dU^T, the X tile
+        // the tile's products: they have read P, dS' and dS and, with dU^T, the X tile
         { TRACE_T0(); if (!mbar_wait(smem_u32(&sm.dx_done), g & 1, abort_flag)) { alive = false; break; } TRACE_ADD(9); }
         tc_fence_after();
         {
@@ -459,6 +478,16 @@ long long* vafa_trace_buffer_dxu = nullptr;
 namespace {
 #endif
 
+// The smallest power of two at or above the scale, upside down, between 1 and 2^8.  From a scale of 1 on dS' is no smaller than dS.
+// Below, w dS' lies between dS / 2 and dS, so that it leaves the range of fp16 on either side no sooner than dS in dU does; w P
+// ends at 2^8.
+float range_factor(float scale) {
+  int e;
+  const float f = frexpf(scale, &e);
+  if (f == 0.5f) --e;
+  return ldexpf(1.f, e >= 0 ? 0 : e <= -8 ? 8 : -e);
+}
+
 template <typename T>
 int launch_dxu(const AbsorbDxuLaunch& L, cudaStream_t s) {
   CUtensorMap tu, tg, tx, tdx;
@@ -468,10 +497,10 @@ int launch_dxu(const AbsorbDxuLaunch& L, cudaStream_t s) {
   if ((rc = encode_tmap_rows(&tx, L.x, L.dtype, L.total_k, 1, L.x_width, kTile))) return rc;
   if ((rc = encode_tmap_rows(&tdx, L.dx, L.dtype, L.total_k, 1, L.x_width, kTile))) return rc;
   DxuParams p;
-  p.du = L.du; p.dx = L.dx; p.nl = L.nl; p.nd = L.nd;
+  p.du = L.du; p.dx = L.dx; p.ld = L.ld; p.nl = L.nl; p.nds = L.nds;
   p.header = (const SchedHeader*)L.header; p.items = (const WorkItem*)L.items;
   p.H = L.H; p.x_width = L.x_width; p.which = L.which;
-  p.scale = L.scale; p.scale_log2 = L.scale * kLog2e; p.log2_scale = log2f(L.scale);
+  p.scale = L.scale; p.scale_log2 = L.scale * kLog2e; p.range = range_factor(L.scale); p.inv_range = 1.f / p.range;
   p.status = L.status;
   p.wait_limit = wait_limit_units();
   p.trace = nullptr;

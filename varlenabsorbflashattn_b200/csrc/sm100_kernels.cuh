@@ -80,7 +80,7 @@ struct AbsorbCoreBwdArgs {
 // dU and dX of the users in the list (1 to 64 / H queries, at least one key) in one kernel.
 struct AbsorbDxuLaunch {
   const void* u; const void* x; const void* dax;
-  const float* nl; const float* nd;  // planar rows of sm100_absorb_ld()
+  const float2* ld; const float* nl; const float* nds;  // the rows of sm100_absorb_ld(): (lse, delta), and planar
   void* du; void* dx;
   const void* header; const void* items;
   int total_q, total_k, H, dtype, x_width, sms;
@@ -91,8 +91,7 @@ struct AbsorbDxuLaunch {
 int sm100_absorb_dxu_launch(const AbsorbDxuLaunch& L, cudaStream_t s);
 size_t sm100_absorb_core_bwd_workspace_bytes(int total_q, int total_k, int n_seg, int H);
 int sm100_absorb_core_bwd(const AbsorbCoreBwdArgs& a, cudaStream_t s);
-// The users of few queries, which sm100_absorb_core_bwd() leaves out where this is true: on any stream, lists built before.
-bool sm100_absorb_one_pass(const AbsorbCoreBwdArgs& a);
+// The users of few queries, which sm100_absorb_core_bwd() leaves out: on any stream, lists built before.
 int sm100_absorb_core_bwd_one_pass(const AbsorbCoreBwdArgs& a, cudaStream_t s);
 // The tile lists depend on cu_seqlens only: these build them on their own (on any stream the caller
 // orders before the core call), so that the single-CTA list builder runs beside the projections.

@@ -914,10 +914,6 @@ struct AbsorbBwdSched {
   SchedParams du, dx, dxu;
 };
 
-// Users whose stacked query rows fill at most half a tile go through one kernel for dU and dX
-// (sm100_absorb_bwd.cu).  It rounds P / scale, which a 16-bit type holds as well as P unless the scale is extreme.
-bool absorb_one_pass(float scale) { return scale >= 1.f / 256.f && scale <= 256.f; }
-
 AbsorbBwdSched absorb_bwd_sched_params(const AbsorbCoreBwdArgs& a, int sms) {
   const AbsorbBwdWs ws = absorb_bwd_ws(a.total_q, a.total_k, a.n_seg, a.H);
   char* base = (char*)a.workspace;
@@ -934,12 +930,9 @@ AbsorbBwdSched absorb_bwd_sched_params(const AbsorbCoreBwdArgs& a, int sms) {
   r.dxu = sq;
   r.dxu.tile_rows = kInner / a.H; r.dxu.cap_items = ws.cap_dxu;
   r.dxu.header = (SchedHeader*)(base + ws.hdr_dxu); r.dxu.items = (WorkItem*)(base + ws.items_dxu);
-  if (absorb_one_pass(a.scale)) {
-    r.dxu.short_rows = kInner / a.H;
-    sq.short_rows = sk.short_rows = -(kInner / a.H);
-  } else {
-    r.dxu.n_seg = 0;
-  }
+  // users whose stacked query rows fill at most half a tile go through one kernel for dU and dX (sm100_absorb_bwd.cu)
+  r.dxu.short_rows = kInner / a.H;
+  sq.short_rows = sk.short_rows = -(kInner / a.H);
   return r;
 }
 
@@ -1006,14 +999,12 @@ int sm100_absorb_core_bwd_lists(const AbsorbCoreBwdArgs& a, cudaStream_t s) {
   return launch_scheduler_three(sch.du, sch.dx, sch.dxu, s);
 }
 
-bool sm100_absorb_one_pass(const AbsorbCoreBwdArgs& a) { return absorb_one_pass(a.scale); }
-
 int sm100_absorb_core_bwd_one_pass(const AbsorbCoreBwdArgs& a, cudaStream_t s) {
   const int sms = resolve_sm_count_bwd(a.sm_count);
   const SchedParams list = absorb_bwd_sched_params(a, sms).dxu;
   const long long pad = sm100_absorb_ld_pad((long long)a.total_q * a.H);
   const float* nl = reinterpret_cast<const float*>((const float2*)a.ld + pad);
-  return sm100_absorb_dxu_launch({a.u, a.x, a.dax, nl, nl + pad, a.du, a.dx, list.header, list.items, a.total_q, a.total_k, a.H, a.dtype,
+  return sm100_absorb_dxu_launch({a.u, a.x, a.dax, (const float2*)a.ld, nl, nl + pad, a.du, a.dx, list.header, list.items, a.total_q, a.total_k, a.H, a.dtype,
                                   a.x_width, sms, a.which, a.scale, a.status}, s);
 }
 

@@ -402,12 +402,10 @@ bool absorb_bwd_core_fast(const vafa_absorb_args* a, bool inner) {
 int absorb_core_bwd(const AbsorbCoreBwdArgs& cb, cudaStream_t s) {
   SideGuard side(s);
   int rc;
-  if (sm100_absorb_one_pass(cb)) {
-    if ((rc = side_fork(s, &side.ss))) return rc;
-    rc = sm100_absorb_core_bwd_one_pass(cb, side.ss->stream);
-    const int rd = side_done(side.ss);
-    if (rc || rd) return rc ? rc : rd;
-  }
+  if ((rc = side_fork(s, &side.ss))) return rc;
+  rc = sm100_absorb_core_bwd_one_pass(cb, side.ss->stream);
+  const int rd = side_done(side.ss);
+  if (rc || rd) return rc ? rc : rd;
   if ((rc = sm100_absorb_core_bwd(cb, s))) return rc;
   return side.join();
 }
