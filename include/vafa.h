@@ -216,8 +216,9 @@ int vafa_check_cu_seqlens(const int32_t* cu_q, const int32_t* cu_k, int32_t n_se
                           int32_t need_keys, vafa_stream_t stream);
 /* The forward calls with that check in them, done on the device by the first kernel of the call; the host reads
  * the verdict while the kernels queued behind it run.  Same arguments as vafa_varlen_fwd, vafa_absorb_fwd and
- * vafa_absorb_inner_fwd (the latter two with need_keys).  Return 1 for bad prefix sums: nothing has been read or
- * written by them, and the outputs are undefined. */
+ * vafa_absorb_inner_fwd (the latter two with need_keys).  Return 1 for bad prefix sums: the outputs are undefined then,
+ * and nothing outside the tensors has been read or written.  (The tensor-core kernels do no row of such a call, the fp32
+ * kernels the segments that lie within the tensors.) */
 int vafa_varlen_fwd_checked(const vafa_varlen_args* a, vafa_stream_t stream);
 int vafa_absorb_fwd_checked(const vafa_absorb_args* a, vafa_stream_t stream);
 int vafa_absorb_inner_fwd_checked(const vafa_absorb_args* a, vafa_stream_t stream);

@@ -57,6 +57,35 @@ def test_bad_arrays_are_refused_and_leave_nothing_behind(name):
         assert torch.equal(call(*good, True), want)
 
 
+@pytest.mark.parametrize("name", ["varlen", "absorb"])
+def test_sums_that_fall_and_rise_again(name):
+    """Two batches put together whose second was not offset: a tile of the fp32 kernels lies in two segments, and clusters
+    (several hundred keys a segment, one head) share it."""
+    rng = torch.Generator().manual_seed(4)
+    lens = torch.randint(150, 450, (130,), generator=rng).tolist()
+    qlens = lens if name == "varlen" else torch.randint(8, 24, (130,), generator=rng).tolist()
+    good = _cu(_sum(qlens)), _cu(_sum(lens))
+    T, Tk, g = sum(qlens), sum(lens), torch.Generator(device="cuda").manual_seed(4)
+    r = lambda *s: torch.randn(*s, device="cuda", generator=g)
+    if name == "varlen":
+        q, k, v = r(T, 1, 64), r(Tk, 1, 64), r(Tk, 1, 64)
+        call = lambda cq, ck: vb.packed_varlen_attn(q, k, v, cu_seqlens_q=cq, cu_seqlens_k=ck)
+    else:
+        q_raw, X, W = r(T, 64), r(Tk, 64), [r(64, 2, 32) / 8 for _ in range(3)]
+        call = lambda cq, ck: vb.packed_target_attn(q_raw, X, *W, cu_seqlens_q=cq, cu_seqlens_k=ck)
+    want = call(*good)
+
+    def twice(cu, at):  # rises for `at` segments, starts again, ends where it should
+        v = cu.tolist()
+        return _cu(v[:at + 1] + [x - v[at] for x in v[at + 1:-1]] + [v[-1]])
+
+    for at in (40, 64, 65, 100, 128):
+        for bad in ((twice(good[0], at), good[1]), (good[0], twice(good[1], at)), (twice(good[0], at), twice(good[1], at))):
+            with pytest.raises(ValueError):
+                call(*bad)
+        assert torch.equal(call(*good), want)
+
+
 def test_threads_and_streams():
     call, good, bad = _operators()["absorb"], (_cu(_sum(QL)), _cu(_sum(KL))), _cu((0, 3, 200, 133, 134))
     want, errors = call(*good, False), []

@@ -14,7 +14,7 @@
 // outer tile, so that a block of X is loaded once for all of them.
 // A cluster of 1-8 CTAs shares one outer tile, rank i taking blocks i, i + N, ...; the partial results are
 // merged through distributed shared memory in rank order (no atomics, no workspace, run-to-run identical).
-// Outer tiles are found without a list: tile t of segment s has slot floor(first_row(s) / 64) + s + t.
+// Outer tiles are found without a list (seg_search.cuh).
 //
 // Measured on a B200, 64 users of 1-16 targets over 8-2048 keys, 8 heads, d_kv = 256, fp32 (forward / dQ / dX): 189 /
 // 232 / 229 us, against 1746 / 2251 / 1155 us with one warp per output row (simt_kernels.cu), which spends five
@@ -24,6 +24,7 @@
 #include <type_traits>
 
 #include "profile.cuh"
+#include "seg_search.cuh"
 #include "simt_kernels.cuh"
 #include "sm100_ptx.cuh"
 
@@ -32,7 +33,6 @@ namespace tiles {
 
 namespace cg = cooperative_groups;
 
-constexpr int kRows = 64;      // outer rows per CTA
 constexpr int kThreads = 256;  // eight warps of eight outer rows
 constexpr int kMaxSplits = 8;  // portable cluster size
 
@@ -229,23 +229,11 @@ __device__ __forceinline__ Tile find_tile(const TileParams& p, const int32_t* cu
   const long long unit = blockIdx.x / (unsigned)p.splits;
   t.h = (int)(unit % p.heads);
   const long long slot = unit / p.heads;
-  // First slots grow from segment to segment; all threads look at once.  (A binary search is a chain of global loads, a
-  // third of a microsecond each.)
-  __shared__ int seg;
-  if (threadIdx.x == 0) seg = -1;
-  __syncthreads();
-  for (int i = threadIdx.x; i < p.n_seg; i += kThreads) {
-    const long long lo = (long long)cu[i] * stack / kRows + i, hi = (long long)cu[i + 1] * stack / kRows + i + 1;
-    if (lo <= slot && slot < hi) seg = i;
-  }
-  __syncthreads();
-  t.seg = seg;
-  t.any = t.seg >= 0;
-  t.row0 = 0;
-  if (t.any) {
-    t.row0 = (slot - ((long long)cu[t.seg] * stack / kRows + t.seg)) * kRows;
-    t.any = t.row0 < (long long)(cu[t.seg + 1] - cu[t.seg]) * stack;
-  }
+  SegSearch find(p.n_seg, kThreads);
+  while (!find.done()) find.narrow(__syncthreads_count(find.starts_by(cu, stack, slot, threadIdx.x)), kThreads);
+  t.seg = (int)find.lo;
+  t.row0 = (slot - first_slot(cu, t.seg, stack)) * kRows;
+  t.any = t.row0 >= 0 && t.row0 < ((long long)cu[t.seg + 1] - cu[t.seg]) * stack;
   return t;
 }
 
@@ -358,7 +346,7 @@ __global__ void __launch_bounds__(kThreads) tile_fwd_kernel(const TileParams p) 
   const Tile t = find_tile(p, p.cu_q, p.stack);
   if (!t.any) return;  // the same for the whole cluster
   const int q0 = p.cu_q[t.seg], Lq = p.cu_q[t.seg + 1] - q0, k0 = p.cu_k[t.seg], Lk = p.cu_k[t.seg + 1] - k0;
-  if (p.guard && (t.row0 < 0 || q0 < 0 || k0 < 0 || p.cu_q[t.seg + 1] < q0 || p.cu_q[t.seg + 1] > p.total_q ||
+  if (p.guard && (q0 < 0 || k0 < 0 || p.cu_q[t.seg + 1] < q0 || p.cu_q[t.seg + 1] > p.total_q ||
                   p.cu_k[t.seg + 1] < k0 || p.cu_k[t.seg + 1] > p.total_k))
     return;
   const long long row0 = (long long)q0 * p.stack + t.row0;  // first row of the tile in the whole batch
