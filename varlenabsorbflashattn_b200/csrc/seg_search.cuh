@@ -3,7 +3,9 @@
 //
 // All threads of a CTA look at once, each at one candidate, and the number of them whose segment starts at or before the slot
 // narrows the candidates to one of `threads` pieces: one round up to 256 segments, two up to 65 536.  (A binary search is a chain of
-// global loads, a third of a microsecond each; a look at every segment by every CTA grows with the square of the segments.)  The answer
+// global loads, a third of a microsecond each; a look at every segment by every CTA grows with the square of the segments: fp32
+// self-attention over segments of 8-64 rows, 2 heads of 64, forward with a binary search | with a look at every segment | now:
+// 64 segments 52 | 55 | 55 us, 1000 111 | 100 | 96, 4096 371 | 311 | 279, 16 384 1390 | 1843 | 1000.)  The answer
 // follows from the prefix sums alone, whatever they hold: CTAs of one cluster, which ask for the same slot, get the same one.
 //
 // No CUDA in here beyond the two qualifiers: the CPU tests compile it as it is.
