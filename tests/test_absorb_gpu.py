@@ -228,3 +228,22 @@ def test_weight_grad_group_path_matches_the_plain_backward():
     finally:
         if created:
             dist.destroy_process_group()
+
+
+@pytest.mark.parametrize("which", ["W_Q", "W_K", "W_V"])
+@pytest.mark.parametrize("d_q,d_kv", [(256, 256), (512, 216)])
+def test_weights_off_the_16_byte_boundary(which, d_q, d_kv):
+    """A weight that is a view into a flat buffer, one element off the boundary that TMA reads from."""
+    ins = make_absorb_inputs([7, 20, 1], [130, 64, 300], d_q, d_kv, 8, 32, torch.bfloat16, 9, x_std=0.1, w_std=0.1)
+    q_raw, X, W_Q, W_K, W_V, dO, cu_q, cu_k = ins
+
+    def off(t):
+        flat = torch.empty(t.numel() + 1, dtype=t.dtype, device=DEV)
+        flat[1:] = t.reshape(-1).to(DEV)
+        return flat[1:].view(t.shape)
+
+    place = {n: off if n == which else (lambda t: t.to(DEV)) for n in ("W_Q", "W_K", "W_V")}
+    g = [q_raw.to(DEV), X.to(DEV), place["W_Q"](W_Q), place["W_K"](W_K), place["W_V"](W_V)]
+    g = [t.detach().requires_grad_(True) for t in g]
+    O = vb.packed_target_attn(*g, cu_seqlens_q=cu_q, cu_seqlens_k=cu_k)
+    _compare(ins, O, torch.autograd.grad(O, g, dO.to(DEV)), torch.bfloat16)

@@ -410,8 +410,8 @@ int absorb_core_bwd(const AbsorbCoreBwdArgs& cb, cudaStream_t s) {
   return side.join();
 }
 
-// The parts of the backward that wait for nothing but the forward: dW_V, p = q_raw W_Q (into `saved`), and W_Q^T (at `wqt`, with
-// dW_V's scratch behind it).
+// The parts of the backward that wait for nothing but the forward: dW_V, p = q_raw W_Q (into `saved`, unless the forward left it
+// there), and W_Q^T (at `wqt`, with dW_V's scratch behind it).
 int absorb_bwd_beside(const vafa_absorb_args* a, bool inner, const void* axn, char* wqt, float* dWV, cudaStream_t s) {
   const int H = a->num_heads, dh = a->head_dim, Tq = a->total_q, dq = a->d_q;
   int rc;
@@ -419,8 +419,10 @@ int absorb_bwd_beside(const vafa_absorb_args* a, bool inner, const void* axn, ch
   GemmTNArgs tv{axn, a->d_o, dWV, wqt + absorb_bwd_extra(a).wqt, Tq, a->dtype, H, H, 64, 32, H * dh, dh, dh, (long long)H * dh, a->sm_count};
   if ((rc = sm100_gemm_tn(tv, s))) return rc;
   if (inner) return 0;
-  GemmNNArgs gp{a->q_raw, a->w_q, a->saved, Tq, H * dh, dq, H * dh, H * dh, a->dtype, 0, a->sm_count};
-  if ((rc = sm100_gemm_nn_k256(gp, s))) return rc;
+  if (absorb_fast(a, false).prologue) {  // (it has seen that W_Q lies as the product reads it)
+    GemmNNArgs gp{a->q_raw, a->w_q, a->saved, Tq, H * dh, dq, H * dh, H * dh, a->dtype, 0, a->sm_count};
+    if ((rc = sm100_gemm_nn_k256(gp, s))) return rc;
+  }
   return sm100_transpose(a->w_q, wqt, dq, H * dh, a->dtype, s);
 }
 
@@ -444,8 +446,9 @@ int absorb_backward(const vafa_absorb_args* a, bool inner, int phase, cudaStream
   float* dWV = inner ? a->dw : a->dw + (size_t)(dq + dkv) * H * dh;
   int rc;
   // weight-gradient chain on the tensor-core GEMMs: needs the dU/dX fast path's preconditions, D_H = 32
-  // (the 64-column box trick of the token reductions) and, for the full operator, d_q = 256
-  const bool fast_chain = absorb_bwd_core_fast(a, inner) && dh == 32 && (inner || (dq >= 256 && dq % 256 == 0));
+  // (the 64-column box trick of the token reductions) and, for the full operator, d_q a multiple of 256 and a W_K that TMA can read
+  const bool fast_chain = absorb_bwd_core_fast(a, inner) && dh == 32 &&
+                          (inner || (dq >= 256 && dq % 256 == 0 && (reinterpret_cast<uintptr_t>(a->w_k) & 15) == 0));
   const bool cut = fast_chain && !inner && phase != 0;
   if (phase == 2 && !cut) return 0;
   // tile lists of the dU and dX kernels: built on the side stream beside the products below
