@@ -181,64 +181,152 @@ AbsorbFast absorb_fast(const vafa_absorb_args* a, bool inner) {
   return f;
 }
 
-// A second stream per device for the tile-list builders of the absorb operator.  The lists depend on
-// cu_seqlens only and their builder is latency-bound on one or two SMs, so it runs beside the
-// projections instead of in front of the attention kernels: fork() orders the side stream after
-// everything already queued on the caller's stream, join() orders the caller's stream after the side
-// stream.  Both are event waits (legal inside a stream capture, where the side stream joins the capture
-// and is rejoined before the call returns).  Created on first use; no device memory is allocated.
+// Second streams for what an absorb call can run beside its main chain: the tile-list builders, which depend on cu_seqlens only, and
+// in the backward whole kernels.  fork() orders the side stream after everything queued on the caller's stream so far, join() the
+// caller's stream after the side stream.  Both are event waits (legal inside a stream capture, where the side stream joins the
+// capture and is rejoined before the call returns).  No device memory is allocated.
+//
+// A call holds its side stream while it queues, and a caller's stream gets the same one each time, of its own priority: calls
+// on different streams wait for one another no more than their kernels do.  With one stream per device for all, a call
+// queued its list builder behind whatever another caller's stream was still waiting for.  The streams are made on first use
+// and kept, eight per device beyond which the one unused longest serves another caller (which shares it then: slower, not wrong).
 struct SideStream {
+  int dev = -1, priority = 0;
+  cudaStream_t caller = nullptr;  // the stream that it served last
+  unsigned long long used = 0;    // when
+  bool held = false;
   cudaStream_t stream = nullptr;
   cudaEvent_t forked = nullptr, joined = nullptr;
+  SideStream* next = nullptr;
 };
-constexpr int kMaxSideDevices = 64;
+constexpr int kMaxDevices = 64;
+constexpr int kKeptSides = 8;
 std::mutex g_side_mu;
-SideStream g_side[kMaxSideDevices];
+SideStream* g_sides[kMaxDevices];
+unsigned long long g_side_clock = 0;
 
-int side_fork(cudaStream_t s, SideStream** out) {
-  int dev = -1;
+bool is_capturing(cudaStream_t s) {
+  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+  return cudaStreamIsCapturing(s, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone;
+}
+
+// Streams and events come and go whether or not some stream of the process is being captured.
+struct RelaxedCapture {
+  cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+  RelaxedCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
+  ~RelaxedCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
+};
+
+void side_delete(SideStream* ss) {
+  RelaxedCapture relaxed;
+  if (ss->stream) cudaStreamDestroy(ss->stream);  // (what is queued on it is finished first, without a wait here)
+  if (ss->forked) cudaEventDestroy(ss->forked);
+  if (ss->joined) cudaEventDestroy(ss->joined);
+  delete ss;
+}
+
+int side_acquire(cudaStream_t s, SideStream** out) {
+  int dev = -1, priority = 0;
   VAFA_CUDA_CHECK(cudaGetDevice(&dev));
-  if (dev < 0 || dev >= kMaxSideDevices) return fail(VAFA_ERR_UNSUPPORTED, "device ordinal %d out of range", dev);
+  if (dev < 0 || dev >= kMaxDevices) return fail(VAFA_ERR_UNSUPPORTED, "device ordinal %d out of range", dev);
+  // (a stream that is being captured is asked nothing else: a refused question would end the capture)
+  const bool captured = is_capturing(s);
+  if (!captured) VAFA_CUDA_CHECK(cudaStreamGetPriority(s, &priority));
   std::lock_guard<std::mutex> lk(g_side_mu);
-  SideStream& ss = g_side[dev];
-  if (ss.stream == nullptr) {
-    VAFA_CUDA_CHECK(cudaStreamCreateWithFlags(&ss.stream, cudaStreamNonBlocking));
-    VAFA_CUDA_CHECK(cudaEventCreateWithFlags(&ss.forked, cudaEventDisableTiming));
-    VAFA_CUDA_CHECK(cudaEventCreateWithFlags(&ss.joined, cudaEventDisableTiming));
+  SideStream* oldest = nullptr;
+  int n = 0;
+  for (SideStream* t = g_sides[dev]; t; t = t->next, ++n) {
+    if (t->held || (!captured && t->priority != priority)) continue;
+    if (t->caller == s) {
+      t->held = true;
+      *out = t;
+      return 0;
+    }
+    if (!oldest || t->used < oldest->used) oldest = t;
   }
-  // record and wait under one lock: a wait refers to the latest record of its event
-  VAFA_CUDA_CHECK(cudaEventRecord(ss.forked, s));
-  VAFA_CUDA_CHECK(cudaStreamWaitEvent(ss.stream, ss.forked, 0));
-  *out = &ss;
+  if (n >= kKeptSides && oldest && !is_capturing(oldest->stream)) {
+    oldest->held = true;
+    oldest->caller = s;
+    *out = oldest;
+    return 0;
+  }
+  SideStream* t = new (std::nothrow) SideStream;
+  if (!t) return fail(VAFA_ERR_CUDA, "out of host memory");
+  t->dev = dev;
+  t->priority = priority;
+  t->caller = s;
+  t->held = true;
+  cudaError_t e;
+  {
+    RelaxedCapture relaxed;
+    e = cudaStreamCreateWithPriority(&t->stream, cudaStreamNonBlocking, priority);
+    if (e == cudaSuccess) e = cudaEventCreateWithFlags(&t->forked, cudaEventDisableTiming);
+    if (e == cudaSuccess) e = cudaEventCreateWithFlags(&t->joined, cudaEventDisableTiming);
+  }
+  if (e != cudaSuccess) side_delete(t);
+  VAFA_CUDA_CHECK(e);
+  t->next = g_sides[dev];
+  g_sides[dev] = t;
+  *out = t;
   return 0;
 }
 
-// Marks the end of this call's work on the side stream.  The later wait may see a newer record of the
-// same event (another call's): the side stream runs in order, so that one is behind this call's work too.
-int side_done(SideStream* ss) {
-  std::lock_guard<std::mutex> lk(g_side_mu);
-  VAFA_CUDA_CHECK(cudaEventRecord(ss->joined, ss->stream));
-  return 0;
+// Gives a side stream back; of more than are kept, one that nobody holds goes.
+void side_release(SideStream* ss) {
+  SideStream* gone = nullptr;
+  {
+    std::lock_guard<std::mutex> lk(g_side_mu);
+    ss->held = false;
+    ss->used = ++g_side_clock;
+    int n = 0;
+    SideStream** oldest = nullptr;
+    for (SideStream** at = &g_sides[ss->dev]; *at; at = &(*at)->next, ++n)
+      if (!(*at)->held && (!oldest || (*at)->used < (*oldest)->used) && !is_capturing((*at)->stream)) oldest = at;
+    if (n > kKeptSides && oldest) {
+      gone = *oldest;
+      *oldest = gone->next;
+    }
+  }
+  if (gone) side_delete(gone);
 }
 
-int side_join(cudaStream_t s, SideStream* ss) {
-  std::lock_guard<std::mutex> lk(g_side_mu);
-  VAFA_CUDA_CHECK(cudaStreamWaitEvent(s, ss->joined, 0));
-  return 0;
-}
-
-// Rejoins the side stream on every way out of a call (an error return included: a stream capture must
-// not end with the side stream still forked).
-struct SideGuard {
-  cudaStream_t s;
-  SideStream* ss = nullptr;
-  explicit SideGuard(cudaStream_t stream) : s(stream) {}
+// A call's side stream, forked and joined as often as it likes.  Rejoined on every way out of the call (an error return included: a
+// stream capture must not end with the side stream still forked).
+class SideGuard {
+ public:
+  explicit SideGuard(cudaStream_t stream) : s_(stream) {}
+  ~SideGuard() {
+    join();
+    if (ss_) side_release(ss_);
+  }
+  // Orders the side stream after what is queued on the caller's.
+  int fork() {
+    int rc;
+    if (!ss_ && (rc = side_acquire(s_, &ss_))) return rc;
+    VAFA_CUDA_CHECK(cudaEventRecord(ss_->forked, s_));
+    VAFA_CUDA_CHECK(cudaStreamWaitEvent(ss_->stream, ss_->forked, 0));
+    pending_ = true;
+    return 0;
+  }
+  // Has `queue(stream)` queue work on the side stream, behind what is there (after a fork()).
+  template <typename F>
+  int run(F queue) {
+    pending_ = true;
+    return queue(ss_->stream);
+  }
+  // Orders the caller's stream after what is queued on the side stream.
   int join() {
-    SideStream* t = ss;
-    ss = nullptr;
-    return t ? side_join(s, t) : 0;
+    if (!pending_) return 0;
+    pending_ = false;
+    VAFA_CUDA_CHECK(cudaEventRecord(ss_->joined, ss_->stream));
+    VAFA_CUDA_CHECK(cudaStreamWaitEvent(s_, ss_->joined, 0));
+    return 0;
   }
-  ~SideGuard() { join(); }
+
+ private:
+  cudaStream_t s_;
+  SideStream* ss_ = nullptr;
+  bool pending_ = false;
 };
 
 size_t absorb_fwd_ws_bytes(const vafa_absorb_args* a, bool inner) {
@@ -269,10 +357,8 @@ int absorb_forward(const vafa_absorb_args* a, bool inner, cudaStream_t s, CuChec
   if (fast.core) {
     c.workspace = ws + ((!inner && fast.prologue) ? align_up((size_t)a->d_q * H * dkv * elem_size(a->dtype), 256) : 0);
     if (!inner) {
-      if ((rc = side_fork(s, &side.ss))) return rc;
-      rc = sm100_absorb_core_fwd_lists(c, side.ss->stream);
-      const int rd = side_done(side.ss);
-      if (rc || rd) return rc ? rc : rd;
+      if ((rc = side.fork())) return rc;
+      if ((rc = side.run([&](cudaStream_t t) { return sm100_absorb_core_fwd_lists(c, t); }))) return rc;
       c.lists_built = 1;
     }
   }
@@ -340,10 +426,10 @@ struct VerdictSlot {
 // to the host and walked there first, it stood idle for the 60-100 us until the first launch, on every call.
 template <typename F>
 int checked(int total_q, int total_k, int need_keys, F launch) {
-  static thread_local VerdictSlot slots[kMaxSideDevices];
+  static thread_local VerdictSlot slots[kMaxDevices];
   int dev = -1;
   VAFA_CUDA_CHECK(cudaGetDevice(&dev));
-  if (dev < 0 || dev >= kMaxSideDevices) return fail(VAFA_ERR_UNSUPPORTED, "device ordinal %d out of range", dev);
+  if (dev < 0 || dev >= kMaxDevices) return fail(VAFA_ERR_UNSUPPORTED, "device ordinal %d out of range", dev);
   VerdictSlot& slot = slots[dev];
   if (!slot.word) {
     // (another thread may be capturing a stream, which an allocation would otherwise break)
@@ -399,13 +485,10 @@ bool absorb_bwd_core_fast(const vafa_absorb_args* a, bool inner) {
 
 // The attention core's backward: the users of few queries on the side stream, the others on the caller's.  Each of the three
 // kernels fills the GPU; which is queued where decides only whose blocks take over the SMs as the other's run out.
-int absorb_core_bwd(const AbsorbCoreBwdArgs& cb, cudaStream_t s) {
-  SideGuard side(s);
+int absorb_core_bwd(const AbsorbCoreBwdArgs& cb, SideGuard& side, cudaStream_t s) {
   int rc;
-  if ((rc = side_fork(s, &side.ss))) return rc;
-  rc = sm100_absorb_core_bwd_one_pass(cb, side.ss->stream);
-  const int rd = side_done(side.ss);
-  if (rc || rd) return rc ? rc : rd;
+  if ((rc = side.fork())) return rc;
+  if ((rc = side.run([&](cudaStream_t t) { return sm100_absorb_core_bwd_one_pass(cb, t); }))) return rc;
   if ((rc = sm100_absorb_core_bwd(cb, s))) return rc;
   return side.join();
 }
@@ -463,7 +546,7 @@ int absorb_backward(const vafa_absorb_args* a, bool inner, int phase, cudaStream
     cb.ld = ex;
     cb.lists_built = 1;
     cb.which = 2;
-    if ((rc = absorb_core_bwd(cb, s))) return rc;
+    if ((rc = absorb_core_bwd(cb, side, s))) return rc;
     void* wqt = ex + x.ld + x.bexp + x.sched + x.tn;  // transposed in phase 1
     GemmNNArgs gq{dp, wqt, a->dq_raw, Tq, dq, H * dh, dq, dq, a->dtype, 0, a->sm_count};
     return sm100_gemm_nn_k256(gq, s);
@@ -471,10 +554,8 @@ int absorb_backward(const vafa_absorb_args* a, bool inner, int phase, cudaStream
   if (absorb_bwd_core_fast(a, inner)) {
     const AbsorbBwdExtra x = absorb_bwd_extra(a);
     cb.workspace = ws + z.dax + z.delta + z.du + z.dp + x.ld + x.bexp;
-    if ((rc = side_fork(s, &side.ss))) return rc;
-    rc = sm100_absorb_core_bwd_lists(cb, side.ss->stream);
-    const int rd = side_done(side.ss);
-    if (rc || rd) return rc ? rc : rd;
+    if ((rc = side.fork())) return rc;
+    if ((rc = side.run([&](cudaStream_t t) { return sm100_absorb_core_bwd_lists(cb, t); }))) return rc;
     cb.lists_built = 1;
   }
   if (!inner && absorb_fast(a, false).prologue && !fast_chain) {
@@ -495,18 +576,14 @@ int absorb_backward(const vafa_absorb_args* a, bool inner, int phase, cudaStream
     if ((rc = sm100_absorb_ld(a->o, a->d_o, a->lse, ld, (long long)Tq * H, dh, a->scale, a->dtype, s))) return rc;
     cb.ld = ld;
     cb.which = cut ? 1 : 0;
-    SideStream* const ss = side.ss;
     if ((rc = side.join())) return rc;  // the lists
     if (fast_chain) {
       // what needs the forward's results only, beside the products above and the kernels below (1024 users of 1-16 queries: about
       // 30 us of launches and gaps that stood in the row before)
-      rc = absorb_bwd_beside(a, inner, axn, ex + x.ld + x.bexp + x.sched + x.tn, dWV, ss->stream);
-      const int rd = side_done(ss);
-      side.ss = ss;
-      if (rc || rd) return rc ? rc : rd;
+      char* const wqt = ex + x.ld + x.bexp + x.sched + x.tn;
+      if ((rc = side.run([&](cudaStream_t t) { return absorb_bwd_beside(a, inner, axn, wqt, dWV, t); }))) return rc;
     }
-    if ((rc = absorb_core_bwd(cb, s))) return rc;
-    if ((rc = side.join())) return rc;
+    if ((rc = absorb_core_bwd(cb, side, s))) return rc;
   } else {
     // dax_h = dO_h W_V_h^T                  fp32 [T_q, H, d_kv]
     SimtGemm g1{a->d_o, a->w_v, dax, a->dtype, a->dtype, VAFA_F32, Tq, dkv, dh, H,
@@ -537,18 +614,12 @@ int absorb_backward(const vafa_absorb_args* a, bool inner, int phase, cudaStream
                   (long long)256 * H * dh, (long long)H * dh, a->sm_count};
     // dq_raw = dp W_Q^T   (W_Q is [d_q, H*D_H]; its transpose [H*D_H, d_q])
     GemmNNArgs gq{dp, wqt, a->dq_raw, Tq, dq, H * dh, dq, dq, a->dtype, 0, a->sm_count};
-    SideStream* ss = nullptr;
-    if ((rc = side_fork(s, &ss))) return rc;
-    rc = sm100_gemm_tn(tk, ss->stream);
-    int rd = side_done(ss);
-    side.ss = ss;
-    if (rc || rd) return rc ? rc : rd;
+    if ((rc = side.fork())) return rc;
+    if ((rc = side.run([&](cudaStream_t t) { return sm100_gemm_tn(tk, t); }))) return rc;
     if ((rc = sm100_gemm_nn_k256(gdp, s))) return rc;
     if (!cut) {  // phase 1 ends with the last weight gradient
-      if ((rc = side_fork(s, &ss))) return rc;
-      rc = sm100_gemm_nn_k256(gq, ss->stream);
-      rd = side_done(ss);
-      if (rc || rd) return rc ? rc : rd;
+      if ((rc = side.fork())) return rc;
+      if ((rc = side.run([&](cudaStream_t t) { return sm100_gemm_nn_k256(gq, t); }))) return rc;
     }
     if ((rc = sm100_gemm_tn(tq, s))) return rc;
     return side.join();
