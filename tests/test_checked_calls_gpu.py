@@ -1,6 +1,8 @@
 """Forward calls that look over cu_seqlens on the device: what they refuse, that a refused call leaves nothing behind, and that
 good calls give what unchecked ones give, from several threads and streams."""
+import os
 import threading
+import time
 
 import pytest
 import torch
@@ -108,3 +110,34 @@ def test_threads_and_streams():
     [t.start() for t in threads]
     [t.join() for t in threads]
     assert not errors, errors[:3]
+
+
+def test_a_threads_end_does_not_wait_for_the_gpu():
+    """The end of a thread that has made checked calls, while the GPU is busy for about a second."""
+    call, good = _operators()["varlen fp32"], (_cu(_sum(QL)), _cu(_sum(KL)))
+    want, got, ids = call(*good, True), [], []
+    called, leave = threading.Event(), threading.Event()
+
+    def work():
+        ids.append(threading.get_native_id())
+        with torch.cuda.stream(torch.cuda.Stream()):
+            got.append(call(*good, True))
+            torch.cuda.current_stream().synchronize()
+        called.set()
+        leave.wait(10)
+
+    thread = threading.Thread(target=work)
+    thread.start()
+    assert called.wait(60)
+    with torch.cuda.stream(torch.cuda.Stream()):
+        torch.cuda._sleep(2_000_000_000)
+        end = torch.cuda.current_stream().record_event()
+    leave.set()
+    thread.join()
+    t0 = time.monotonic()
+    while time.monotonic() - t0 < 0.4 and os.path.exists(f"/proc/self/task/{ids[0]}"):
+        time.sleep(0.01)
+    gone, asleep = not os.path.exists(f"/proc/self/task/{ids[0]}"), not end.query()
+    torch.cuda.synchronize()
+    assert asleep, "the sleep was too short for the test"
+    assert gone and torch.equal(got[0], want)

@@ -3,6 +3,7 @@
 #include <cstdio>
 #include <cstring>
 #include <atomic>
+#include <condition_variable>
 #include <mutex>
 #include <new>
 #include <vector>
@@ -410,43 +411,72 @@ int absorb_forward(const vafa_absorb_args* a, bool inner, cudaStream_t s, CuChec
   return simt_gemm(g3, s);
 }
 
-// Where the verdict of a checked forward call arrives: one pinned word and one event per thread and device (a call
-// waits for its verdict before it returns, so a thread has one at a time).  Given back when the thread ends.
-struct VerdictSlot {
-  int32_t* word = nullptr;
-  cudaEvent_t done = nullptr;
-  ~VerdictSlot() {
-    if (done) cudaEventDestroy(done);
-    if (word) cudaFreeHost(word);
-  }
+// Where the verdict of a checked forward call arrives: a word of pinned memory and an event, held by a call until it returns.  A
+// device has a page of words, pinned by its first checked call and kept; an event comes with a word's first use.  (One word per
+// thread, given back at its end, made every new thread pin memory and its end wait for the device.)
+struct Verdict {
+  int32_t* word;
+  cudaEvent_t done;
 };
+constexpr int kVerdicts = 1024;  // calls at a time; another one waits for the first of them to return
+struct VerdictPool {
+  std::mutex mu;
+  std::condition_variable returned;
+  int32_t* page = nullptr;
+  int made = 0, n_free = 0;
+  Verdict free[kVerdicts];
+};
+// (never destroyed: a thread may be in a call when the process ends)
+VerdictPool* verdict_pools() {
+  static VerdictPool* const pools = new (std::nothrow) VerdictPool[kMaxDevices];
+  return pools;
+}
+
+int verdict_acquire(VerdictPool& pool, Verdict* v) {
+  std::unique_lock<std::mutex> lk(pool.mu);
+  while (pool.n_free == 0 && pool.made == kVerdicts) pool.returned.wait(lk);
+  if (pool.n_free > 0) {
+    *v = pool.free[--pool.n_free];
+    return 0;
+  }
+  RelaxedCapture relaxed;
+  if (!pool.page)
+    VAFA_CUDA_CHECK(cudaHostAlloc((void**)&pool.page, kVerdicts * sizeof(int32_t), cudaHostAllocPortable | cudaHostAllocMapped));
+  VAFA_CUDA_CHECK(cudaEventCreateWithFlags(&v->done, cudaEventDisableTiming));
+  v->word = pool.page + pool.made++;
+  return 0;
+}
+
+void verdict_release(VerdictPool& pool, const Verdict& v) {
+  {
+    std::lock_guard<std::mutex> lk(pool.mu);
+    pool.free[pool.n_free++] = v;
+  }
+  pool.returned.notify_one();
+}
 
 // Runs `launch(CuCheck*)`, which queues the list builder and the kernels behind it, then waits for the builder's verdict.
 // Returns 1 for bad prefix sums.  The GPU has the call's kernels to run while the host waits: with the arrays copied
 // to the host and walked there first, it stood idle for the 60-100 us until the first launch, on every call.
 template <typename F>
 int checked(int total_q, int total_k, int need_keys, F launch) {
-  static thread_local VerdictSlot slots[kMaxDevices];
-  int dev = -1;
+  int dev = -1, rc;
   VAFA_CUDA_CHECK(cudaGetDevice(&dev));
   if (dev < 0 || dev >= kMaxDevices) return fail(VAFA_ERR_UNSUPPORTED, "device ordinal %d out of range", dev);
-  VerdictSlot& slot = slots[dev];
-  if (!slot.word) {
-    // (another thread may be capturing a stream, which an allocation would otherwise break)
-    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
-    VAFA_CUDA_CHECK(cudaThreadExchangeStreamCaptureMode(&mode));
-    cudaError_t e = slot.done ? cudaSuccess : cudaEventCreateWithFlags(&slot.done, cudaEventDisableTiming);
-    if (e == cudaSuccess) e = cudaHostAlloc((void**)&slot.word, sizeof(int32_t), cudaHostAllocPortable | cudaHostAllocMapped);
-    cudaThreadExchangeStreamCaptureMode(&mode);
-    VAFA_CUDA_CHECK(e);
-  }
-  *(volatile int32_t*)slot.word = 1;
-  CuCheck c{slot.word, slot.done, total_q, total_k, need_keys, false};
-  const int rc = launch(&c);
-  // (on an error behind the builder's launch too: its write must not meet the next call's word)
-  if (c.queued) VAFA_CUDA_CHECK(cudaEventSynchronize(slot.done));
-  if (rc) return rc;
-  return *(volatile int32_t*)slot.word != 0 ? 1 : 0;
+  if (!verdict_pools()) return fail(VAFA_ERR_CUDA, "out of host memory");
+  VerdictPool& pool = verdict_pools()[dev];
+  Verdict v;
+  if ((rc = verdict_acquire(pool, &v))) return rc;
+  volatile int32_t* const word = v.word;
+  *word = 1;
+  CuCheck c{v.word, v.done, total_q, total_k, need_keys, false};
+  rc = launch(&c);
+  // (on an error behind the builder's launch too: its write must not meet the next call's word.  A wait that fails leaves a
+  // broken context, and the word is not used again.)
+  if (c.queued) VAFA_CUDA_CHECK(cudaEventSynchronize(v.done));
+  const bool bad = *word != 0;
+  verdict_release(pool, v);
+  return rc ? rc : bad ? 1 : 0;
 }
 
 int not_while_captured(cudaStream_t s) {
