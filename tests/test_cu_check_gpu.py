@@ -27,3 +27,17 @@ def test_good_arrays_pass(n_seg):
     a = vb.packed_varlen_attn(x, x, x, cu_seqlens_q=cu, cu_seqlens_k=cu.clone())
     c32 = cu.to(torch.int32)
     assert torch.equal(a, vb.packed_varlen_attn(x, x, x, cu_seqlens_q=c32, cu_seqlens_k=c32))
+
+
+def test_more_rows_than_32_bits_count_are_refused():
+    """2^32 + 1 keys (17 GB that nobody writes or reads) must not arrive in the library as one."""
+    torch.cuda.empty_cache()
+    X = torch.empty(2 ** 32 + 1, 1, device="cuda")
+    q_raw, W = torch.randn(3, 8, device="cuda"), [torch.randn(d, 1, 16, device="cuda") for d in (8, 1, 1)]
+    for validate in (True, False):
+        with pytest.raises(ValueError, match="int32"):
+            vb.packed_target_attn(q_raw, X, *W, cu_seqlens_q=_cu(0, 3), cu_seqlens_k=_cu(0, 1), validate=validate)
+    with pytest.raises(ValueError, match="int32"):
+        vb.target_attn_inner(torch.randn(3, 1, 1, device="cuda"), X, W[2], _cu(0, 3), _cu(0, 1))
+    del X
+    torch.cuda.empty_cache()

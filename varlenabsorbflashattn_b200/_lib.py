@@ -199,6 +199,12 @@ def maybe_check_status(device: torch.device) -> None:
         check_status(device)
 
 
+def check_rows(T_q: int, T_k: int) -> None:
+    """The library counts rows in 32 bits; a larger batch must not arrive there as a smaller one."""
+    if max(T_q, T_k) > 2**31 - 1:
+        raise ValueError(f"total tokens {max(T_q, T_k)} exceeds int32 range")
+
+
 def workspace(nbytes: int, device: torch.device) -> torch.Tensor | None:
     if nbytes <= 0:
         return None

@@ -338,6 +338,7 @@ def target_attn_inner(
         scale = 1.0 / math.sqrt(D_H)
     cu_q = cu_seqlens_q.to(device=u.device, dtype=torch.int32).contiguous()
     cu_k = cu_seqlens_k.to(device=u.device, dtype=torch.int32).contiguous()
+    _lib.check_rows(T_q, T_k)
     if validate and (cu_q.dim() != 1 or cu_q.numel() < 2 or cu_q.shape != cu_k.shape):
         _validate(cu_q, cu_k, T_q, T_k)
     impl = _impl_code()
@@ -405,6 +406,7 @@ def packed_target_attn(
         scale = 1.0 / math.sqrt(D_H)
     cu_q = cu_seqlens_q.to(device=q_raw.device, dtype=torch.int32).contiguous()
     cu_k = cu_seqlens_k.to(device=q_raw.device, dtype=torch.int32).contiguous()
+    _lib.check_rows(T_q, T_k)
     if validate and (cu_q.dim() != 1 or cu_q.numel() < 2 or cu_q.shape != cu_k.shape):
         _validate(cu_q, cu_k, T_q, T_k)
     impl = _impl_code()

@@ -30,7 +30,7 @@ LN2 = math.log(2.0)
 
 
 def set_validate_cu_seqlens(enabled: bool) -> None:
-    """Switch the host-side cu_seqlens check (one small device-to-host copy) on or off."""
+    """Switch the check of cu_seqlens (on the device, the call waits for its verdict) on or off."""
     global _validate
     _validate = bool(enabled)
 
@@ -145,6 +145,7 @@ class _PackedVarlenAttn(torch.autograd.Function):
         assert q.is_cuda, "packed_varlen_attn requires CUDA tensors (there is no CPU path)"
         assert k.device == q.device and v.device == q.device, "q/k/v must be on the same device"
         assert D in _SUPPORTED_HEAD_DIMS, f"head_dim {D} not supported (try 64/128/256)"
+        _lib.check_rows(T_q, T_k)
 
         cu_q = cu_q.to(device=q.device, dtype=torch.int32).contiguous()
         cu_k = cu_k.to(device=q.device, dtype=torch.int32).contiguous()
