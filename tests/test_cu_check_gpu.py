@@ -1,8 +1,9 @@
-"""The host-side cu_seqlens check of tensors on the GPU: what it refuses, and with which error."""
+"""The check of cu_seqlens on the GPU: what a checked call refuses, and with which error; vafa_check_cu_seqlens on its own."""
 import pytest
 import torch
 
 import varlenabsorbflashattn_b200 as vb
+from varlenabsorbflashattn_b200 import _lib
 
 pytestmark = pytest.mark.gpu
 
@@ -41,3 +42,20 @@ def test_more_rows_than_32_bits_count_are_refused():
         vb.target_attn_inner(torch.randn(3, 1, 1, device="cuda"), X, W[2], _cu(0, 3), _cu(0, 1))
     del X
     torch.cuda.empty_cache()
+
+
+@pytest.mark.parametrize("cu_q,cu_k,need_keys,rc", [
+    ((0, 4), (0, 6), 0, 0), ((0, 2, 2, 4), (0, 0, 6, 6), 0, 0), ((0, 2, 4), (0, 3, 6), 1, 0), ((0, 0, 4), (0, 0, 6), 1, 0),
+    ((1, 4), (0, 6), 0, 1), ((0, 4), (1, 6), 0, 1), ((0, 3), (0, 6), 0, 1), ((0, 4), (0, 7), 0, 1), ((0, 5, 4), (0, 2, 6), 0, 1),
+    ((0, 2, 4), (0, 7, 6), 0, 1), ((0, 2, 4), (0, 0, 6), 1, 1), ((0, 2, 4), (0, 6, 6), 1, 1)])
+def test_the_check_as_a_call_of_its_own(cu_q, cu_k, need_keys, rc):
+    a, b = _cu(*cu_q), _cu(*cu_k)
+    stream = _lib.raw_stream(a.device)
+    assert _lib.load().vafa_check_cu_seqlens(a.data_ptr(), b.data_ptr(), len(cu_q) - 1, 4, 6, need_keys, stream) == rc
+
+
+def test_the_check_as_a_call_of_its_own_wants_arrays():
+    a = _cu(0, 4)
+    lib, stream = _lib.load(), _lib.raw_stream(a.device)
+    assert lib.vafa_check_cu_seqlens(a.data_ptr(), None, 1, 4, 4, 0, stream) < 0
+    assert lib.vafa_check_cu_seqlens(a.data_ptr(), a.data_ptr(), 0, 4, 4, 0, stream) < 0
