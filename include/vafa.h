@@ -208,7 +208,7 @@ int vafa_absorb_inner_bwd(const vafa_absorb_args* a, vafa_stream_t stream);
 int vafa_cast_from_f32(const float* src, void* dst, size_t n, int32_t dtype, vafa_stream_t stream);
 
 /* ---- housekeeping ------------------------------------------------------------------ */
-/* The host-side check of two prefix-sum arrays of n_seg + 1 entries on the device: both start at 0, end at their
+/* A check on the host of two prefix-sum arrays of n_seg + 1 entries on the device: both start at 0, end at their
  * total, never decrease, and, with need_keys, every segment with query rows has keys.  Copies both to the host
  * behind the work already queued on `stream` and waits for them.  Returns 0 when all holds, 1 when something does
  * not (the caller words the error), a negative code when the copy failed or the stream is being captured. */

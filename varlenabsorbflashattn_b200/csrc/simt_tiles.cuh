@@ -16,9 +16,10 @@
 // merged through distributed shared memory in rank order (no atomics, no workspace, run-to-run identical).
 // Outer tiles are found without a list (seg_search.cuh).
 //
-// Measured on a B200, 64 users of 1-16 targets over 8-2048 keys, 8 heads, d_kv = 256, fp32 (forward / dQ / dX): 189 /
-// 232 / 229 us, against 1746 / 2251 / 1155 us with one warp per output row (simt_kernels.cu), which spends five
-// shuffles per (row, key) and reads every key once per row.  At most four CTAs per tile: 195 / 261 / 232 us.
+// Measured on a B200, 64 users of 1-16 targets over 8-2048 keys, 8 heads, d_kv = 256, fp32 (forward / dQ / dX): 160 /
+// 211 / 185 us, against 1746 / 2251 / 1155 us with one warp per output row (simt_kernels.cu), which spends five
+// shuffles per (row, key) and reads every key once per row.  (Before the rows were copied asynchronously, see load_tile: 189 / 232 /
+// 229 us, with at most four CTAs per tile 195 / 261 / 232.)
 #pragma once
 #include <cooperative_groups.h>
 #include <type_traits>
